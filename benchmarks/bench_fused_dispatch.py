@@ -115,17 +115,6 @@ def main():
             best[k] = min(best[k], run(fn))
     buf.check()
     gemm.check_status()
-    if os.environ.get("MOONEP_B200_FD_EXPERIMENT") is not None:
-        # a build with -DMEP_GEMM_EXPERIMENTS records the longest copy-warp run and the summed
-        # arrival waits of the last launches in the GEMM status words 7 and 6 (microseconds)
-        for name, fn in (("gateup.fused", fused_fwd), ("dgrad.fused", fused_bwd)):
-            gemm.reset_status()
-            fn()
-            torch.cuda.synchronize()
-            st = gemm.status_word(dev).tolist()
-            print(f"[experiment] {name}: longest copy warp {st[7]} us, arrival waits summed over CTAs {st[6]} us",
-                  flush=True)
-        gemm.reset_status()
     real = int(cu[-1])
     fl_gu = 2.0 * real * H * 2 * Hp
     fl_dg = 2.0 * real * H * Hp

@@ -32,8 +32,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fno-strict-aliasing",
     "-Xcompiler", "-Wno-psabi", "-DNDEBUG",
 ]
-# extra nvcc flags for one-off builds (e.g. -DMEP_GEMM_EXPERIMENTS, which compiles the timing
-# experiment switches of the GEMM in; a normal build has none of those branches)
+# extra nvcc flags for one-off builds (e.g. -DMEP_PHASE_STAMPS)
 NVCC_FLAGS += os.environ.get("MOONEP_B200_NVCC_FLAGS", "").split()
 
 

@@ -55,16 +55,7 @@ struct FusedDispatch {
   long long meta_stride;           // int32 elements
   long long weights_off, link_off, src_off, arrive_off, NvS;
   int N, K, epn, rank, R, fresh, row_bytes, nsplit;
-  int debug;   // timing experiments, compiled in only with -DMEP_GEMM_EXPERIMENTS (see fd_dbg)
 };
-
-// Timing experiments (results are wrong when set): 1 = arrival signals without the release fence,
-// 4 = the copy warp issues no stores, 8 = neither loads nor stores.  A constant false in a normal build.
-#ifdef MEP_GEMM_EXPERIMENTS
-__device__ __forceinline__ bool fd_dbg(const FusedDispatch& d, int bit) { return (d.debug & bit) != 0; }
-#else
-__device__ __forceinline__ constexpr bool fd_dbg(const FusedDispatch&, int) { return false; }
-#endif
 
 // One warp.  `ring` holds NST stages of FD_PART_CAP bytes and `full` NST mbarriers (initialised
 // with count 1 by the caller): lane i < NST owns stage i.  The warp works in lockstep rounds of
@@ -168,7 +159,7 @@ __device__ __forceinline__ void fused_dispatch_copy_warp(const FusedDispatch& d,
     // is enough per round.  (A release per round cost a full drain of the SM's stores each time
     // and made the copy warp, not NVLink, the limit.)
     __syncwarp();
-    if (lane == 0 && !fd_dbg(d, 1)) fence_sys();
+    if (lane == 0) fence_sys();
     __syncwarp();
     // ---- rounds of NST units: lane i < NST moves unit u0 + r0 + i through stage i ---------------
     for (int r0 = 0; r0 < PER_BATCH && u0 + r0 < n_units; r0 += NST) {
@@ -179,20 +170,16 @@ __device__ __forceinline__ void fused_dispatch_copy_warp(const FusedDispatch& d,
       const bool act = lane < NST && u0 + from < n_units && s_src != 0ull;
       bool sent = false;
       if (act) {
-        if (!fd_dbg(d, 8)) {
-          mbar_expect_tx(my_full, (uint32_t)part_bytes);
-          bulk_g2s(my_stage, reinterpret_cast<const void*>(s_src), (uint32_t)part_bytes, my_full);
-          sent = wait_full(my_full, parity);
-          parity ^= 1u;
-          if (sent && !fd_dbg(d, 4)) {
-            bulk_s2g(reinterpret_cast<void*>(s_dst), my_stage, (uint32_t)part_bytes);
-            bulk_commit();
-            bulk_wait<0>();          // complete, not just read: the rows may now be announced
-          }
-        } else {
-          sent = true;
+        mbar_expect_tx(my_full, (uint32_t)part_bytes);
+        bulk_g2s(my_stage, reinterpret_cast<const void*>(s_src), (uint32_t)part_bytes, my_full);
+        sent = wait_full(my_full, parity);
+        parity ^= 1u;
+        if (sent) {
+          bulk_s2g(reinterpret_cast<void*>(s_dst), my_stage, (uint32_t)part_bytes);
+          bulk_commit();
+          bulk_wait<0>();          // complete, not just read: the rows may now be announced
         }
-        if (sent && !fd_dbg(d, 1)) fence_proxy_async();
+        if (sent) fence_proxy_async();
       }
       // a load that never landed ends this warp's work (the status is already recorded)
       if (__any_sync(0xffffffffu, act && !sent)) ok = false;

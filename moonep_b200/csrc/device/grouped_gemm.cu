@@ -85,11 +85,7 @@ struct GemmKParams {
   CUtensorMap o;           // bf16 output of the token-major epilogue (32 x 64 store boxes)
   const int32_t* cu_seqlens;
   int ngroups, split, total_rows, N, K, nseg, rows_per_expert, Mw, accumulate, zero_empty_below;
-  // Timing experiments, compiled in only with -DMEP_GEMM_EXPERIMENTS (results are wrong when
-  // non-zero), a bit mask: 1 = skip the epilogue's global stores, 2 = skip its TMEM loads, 4 =
-  // issue no MMAs (barriers only), 8 = issue no TMA loads (barriers only).  In a normal build
-  // gemm_dbg() is a constant false and none of those branches exists.  Bit 16 (plain-store
-  // epilogues, results stay correct) is a host-side choice of the epilogue and always available.
+  // bit 16: per-row plain stores in the bf16 epilogue (A/B of benchmarks; a host-side choice)
   int debug;
   int stages, wb;   // SGD kernels: operand stages and weight blocks per epilogue warp of this launch
   // SGD kernels: 1 = only the tiles whose grads are STORED (experts with replicas, slot groups),
@@ -123,12 +119,6 @@ struct GemmKParams {
   // accumulator), so that a missing row is reported as what it is.
   unsigned long long arrive_timeout_ns;
 };
-
-#ifdef MEP_GEMM_EXPERIMENTS
-__device__ __forceinline__ bool gemm_dbg(const GemmKParams& p, int bit) { return (p.debug & bit) != 0; }
-#else
-__device__ __forceinline__ constexpr bool gemm_dbg(const GemmKParams&, int) { return false; }
-#endif
 
 struct Tile {
   int g, row0, rows, n0, num_kb, alloc, g_local, m0;
@@ -375,9 +365,6 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
           // every CTA enter a group at about the same time, as CTAs that start together do: the
           // tiles in flight then share one group's rows and weights in L2 instead of two groups'.
           if (p.disp.arrive != nullptr && t.rows > 0 && t.g >= groups_ready) {
-#ifdef MEP_GEMM_EXPERIMENTS
-            const unsigned long long t_begin = globaltimer_ns();
-#endif
             unsigned long long t0 = 0ull;
             unsigned spins = 0;
             while ((groups_ready = *(volatile int*)&s_groups_ready) <= t.g) {
@@ -390,10 +377,6 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
             __threadfence_block();
             fence_proxy_async();   // the rows were written through the async proxy (or by plain stores)
             if (!stamped_first) { phase_stamp(p.trace, 2, (int)blockIdx.x, 1); stamped_first = true; }   // first group arrived
-#ifdef MEP_GEMM_EXPERIMENTS
-            if (p.status != nullptr)                   // experiments: total arrival wait of all CTAs, in microseconds
-              atomicAdd(p.status + 6, (int)((globaltimer_ns() - t_begin) / 1000ull));
-#endif
           }
         }
         for (int kb = 0; kb < t.num_kb; ++kb, ++it) {
@@ -407,10 +390,6 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
           uint8_t* sb = sa + A_TILE_BYTES;
           uint32_t lead_bar = 0;
           if constexpr (TWO) lead_bar = mapa_u32(&full[s], 0);
-          if (gemm_dbg(p, 8)) {
-            if (crank == 0) mbar_arrive(&full[s]);
-            continue;
-          }
           // the peer's bytes may land before this arrival: the pending count keeps the phase open
           if (crank == 0) mbar_expect_tx(&full[s], TWO ? 2 * STAGE_BYTES : STAGE_BYTES);
           const int seg = kb / kb_per_seg;
@@ -507,7 +486,6 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
           const uint32_t sb = sa + A_TILE_BYTES;
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
-            if (gemm_dbg(p, 4)) break;
             const uint64_t da = A_MN ? make_smem_desc(sa + kk * 2048, 8192, 1024)
                                      : make_smem_desc(sa + kk * 32, 16, 1024);
             const uint64_t db = B_MN ? make_smem_desc(sb + kk * 2048, 8192, 1024)
@@ -530,18 +508,11 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
     if constexpr (DISP) {
       if (p.disp.x != nullptr) {
         uint8_t* ring = tiles + (size_t)nst * STAGE_BYTES;
-#ifdef MEP_GEMM_EXPERIMENTS
-        const unsigned long long t_begin = globaltimer_ns();
-#endif
         if (lane == 0) phase_stamp(p.trace, 3, (int)blockIdx.x, 0);          // copy warp starts
         fused_dispatch_copy_warp<FD_NST>(
             p.disp, ring, fd_full, (int)blockIdx.x, (int)gridDim.x,
             [&](uint64_t* bar, uint32_t parity) { return gemm_wait(bar, parity, abortp, p, 7); });
         if (lane == 0) phase_stamp(p.trace, 3, (int)blockIdx.x, 1);          // all rows sent and announced
-#ifdef MEP_GEMM_EXPERIMENTS
-        if (lane == 0 && p.status != nullptr)      // experiments: longest copy-warp run, in microseconds
-          atomicMax(p.status + 7, (int)((globaltimer_ns() - t_begin) / 1000ull));
-#endif
       }
     }
   } else {
@@ -617,14 +588,9 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
           uint32_t rg[32], ru[32];
-          if (!gemm_dbg(p, 2)) {
-            tmem_ld_32x32(tacc + c * 32, rg);
-            tmem_ld_32x32(tacc + 128 + c * 32, ru);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) rg[i] = ru[i] = 0u;
-          }
+          tmem_ld_32x32(tacc + c * 32, rg);
+          tmem_ld_32x32(tacc + 128 + c * 32, ru);
+          tmem_ld_wait();
           const int col = t.n0 + c * 32;
           if (row_ok && col < p.N) {
             uint32_t pg[16], pu[16], pa[16];
@@ -645,8 +611,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
               pa[i] = *reinterpret_cast<uint32_t*>(&ha);
             }
             const long long off = row * p.ldc + col;
-            if (gemm_dbg(p, 1)) {
-            } else if (col + 32 <= p.N) {
+            if (col + 32 <= p.N) {
 #pragma unroll
               for (int v = 0; v < 4; ++v) {
                 if (og) reinterpret_cast<uint4*>(og + off)[v] = make_uint4(pg[4 * v], pg[4 * v + 1], pg[4 * v + 2], pg[4 * v + 3]);
@@ -748,21 +713,14 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
               const int b = wseq % WB;
               uint8_t* wbuf = wring + b * WBLK;
               uint32_t ra[32], rb[32];
-              if (!gemm_dbg(p, 2)) {
-                tmem_ld_32x32(tacc + cofs + c * WCOLS, ra);
-                tmem_ld_32x32(tacc + cofs + c * WCOLS + 32, rb);
-              }
+              tmem_ld_32x32(tacc + cofs + c * WCOLS, ra);
+              tmem_ld_32x32(tacc + cofs + c * WCOLS + 32, rb);
               if (!gemm_wait(&wbar[ew][b], (uint32_t)(wseq / WB) & 1u, abortp, p, 5)) {
-                if (!gemm_dbg(p, 2)) tmem_ld_wait();
+                tmem_ld_wait();
                 wok = false;
                 break;
               }
-              if (!gemm_dbg(p, 2)) {
-                tmem_ld_wait();
-              } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) ra[i] = rb[i] = 0u;
-              }
+              tmem_ld_wait();
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 const uint32_t* g = j < 4 ? ra + 8 * j : rb + 8 * (j - 4);
@@ -780,10 +738,8 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
               fence_proxy_async_smem();
               __syncwarp();
               if (lane == 0) {
-                if (!gemm_dbg(p, 1)) {
-                  tma_store_2d(&p.wmap, col_base + cofs + c * WCOLS, y0, wbuf);
-                  bulk_commit();
-                }
+                tma_store_2d(&p.wmap, col_base + cofs + c * WCOLS, y0, wbuf);
+                bulk_commit();
                 bulk_wait_read<0>();                // the store has read the buffer: it may be refilled
               }
               ++wseq;
@@ -794,7 +750,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
 #pragma unroll 1
           for (int c = 0; c < BN / 32; ++c) {
             uint32_t r[32];
-            if (have_acc && !gemm_dbg(p, 2)) {
+            if (have_acc) {
               tmem_ld_32x32(tacc + c * 32, r);
               tmem_ld_wait();
             } else {
@@ -810,7 +766,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
             fence_proxy_async_smem();
             __syncwarp();
             const int x0 = col_base + c * 32;
-            if (lane == 0 && x0 < p.N && !gemm_dbg(p, 1)) {
+            if (lane == 0 && x0 < p.N) {
               if (p.accumulate) tma_reduce_add_2d(cmap, x0, y0, pad);
               else tma_store_2d(cmap, x0, y0, pad);
               bulk_commit();
@@ -828,7 +784,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
 #pragma unroll 1
           for (int c = 0; c < BN / 32; ++c) {
             uint32_t r[32];
-            if (have_acc && !gemm_dbg(p, 2)) {
+            if (have_acc) {
               tmem_ld_32x32(tacc + c * 32, r);
               tmem_ld_wait();
             } else {
@@ -839,7 +795,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) pad[lane * 33 + i] = __uint_as_float(r[i]);
             __syncwarp();
-            if (col < p.N && !gemm_dbg(p, 1)) {
+            if (col < p.N) {
               float* o = (float*)outp + off_warp + col;
 #pragma unroll 8
               for (int rr = 0; rr < 32; ++rr) {
@@ -862,7 +818,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
             const int col = col_base + c2 * 64;
             if (col >= p.N) break;
             uint32_t ra[32], rb[32];
-            if (have_acc && !gemm_dbg(p, 2)) {
+            if (have_acc) {
               tmem_ld_32x32(tacc + c2 * 64, ra);
               tmem_ld_32x32(tacc + c2 * 64 + 32, rb);
               tmem_ld_wait();
@@ -886,7 +842,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
             }
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0 && !gemm_dbg(p, 1)) {
+            if (lane == 0) {
               tma_store_2d(&p.o, col, y0, pad);
               bulk_commit();
             }
@@ -895,7 +851,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
           uint32_t r[32];
-          if (have_acc && !gemm_dbg(p, 2)) {
+          if (have_acc) {
             tmem_ld_32x32(tacc + c * 32, r);
             tmem_ld_wait();
           } else {
@@ -903,7 +859,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
             for (int i = 0; i < 32; ++i) r[i] = 0u;
           }
           const int col = col_base + c * 32;
-          if (!row_ok || col >= p.N || gemm_dbg(p, 1)) continue;
+          if (!row_ok || col >= p.N) continue;
           if constexpr (EPI == EPI_F32) {
             // unreachable: the fp32 epilogue is the transposed loop below
           } else {
@@ -1181,9 +1137,6 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
   kp.rows_per_expert = d->rows_per_expert; kp.Mw = d->Mw; kp.accumulate = d->accumulate;
   kp.zero_empty_below = d->zero_empty_below;
   kp.debug = d->debug; kp.g_begin = d->g_begin;
-#ifdef MEP_GEMM_EXPERIMENTS
-  if (const char* e = getenv("MOONEP_B200_GEMM_EXPERIMENT")) kp.debug |= atoi(e);   // timing only: results are wrong
-#endif
   kp.src_info = d->src_info; kp.push_base = d->push_base; kp.push_rank_stride = d->push_rank_stride;
   kp.push_entries = d->push_entries; kp.push_ranks = d->push_ranks;
   kp.out[0] = d->out[0]; kp.out[1] = d->out[1]; kp.out[2] = d->out[2];
@@ -1288,9 +1241,6 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
     kp.trace = c.trace;
     kp.arrive_timeout_ns = c.timeout_ns;                       // waits on other ranks: the Buffer's budget
     kp.timeout_ns = c.timeout_ns + c.timeout_ns / 2 + 200000000ull;
-#ifdef MEP_GEMM_EXPERIMENTS
-    if (const char* e = getenv("MOONEP_B200_FD_EXPERIMENT")) f.debug = atoi(e);
-#endif
     if (d->epi == EPI_SWIGLU) {
       if (two) return launch_gemm2<false, true, EPI_SWIGLU, false, false, true>(kp, grid, stream);
       return launch_gemm<false, false, true, EPI_SWIGLU, false, true>(kp, grid, stream);
