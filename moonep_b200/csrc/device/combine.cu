@@ -399,12 +399,8 @@ __global__ void __launch_bounds__(PUSH_REDUCE_THREADS, 1) ep_push_reduce_kernel(
 
 template <int ST, int NV>
 static int launch_combine_t(const BufferCtx& c, CombineParams& p, size_t smem, cudaStream_t stream) {
-  static thread_local size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    MEP_CUDA_OK(cudaFuncSetAttribute((const void*)ep_combine_kernel<ST, NV>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static std::atomic<unsigned long long> raised{0};
+  MEP_CUDA_OK(raise_smem_limit((const void*)ep_combine_kernel<ST, NV>, raised));
   dim3 grid(c.num_sms, c.Rv());
   MEP_CUDA_OK(launch_chained((const void*)ep_combine_kernel<ST, NV>, grid, dim3(COMBINE_THREADS), smem,
                              stream, p, /*coop=*/1, c.pdl));
@@ -424,12 +420,8 @@ static int launch_combine_nv(const BufferCtx& c, CombineParams& p, cudaStream_t 
 
 template <int ST, int NV>
 static int launch_prologue_t(const BufferCtx& c, PrologueParams& p, size_t smem, cudaStream_t stream) {
-  static thread_local size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    MEP_CUDA_OK(cudaFuncSetAttribute((const void*)ep_combine_prologue_kernel<ST, NV>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static std::atomic<unsigned long long> raised{0};
+  MEP_CUDA_OK(raise_smem_limit((const void*)ep_combine_prologue_kernel<ST, NV>, raised));
   // one CTA per SM (a virtual group shares the SMs between its ranks)
   int gx = c.num_sms_local / c.Rv();
   if (gx < 1) gx = 1;

@@ -296,12 +296,8 @@ __global__ void __launch_bounds__(256) ep_plan_snapshot_kernel(const SnapshotPar
 template <int ST>
 static int launch_dispatch_t(const BufferCtx& c, DispatchParams& p, size_t smem,
                              cudaStream_t stream) {
-  static thread_local size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    MEP_CUDA_OK(cudaFuncSetAttribute((const void*)ep_dispatch_kernel<ST>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static std::atomic<unsigned long long> raised{0};
+  MEP_CUDA_OK(raise_smem_limit((const void*)ep_dispatch_kernel<ST>, raised));
   dim3 grid(c.num_sms, c.Rv());
   MEP_CUDA_OK(launch_chained((const void*)ep_dispatch_kernel<ST>, grid, dim3(DISPATCH_THREADS), smem,
                              stream, p, /*coop=*/1, c.pdl && p.fresh));
@@ -363,12 +359,9 @@ int mep_launch_expand(const void* ctx_, const int32_t* link, const int32_t* cu_s
   else if (4 * row <= 200 * 1024) { kern = (const void*)ep_expand_kernel<4>; smem = 4 * row; }
   else if (2 * row <= 200 * 1024) { kern = (const void*)ep_expand_kernel<2>; smem = 2 * row; }
   else return fail(-2, "expand: H=%d does not fit a 2-stage ring", c.H);
-  static thread_local size_t configured[3] = {0, 0, 0};
+  static std::atomic<unsigned long long> raised[3];
   const int which = kern == (const void*)ep_expand_kernel<8> ? 0 : (kern == (const void*)ep_expand_kernel<4> ? 1 : 2);
-  if (smem > 48 * 1024 && smem > configured[which]) {
-    MEP_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured[which] = smem;
-  }
+  MEP_CUDA_OK(raise_smem_limit(kern, raised[which]));
   MEP_CUDA_OK(launch_chained(kern, grid, dim3(EXPAND_THREADS), smem, stream, p, /*coop=*/0, c.pdl));
   return 0;
 }

@@ -8,45 +8,80 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "host/ctx.h"
 #include "host/errors.h"
 
 namespace mep {
 
 // ---- router: top-k over (logits + bias), softmax over the selected unbiased logits ------------
-constexpr int ROUTER_WARPS = 4;
+// One warp per token.  The biased logits are turned into order-preserving unsigned keys and, up to
+// 32 * ROUTER_VPL experts, stay in registers; a selection round is then ROUTER_VPL compares, one
+// warp-wide redux for the largest key and one for its smallest expert index.  (With the keys in
+// shared memory and ten shuffles a round the kernel was bound by that chain: 18 us for 4096 tokens
+// x 32 experts, top-8.)  A NaN gets the lowest key of all: it is chosen only when nothing else is
+// left, and no input makes an index leave [0, E).  Selections are counted per block in shared memory:
+// one global atomic per selection made the popular experts' counters the limit (15 us of 18).
+constexpr int ROUTER_WARPS = 8;
+constexpr int ROUTER_VPL = 8;                 // keys per lane kept in registers
 
+__device__ __forceinline__ uint32_t router_key(float x) {
+  const uint32_t b = __float_as_uint(x);
+  if ((b & 0x7FFFFFFFu) > 0x7F800000u) return 1u;                 // NaN; 0 marks "already selected"
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);              // (-inf maps to 0x007FFFFF)
+}
+
+template <bool REGS>
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
 ep_router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int S, int E,
                       int K, int32_t* __restrict__ topk, float* __restrict__ weights,
                       int32_t* __restrict__ tpe) {
-  extern __shared__ float s_vals[];   // [ROUTER_WARPS][E]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float* v = s_vals + (size_t)warp * E;
-  for (int s = blockIdx.x * ROUTER_WARPS + warp; s < S; s += gridDim.x * ROUTER_WARPS) {
+  extern __shared__ uint32_t s_hist[];   // [E] selections, then [warps][E] keys unless they fit in registers
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (int)(blockDim.x >> 5);
+  uint32_t* sk = REGS ? nullptr : s_hist + E + (size_t)warp * E;
+  for (int e = threadIdx.x; e < E; e += (int)blockDim.x) s_hist[e] = 0u;
+  __syncthreads();
+  for (int s = blockIdx.x * nwarps + warp; s < S; s += gridDim.x * nwarps) {
     const float* row = logits + (size_t)s * E;
-    for (int e = lane; e < E; e += 32) v[e] = row[e] + (bias ? bias[e] : 0.f);
-    __syncwarp();
-    float sel_logit = 0.f;   // lane k keeps the k-th selected raw logit
-    int sel_idx = -1;
-    for (int k = 0; k < K; ++k) {
-      float bv = -FLT_MAX;
-      int bi = 0x7fffffff;
-      for (int e = lane; e < E; e += 32) {
-        float x = v[e];
-        if (x > bv) { bv = x; bi = e; }
-      }
+    uint32_t key[ROUTER_VPL];
+    if constexpr (REGS) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+      for (int i = 0; i < ROUTER_VPL; ++i) {
+        const int e = i * 32 + lane;
+        key[i] = e < E ? router_key(row[e] + (bias ? bias[e] : 0.f)) : 0u;
       }
-      if (lane == k) { sel_idx = bi; sel_logit = row[bi]; }
-      if (lane == 0) v[bi] = -FLT_MAX;
+    } else {
+      for (int e = lane; e < E; e += 32) sk[e] = router_key(row[e] + (bias ? bias[e] : 0.f));
       __syncwarp();
     }
+    int sel_idx = 0;         // lane k keeps the k-th selected expert
+    for (int k = 0; k < K; ++k) {
+      uint32_t best = 0u;
+      int at = E - 1;        // smallest index of this lane's largest key
+      if constexpr (REGS) {
+#pragma unroll
+        for (int i = 0; i < ROUTER_VPL; ++i)
+          if (key[i] > best) { best = key[i]; at = i * 32 + lane; }
+      } else {
+        for (int e = lane; e < E; e += 32) {
+          const uint32_t x = sk[e];
+          if (x > best) { best = x; at = e; }
+        }
+      }
+      const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+      const int idx = (int)__reduce_min_sync(0xffffffffu, best == top ? (uint32_t)at : (uint32_t)(E - 1));
+      if (lane == k) sel_idx = idx;
+      if constexpr (REGS) {
+#pragma unroll
+        for (int i = 0; i < ROUTER_VPL; ++i)
+          if (i * 32 + lane == idx) key[i] = 0u;
+      } else {
+        if (lane == 0) sk[idx] = 0u;
+        __syncwarp();
+      }
+    }
     // softmax over the K selected logits (lanes 0..K-1)
-    float m = lane < K ? sel_logit : -FLT_MAX;
+    const float sel_logit = lane < K ? row[sel_idx] : -FLT_MAX;
+    float m = sel_logit;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     float ex = lane < K ? __expf(sel_logit - m) : 0.f;
@@ -56,10 +91,13 @@ ep_router_topk_kernel(const float* __restrict__ logits, const float* __restrict_
     if (lane < K) {
       topk[(size_t)s * K + lane] = sel_idx;
       weights[(size_t)s * K + lane] = ex / sum;
-      atomicAdd(&tpe[sel_idx], 1);
+      atomicAdd(&s_hist[sel_idx], 1u);
     }
-    __syncwarp();
+    if constexpr (!REGS) __syncwarp();
   }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += (int)blockDim.x)
+    if (s_hist[e] != 0u) atomicAdd(&tpe[e], (int)s_hist[e]);
 }
 
 // d logits = softmax backward scattered to the selected experts (zero elsewhere), bf16 so that
@@ -178,18 +216,21 @@ extern "C" {
 int mep_router_topk(const float* logits, const float* bias, int S, int E, int K, int32_t* topk,
                     float* weights, int32_t* tpe, cudaStream_t stream) {
   if (K > 32 || K < 1 || E < K) return fail(-1, "router: need 1 <= K <= min(32, E)");
-  size_t smem = (size_t)ROUTER_WARPS * E * sizeof(float);
-  if (smem > 200 * 1024) return fail(-2, "router: E=%d too large", E);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    MEP_CUDA_OK(cudaFuncSetAttribute((const void*)ep_router_topk_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
-  MEP_CUDA_OK(cudaMemsetAsync(tpe, 0, sizeof(int32_t) * E, stream));
   int blocks = (S + ROUTER_WARPS - 1) / ROUTER_WARPS;
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  ep_router_topk_kernel<<<blocks, ROUTER_WARPS * 32, smem, stream>>>(logits, bias, S, E, K, topk, weights, tpe);
+  if (blocks > 148 * 2) blocks = 148 * 2;
+  MEP_CUDA_OK(cudaMemsetAsync(tpe, 0, sizeof(int32_t) * E, stream));
+  if (E <= 32 * ROUTER_VPL) {
+    ep_router_topk_kernel<true><<<blocks, ROUTER_WARPS * 32, E * sizeof(uint32_t), stream>>>(logits, bias, S, E, K, topk, weights, tpe);
+  } else {
+    // as many warps as the keys leave room for
+    int warps = (int)(200 * 1024 / (sizeof(uint32_t) * (size_t)E)) - 1;
+    if (warps < 1) return fail(-2, "router: E=%d too large", E);
+    if (warps > ROUTER_WARPS) warps = ROUTER_WARPS;
+    const size_t smem = (size_t)(warps + 1) * E * sizeof(uint32_t);
+    static std::atomic<unsigned long long> raised{0};
+    MEP_CUDA_OK(raise_smem_limit((const void*)ep_router_topk_kernel<false>, raised));
+    ep_router_topk_kernel<false><<<blocks, warps * 32, smem, stream>>>(logits, bias, S, E, K, topk, weights, tpe);
+  }
   MEP_CUDA_OK(cudaGetLastError());
   return 0;
 }

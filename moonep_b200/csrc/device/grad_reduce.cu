@@ -217,12 +217,8 @@ template <int ST, uint32_t GR_CHUNK>
 static int launch_gr_t(const BufferCtx& c, GradReduceParams& p, int grid_x, cudaStream_t stream) {
   size_t smem = (size_t)ST * GR_CHUNK + sizeof(int32_t) * ((size_t)3 * c.epn + (size_t)c.epn * c.R);
   if (smem > 220 * 1024) return fail(-2, "reduce_grad: E=%d is too large for the slot lists", c.E);
-  static thread_local size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    MEP_CUDA_OK(cudaFuncSetAttribute((const void*)ep_grad_reduce_kernel<ST, GR_CHUNK>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static std::atomic<unsigned long long> raised{0};
+  MEP_CUDA_OK(raise_smem_limit((const void*)ep_grad_reduce_kernel<ST, GR_CHUNK>, raised));
   dim3 grid(grid_x > 0 ? grid_x : c.num_sms_weights, c.Rv());
   MEP_CUDA_OK(launch_coop_paired((const void*)ep_grad_reduce_kernel<ST, GR_CHUNK>, grid, dim3(GR_THREADS), smem, stream, p));
   return 0;

@@ -130,7 +130,7 @@ extern "C" int mep_plan_local_noalloc(const int32_t* tpe_all, const int32_t* top
   p.send_order = nullptr; p.arrive_off = 0; p.n_arrive = 0;
   lp.tpe_all = tpe_all; lp.rank = rank; lp.status_out = status;
   const size_t smem = sizeof(int32_t) * (2 * (size_t)E + 4 * (size_t)R + (size_t)PLAN_WARPS * R);
-  if (smem > 48 * 1024) {
+  if (smem > 40 * 1024) {     // (beside the kernel's static part)
     // E <= 16384 keeps this below 133 KB; raising the limit is not an allocation
     MEP_CUDA_OK(cudaFuncSetAttribute((const void*)ep_plan_local_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -204,12 +204,8 @@ int mep_launch_plan(const void* ctx_, const int32_t* topk, const int32_t* tpe, i
   p.scratch = c.plan_scratch; p.scratch_ints = c.plan_scratch_ints;
   p.send_order = send_order; p.arrive_off = c.ml.arrive_off; p.n_arrive = (int)(c.NvS / 128 + 1);
   size_t smem = (size_t)mep_plan_smem_bytes(c.R, c.E);
-  static thread_local size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    MEP_CUDA_OK(cudaFuncSetAttribute((const void*)ep_plan_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static std::atomic<unsigned long long> raised{0};
+  MEP_CUDA_OK(raise_smem_limit((const void*)ep_plan_kernel, raised));
   dim3 grid(c.num_sms, c.Rv());
   MEP_CUDA_OK(launch_coop((const void*)ep_plan_kernel, grid, dim3(PLAN_THREADS), smem, stream, p));
   return 0;

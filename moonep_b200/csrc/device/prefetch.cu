@@ -166,12 +166,8 @@ template <int ST, uint32_t PF_CHUNK>
 static int launch_prefetch_t(const BufferCtx& c, PrefetchParams& p, cudaStream_t stream) {
   size_t smem = (size_t)ST * PF_CHUNK + sizeof(int32_t) * ((size_t)4 * c.epn + (size_t)c.epn * c.R);
   if (smem > 220 * 1024) return fail(-2, "prefetch: E=%d is too large for the slot lists", c.E);
-  static thread_local size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    MEP_CUDA_OK(cudaFuncSetAttribute((const void*)ep_prefetch_kernel<ST, PF_CHUNK>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static std::atomic<unsigned long long> raised{0};
+  MEP_CUDA_OK(raise_smem_limit((const void*)ep_prefetch_kernel<ST, PF_CHUNK>, raised));
   dim3 grid(c.num_sms_weights, c.Rv());
   MEP_CUDA_OK(launch_coop_paired((const void*)ep_prefetch_kernel<ST, PF_CHUNK>, grid, dim3(PF_THREADS), smem, stream, p));
   return 0;

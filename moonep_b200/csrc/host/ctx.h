@@ -8,6 +8,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include <cstdint>
 
 #include "common/layout.h"
@@ -62,6 +64,25 @@ struct BufferCtx {
 // alloc_cumsum[E*R] + expert_off[R*E] + per-CTA histograms [num_sms*E].
 inline int64_t plan_scratch_ints(int R, int E, int num_sms) {
   return (int64_t)4 * R * E + (int64_t)num_sms * E;
+}
+
+// Lets `kernel` be launched with all the dynamic shared memory that the device has beside the kernel's
+// static part, once per kernel and device (`done`: one bit per device).  It is raised for every
+// launch size: a launch whose dynamic part stays within 48 KB but whose sum with the static part
+// does not is refused by the driver, and a limit that followed the sizes of one thread's launches
+// could be lowered under another thread's.
+inline cudaError_t raise_smem_limit(const void* kernel, std::atomic<unsigned long long>& done) {
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  cudaFuncAttributes fa;
+  if ((e = cudaFuncGetAttributes(&fa, kernel)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
 }
 
 // Cooperative launch helper: all CTAs of grid (gx, gy) must be co-resident.
