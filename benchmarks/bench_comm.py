@@ -138,13 +138,13 @@ class OursArm:
             nat.call("mep_launch_sync", buf._ctx, st())))
         r["k_dispatch_us"] = timed(lambda: nat.call(
             "mep_launch_dispatch", buf._ctx, x.data_ptr(), 0, plan.dst.data_ptr(),
-            plan.zero_fill_ranges.data_ptr(), 0, 0, 1, 0, 0, st()))
+            plan.zero_fill_ranges.data_ptr(), 0, 0, 1, 0, 0, 0, st()))
         r["k_expand_us"] = timed(lambda: nat.call(
             "mep_launch_expand", buf._ctx, plan.link.data_ptr(), plan.cu_seqlens.data_ptr(), 0, st()))
         r["k_prologue_us"] = timed(lambda: nat.call(
             "mep_launch_combine_prologue", buf._ctx, plan.link.data_ptr(), plan.cu_seqlens.data_ptr(), st()))
         r["k_combine_us"] = timed(lambda: nat.call(
-            "mep_launch_combine", buf._ctx, plan.dst.data_ptr(), out_sh.data_ptr(), 0, st()))
+            "mep_launch_combine", buf._ctx, plan.dst.data_ptr(), out_sh.data_ptr(), 0, 0, st()))
         if self.R > 1:
             # the conventional exchange at the same shape: all_to_all_single over NCCL + permute
             from moonep_b200.parallel.nccl_baseline import NcclAllToAllEP

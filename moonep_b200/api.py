@@ -51,11 +51,11 @@ nat.declare("mep_ctx_set_trace", None, [P, P])
 nat.declare("mep_launch_plan", I, [P, P, P, P, P, P, P, P, P, P])
 nat.declare("mep_launch_arrive_reset", I, [P, P])
 nat.declare("mep_launch_plan_snapshot", I, [P, P, P, P])
-nat.declare("mep_launch_dispatch", I, [P, P, P, P, P, P, P, I, I, I, P])
+nat.declare("mep_launch_dispatch", I, [P, P, P, P, P, P, P, I, I, I, I, P])
 nat.declare("mep_launch_push_reduce", I, [P, P, L, P, L, P, P, P, P, P, I, P])
 nat.declare("mep_launch_expand", I, [P, P, P, I, P])
 nat.declare("mep_launch_combine_prologue", I, [P, P, P, P])
-nat.declare("mep_launch_combine", I, [P, P, P, P, P])
+nat.declare("mep_launch_combine", I, [P, P, P, P, I, P])
 nat.declare("mep_launch_prefetch", I, [P, P, I, P, P, P, P, P])
 nat.declare("mep_launch_grad_reduce", I, [P, P, I, P, P, P, P, I, I, I, P])
 nat.declare("mep_launch_sync", I, [P, P])
@@ -152,6 +152,10 @@ class Buffer:
         # ---- symmetric buffers ----------------------------------------------------------
         meta_ints = int(nat.call("mep_meta_chunk_ints", self.NvS, R, E))
         self._solo = self.virtual or R == 1
+        # Every rank's buffers are memory of this device: a token's duplicate rows cross no link, so
+        # dispatch stores and combine reads them directly (no expansion, no pre-reduction), and
+        # stream order stands in for the barriers between launches.
+        self._one_device = self._solo
         if self._solo:
             self.hidden_buf = symm.create_local_group_tensor((self.NvS, H), torch.bfloat16, R, self.device)
             self.meta_buf = symm.create_local_group_tensor((meta_ints,), torch.int32, R, self.device)
@@ -394,9 +398,11 @@ class Buffer:
                           plan.dst.data_ptr(), plan.zero_fill_ranges.data_ptr(),
                           plan.link.data_ptr() if fresh else 0,
                           plan.src_info.data_ptr() if fresh else 0,
-                          int(bool(inter_rank_sync) and not fresh), int(fresh), shard, st), "dispatch")
-        self._rc(nat.call("mep_launch_expand", self._ctx, plan.link.data_ptr(),
-                          plan.cu_seqlens.data_ptr(), shard, st), "dispatch expand")
+                          int(bool(inter_rank_sync) and not fresh), int(fresh), shard,
+                          int(self._one_device), st), "dispatch")
+        if not self._one_device:
+            self._rc(nat.call("mep_launch_expand", self._ctx, plan.link.data_ptr(),
+                              plan.cu_seqlens.data_ptr(), shard, st), "dispatch expand")
         view = self.hidden_view(shard)
         hidden = view if zero_copy else view.clone()
         weights = None
@@ -531,20 +537,21 @@ class Buffer:
     def _combine_on_current_stream(self, plan, hidden_nvsh, w_nvs, inter_rank_sync, zero_copy, w_zero_copy):
         st = self._stream()
         dev = hidden_nvsh.device
-        if inter_rank_sync:
+        if inter_rank_sync and not self._one_device:
             self._rc(nat.call("mep_launch_sync", self._ctx, st), "inter_rank_sync")
         if not zero_copy:
             self.hidden_nvsh_buffer_view.copy_(hidden_nvsh)
         if w_nvs is not None and not w_zero_copy:
             self.router_weight_buffer_view.copy_(w_nvs)
-        self._rc(nat.call("mep_launch_combine_prologue", self._ctx, plan.link.data_ptr(),
-                          plan.cu_seqlens.data_ptr(), st), "combine prologue")
+        if not self._one_device:
+            self._rc(nat.call("mep_launch_combine_prologue", self._ctx, plan.link.data_ptr(),
+                              plan.cu_seqlens.data_ptr(), st), "combine prologue")
         out = torch.empty(self._shape(self.S, self.H), dtype=torch.bfloat16, device=dev)
         w_out = None
         if w_nvs is not None:
             w_out = torch.empty(self._shape(self.S, self.K), dtype=torch.float32, device=dev)
         self._rc(nat.call("mep_launch_combine", self._ctx, plan.dst.data_ptr(), out.data_ptr(),
-                          nat.ptr(w_out), st), "combine")
+                          nat.ptr(w_out), int(self._one_device), st), "combine")
         self._stats["combine"] += 1
         self._stats["bytes_combine"] += self.N * self.H * 2 * self.Rv
         self._maybe_check()

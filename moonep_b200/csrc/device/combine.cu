@@ -1,5 +1,7 @@
 // Combine: local fp32 pre-reduction of duplicate rows, then every rank PULLS the rows of its
-// own tokens from the peers' shards and sums them in fp32 in ascending k.
+// own tokens from the peers' shards and sums them in fp32 in ascending k.  When every shard is on
+// this device (one rank, or a virtual group) the pull reads the duplicates itself and there is no
+// pre-reduction pass (template DIRECT).
 //
 // Reference counterparts: CombinePrologueKernel (moonep/combine_prologue.py:196-484) and
 // CombineKernel (moonep/combine.py:210-511).  The sum is unweighted, as in the reference:
@@ -223,8 +225,29 @@ struct CombineParams {
 constexpr int COMBINE_ACC_THREADS = ACC_THREADS;
 constexpr int COMBINE_THREADS = 32 + COMBINE_ACC_THREADS + 32;  // loader, accumulator warps, weights
 
-// NV: 16-byte vectors per accumulator thread (H <= NV * 128 * 8)
-template <int ST, int NV>
+// What the accumulators do with a staged row.
+enum : int { ROW_STARTS_GROUP = 1, ROW_ENDS_GROUP = 2, ROW_ENDS_TOKEN = 4 };
+
+// acc (+)= the bf16-rounded sum of one duplicate group: what the pre-reduction would have stored
+template <int NV>
+__device__ __forceinline__ void fold_group(unsigned long long (&tot)[NV][4], const unsigned long long (&grp)[NV][4],
+                                           bool first) {
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    unsigned long long t[4];
+    bf16x8_to_f32x2(f32x2_to_bf16x8(grp[i]), t);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) tot[i][q] = first ? t[q] : add_f32x2(tot[i][q], t[q]);
+  }
+}
+
+// NV: 16-byte vectors per accumulator thread (H <= NV * 128 * 8).
+// DIRECT (every shard is memory of this device): the loader also reads the duplicates, group by group
+// in the order of the primaries' k, and the accumulators sum a group in registers, round it to
+// bf16 once and add it to the token's sum: the same additions and roundings, in the same order, as
+// pre-reduction + pull, without the pass that reads every duplicate group and writes its primary back,
+// and without the barriers, since launches of one stream already order the rows.
+template <int ST, int NV, bool DIRECT>
 __global__ void __launch_bounds__(COMBINE_THREADS, 1) ep_combine_kernel(const CombineParams p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full[ST];
@@ -245,13 +268,50 @@ __global__ void __launch_bounds__(COMBINE_THREADS, 1) ep_combine_kernel(const Co
   __syncthreads();
   pdl_wait();                 // this rank's pre-reduction kernel has completed
   if (tid == 0) phase_stamp(sc.trace, 1, c, 0);
-  cross_rank_barrier(sc, 1);  // every rank's shard (and its pre-reduction) is final
+  if constexpr (!DIRECT) cross_rank_barrier(sc, 1);  // every rank's shard (and its pre-reduction) is final
   if (tid == 0) phase_stamp(sc.trace, 1, c, 1);          // past the entry barrier: pulls start
 
   const int32_t* dst = p.dst + (size_t)vr * p.N;
   const int n_tok = c < p.S ? (p.S - c + G - 1) / G : 0;
 
-  if (warp == 0) {
+  if (DIRECT && warp == 0) {
+    // ---- loader: all K rows of a token, one lane each ----------------------------------------
+    // The rows travel in the order (k of the group's primary, k): a lane's place among its token's
+    // rows is the number of rows ahead of its own in that order.
+    const uint32_t NvS = (uint32_t)p.NvS;
+    int prod = 0;
+    int d_next = (n_tok > 0 && lane < p.K) ? dst[(size_t)c * p.K + lane] : 0;
+    for (int j = 0; j < n_tok; ++j, prod += p.K) {
+      const int d = d_next;
+      d_next = (j + 1 < n_tok && lane < p.K) ? dst[(size_t)(c + (int64_t)(j + 1) * G) * p.K + lane] : 0;
+      const uint32_t raw = (uint32_t)(d >= 0 ? d : -d - 1);
+      uint32_t dr = raw / NvS;
+      const uint32_t row = raw - dr * NvS;
+      const bool mine = lane < p.K;
+      if (mine && dr >= (uint32_t)sc.R) { report_failure(sc, ST_BAD_INDEX, 21, (int)dr, d, (int)p.NvS); dr = 0; }
+      const unsigned grp = __match_any_sync(0xffffffffu, mine ? (int)dr : (0x40000000 | lane));
+      const int prim = __ffs(grp) - 1;
+      int place = 0;
+      for (int i = 0; i < p.K; ++i) {
+        const int pi = __shfl_sync(0xffffffffu, prim, i);
+        place += (pi < prim || (pi == prim && i < lane)) ? 1 : 0;
+      }
+      // at most ST rows at a time: a lane that waits for a stage then never waits for a row that
+      // another lane of its own round has yet to issue
+      for (int p0 = 0; p0 < p.K; p0 += ST) {
+        if (mine && place >= p0 && place < p0 + ST) {
+          const int q = prod + place, s = q % ST;
+          if (q >= ST) mbar_wait(sc, &empty[s], ((uint32_t)(q / ST) & 1u) ^ 1u, 20);
+          last_flag[s] = (lane == prim ? ROW_STARTS_GROUP : 0) | ((grp >> lane) == 1u ? ROW_ENDS_GROUP : 0) |
+                         (place == p.K - 1 ? ROW_ENDS_TOKEN : 0);
+          mbar_expect_tx(&full[s], row_bytes);
+          bulk_g2s(ring + (size_t)s * row_bytes, p.hidden + ((size_t)dr * p.hidden_stride + row) * p.H, row_bytes,
+                   &full[s]);
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp == 0) {
     // ---- loader: one remote bulk read per primary entry -----------------------------------
     int prod = 0;
     int d_next = (n_tok > 0 && lane < p.K) ? dst[(size_t)c * p.K + lane] : -1;
@@ -283,14 +343,28 @@ __global__ void __launch_bounds__(COMBINE_THREADS, 1) ep_combine_kernel(const Co
     int cons = 0;
     for (int j = 0; j < n_tok; ++j) {
       unsigned long long acc[NV][4];
+      [[maybe_unused]] unsigned long long grp[DIRECT ? NV : 1][4];
       bool first = true;
       for (int guard = 0; guard < MAX_TOPK; ++guard) {
         const int s = cons % ST;
         bool ok = mbar_wait(sc, &full[s], (uint32_t)(cons / ST) & 1u, 30);
         const uint4* src = reinterpret_cast<const uint4*>(ring + (size_t)s * row_bytes);
-        const int is_last = ok ? last_flag[s] : 1;
-        accumulate_row<NV>(acc, src, ta, nvec, first);
-        first = false;
+        bool is_last;
+        if constexpr (DIRECT) {
+          const int f = ok ? last_flag[s] : (ROW_STARTS_GROUP | ROW_ENDS_GROUP | ROW_ENDS_TOKEN);
+          is_last = (f & ROW_ENDS_TOKEN) != 0;
+          if ((f & ROW_STARTS_GROUP) && (f & ROW_ENDS_GROUP)) {
+            accumulate_row<NV>(acc, src, ta, nvec, first);      // a lone row is its own rounded sum
+            first = false;
+          } else {
+            accumulate_row<NV>(grp, src, ta, nvec, (f & ROW_STARTS_GROUP) != 0);
+            if (f & ROW_ENDS_GROUP) { fold_group<NV>(acc, grp, first); first = false; }
+          }
+        } else {
+          is_last = !ok || last_flag[s] != 0;
+          accumulate_row<NV>(acc, src, ta, nvec, first);
+          first = false;
+        }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
         ++cons;
@@ -341,9 +415,12 @@ struct PushReduceParams {
   const int32_t* cu_seqlens;       // [Rv][2epn]
   __nv_bfloat16* out;              // [Rv][S][H]
   float* w_out;                    // [Rv][S][K] or null
+  int one_device;                  // every rank's staging is memory of this device
 };
 
-constexpr int PUSH_REDUCE_THREADS = 256;
+// 1024 threads, eight 16-byte loads each in flight: one CTA an SM with 256 threads kept 32 KB in
+// flight and ran at 3.4 TB/s (4096 tokens x 7168, top-8: 154 us).
+constexpr int PUSH_REDUCE_THREADS = 1024;
 
 __global__ void __launch_bounds__(PUSH_REDUCE_THREADS, 1) ep_push_reduce_kernel(const PushReduceParams p) {
   const SyncCtx& sc = p.sync;
@@ -362,32 +439,38 @@ __global__ void __launch_bounds__(PUSH_REDUCE_THREADS, 1) ep_push_reduce_kernel(
       if (sr < sc.R) p.wpush[(size_t)sr * p.wpush_stride + ent] = rs[r];
     }
   }
-  fence_sys();
-  cross_rank_barrier(sc, 1);
+  if (!p.one_device || p.row_scalar != nullptr) {      // (on one device the launch boundary ordered the rows)
+    fence_sys();
+    cross_rank_barrier(sc, 1);
+  }
   const uint4* mine = reinterpret_cast<const uint4*>(p.push + (size_t)rank * p.push_stride);
   uint4* out = reinterpret_cast<uint4*>(p.out + (size_t)vr * p.S * p.H);
+  // one 16-byte vector v of one token s per thread and step; (s, v) advance without a division
   const int nvec = p.H / 8;
-  for (int s = c; s < p.S; s += G) {
-    const uint4* base = mine + (size_t)s * p.K * nvec;
-    for (int v = tid; v < nvec; v += PUSH_REDUCE_THREADS) {
-      float acc[8];
+  const int step_s = G * PUSH_REDUCE_THREADS / nvec, step_v = G * PUSH_REDUCE_THREADS - step_s * nvec;
+  int s = (c * PUSH_REDUCE_THREADS + tid) / nvec, v = c * PUSH_REDUCE_THREADS + tid - s * nvec;
+  while (s < p.S) {
+    const uint4* base = mine + (size_t)s * p.K * nvec + v;
+    float acc[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] = 0.f;
-      for (int k0 = 0; k0 < p.K; k0 += 8) {
-        uint4 raw[8];
+    for (int q = 0; q < 8; ++q) acc[q] = 0.f;
+    for (int k0 = 0; k0 < p.K; k0 += 8) {
+      uint4 raw[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          raw[u] = k0 + u < p.K ? base[(size_t)(k0 + u) * nvec + v] : make_uint4(0, 0, 0, 0);
+      for (int u = 0; u < 8; ++u)
+        raw[u] = k0 + u < p.K ? base[(size_t)(k0 + u) * nvec] : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          float t[8];
-          bf16x8_to_f32(raw[u], t);
+      for (int u = 0; u < 8; ++u) {
+        float t[8];
+        bf16x8_to_f32(raw[u], t);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) acc[q] += t[q];
-        }
+        for (int q = 0; q < 8; ++q) acc[q] += t[q];
       }
-      out[(size_t)s * nvec + v] = f32_to_bf16x8(acc);
     }
+    out[(size_t)s * nvec + v] = f32_to_bf16x8(acc);
+    s += step_s;
+    v += step_v;
+    if (v >= nvec) { v -= nvec; ++s; }
   }
   if (p.w_out != nullptr) {
     const float* wm = p.wpush + (size_t)rank * p.wpush_stride;
@@ -397,25 +480,31 @@ __global__ void __launch_bounds__(PUSH_REDUCE_THREADS, 1) ep_push_reduce_kernel(
   }
 }
 
-template <int ST, int NV>
+template <int ST, int NV, bool DIRECT>
 static int launch_combine_t(const BufferCtx& c, CombineParams& p, size_t smem, cudaStream_t stream) {
   static std::atomic<unsigned long long> raised{0};
-  MEP_CUDA_OK(raise_smem_limit((const void*)ep_combine_kernel<ST, NV>, raised));
+  MEP_CUDA_OK(raise_smem_limit((const void*)ep_combine_kernel<ST, NV, DIRECT>, raised));
   dim3 grid(c.num_sms, c.Rv());
-  MEP_CUDA_OK(launch_chained((const void*)ep_combine_kernel<ST, NV>, grid, dim3(COMBINE_THREADS), smem,
-                             stream, p, /*coop=*/1, c.pdl));
+  // (DIRECT follows no kernel of its own chain and has no barrier inside)
+  MEP_CUDA_OK(launch_chained((const void*)ep_combine_kernel<ST, NV, DIRECT>, grid, dim3(COMBINE_THREADS), smem,
+                             stream, p, /*coop=*/!DIRECT, c.pdl && !DIRECT));
   return 0;
 }
 
-template <int NV>
+template <int NV, bool DIRECT>
 static int launch_combine_nv(const BufferCtx& c, CombineParams& p, cudaStream_t stream) {
   const size_t row = (size_t)c.H * 2;
-  const size_t budget = c.virt ? 100 * 1024 : 210 * 1024;
-  if (14 * row <= budget) return launch_combine_t<14, NV>(c, p, 14 * row, stream);
-  if (10 * row <= budget) return launch_combine_t<10, NV>(c, p, 10 * row, stream);
-  if (6 * row <= budget) return launch_combine_t<6, NV>(c, p, 6 * row, stream);
-  if (3 * row <= 220 * 1024) return launch_combine_t<3, NV>(c, p, 3 * row, stream);
+  const size_t budget = c.ring_budget(210 * 1024);
+  if (14 * row <= budget) return launch_combine_t<14, NV, DIRECT>(c, p, 14 * row, stream);
+  if (10 * row <= budget) return launch_combine_t<10, NV, DIRECT>(c, p, 10 * row, stream);
+  if (6 * row <= budget) return launch_combine_t<6, NV, DIRECT>(c, p, 6 * row, stream);
+  if (3 * row <= 220 * 1024) return launch_combine_t<3, NV, DIRECT>(c, p, 3 * row, stream);
   return fail(-2, "combine: H=%d does not fit a 2-stage ring", c.H);
+}
+
+template <int NV>
+static int launch_combine_d(const BufferCtx& c, CombineParams& p, int direct, cudaStream_t stream) {
+  return direct ? launch_combine_nv<NV, true>(c, p, stream) : launch_combine_nv<NV, false>(c, p, stream);
 }
 
 template <int ST, int NV>
@@ -477,15 +566,18 @@ int mep_launch_push_reduce(const void* ctx_, const void* push, int64_t push_stri
   p.push_stride = push_stride; p.wpush_stride = wpush_stride;
   p.push = (const __nv_bfloat16*)push; p.wpush = (float*)wpush; p.src_info = src_info;
   p.row_scalar = row_scalar; p.cu_seqlens = cu_seqlens; p.out = (__nv_bfloat16*)out; p.w_out = w_out;
+  p.one_device = c.one_device();
   dim3 grid(grid_x > 0 ? grid_x : c.num_sms, c.Rv());
   MEP_CUDA_OK(launch_coop((const void*)ep_push_reduce_kernel, grid, dim3(PUSH_REDUCE_THREADS), 0, stream, p));
   return 0;
 }
 
-// dst [Rv][N], out [Rv][S][H] bf16, w_out [Rv][S][K] fp32 or null.
-int mep_launch_combine(const void* ctx_, const int32_t* dst, void* out, float* w_out,
+// dst [Rv][N], out [Rv][S][H] bf16, w_out [Rv][S][K] fp32 or null.  direct != 0 (only where every
+// rank's shard is on this device): no pre-reduction has run, the duplicates are summed here.
+int mep_launch_combine(const void* ctx_, const int32_t* dst, void* out, float* w_out, int direct,
                        cudaStream_t stream) {
   const BufferCtx& c = *(const BufferCtx*)ctx_;
+  if (direct && !c.one_device()) return fail(-4, "combine: duplicates are read only within one device");
   if (c.H % 8 != 0) return fail(-1, "combine needs H %% 8 == 0 (got %d)", c.H);
   CombineParams p;
   p.sync = c.sync(KID_COMBINE);
@@ -495,10 +587,10 @@ int mep_launch_combine(const void* ctx_, const int32_t* dst, void* out, float* w
   p.out = (__nv_bfloat16*)out; p.w_out = w_out;
   const int nvec = c.H / 8;
   const int nv = (nvec + COMBINE_ACC_THREADS - 1) / COMBINE_ACC_THREADS;
-  if (nv <= 1) return launch_combine_nv<1>(c, p, stream);
-  if (nv <= 2) return launch_combine_nv<2>(c, p, stream);
-  if (nv <= 4) return launch_combine_nv<4>(c, p, stream);
-  if (nv <= 10) return launch_combine_nv<10>(c, p, stream);
+  if (nv <= 1) return launch_combine_d<1>(c, p, direct, stream);
+  if (nv <= 2) return launch_combine_d<2>(c, p, direct, stream);
+  if (nv <= 4) return launch_combine_d<4>(c, p, direct, stream);
+  if (nv <= 10) return launch_combine_d<10>(c, p, direct, stream);
   return fail(-3, "combine: H=%d is larger than 16384", c.H);
 }
 

@@ -10,7 +10,9 @@
 //  * there is no dedup builder: the chain links were written by the planner (source side);
 //    the kernel only snapshots this rank's links into the plan after its exit barrier;
 //  * padding rows are zeroed with bulk stores from one zero row, and their weight and link
-//    slots are reset locally.
+//    slots are reset locally;
+//  * when every destination's buffer is on this device (one rank, or a virtual group) there is no
+//    link to save: the duplicates are stored from the staged row too, and no expansion follows.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -36,6 +38,11 @@ struct DispatchParams {
   int32_t* src_out;           // [Rv][NvS] or null
   int entry_barrier;
   int fresh;                  // plan made by the preceding planner launch
+  // Every destination's row buffer is on this device: duplicates are stored from the staged row, and
+  // launches of one stream order what the cross-rank entry barrier would.  8 ranks x 4096 tokens x
+  // 7168, top-8: one launch of 0.59 ms and an expansion of 0.95 ms (which reads every primary row
+  // back from HBM) became one launch, bound by its stores; see mep_launch_dispatch.
+  int direct;
 };
 
 constexpr int DISPATCH_THREADS = 128;
@@ -64,7 +71,7 @@ __global__ void __launch_bounds__(DISPATCH_THREADS, 1) ep_dispatch_kernel(const 
   pdl_launch_dependents();   // the expansion kernel may be scheduled; it waits for this one to end
   pdl_wait();                // a preceding planner launch has completed: its plan is readable
   if (tid == 0) phase_stamp(sc.trace, 0, c, 0);          // set up, predecessor complete
-  if (p.entry_barrier) cross_rank_barrier(sc, 1);
+  if (p.entry_barrier && !p.direct) cross_rank_barrier(sc, 1);
   if (tid == 0) phase_stamp(sc.trace, 0, c, 1);          // past the entry barrier
 
   const __nv_bfloat16* x = p.x + (size_t)vr * p.S * p.H;
@@ -81,14 +88,17 @@ __global__ void __launch_bounds__(DISPATCH_THREADS, 1) ep_dispatch_kernel(const 
       }
     }
     __syncwarp();
+    const uint32_t NvS = (uint32_t)p.NvS;          // R * NvS < 2^31: 32-bit arithmetic is enough
+    int d_next = n_tok > 0 && lane < p.K ? dst[(size_t)c * p.K + lane] : 0;
     for (int j = 0; j < n_tok; ++j) {
       const int s = j % ST;
-      const int t = c + j * G;
-      int d = lane < p.K ? dst[(size_t)t * p.K + lane] : -1;
+      const int d = d_next;                        // the next token's entries load while this one moves
+      d_next = j + 1 < n_tok && lane < p.K ? dst[(size_t)(c + (int64_t)(j + 1) * G) * p.K + lane] : 0;
       mbar_wait(sc, &full[s], (uint32_t)(j / ST) & 1u, 10);
-      if (d >= 0) {
-        int64_t dr = d / p.NvS, row = d - dr * p.NvS;
-        if (dr < sc.R) {
+      if (lane < p.K && (d >= 0 || p.direct)) {
+        const uint32_t raw = (uint32_t)(d >= 0 ? d : -d - 1);
+        const uint32_t dr = raw / NvS, row = raw - dr * NvS;
+        if (dr < (uint32_t)sc.R) {
           bulk_s2g(p.hidden + ((size_t)dr * p.hidden_stride + row) * p.H,
                    ring + (size_t)s * row_bytes, row_bytes);
         } else {
@@ -127,31 +137,44 @@ __global__ void __launch_bounds__(DISPATCH_THREADS, 1) ep_dispatch_kernel(const 
     }
   } else {
     // ---- padding rows of MY shard: zero payload, weight 0, link NONE ----------------------
+    // The lanes fetch 32 groups' ranges at once: one group at a time, the two dependent loads a
+    // group cost ~0.6 us each and were the kernel at 256 groups and more.
     const int32_t* zf = p.zero_fill + (size_t)vr * 2 * p.epn * 2;
     int32_t* my_meta = sc.meta + (size_t)rank * sc.meta_stride;
     __nv_bfloat16* my_shard = p.hidden + (size_t)rank * p.hidden_stride * p.H;
     int pending = 0;
-    for (int g = 0; g < 2 * p.epn; ++g) {
-      const int first = zf[2 * g], n = zf[2 * g + 1];
-      if (n <= 0 || first < 0 || (int64_t)first + n > p.NvS) continue;
-      if (warp == 2) {
-        // one elected thread issues the row stores of this CTA's share
-        if (lane == 0) {
-          for (int r = first + c; r < first + n; r += G) {
-            bulk_s2g(my_shard + (size_t)r * p.H, zero_row, row_bytes);
-            if (++pending == 16) { bulk_commit(); bulk_wait_read<4>(); pending = 0; }
+    for (int g0 = 0; g0 < 2 * p.epn; g0 += 32) {
+      const int g = g0 + lane;
+      const int2 mine = g < 2 * p.epn ? make_int2(zf[2 * g], zf[2 * g + 1]) : make_int2(0, 0);
+      unsigned some = __ballot_sync(0xffffffffu, mine.y > 0 && mine.x >= 0 && (int64_t)mine.x + mine.y <= p.NvS);
+      while (some) {
+        const int i = __ffs(some) - 1;
+        some &= some - 1;
+        const int first = __shfl_sync(0xffffffffu, mine.x, i), n = __shfl_sync(0xffffffffu, mine.y, i);
+        // group i starts its round over the CTAs at CTA i * 7: short ranges do not all end up on the first ones
+        const int c_rot = (int)((unsigned)(c + (g0 + i) * 7) % (unsigned)G);
+        if (warp == 2) {
+          // one elected thread issues the row stores of this CTA's share
+          if (lane == 0) {
+            for (int r = first + c_rot; r < first + n; r += G) {
+              bulk_s2g(my_shard + (size_t)r * p.H, zero_row, row_bytes);
+              if (++pending == 16) { bulk_commit(); bulk_wait_read<4>(); pending = 0; }
+            }
           }
-        }
-      } else {
-        for (int r = first + c * 32 + lane; r < first + n; r += G * 32) {
-          if (p.w != nullptr) my_meta[p.weights_off + r] = 0;
-          if (p.fresh) { my_meta[p.link_off + r] = LINK_NONE; my_meta[p.src_off + r] = -1; }
+        } else {
+          for (int r = first + c_rot * 32 + lane; r < first + n; r += G * 32) {
+            if (p.w != nullptr) my_meta[p.weights_off + r] = 0;
+            if (p.fresh) { my_meta[p.link_off + r] = LINK_NONE; my_meta[p.src_off + r] = -1; }
+          }
         }
       }
     }
     if (warp == 2 && lane == 0) { bulk_commit(); bulk_wait<0>(); fence_proxy_async(); }
   }
   if (tid == 0) phase_stamp(sc.trace, 0, c, 2);          // this CTA's rows, weights and padding issued
+  // With everything on one device the end of the launch orders the rows; the barrier is then only
+  // needed ahead of the snapshots below, which read what other CTAs wrote.
+  if (p.direct && p.link_out == nullptr && p.src_out == nullptr) return;
   fence_sys();
   cross_rank_barrier(sc, 2);
   if (tid == 0) phase_stamp(sc.trace, 0, c, 3);          // past the exit barrier
@@ -313,13 +336,15 @@ extern "C" {
 // x [Rv][S][H] bf16, w [Rv][S][K] fp32 or null, dst [Rv][N], zero_fill [Rv][2epn][2],
 // link_out [Rv][NvS] or null.  fresh != 0: the plan comes from the planner launch that
 // precedes this one on the stream (its barrier stands in for the entry sync).  shard selects
-// the row buffer the rows land in (0, or 1 once a second shard is registered).
+// the row buffer the rows land in (0, or 1 once a second shard is registered).  direct != 0 (only
+// where every rank's buffer is on this device) also stores the duplicates; no expansion follows.
 int mep_launch_dispatch(const void* ctx_, const void* x, const float* w, const int32_t* dst,
                         const int32_t* zero_fill, int32_t* link_out, int32_t* src_out, int entry_barrier,
-                        int fresh, int shard, cudaStream_t stream) {
+                        int fresh, int shard, int direct, cudaStream_t stream) {
   const BufferCtx& c = *(const BufferCtx*)ctx_;
   if (c.H % 8 != 0) return fail(-1, "dispatch needs H %% 8 == 0 (got %d)", c.H);
   if (c.shard_base(shard) == nullptr) return fail(-4, "dispatch: shard %d does not exist", shard);
+  if (direct && !c.one_device()) return fail(-5, "dispatch: duplicates travel only within one device");
   DispatchParams p;
   p.sync = c.sync(KID_DISPATCH);
   p.S = c.S; p.K = c.K; p.H = c.H; p.epn = c.epn;
@@ -327,10 +352,10 @@ int mep_launch_dispatch(const void* ctx_, const void* x, const float* w, const i
   p.weights_off = c.ml.weights_off; p.link_off = c.ml.link_off; p.src_off = c.ml.src_off;
   p.x = (const __nv_bfloat16*)x; p.w = w; p.dst = dst; p.zero_fill = zero_fill;
   p.hidden = (__nv_bfloat16*)c.shard_base(shard); p.link_out = link_out; p.src_out = src_out;
-  p.entry_barrier = entry_barrier; p.fresh = fresh;
+  p.entry_barrier = entry_barrier; p.fresh = fresh; p.direct = direct;
   const size_t row = (size_t)c.H * 2;
-  // virtual groups must keep gridDim.x * R CTAs co-resident: leave room for 2 CTAs per SM
-  const size_t budget = c.virt ? 100 * 1024 : 200 * 1024;
+  const size_t budget = c.ring_budget(200 * 1024);
+  if (17 * row <= budget) return launch_dispatch_t<16>(c, p, 17 * row, stream);
   if (9 * row <= budget) return launch_dispatch_t<8>(c, p, 9 * row, stream);
   if (5 * row <= budget) return launch_dispatch_t<4>(c, p, 5 * row, stream);
   if (3 * row <= 220 * 1024) return launch_dispatch_t<2>(c, p, 3 * row, stream);

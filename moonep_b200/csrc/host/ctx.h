@@ -37,6 +37,13 @@ struct BufferCtx {
   int pdl;                 // chain plan -> dispatch -> expand and prologue -> combine programmatically
 
   int Rv() const { return virt ? R : 1; }
+  // Every rank's buffers are memory of this device: a lone rank, or a virtual group.
+  bool one_device() const { return virt != 0 || R == 1; }
+  // Shared memory a copy ring may take: `most`, unless a virtual group's num_sms * R co-resident
+  // CTAs outnumber the SMs, which then have to hold two each.
+  size_t ring_budget(size_t most) const {
+    return virt && num_sms * R > sm_count ? 100 * 1024 : most;
+  }
   // Row buffer that a launch with the given shard index works on (null when it does not exist).
   // The choice is a launch ARGUMENT: nothing in the context changes between launches, so
   // dispatches into different shards may be issued from different threads or streams.
