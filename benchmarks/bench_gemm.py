@@ -112,7 +112,7 @@ def ab(args, ops, x, act, cu, grad, w, out):
         torch.cuda.synchronize()
         return a.elapsed_time(b) / n
 
-    variants = [("single", 0, False), ("single_plain_epilogue", 0, True), ("pair", 1, False), ("pair_plain_epilogue", 1, True)]
+    variants = [("single", 0), ("pair", 1)]
     ops = dict(ops)
     ops.pop("cublas_ref_down(torch.bmm)", None)
     flops_w = ops["wgrad"][1]
@@ -120,18 +120,15 @@ def ab(args, ops, x, act, cu, grad, w, out):
     for name, (fn, flops) in ops.items():
         if args.only and args.only not in name:
             continue
-        vs = [v for v in variants if "wgrad" not in name or not v[2]]
-        for _, two, dbg in vs:
-            gemm.TWO_CTA, gemm.PLAIN_EPILOGUE = two, dbg
+        for _, gemm.TWO_CTA in variants:
             fn()
         torch.cuda.synchronize()
-        best = {v[0]: 1e9 for v in vs}
+        best = {v: 1e9 for v, _ in variants}
         for _ in range(6):
-            for v, two, dbg in vs:
-                gemm.TWO_CTA, gemm.PLAIN_EPILOGUE = two, dbg
+            for v, gemm.TWO_CTA in variants:
                 best[v] = min(best[v], run(fn))
         out[name] = {v: {"ms": round(t, 4), "tflops": round(flops / t / 1e9)} for v, t in best.items()}
-    gemm.TWO_CTA, gemm.PLAIN_EPILOGUE = 2, False
+    gemm.TWO_CTA = 2
     gemm.check_status()
     print(json.dumps(out))
 

@@ -3,25 +3,16 @@
 // fp32 accumulators in tensor memory, read back with tcgen05.ld for fused epilogues.
 //
 // The reference ships no GEMM: it hands cu_seqlens and the [2*epn, H, H'] compute view to the
-// host framework's "VM group GEMM" (README.md:45-68).  This kernel is that GEMM.  One
-// persistent CTA per SM walks a static tile list derived on the device from cu_seqlens (no
-// host synchronisation), with three warp roles:
-//   warp 0      TMA producer        (4-stage ring of 128x64 A and 256x64 B tiles, 48 KB each)
-//   warp 1      MMA issuer          (128x256x16 UMMAs, two 256-column TMEM accumulators)
-//   warps 2..5  epilogue            (TMEM -> registers -> global, plain stores or staged TMA
-//                                   stores), overlapped with the next tile's main loop through
-//                                   the second accumulator
-// Modes:
-//   token-major (groups partition the rows of A and C):
-//        C[rows of g] = A[rows of g] * B[g]     B K-major ([N][K]) or MN-major ([K][N])
-//        epilogues: bf16 store, fp32 store, or SwiGLU: the tile holds 128 gate and 128 up
-//        columns of the same output columns; writes gate, up and silu(gate)*up*row_scale.
-//        Up to two K segments accumulate into one tile (dX = dG*Wg^T + dU*Wu^T).
-//        PUSH epilogue (GEMM fused with the combine all-to-all): each finished row segment is
-//        stored, over NVLink, straight into the slot of its (token, k) entry in the token's
-//        HOME rank's staging buffer, so the transfer overlaps the math tile by tile; the home
-//        rank then only sums K local rows per token.
-//   weight-grad (groups partition the REDUCTION dimension):
+// host framework's "VM group GEMM" (README.md:45-68).  These kernels are that GEMM.  One
+// persistent CTA (or CTA pair) per SM walks a static tile list derived on the device from
+// cu_seqlens (no host synchronisation), with three warp roles: warp 0 TMA producer, warp 1 MMA
+// issuer (two 256-column TMEM accumulators), warps 2.. epilogue, overlapped with the next tile's
+// main loop through the second accumulator.  Kernels:
+//   ep_token_gemm_kernel (token_gemm.cuh): token-major products with bf16 output -- gate/up with
+//        SwiGLU, down, both dgrads, the pushed combine, the fused dispatch.
+//   ep_grouped_gemm_kernel (this file):
+//     token-major with fp32 output (router logits; 128 x 256 tiles, plain transposed stores)
+//     weight-grad (groups partition the REDUCTION dimension):
 //        D[g] (+)= A[rows of g]^T * B[rows of g]   both operands MN-major, fp32 output by TMA
 //        store / reduce-add; or (template SGD) the optimizer step fused in: the accumulator is
 //        applied straight to the bf16 weights, w = bf16(w - lr * acc), through a per-warp TMA
@@ -31,18 +22,12 @@
 // Group g < split reads/writes allocation 0 (local experts), g >= split allocation 1 (this
 // rank's prefetch / reduce slots): the [2*epn] compute view never has to be contiguous.
 // CTA pairs (template TWO, clusters of two CTAs, tcgen05 cta_group::2): the leader issues
-// 256x256x16 MMAs over both CTAs' shared memory; each CTA stages its own 128 rows of A and half
+// 256-row MMAs over both CTAs' shared memory; each CTA stages its own 128 rows of A and half
 // of the B tile (32 KB per k-block instead of 48 KB, six stages), which lifts the single-CTA
 // kernel's limit of 12 KB of operand reads per MMA.  Both CTAs' loads count on the LEADER's full
 // barrier, on which only the leader's producer arrives (expecting the bytes of both): a per-stage
-// arrival from the peer over the cluster network measured 2x slower overall.  Token-major pairs
-// cover 256 rows of one group; weight-grad pairs 256 rows of the weight matrix.
-// Measured A/B (32 groups x 1024 rows, H=7168, H'=2048, interleaved runs under the power cap):
-// pairs +13% gate/up, +13% down, +18% down dgrad, +7% gate/up dgrad, +24% weight grad.
-// Fused dispatch (template DISP, token-major kernels whose A operand is the dispatched rows): a
-// seventh warp per CTA sends this rank's token rows to their destination ranks while the other
-// warps compute, and the TMA producer waits for a tile's rows to have arrived before it loads
-// them (device/fused_dispatch.cuh).  That variant gives up one operand stage for the copy ring.
+// arrival from the peer over the cluster network measured 2x slower overall.  Weight-grad pairs
+// cover 256 rows of the weight matrix (+24% over single CTAs, 32 groups x 1024 rows, H=7168, H'=2048).
 // Every mbarrier wait is bounded; on expiry the CTA records an error, drains and frees TMEM.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -77,23 +62,24 @@ constexpr int STAGE_BYTES2 = A_TILE_BYTES + B_TILE_BYTES / 2;
 
 enum { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_F32 = 2, EPI_PUSH = 3 };
 
+constexpr int TG_BOXES = 4;
+
 struct GemmKParams {
-  CUtensorMap a[2];
+  CUtensorMap a[2];        // 128-row boxes (weight grad: 64 x 64)
+  CUtensorMap tok[2][TG_BOXES];   // token rows in boxes of 32, 64, 96 and 128 rows (token_gemm.cuh)
   CUtensorMap b[2][2];
   CUtensorMap c[2];        // weight-grad output (fp32), per allocation
-  CUtensorMap b2[2][2];    // K-major B with a 128-row box (CTA-pair variant)
-  CUtensorMap o;           // bf16 output of the token-major epilogue (32 x 64 store boxes)
+  CUtensorMap b2[2][2];    // K-major B with a 128-row box
   const int32_t* cu_seqlens;
+  const int32_t* pads;     // [ngroups][2] first padding row and their number, per group; or null
   int ngroups, split, total_rows, N, K, nseg, rows_per_expert, Mw, accumulate, zero_empty_below;
-  // bit 16: per-row plain stores in the bf16 epilogue (A/B of benchmarks; a host-side choice)
-  int debug;
   int stages, wb;   // SGD kernels: operand stages and weight blocks per epilogue warp of this launch
   // SGD kernels: 1 = only the tiles whose grads are STORED (experts with replicas, slot groups),
   // 2 = only the tiles that are applied to the weights, 0 = all.  Lets the grads that have to
   // travel be computed first, so that their reduce runs beside the rest of the weight grad.
   int wg_select;
   int g_begin; // groups below this index are skipped (a launch may cover a suffix of the groups)
-  int tma_out; // outputs are 16-byte aligned: whole 32-row blocks leave through TMA stores
+  int tma_out; // outputs allow 16-byte stores
   // weight grad fused with the SGD step: a local expert's tile is applied straight to its bf16
   // weights, w = bf16(w - lr * acc), instead of being stored as an fp32 grad.  Experts whose
   // sgd_keep flag is set (they have replicas elsewhere, whose grads must be added first) and the
@@ -180,10 +166,16 @@ __device__ __forceinline__ bool arrive_wait(const int32_t* ctr, int expect, int 
   return true;
 }
 
-// TWO: the tile list counts PAIRS of 128-row tiles (256 rows of one group); CTA `crank` of the
-// pair takes the rows [256*mi + 128*crank, +128) and may end up with none in a group's last pair.
-template <bool WGRAD, int EPI, bool TWO = false>
-__device__ __forceinline__ Tile get_tile(const GemmKParams& p, int id, const int* s_end,
+// Rows of a group that hold tokens (its real rows if the padding ranges are known); at least one
+// for a group that is not empty.
+__device__ __forceinline__ int group_valid(const GemmKParams& p, int g, int start, int end) {
+  if (p.pads == nullptr || end <= start) return end - start;
+  const int first = p.pads[2 * g], n = p.pads[2 * g + 1];
+  return (n > 0 && first >= start && first < end) ? max(1, first - start) : end - start;
+}
+
+template <bool WGRAD, bool TWO = false>
+__device__ __forceinline__ Tile get_tile(const GemmKParams& p, int id, const int* s_end, const int* s_valid,
                                          const int* s_prefix, int n_tiles_n, int crank = 0) {
   Tile t;
   t.valid = true;
@@ -194,9 +186,8 @@ __device__ __forceinline__ Tile get_tile(const GemmKParams& p, int id, const int
     t.g = id / tpg;
     int local = id - t.g * tpg;
     int ni = local / mt, mi = local - ni * mt;
-    int start = t.g == 0 ? 0 : s_end[t.g - 1];
-    t.row0 = start;
-    t.rows = s_end[t.g] - start;
+    t.row0 = t.g == 0 ? 0 : s_end[t.g - 1];
+    t.rows = s_valid[t.g];                       // padding rows are zero: blocks of nothing else are skipped
     t.m0 = mi * TMW + crank * BM;
     t.n0 = ni * BN;
     t.num_kb = (t.rows + BK - 1) / BK;
@@ -214,14 +205,13 @@ __device__ __forceinline__ Tile get_tile(const GemmKParams& p, int id, const int
     t.g = lo;
     int start = t.g == 0 ? 0 : s_end[t.g - 1];
     int len = s_end[t.g] - start;
-    constexpr int TM = TWO ? 2 * BM : BM;
-    int mt = max(1, (len + TM - 1) / TM);
+    int mt = max(1, (len + BM - 1) / BM);
     int local = id - s_prefix[t.g] * n_tiles_n;
     int ni = local / mt, mi = local - ni * mt;
-    t.row0 = start + mi * TM + crank * BM;
+    t.row0 = start + mi * BM;
     t.rows = max(0, min(BM, s_end[t.g] - t.row0));
     t.m0 = 0;
-    t.n0 = ni * (EPI == EPI_SWIGLU ? BN / 2 : BN);
+    t.n0 = ni * BN;
     t.num_kb = p.nseg * ((p.K + BK - 1) / BK);
   }
   t.alloc = t.g >= p.split ? 1 : 0;
@@ -235,32 +225,25 @@ __device__ __forceinline__ Tile get_tile(const GemmKParams& p, int id, const int
   return t;
 }
 
-// Operand stages of the kernels whose geometry is fixed at compile time; the fused dispatch gives
-// one up for its copy ring.
-template <bool TWO, bool DISP = false> __host__ __device__ constexpr int gemm_stages() {
-  return (TWO ? GEMM_STAGES2 : GEMM_STAGES) - (DISP ? 1 : 0);
-}
+// Operand stages of the kernels whose geometry is fixed at compile time.
+template <bool TWO> __host__ __device__ constexpr int gemm_stages() { return TWO ? GEMM_STAGES2 : GEMM_STAGES; }
 // The SGD kernels (weight grad with the optimizer step in the epilogue) take their geometry at
 // launch instead (GemmKParams::stages / wb, sgd_geometry() below): how the shared memory is best
 // split between operand stages and weight blocks depends on the group length.
 constexpr int SGD_RING_MAX = 8;      // 4 KB weight blocks per epilogue warp, at most
-// Fused dispatch: stages of the copy ring (the pair kernel with the staged bf16 epilogue has less
-// shared memory to spare).
-template <bool TWO, int EPI> __host__ __device__ constexpr int fd_stages() { return (TWO && EPI == EPI_BF16) ? 5 : 8; }
-template <bool TWO, bool DISP = false, int EPI = EPI_BF16> __host__ __device__ constexpr int gemm_smem() {   // dynamic shared memory
-  return gemm_stages<TWO, DISP>() * (TWO ? STAGE_BYTES2 : STAGE_BYTES) + 1024 +
-         (DISP ? fd_stages<TWO, EPI>() * FD_PART_CAP : 0);
+template <bool TWO> __host__ __device__ constexpr int gemm_smem() {   // dynamic shared memory
+  return gemm_stages<TWO>() * (TWO ? STAGE_BYTES2 : STAGE_BYTES) + 1024;
 }
 
-template <bool WGRAD, bool A_MN, bool B_MN, int EPI, bool TWO = false, bool SGD = false, bool DISP = false>
-__global__ void __launch_bounds__(SGD ? GEMM_THREADS_SGD : (DISP ? GEMM_THREADS_DISP : GEMM_THREADS), 1)
+// WGRAD: the weight grads.  Otherwise the token-major kernel with fp32 output (router logits), tokens on
+// the M side; the other token-major products are in token_gemm.cuh.
+template <bool WGRAD, bool A_MN, bool B_MN, bool TWO = false, bool SGD = false>
+__global__ void __launch_bounds__(SGD ? GEMM_THREADS_SGD : GEMM_THREADS, 1)
 ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
-  static_assert(!SGD || (WGRAD && EPI == EPI_F32), "the fused SGD step belongs to the weight grad");
-  static_assert(!DISP || (!WGRAD && !SGD), "the fused dispatch feeds a token-major GEMM");
+  static_assert(WGRAD || (!TWO && !SGD), "pairs and the fused SGD step belong to the weight grad");
   // operand stages: a constant, except in the SGD kernels (upper bound; p.stages are used)
-  constexpr int GEMM_STAGES = SGD ? (TWO ? GEMM_STAGES2 : mep::GEMM_STAGES) : gemm_stages<TWO, DISP>();
+  constexpr int GEMM_STAGES = gemm_stages<TWO>();
   const int nst = SGD ? p.stages : GEMM_STAGES;
-  constexpr int FD_NST = fd_stages<TWO, EPI>();
   constexpr int STAGE_BYTES = TWO ? STAGE_BYTES2 : mep::STAGE_BYTES;
   constexpr int WB_MAX = SGD ? SGD_RING_MAX : 1;
   const int WB = SGD ? p.wb : 1;
@@ -274,20 +257,15 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
   __shared__ __align__(8) uint64_t acc_empty[2];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
-  __shared__ int s_groups_ready;   // DISP: written by the arrival watchers, read by the producer
   __shared__ int s_end[MAX_GROUPS];
+  __shared__ int s_valid[WGRAD ? MAX_GROUPS : 1];
   __shared__ int s_prefix[WGRAD ? 1 : MAX_GROUPS + 1];
   // per-warp staging of the fp32 epilogues: 32 x 33 floats token-major, a 4 KB swizzled block for
   // the weight grad
-  __shared__ __align__(1024) float s_epi[(EPI == EPI_F32) ? 4 * 32 * 33 : 1];
+  __shared__ __align__(1024) float s_epi[4 * 32 * 33];
   // fused SGD: per epilogue warp a ring of WB 32 x 32 bf16 weight blocks (in dynamic shared
   // memory, behind the operand stages) and their "landed" barriers
   __shared__ __align__(8) uint64_t wbar[SGD ? 8 : 4][WB_MAX];
-  __shared__ __align__(128) uint8_t s_push[(EPI == EPI_PUSH) ? 4 * 4096 : 16];
-  // staging of the bf16 epilogue: per warp one 32 x 64 block (128-byte rows, 128B swizzle)
-  __shared__ __align__(1024) uint8_t s_out[(!WGRAD && EPI == EPI_BF16) ? 4 * 4096 : 16];
-  // fused dispatch: "landed" barriers of the copy ring
-  __shared__ __align__(8) uint64_t fd_full[DISP ? FD_NST : 1];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
@@ -299,24 +277,25 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
     for (int s = 0; s < GEMM_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], (TWO ? 8 : 4) * (SGD ? 2 : 1)); }
     for (int a = 0; a < (SGD ? 8 : 4) * WB_MAX; ++a) mbar_init(&wbar[a / WB_MAX][a % WB_MAX], 1);
-    if constexpr (DISP) for (int a = 0; a < FD_NST; ++a) mbar_init(&fd_full[a], 1);
     mbar_fence_init();
     s_abort = 0;
-    s_groups_ready = 0;
   }
   // group table
   for (int g = tid; g < p.ngroups; g += (int)blockDim.x)
     s_end[g] = p.cu_seqlens != nullptr ? p.cu_seqlens[g] : p.total_rows;
   __syncthreads();
-  if (warp == 0) {
+  if constexpr (WGRAD) {
+    for (int g = tid; g < p.ngroups; g += (int)blockDim.x)
+      s_valid[g] = group_valid(p, g, g == 0 ? 0 : s_end[g - 1], s_end[g]);
+  }
+  if (!WGRAD && warp == 0) {
     // exclusive prefix of M tiles per group (token-major); cheap serial-by-chunks scan
     int run = 0;
     for (int g0 = 0; g0 < p.ngroups; g0 += 32) {
       int g = g0 + lane;
       int len = 0;
       if (g < p.ngroups) len = s_end[g] - (g == 0 ? 0 : s_end[g - 1]);
-      constexpr int TM = TWO ? 2 * BM : BM;
-      int mt = (len > 0 && g >= p.g_begin) ? (len + TM - 1) / TM : 0;
+      int mt = (len > 0 && g >= p.g_begin) ? (len + BM - 1) / BM : 0;
       int incl = mt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -338,8 +317,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
   tc_fence_after();
   const uint32_t tmem_base = s_tmem;
 
-  const int bn_eff = (EPI == EPI_SWIGLU) ? BN / 2 : BN;
-  const int n_tiles_n = (p.N + bn_eff - 1) / bn_eff;
+  const int n_tiles_n = (p.N + BN - 1) / BN;
   long long total_tiles;
   if constexpr (WGRAD) total_tiles = (long long)p.ngroups * (p.Mw / (TWO ? 2 * BM : BM)) * n_tiles_n;
   else total_tiles = (long long)s_prefix[p.ngroups] * n_tiles_n;
@@ -351,34 +329,10 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
       tma_prefetch_desc(&p.b[0][0]);
       int it = 0;
       bool ok = true;
-      int groups_ready = 0;      // DISP: groups [0, groups_ready) are known to have arrived
-      if constexpr (DISP) phase_stamp(p.trace, 2, (int)blockIdx.x, 0);       // producer starts
-      bool stamped_first = false;
       for (long long id = work_id0; id < total_tiles && ok; id += work_stride) {
-        Tile t = get_tile<WGRAD, EPI, TWO>(p, (int)id, s_end, s_prefix, n_tiles_n, crank);
+        Tile t = get_tile<WGRAD, TWO>(p, (int)id, s_end, s_valid, s_prefix, n_tiles_n, crank);
         if (!t.valid) continue;
         const int kb_per_seg = WGRAD ? t.num_kb : (p.K + BK - 1) / BK;
-        if constexpr (DISP) {
-          // The rows of this tile come from other ranks' copy warps.  The other lanes of this warp
-          // watch the arrival counters group by group (below) and publish how many groups are
-          // complete; waiting for the tile's whole GROUP rather than for its own 128 rows makes
-          // every CTA enter a group at about the same time, as CTAs that start together do: the
-          // tiles in flight then share one group's rows and weights in L2 instead of two groups'.
-          if (p.disp.arrive != nullptr && t.rows > 0 && t.g >= groups_ready) {
-            unsigned long long t0 = 0ull;
-            unsigned spins = 0;
-            while ((groups_ready = *(volatile int*)&s_groups_ready) <= t.g) {
-              if ((++spins & 63u) == 0) {
-                if (t0 == 0ull) t0 = globaltimer_ns();
-                if (*abortp || globaltimer_ns() - t0 > p.timeout_ns) { ok = false; break; }
-              }
-            }
-            if (!ok) break;
-            __threadfence_block();
-            fence_proxy_async();   // the rows were written through the async proxy (or by plain stores)
-            if (!stamped_first) { phase_stamp(p.trace, 2, (int)blockIdx.x, 1); stamped_first = true; }   // first group arrived
-          }
-        }
         for (int kb = 0; kb < t.num_kb; ++kb, ++it) {
           const int s = it % nst;
           if (it >= nst &&
@@ -411,53 +365,15 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
             for (int j = 0; j < BN / 64; ++j)
               tma_load_2d(sb + j * 8192, &p.b[0][0], t.n0 + 64 * j, t.row0 + k0, &full[s]);
           } else {
-            if constexpr (TWO) tma_load_2d_pair(sa, &p.a[seg], k0, t.row0, lead_bar);
-            else tma_load_2d(sa, &p.a[seg], k0, t.row0, &full[s]);
+            tma_load_2d(sa, &p.a[seg], k0, t.row0, &full[s]);
             const int erow = t.g_local * p.rows_per_expert;
-            if constexpr (TWO) {
-              // this CTA's half of the B tile: N columns [128*crank, +128) of the pair's tile
-              if constexpr (B_MN) {
+            if constexpr (B_MN) {
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                  if constexpr (EPI == EPI_SWIGLU)   // leader: 128 gate columns, peer: 128 up columns
-                    tma_load_2d_pair(sb + j * 8192, &p.b[crank][t.alloc], t.n0 + 64 * j, erow + k0, lead_bar);
-                  else
-                    tma_load_2d_pair(sb + j * 8192, &p.b[seg][t.alloc], t.n0 + 128 * crank + 64 * j, erow + k0, lead_bar);
-                }
-              } else {
-                tma_load_2d_pair(sb, &p.b2[seg][t.alloc], k0, erow + t.n0 + 128 * crank, lead_bar);
-              }
-            } else if constexpr (B_MN) {
-#pragma unroll
-              for (int j = 0; j < BN / 64; ++j) {
-                if constexpr (EPI == EPI_SWIGLU) {
-                  const int part = j / (BN / 128);
-                  tma_load_2d(sb + j * 8192, &p.b[part][t.alloc],
-                              t.n0 + 64 * (j % (BN / 128)), erow + k0, &full[s]);
-                } else {
-                  tma_load_2d(sb + j * 8192, &p.b[seg][t.alloc], t.n0 + 64 * j, erow + k0, &full[s]);
-                }
-              }
+              for (int j = 0; j < BN / 64; ++j)
+                tma_load_2d(sb + j * 8192, &p.b[seg][t.alloc], t.n0 + 64 * j, erow + k0, &full[s]);
             } else {
               tma_load_2d(sb, &p.b[seg][t.alloc], k0, erow + t.n0, &full[s]);
             }
-          }
-        }
-      }
-      if constexpr (DISP) phase_stamp(p.trace, 2, (int)blockIdx.x, 2);       // last operand load issued
-    } else if (DISP && p.disp.arrive != nullptr) {
-      // ---- arrival watchers (lanes 1..31): group after group, wait until every 128-row block of
-      // the group has all its rows, then publish the number of complete groups to lane 0 --------
-      if constexpr (DISP) {
-        for (int g = 0; g < p.ngroups; ++g) {
-          const int b0 = (g == 0 ? 0 : s_end[g - 1]) >> 7, b1 = s_end[g] >> 7;
-          bool okw = true;
-          for (int b = b0 + lane - 1; b < b1 && okw; b += 31)
-            okw = arrive_wait(p.disp.arrive + b, p.disp.expect, b, abortp, p);
-          if (!__all_sync(0xfffffffeu, okw)) break;
-          if (lane == 1) {
-            __threadfence_block();
-            *(volatile int*)&s_groups_ready = g + 1;
           }
         }
       }
@@ -471,7 +387,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
       int it = 0, tile_n = 0;
       bool ok = true;
       for (long long id = work_id0; id < total_tiles && ok; id += work_stride) {
-        Tile t = get_tile<WGRAD, EPI, TWO>(p, (int)id, s_end, s_prefix, n_tiles_n, crank);
+        Tile t = get_tile<WGRAD, TWO>(p, (int)id, s_end, s_valid, s_prefix, n_tiles_n, crank);
         if (!t.valid) continue;
         const int acc = tile_n & 1;
         if (tile_n >= 2 &&
@@ -503,22 +419,9 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
         ++tile_n;
       }
     }
-  } else if (DISP && warp >= 6) {
-    // ================= fused dispatch: this CTA's share of the all-to-all =================
-    if constexpr (DISP) {
-      if (p.disp.x != nullptr) {
-        uint8_t* ring = tiles + (size_t)nst * STAGE_BYTES;
-        if (lane == 0) phase_stamp(p.trace, 3, (int)blockIdx.x, 0);          // copy warp starts
-        fused_dispatch_copy_warp<FD_NST>(
-            p.disp, ring, fd_full, (int)blockIdx.x, (int)gridDim.x,
-            [&](uint64_t* bar, uint32_t parity) { return gemm_wait(bar, parity, abortp, p, 7); });
-        if (lane == 0) phase_stamp(p.trace, 3, (int)blockIdx.x, 1);          // all rows sent and announced
-      }
-    }
   } else {
     // ================= epilogue (4 warps, one TMEM lane quarter each) =================
     const int q = warp & 3;
-    const int r_in_tile = q * 32 + lane;
     // SGD: warps 2..5 take the tile's first 128 columns, warps 6..9 the other 128
     const int half = SGD ? (warp - 2) >> 2 : 0;
     const int ew = q + 4 * half;
@@ -543,7 +446,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
     auto cursor_settle = [&]() {           // move to the next existing block at or after (lid, lc)
       while (lid < total_tiles) {
         if (!l_have) {
-          const Tile u = get_tile<WGRAD, EPI, TWO>(p, (int)lid, s_end, s_prefix, n_tiles_n, crank);
+          const Tile u = get_tile<WGRAD, TWO>(p, (int)lid, s_end, s_valid, s_prefix, n_tiles_n, crank);
           if (sgd_tile(u)) { l_have = true; l_y0 = u.g_local * p.Mw + u.m0 + q * 32; l_n0 = u.n0; lc = 0; }
         }
         if (l_have && lc < CB && l_n0 + cofs + lc * WCOLS < p.N) return;
@@ -568,7 +471,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
       issue_loads();
     }
     for (long long id = work_id0; id < total_tiles; id += work_stride) {
-      Tile t = get_tile<WGRAD, EPI, TWO>(p, (int)id, s_end, s_prefix, n_tiles_n, crank);
+      Tile t = get_tile<WGRAD, TWO>(p, (int)id, s_end, s_valid, s_prefix, n_tiles_n, crank);
       if (!t.valid) continue;
       const int acc = tile_n & 1;
       bool sgd_fuse = false;
@@ -577,121 +480,9 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
       tc_fence_after();
       const uint32_t tacc = tmem_base + (uint32_t)acc * BN + ((uint32_t)(q * 32) << 16);
       const bool have_acc = t.num_kb > 0;
-      if constexpr (EPI == EPI_SWIGLU) {
-        const bool row_ok = r_in_tile < t.rows;
-        const long long row = (long long)t.row0 + r_in_tile;
-        // (read past L1: with the fused dispatch the scale was written by another rank moments ago)
-        const float rs = (row_ok && p.row_scale != nullptr) ? __ldcg(p.row_scale + row) : 1.f;
-        __nv_bfloat16* og = (__nv_bfloat16*)p.out[0];
-        __nv_bfloat16* ou = (__nv_bfloat16*)p.out[1];
-        __nv_bfloat16* oa = (__nv_bfloat16*)p.out[2];
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t rg[32], ru[32];
-          tmem_ld_32x32(tacc + c * 32, rg);
-          tmem_ld_32x32(tacc + 128 + c * 32, ru);
-          tmem_ld_wait();
-          const int col = t.n0 + c * 32;
-          if (row_ok && col < p.N) {
-            uint32_t pg[16], pu[16], pa[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              float g0 = __uint_as_float(rg[2 * i]), g1 = __uint_as_float(rg[2 * i + 1]);
-              float u0 = __uint_as_float(ru[2 * i]), u1 = __uint_as_float(ru[2 * i + 1]);
-              __nv_bfloat162 hg = __floats2bfloat162_rn(g0, g1);
-              __nv_bfloat162 hu = __floats2bfloat162_rn(u0, u1);
-              // the saved gate/up are bf16; the activation is computed from the rounded values
-              // so that backward recomputes exactly what forward used
-              float2 fg = __bfloat1622float2(hg), fu = __bfloat1622float2(hu);
-              float a0 = fg.x / (1.f + __expf(-fg.x)) * fu.x * rs;
-              float a1 = fg.y / (1.f + __expf(-fg.y)) * fu.y * rs;
-              __nv_bfloat162 ha = __floats2bfloat162_rn(a0, a1);
-              pg[i] = *reinterpret_cast<uint32_t*>(&hg);
-              pu[i] = *reinterpret_cast<uint32_t*>(&hu);
-              pa[i] = *reinterpret_cast<uint32_t*>(&ha);
-            }
-            const long long off = row * p.ldc + col;
-            if (col + 32 <= p.N) {
-#pragma unroll
-              for (int v = 0; v < 4; ++v) {
-                if (og) reinterpret_cast<uint4*>(og + off)[v] = make_uint4(pg[4 * v], pg[4 * v + 1], pg[4 * v + 2], pg[4 * v + 3]);
-                if (ou) reinterpret_cast<uint4*>(ou + off)[v] = make_uint4(pu[4 * v], pu[4 * v + 1], pu[4 * v + 2], pu[4 * v + 3]);
-                reinterpret_cast<uint4*>(oa + off)[v] = make_uint4(pa[4 * v], pa[4 * v + 1], pa[4 * v + 2], pa[4 * v + 3]);
-              }
-            } else {
-              for (int i = 0; i < 32 && col + i < p.N; ++i) {
-                const __nv_bfloat16* sg = reinterpret_cast<const __nv_bfloat16*>(pg);
-                const __nv_bfloat16* su = reinterpret_cast<const __nv_bfloat16*>(pu);
-                const __nv_bfloat16* sa2 = reinterpret_cast<const __nv_bfloat16*>(pa);
-                if (og) og[off + i] = sg[i];
-                if (ou) ou[off + i] = su[i];
-                oa[off + i] = sa2[i];
-              }
-            }
-          }
-        }
-      } else if constexpr (EPI == EPI_PUSH) {
-        // thread = output row.  The row's owner entry (source rank, token*K+k) comes from the
-        // per-slot source record; padding rows have none and are dropped.  64 columns at a time
-        // are staged in a swizzled per-warp pad and leave as full 128-byte lines: every store
-        // instruction covers 4 rows x 128 B, 8 lanes per row, addressed at the home rank.
-        uint8_t* pad = s_push + q * 4096;
-        const bool row_ok = r_in_tile < t.rows;
-        const long long row = (long long)t.row0 + r_in_tile;
-        const int si = row_ok ? p.src_info[row] : -1;
-        unsigned long long dptr = 0ull;
-        if (si >= 0) {
-          const int sr = si / p.push_entries, ent = si - sr * p.push_entries;
-          if (sr < p.push_ranks)
-            dptr = (unsigned long long)((__nv_bfloat16*)p.push_base + (long long)sr * p.push_rank_stride +
-                                        (long long)ent * p.ldc + t.n0);
-        }
-#pragma unroll 1
-        for (int c2 = 0; c2 < BN / 64; ++c2) {
-          uint32_t ra[32], rb[32];
-          tmem_ld_32x32(tacc + c2 * 64, ra);
-          tmem_ld_32x32(tacc + c2 * 64 + 32, rb);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint32_t* src = j < 4 ? ra + 8 * j : rb + 8 * (j - 4);
-            uint32_t pk[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(src[2 * i]), __uint_as_float(src[2 * i + 1]));
-              pk[i] = *reinterpret_cast<uint32_t*>(&h);
-            }
-            *reinterpret_cast<uint4*>(pad + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          }
-          __syncwarp();
-          const int j = lane & 7;
-          const bool col_ok = t.n0 + c2 * 64 + j * 8 < p.N;
-#pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            const int rr = g * 4 + (lane >> 3);
-            const unsigned long long pr = __shfl_sync(0xffffffffu, dptr, rr);
-            const uint4 v = *reinterpret_cast<const uint4*>(pad + rr * 128 + ((j ^ (rr & 7)) << 4));
-            if (pr != 0ull && col_ok)
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(pr) + c2 * 64 + j * 8) = v;
-          }
-          __syncwarp();
-        }
-      } else {
-        bool row_ok;
-        long long off_row;
-        int col_base;
+      {
+        const int col_base = t.n0;
         if constexpr (WGRAD) {
-          row_ok = t.m0 + r_in_tile < p.Mw;
-          off_row = ((long long)t.g_local * p.Mw + t.m0 + r_in_tile) * p.ldc;
-          col_base = t.n0;
-        } else {
-          row_ok = r_in_tile < t.rows;
-          off_row = ((long long)t.row0 + r_in_tile) * p.ldc;
-          col_base = t.n0;
-        }
-        void* outp = WGRAD ? p.out[t.alloc] : p.out[0];
-        if constexpr (EPI == EPI_F32 && WGRAD) {
           // fp32 weight-grad tiles are 128 KB each and the main loop is short (one group's
           // tokens), so the epilogue must move ~30 GB/s per SM.  Four warps of plain stores
           // cannot (measured: ~14 B/clk/SM), so each warp stages 32x32 blocks in shared memory
@@ -772,15 +563,14 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
               bulk_commit();
             }
           }
-        } else if constexpr (EPI == EPI_F32) {
+        } else {
           // token-major fp32 output (router logits): rows of a tile may belong to the next
           // group, so stores stay row-masked; each warp transposes through a padded pad so
           // that every store instruction writes one full 128-byte line.
           float* pad = s_epi + q * (32 * 33);
           const long long row_stride = p.ldc;
-          const long long off_warp = WGRAD ? ((long long)t.g_local * p.Mw + t.m0 + q * 32) * p.ldc
-                                           : ((long long)t.row0 + q * 32) * p.ldc;
-          const int rows_ok = WGRAD ? min(32, p.Mw - (t.m0 + q * 32)) : min(32, t.rows - q * 32);
+          const long long off_warp = ((long long)t.row0 + q * 32) * p.ldc;
+          const int rows_ok = min(32, t.rows - q * 32);
 #pragma unroll 1
           for (int c = 0; c < BN / 32; ++c) {
             uint32_t r[32];
@@ -796,7 +586,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
             for (int i = 0; i < 32; ++i) pad[lane * 33 + i] = __uint_as_float(r[i]);
             __syncwarp();
             if (col < p.N) {
-              float* o = (float*)outp + off_warp + col;
+              float* o = (float*)p.out[0] + off_warp + col;
 #pragma unroll 8
               for (int rr = 0; rr < 32; ++rr) {
                 if (rr < rows_ok) {
@@ -807,77 +597,6 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
               }
             }
             __syncwarp();
-          }
-        } else if (EPI == EPI_BF16 && !WGRAD && p.tma_out != 0 && q * 32 + 32 <= t.rows) {
-          // all 32 rows of this warp belong to the group: stage 32 x 64 blocks (128-byte rows,
-          // 128B swizzle, conflict-free 16-byte stores) and let the TMA engine write full lines
-          uint8_t* pad = s_out + q * 4096;
-          const int y0 = t.row0 + q * 32;
-#pragma unroll 1
-          for (int c2 = 0; c2 < BN / 64; ++c2) {
-            const int col = col_base + c2 * 64;
-            if (col >= p.N) break;
-            uint32_t ra[32], rb[32];
-            if (have_acc) {
-              tmem_ld_32x32(tacc + c2 * 64, ra);
-              tmem_ld_32x32(tacc + c2 * 64 + 32, rb);
-              tmem_ld_wait();
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) ra[i] = rb[i] = 0u;
-            }
-            if (lane == 0) bulk_wait_read<0>();
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const uint32_t* src = j < 4 ? ra + 8 * j : rb + 8 * (j - 4);
-              uint32_t pk[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(src[2 * i]), __uint_as_float(src[2 * i + 1]));
-                pk[i] = *reinterpret_cast<uint32_t*>(&h);
-              }
-              *reinterpret_cast<uint4*>(pad + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                  make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&p.o, col, y0, pad);
-              bulk_commit();
-            }
-          }
-        } else
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          if (have_acc) {
-            tmem_ld_32x32(tacc + c * 32, r);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = 0u;
-          }
-          const int col = col_base + c * 32;
-          if (!row_ok || col >= p.N) continue;
-          if constexpr (EPI == EPI_F32) {
-            // unreachable: the fp32 epilogue is the transposed loop below
-          } else {
-            __nv_bfloat16* o = (__nv_bfloat16*)outp + off_row + col;
-            uint32_t pk[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-              pk[i] = *reinterpret_cast<uint32_t*>(&h);
-            }
-            if (col + 32 <= p.N) {
-#pragma unroll
-              for (int v = 0; v < 4; ++v)
-                reinterpret_cast<uint4*>(o)[v] = make_uint4(pk[4 * v], pk[4 * v + 1], pk[4 * v + 2], pk[4 * v + 3]);
-            } else {
-              const __nv_bfloat16* sp = reinterpret_cast<const __nv_bfloat16*>(pk);
-              for (int i = 0; i < 32 && col + i < p.N; ++i) o[i] = sp[i];
-            }
           }
         }
       }
@@ -898,11 +617,6 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
     while (globaltimer_ns() - t0 < 200000ull) { }
   }
   if (warp >= 2 && lane == 0) bulk_wait<0>();   // epilogue TMA stores have completed
-  // Pushed rows: the kernel that consumes them on the home rank runs behind a cross-rank barrier
-  // that this rank enters from a LATER launch of the same stream, so the end of this kernel
-  // already orders the stores; one fence here (instead of one per tile, which made every epilogue
-  // warp wait for an NVLink round trip per tile) keeps that independent of how the next launch arrives.
-  if constexpr (EPI == EPI_PUSH) { if (warp >= 2) __threadfence_system(); }
   if constexpr (TWO) cluster_sync_all();        // neither CTA leaves while its peer may still touch it
   if (warp == 1) {
     tc_fence_after();
@@ -911,11 +625,17 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
   }
 }
 
+}  // namespace mep
+
+#include "device/token_gemm.cuh"
+
+namespace mep {
+
 // ---- host side -----------------------------------------------------------------------------------
 struct GemmDesc {
   int32_t mode, epi, b_mn, nseg;
   int32_t ngroups, split, total_rows, N, K, rows_per_expert, Mw, accumulate, zero_empty_below, grid;
-  int32_t debug, g_begin;
+  int32_t g_begin;
   int64_t a_rows;
   int64_t lda[2];
   const void* a[2];
@@ -947,6 +667,7 @@ struct GemmDesc {
   const int32_t* disp_order;
   const int32_t* disp_zero_fill;
   int32_t disp_fresh, disp_shard;
+  const int32_t* pads;
 };
 
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1033,46 +754,39 @@ static int sgd_smem_limit(const void* kern) {
   return optin - (int)fa.sharedSizeBytes;
 }
 
-// CTA-pair launch: clusters of two CTAs, one pair per two SMs.
-template <bool A_MN, bool B_MN, int EPI, bool WGRAD = false, bool SGD = false, bool DISP = false>
-static int launch_gemm2(const GemmKParams& kp, int grid, cudaStream_t stream) {
-  auto kern = ep_grouped_gemm_kernel<WGRAD, A_MN, B_MN, EPI, true, SGD, DISP>;
-  const int GEMM_SMEM2 = SGD ? sgd_smem(kp, true) : gemm_smem<true, DISP, EPI>();
-  static bool configured = false;
-  if (!configured) {
-    const int most = SGD ? sgd_smem_limit((const void*)kern) : GEMM_SMEM2;
-    MEP_CUDA_OK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    configured = true;
-  }
-  if (SGD && GEMM_SMEM2 > sgd_smem_limit((const void*)kern))
-    return fail(-3, "gemm: %d operand stages + %d weight blocks do not fit in shared memory", kp.stages, kp.wb);
+// CTA-pair launch: clusters of two CTAs, one pair per two SMs.  `coop`: the whole grid must be
+// resident at once.
+struct PairLaunch {
+  std::atomic<unsigned long long> raised{0};
+  std::atomic<int> max_clusters{-1};
+};
+static int launch_pair(const void* kern, PairLaunch& once, GemmKParams kp, int grid, int threads, int smem, bool coop,
+                       cudaStream_t stream) {
+  MEP_CUDA_OK(raise_smem_limit(kern, once.raised));
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(grid / 2 * 2));
-  cfg.blockDim = dim3(SGD ? GEMM_THREADS_SGD : (DISP ? GEMM_THREADS_DISP : GEMM_THREADS));
-  cfg.dynamicSmemBytes = GEMM_SMEM2;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  // the fused dispatch makes CTAs of different ranks wait for one another's copy warps: the
-  // whole grid must be resident at once, which a cooperative launch guarantees
   attr[1].id = cudaLaunchAttributeCooperative;
   attr[1].val.cooperative = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = (DISP && fused_dispatch_cooperative()) ? 2 : 1;
+  cfg.numAttrs = coop ? 2 : 1;
   // A persistent grid must not exceed what is resident at once: not every SM can be paired
   // into a cluster (GPCs with an odd SM count leave one out), and a second wave of persistent
   // CTAs would double the run time.
-  static int max_clusters = -1;
-  if (max_clusters < 0) {
-    int n = 0;
+  int most = once.max_clusters.load(std::memory_order_relaxed);
+  if (most < 0) {
     cudaLaunchConfig_t probe = cfg;
     probe.gridDim = dim3(2 * 148);
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &probe) != cudaSuccess || n < 1) { cudaGetLastError(); n = 1 << 20; }
-    max_clusters = n;
+    if (cudaOccupancyMaxActiveClusters(&most, kern, &probe) != cudaSuccess || most < 1) { cudaGetLastError(); most = 1 << 20; }
+    once.max_clusters.store(most, std::memory_order_relaxed);
   }
-  int use = max_clusters;
+  int use = most;
   {
     // a launch with a CTA limit shares the GPU with a copy kernel that is placed as SM pairs too:
     // leave it its pairs out of what the device can hold, or this persistent grid would need a
@@ -1080,44 +794,65 @@ static int launch_gemm2(const GemmKParams& kp, int grid, cudaStream_t stream) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (grid < sms && max_clusters < (1 << 20)) use = max_clusters - (sms - grid + 1) / 2;
+    if (grid < sms && most < (1 << 20)) use = most - (sms - grid + 1) / 2;
     if (use < 1) use = 1;
   }
   if ((int)cfg.gridDim.x / 2 > use) cfg.gridDim = dim3((unsigned)(2 * use));
-  MEP_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, kp));
+  void* args[] = {(void*)&kp};
+  MEP_CUDA_OK(cudaLaunchKernelExC(&cfg, kern, args));
+  return 0;
+}
+static int launch_single(const void* kern, std::atomic<unsigned long long>& raised, GemmKParams kp, int grid, int threads,
+                         int smem, bool coop, cudaStream_t stream) {
+  MEP_CUDA_OK(raise_smem_limit(kern, raised));
+  void* args[] = {(void*)&kp};
+  if (coop) MEP_CUDA_OK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(threads), args, (size_t)smem, stream));
+  else MEP_CUDA_OK(cudaLaunchKernel(kern, dim3(grid), dim3(threads), args, (size_t)smem, stream));
   return 0;
 }
 
-template <bool WGRAD, bool A_MN, bool B_MN, int EPI, bool SGD = false, bool DISP = false>
-static int launch_gemm(const GemmKParams& kp, int grid, cudaStream_t stream) {
-  auto kern = ep_grouped_gemm_kernel<WGRAD, A_MN, B_MN, EPI, false, SGD, DISP>;
-  const int GEMM_SMEM = SGD ? sgd_smem(kp, false) : gemm_smem<false, DISP, EPI>();
-  static bool configured = false;
-  if (!configured) {
-    const int most = SGD ? sgd_smem_limit((const void*)kern) : GEMM_SMEM;
-    MEP_CUDA_OK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    configured = true;
-  }
-  if (SGD && GEMM_SMEM > sgd_smem_limit((const void*)kern))
+template <bool SGD>
+static int launch_wgrad(const GemmKParams& kp, bool pair, int grid, cudaStream_t stream) {
+  const void* kern = pair ? (const void*)ep_grouped_gemm_kernel<true, true, true, true, SGD>
+                          : (const void*)ep_grouped_gemm_kernel<true, true, true, false, SGD>;
+  const int smem = SGD ? sgd_smem(kp, pair) : (pair ? gemm_smem<true>() : gemm_smem<false>());
+  if (SGD && smem > sgd_smem_limit(kern))
     return fail(-3, "gemm: %d operand stages + %d weight blocks do not fit in shared memory", kp.stages, kp.wb);
-  if constexpr (DISP) {
+  const int threads = SGD ? GEMM_THREADS_SGD : GEMM_THREADS;
+  if (pair) {
+    static PairLaunch once;
+    return launch_pair(kern, once, kp, grid, threads, smem, false, stream);
+  }
+  static std::atomic<unsigned long long> raised{0};
+  return launch_single(kern, raised, kp, grid, threads, smem, false, stream);
+}
+
+template <bool B_MN>
+static int launch_dense_f32(const GemmKParams& kp, int grid, cudaStream_t stream) {
+  static std::atomic<unsigned long long> raised{0};
+  return launch_single((const void*)ep_grouped_gemm_kernel<false, false, B_MN>, raised, kp, grid, GEMM_THREADS,
+                       gemm_smem<false>(), false, stream);
+}
+
+template <bool A_MN, int EPI, bool DISP>
+static int launch_token(const GemmKParams& kp, bool pair, int grid, cudaStream_t stream) {
+  const int threads = DISP ? GEMM_THREADS_DISP : GEMM_THREADS;
+  const bool coop = DISP && fused_dispatch_cooperative();
+  if (pair) {
+    static PairLaunch once;
+    return launch_pair((const void*)ep_token_gemm_kernel<A_MN, EPI, true, DISP>, once, kp, grid, threads,
+                       tg_smem<true, DISP>(), coop, stream);
+  }
+  if (DISP) {
     // CTAs of different ranks wait for one another's copy warps: all of them must be resident
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (grid > sms) grid = sms;
-    if (fused_dispatch_cooperative()) {
-      GemmKParams kpc = kp;
-      MEP_CUDA_OK(launch_coop((const void*)kern, dim3(grid), dim3(GEMM_THREADS_DISP), GEMM_SMEM, stream, kpc));
-    } else {
-      kern<<<grid, GEMM_THREADS_DISP, GEMM_SMEM, stream>>>(kp);
-      MEP_CUDA_OK(cudaGetLastError());
-    }
-    return 0;
   }
-  kern<<<grid, SGD ? GEMM_THREADS_SGD : GEMM_THREADS, GEMM_SMEM, stream>>>(kp);
-  MEP_CUDA_OK(cudaGetLastError());
-  return 0;
+  static std::atomic<unsigned long long> raised{0};
+  return launch_single((const void*)ep_token_gemm_kernel<A_MN, EPI, false, DISP>, raised, kp, grid, threads,
+                       tg_smem<false, DISP>(), coop, stream);
 }
 
 }  // namespace mep
@@ -1136,7 +871,7 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
   kp.total_rows = d->total_rows; kp.N = d->N; kp.K = d->K; kp.nseg = d->nseg;
   kp.rows_per_expert = d->rows_per_expert; kp.Mw = d->Mw; kp.accumulate = d->accumulate;
   kp.zero_empty_below = d->zero_empty_below;
-  kp.debug = d->debug; kp.g_begin = d->g_begin;
+  kp.g_begin = d->g_begin; kp.pads = d->pads;
   kp.src_info = d->src_info; kp.push_base = d->push_base; kp.push_rank_stride = d->push_rank_stride;
   kp.push_entries = d->push_entries; kp.push_ranks = d->push_ranks;
   kp.out[0] = d->out[0]; kp.out[1] = d->out[1]; kp.out[2] = d->out[2];
@@ -1173,17 +908,21 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
     if (kp.sgd_w != nullptr) sgd_geometry(pair, &kp);
     kp.wg_select = kp.sgd_w != nullptr ? d->wg_select : 0;
     if (kp.sgd_w != nullptr)
-      return pair ? launch_gemm2<true, true, EPI_F32, true, true>(kp, grid, stream)
-                  : launch_gemm<true, true, true, EPI_F32, true>(kp, grid, stream);
-    return pair ? launch_gemm2<true, true, EPI_F32, true>(kp, grid, stream)
-                : launch_gemm<true, true, true, EPI_F32>(kp, grid, stream);
+      return launch_wgrad<true>(kp, pair, grid, stream);
+    return launch_wgrad<false>(kp, pair, grid, stream);
   }
   // A reduction tail is legal: the TMA loads zero-fill A beyond K, which also cancels whatever
   // a MN-major B tile picks up from the next expert's rows.
   if (d->K % 8 != 0) return fail(-4, "gemm: K=%d must be a multiple of 8", d->K);
   if (d->nseg < 1 || d->nseg > 2) return fail(-5, "gemm: nseg=%d", d->nseg);
-  for (int s = 0; s < d->nseg; ++s)
-    if ((rc = make_map(&kp.a[s], d->a[s], d->a_rows, d->K, d->lda[s], BK, BM))) return rc;
+  for (int s = 0; s < d->nseg; ++s) {
+    if (d->epi == EPI_F32) {
+      if ((rc = make_map(&kp.a[s], d->a[s], d->a_rows, d->K, d->lda[s], BK, BM))) return rc;
+      continue;
+    }
+    for (int b = 0; b < TG_BOXES; ++b)
+      if ((rc = make_map(&kp.tok[s][b], d->a[s], d->a_rows, d->K, d->lda[s], BK, 32 * (b + 1)))) return rc;
+  }
   if (d->nseg == 1) kp.a[1] = kp.a[0];
   const int nsel = (d->epi == EPI_SWIGLU) ? 2 : d->nseg;
   for (int s = 0; s < 2; ++s)
@@ -1194,18 +933,13 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
         if ((rc = make_map(&kp.b[s][al], base, rows, d->N, d->ldb, 64, BK))) return rc;
         kp.b2[s][al] = kp.b[s][al];
       } else {         // [N rows][K cols] per expert
-        if ((rc = make_map(&kp.b[s][al], base, rows, d->K, d->ldb, BK, BN))) return rc;
+        if (d->epi == EPI_F32 && (rc = make_map(&kp.b[s][al], base, rows, d->K, d->ldb, BK, BN))) return rc;
         if ((rc = make_map(&kp.b2[s][al], base, rows, d->K, d->ldb, BK, BN / 2))) return rc;
       }
     }
-  // output maps of the staged epilogues (plain stores remain for unaligned outputs and for the
-  // warps whose 32 rows straddle the end of a group)
-  // The SwiGLU epilogue keeps plain stores: staging its three outputs measured no faster.
-  if (d->epi == EPI_BF16 && (d->ldc * 2) % 16 == 0 && ((uintptr_t)d->out[0] & 15) == 0) {
-    if ((rc = make_map(&kp.o, d->out[0], d->a_rows, d->N, d->ldc, 64, 32))) return rc;
-    kp.tma_out = (d->debug & 16) ? 0 : 1;
-  }
-  const bool two = d->two_cta != 0 && grid >= 2;
+  kp.tma_out = d->ldc % 8 == 0 && (((uintptr_t)d->out[0] | (uintptr_t)d->out[1] | (uintptr_t)d->out[2] |
+                                    (uintptr_t)d->push_base) & 15) == 0 && d->push_rank_stride % 8 == 0;
+  const bool two = d->two_cta != 0 && grid >= 2;     // (fp32 output: single CTAs)
   if (d->disp_mode != 0) {
     // ---- fused dispatch: the A operand is a row buffer of the Buffer behind disp_ctx ----------
     if (d->disp_ctx == nullptr) return fail(-20, "gemm: the fused dispatch needs the Buffer's context");
@@ -1241,34 +975,23 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
     kp.trace = c.trace;
     kp.arrive_timeout_ns = c.timeout_ns;                       // waits on other ranks: the Buffer's budget
     kp.timeout_ns = c.timeout_ns + c.timeout_ns / 2 + 200000000ull;
-    if (d->epi == EPI_SWIGLU) {
-      if (two) return launch_gemm2<false, true, EPI_SWIGLU, false, false, true>(kp, grid, stream);
-      return launch_gemm<false, false, true, EPI_SWIGLU, false, true>(kp, grid, stream);
-    }
-    if (two) return launch_gemm2<false, true, EPI_BF16, false, false, true>(kp, grid, stream);
-    return launch_gemm<false, false, true, EPI_BF16, false, true>(kp, grid, stream);
+    return d->epi == EPI_SWIGLU ? launch_token<true, EPI_SWIGLU, true>(kp, two, grid, stream)
+                                : launch_token<true, EPI_BF16, true>(kp, two, grid, stream);
   }
   if (d->epi == EPI_SWIGLU) {
     if (!d->b_mn) return fail(-6, "swiglu epilogue expects MN-major weights");
-    if (two) return launch_gemm2<false, true, EPI_SWIGLU>(kp, grid, stream);
-    return launch_gemm<false, false, true, EPI_SWIGLU>(kp, grid, stream);
+    return launch_token<true, EPI_SWIGLU, false>(kp, two, grid, stream);
   }
-  if (d->epi == EPI_BF16) {
-    if (two) return d->b_mn ? launch_gemm2<false, true, EPI_BF16>(kp, grid, stream)
-                            : launch_gemm2<false, false, EPI_BF16>(kp, grid, stream);
-    return d->b_mn ? launch_gemm<false, false, true, EPI_BF16>(kp, grid, stream)
-                   : launch_gemm<false, false, false, EPI_BF16>(kp, grid, stream);
-  }
+  if (d->epi == EPI_BF16)
+    return d->b_mn ? launch_token<true, EPI_BF16, false>(kp, two, grid, stream)
+                   : launch_token<false, EPI_BF16, false>(kp, two, grid, stream);
   if (d->epi == EPI_F32)
-    return d->b_mn ? launch_gemm<false, false, true, EPI_F32>(kp, grid, stream)
-                   : launch_gemm<false, false, false, EPI_F32>(kp, grid, stream);
+    return d->b_mn ? launch_dense_f32<true>(kp, grid, stream) : launch_dense_f32<false>(kp, grid, stream);
   if (d->epi == EPI_PUSH) {
     if (d->src_info == nullptr || d->push_base == nullptr || d->push_entries <= 0)
       return fail(-9, "gemm: the push epilogue needs src_info and a staging buffer");
-    if (two) return d->b_mn ? launch_gemm2<false, true, EPI_PUSH>(kp, grid, stream)
-                            : launch_gemm2<false, false, EPI_PUSH>(kp, grid, stream);
-    return d->b_mn ? launch_gemm<false, false, true, EPI_PUSH>(kp, grid, stream)
-                   : launch_gemm<false, false, false, EPI_PUSH>(kp, grid, stream);
+    return d->b_mn ? launch_token<true, EPI_PUSH, false>(kp, two, grid, stream)
+                   : launch_token<false, EPI_PUSH, false>(kp, two, grid, stream);
   }
   return fail(-7, "gemm: unknown epilogue %d", d->epi);
 }

@@ -101,20 +101,22 @@ class _MoEFn(torch.autograd.Function):
             split, cu_use = epn, cu
             with tr.span("f.gateup_local"):
                 outs = gemm.gateup_swiglu(hidden, layer.w_gate, layer.w_up, cu[:epn], row_scale=w_nvs,
-                                          save_gate_up=layer.training, grid=layer.overlap_grid(), dispatch=disp)
+                                          save_gate_up=layer.training, grid=layer.overlap_grid(), dispatch=disp,
+                                          pads=plan.zero_fill_ranges)
             with tr.span("f.wait_prefetch"):
                 torch.cuda.current_stream().wait_event(ev)
             with tr.span("f.gateup_slots"):
                 act, gate, up = gemm.gateup_swiglu(hidden, layer.w_gate, layer.w_up, cu, wg_slot=slots["g"],
                                                    wu_slot=slots["u"], split=epn, row_scale=w_nvs,
                                                    save_gate_up=layer.training, out=outs, g_begin=epn,
-                                                   dispatch=wait_only)
+                                                   dispatch=wait_only, pads=plan.zero_fill_ranges)
         else:
             slots = dict(g=None, u=None, d=None)
             split, cu_use = None, cu[:epn]
             with tr.span("f.gateup"):
                 act, gate, up = gemm.gateup_swiglu(hidden, layer.w_gate, layer.w_up, cu_use, row_scale=w_nvs,
-                                                   save_gate_up=layer.training, dispatch=disp)
+                                                   save_gate_up=layer.training, dispatch=disp,
+                                                   pads=plan.zero_fill_ranges)
         if fused:
             w_nvs = buf.dispatch_fused_end(plan, disp)     # plan records + a private copy of the weights
             if not layer.hidden_in_place:
@@ -124,12 +126,13 @@ class _MoEFn(torch.autograd.Function):
             # into its entry's slot on the token's home rank while later tiles are still computing
             with tr.span("f.down_push"):
                 gemm.down(act, layer.w_down, cu_use, wd_slot=slots["d"], split=split,
-                          push=buf.push_target(plan))
+                          push=buf.push_target(plan), pads=plan.zero_fill_ranges)
             with tr.span("f.combine_pushed"):
                 y, _ = buf.combine_pushed(plan)
         else:
             shard = buf.hidden_nvsh_buffer_view
-            gemm.down(act, layer.w_down, cu_use, wd_slot=slots["d"], split=split, out=shard)
+            gemm.down(act, layer.w_down, cu_use, wd_slot=slots["d"], split=split, out=shard,
+                      pads=plan.zero_fill_ranges)
             y, _, _ = buf.combine(plan, shard, None, zero_copy=True)
         ctx.layer, ctx.plan, ctx.split = layer, plan, split
         ctx.save_for_backward(x, hidden, w_nvs, cu_use, act, gate, up, topk, w)
@@ -145,6 +148,7 @@ class _MoEFn(torch.autograd.Function):
         have_slots = split is not None
         slot = (lambda n: pools.slot(n)) if have_slots else (lambda n: None)
         gslot = (lambda n: pools.grad_slot(n)) if have_slots else (lambda n: None)
+        pads = plan.zero_fill_ranges
         dy = dy.contiguous()
         # combine backward = dispatch with the saved plan; the view is consumed before the shard
         # is overwritten further down (same stream)
@@ -167,14 +171,15 @@ class _MoEFn(torch.autograd.Function):
                 ev_p = layer.prefetch(plan)
         with tr.span("b.down_dgrad"):
             if ev_p is None:
-                d_act = gemm.down_dgrad(d_out, layer.w_down, cu, wd_slot=slot("down"), split=split, dispatch=disp)
+                d_act = gemm.down_dgrad(d_out, layer.w_down, cu, wd_slot=slot("down"), split=split, dispatch=disp,
+                                        pads=pads)
             else:      # local experts first, next to the copy kernel; the slot groups once it is done
                 d_act = gemm.down_dgrad(d_out, layer.w_down, cu[:buf.epn], grid=layer.overlap_grid(),
-                                        dispatch=disp)
+                                        dispatch=disp, pads=pads)
                 torch.cuda.current_stream().wait_event(ev_p)
                 d_act = gemm.down_dgrad(d_out, layer.w_down, cu, wd_slot=slot("down"), split=split,
                                         out=d_act, g_begin=buf.epn,
-                                        dispatch=None if disp is None else dict(disp, mode=1))
+                                        dispatch=None if disp is None else dict(disp, mode=1), pads=pads)
         if disp is not None:
             buf.dispatch_fused_end(plan, disp)
         acc = layer.accumulate_grads
@@ -197,15 +202,17 @@ class _MoEFn(torch.autograd.Function):
             sgd = lambda w: (w, fused_lr, keep)
         with tr.span("b.wgrad_down"):
             gemm.wgrad(d_out, act, cu, layer.g_down, grad_slot=gslot("down"), split=split, accumulate=acc,
-                       sgd=sgd(layer.w_down))
+                       sgd=sgd(layer.w_down), pads=pads)
         with tr.span("b.swiglu_bwd"):
             d_gate, d_up, d_scale = ew.swiglu_bwd(d_act, gate, up, w_nvs, rows_ptr=cu[-1:])
         ev_r = None
         zc = layer.accumulate_grads            # the slots are overwritten next step otherwise
         if fused_lr is None:
             with tr.span("b.wgrad_gateup"):
-                gemm.wgrad(hidden, d_gate, cu, layer.g_gate, grad_slot=gslot("gate"), split=split, accumulate=acc)
-                gemm.wgrad(hidden, d_up, cu, layer.g_up, grad_slot=gslot("up"), split=split, accumulate=acc)
+                gemm.wgrad(hidden, d_gate, cu, layer.g_gate, grad_slot=gslot("gate"), split=split, accumulate=acc,
+                           pads=pads)
+                gemm.wgrad(hidden, d_up, cu, layer.g_up, grad_slot=gslot("up"), split=split, accumulate=acc,
+                           pads=pads)
             if layer.hidden_in_place:  # the forward rows have had their last reader
                 buf.release_second_shard(layer)
             # the replicas' weight grads travel home on the comm stream while this stream computes dX
@@ -224,14 +231,15 @@ class _MoEFn(torch.autograd.Function):
         if layer.fused_combine:
             with tr.span("b.gateup_dgrad_push"):
                 gemm.gateup_dgrad(d_gate, d_up, layer.w_gate, layer.w_up, cu, wg_slot=slot("gate"),
-                                  wu_slot=slot("up"), split=split, push=buf.push_target(plan), grid=grid)
+                                  wu_slot=slot("up"), split=split, push=buf.push_target(plan), grid=grid,
+                                  pads=pads)
             ev_r = _MoEFn._late_wgrads(layer, plan, hidden, d_gate, d_up, cu, gslot, split, ev_r, do_reduce, sgd)
             with tr.span("b.combine_pushed"):
                 dx, dw_sk = buf.combine_pushed(plan, d_scale)
         else:
             shard = buf.hidden_nvsh_buffer_view
             gemm.gateup_dgrad(d_gate, d_up, layer.w_gate, layer.w_up, cu, wg_slot=slot("gate"),
-                              wu_slot=slot("up"), split=split, out=shard, grid=grid)
+                              wu_slot=slot("up"), split=split, out=shard, grid=grid, pads=pads)
             ev_r = _MoEFn._late_wgrads(layer, plan, hidden, d_gate, d_up, cu, gslot, split, ev_r, do_reduce, sgd)
             dx, dw_sk, _ = buf.combine(plan, shard, d_scale, zero_copy=True)
         # router backward
@@ -253,7 +261,8 @@ class _MoEFn(torch.autograd.Function):
             return ev_r
         pools, zc = layer.pools, layer.accumulate_grads
         wg = lambda a, g, w, **kw: gemm.wgrad(hidden, a, cu, g, grad_slot=gslot(w), split=split,
-                                              sgd=sgd(getattr(layer, "w_" + w)), **kw)
+                                              sgd=sgd(getattr(layer, "w_" + w)),
+                                              pads=plan.zero_fill_ranges, **kw)
         with layer.tracer.span("b.wgrad_gateup"):
             wg(d_gate, layer.g_gate, "gate")
             if do_reduce:     # the gate grads travel home under the up projection's weight grad

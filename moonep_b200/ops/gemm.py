@@ -40,7 +40,7 @@ class _GemmDesc(ctypes.Structure):
         ("total_rows", ctypes.c_int32), ("N", ctypes.c_int32), ("K", ctypes.c_int32),
         ("rows_per_expert", ctypes.c_int32), ("Mw", ctypes.c_int32),
         ("accumulate", ctypes.c_int32), ("zero_empty_below", ctypes.c_int32),
-        ("grid", ctypes.c_int32), ("debug", ctypes.c_int32), ("g_begin", ctypes.c_int32),
+        ("grid", ctypes.c_int32), ("g_begin", ctypes.c_int32),
         ("a_rows", ctypes.c_int64), ("lda", ctypes.c_int64 * 2), ("a", ctypes.c_void_p * 2),
         ("b", (ctypes.c_void_p * 2) * 2), ("b_rows", ctypes.c_int64 * 2), ("ldb", ctypes.c_int64),
         ("cu_seqlens", ctypes.c_void_p), ("out", ctypes.c_void_p * 3), ("ldc", ctypes.c_int64),
@@ -52,6 +52,7 @@ class _GemmDesc(ctypes.Structure):
         ("disp_mode", ctypes.c_int32), ("disp_ctx", ctypes.c_void_p), ("disp_x", ctypes.c_void_p),
         ("disp_w", ctypes.c_void_p), ("disp_dst", ctypes.c_void_p), ("disp_order", ctypes.c_void_p),
         ("disp_zero_fill", ctypes.c_void_p), ("disp_fresh", ctypes.c_int32), ("disp_shard", ctypes.c_int32),
+        ("pads", ctypes.c_void_p),
     ]
 
 
@@ -83,31 +84,27 @@ def reset_status(device="cuda") -> None:
     status_word(device).zero_()
 
 
-PLAIN_EPILOGUE = False   # A/B switch of benchmarks: per-row 16-byte stores instead of staged TMA stores
 # CTA pairs (tcgen05 cta_group::2: clusters of two CTAs issue one 256-row MMA and each stages only
-# half of the B tile, which cuts the shared-memory reads per MMA from 12 KB to 8 KB, the limit of
-# the single-CTA kernel).  ``MOONEP_B200_TWO_CTA``: ``auto`` (default) uses pairs when the groups
-# are long enough on average (see ``_launch``); ``1`` always, ``0`` never.  A launch with a CTA
-# limit (one that runs next to a copy kernel) needs an even limit; the copy kernels are placed
-# as SM pairs too, so the SMs they leave free can all be paired.
+# half of the second operand's tile).  ``MOONEP_B200_TWO_CTA``: ``auto`` (default) uses pairs for the
+# token-major products always and for the weight grads when the groups are long enough on average
+# (see ``_launch``); ``1`` always, ``0`` never.  A launch with a CTA limit (one that runs next to a
+# copy kernel) needs an even limit; the copy kernels are placed as SM pairs too, so the SMs they
+# leave free can all be paired.
 _two = __import__("os").environ.get("MOONEP_B200_TWO_CTA", "auto").strip().lower()
 TWO_CTA = {"auto": 2, "": 2}.get(_two, None)
 if TWO_CTA is None:
     TWO_CTA = int(_two)
-PAIR_MIN_AVG_ROWS = 768
 PAIR_MIN_AVG_ROWS_WGRAD = 512   # 64 groups x 512 rows, fused SGD: pairs 1.16 ms, single CTAs 1.44 ms
 
 
 def _launch(d: _GemmDesc) -> None:
     global _checked_layout
-    d.debug = 16 if PLAIN_EPILOGUE else 0
     if TWO_CTA == 2:
-        # token-major: a pair covers 256 rows of ONE group, so short groups would leave the second
-        # CTA idle; the host only knows the average (over the local groups, the slot groups hold
-        # rows taken from those).  Weight-grad tiles split the weight rows instead, but with short
-        # groups (a few k-blocks per tile) the pair's extra hand-shakes cost more than they save.
+        # Weight-grad tiles split the weight rows between the pair's CTAs; with short groups (a few
+        # k-blocks per tile) the pair's extra hand-shakes cost more than they save.  The host only
+        # knows the average (over the local groups, the slot groups hold rows taken from those).
         local_groups = max(1, min(d.ngroups, d.split))
-        least = PAIR_MIN_AVG_ROWS_WGRAD if d.mode == 1 else PAIR_MIN_AVG_ROWS
+        least = PAIR_MIN_AVG_ROWS_WGRAD if d.mode == 1 else 0
         d.two_cta = int(d.grid % 2 == 0 and d.total_rows >= least * local_groups)
     else:
         d.two_cta = TWO_CTA
@@ -125,6 +122,15 @@ def _bf16(t: torch.Tensor, name: str) -> torch.Tensor:
     return t
 
 
+def _pads(pads, cu_seqlens):
+    """Pointer of the plan's padding ranges (``zero_fill_ranges [>= groups, 2]``), or ``None``."""
+    if pads is None:
+        return None
+    assert pads.dtype == torch.int32 and pads.is_cuda and pads.is_contiguous() and cu_seqlens is not None
+    assert pads.dim() == 2 and pads.shape[1] == 2 and pads.shape[0] >= cu_seqlens.numel()
+    return pads.data_ptr()
+
+
 def _groups(cu_seqlens, rows):
     if cu_seqlens is None:
         return None, 1
@@ -133,7 +139,7 @@ def _groups(cu_seqlens, rows):
 
 
 def _tokens_gemm(a_segs, b_sel, b_slot_sel, cu_seqlens, split, N, K, rows_per_expert, b_mn, epi,
-                 outs, ldc, row_scale=None, total_rows=None, grid=0, push=None, g_begin=0, dispatch=None):
+                 outs, ldc, row_scale=None, total_rows=None, grid=0, push=None, g_begin=0, dispatch=None, pads=None):
     d = _GemmDesc()
     d.mode, d.epi, d.b_mn, d.nseg = 0, epi, int(b_mn), len(a_segs)
     cu_ptr, ngroups = _groups(cu_seqlens, None)
@@ -144,6 +150,7 @@ def _tokens_gemm(a_segs, b_sel, b_slot_sel, cu_seqlens, split, N, K, rows_per_ex
     d.N, d.K, d.rows_per_expert, d.Mw = N, K, rows_per_expert, 0
     d.grid = grid
     d.g_begin = g_begin
+    d.pads = _pads(pads, cu_seqlens)
     d.a_rows = a0.shape[0]
     for i, a in enumerate(a_segs):
         _bf16(a, "A")
@@ -191,7 +198,8 @@ def _tokens_gemm(a_segs, b_sel, b_slot_sel, cu_seqlens, split, N, K, rows_per_ex
 
 
 def gateup_swiglu(x, wg, wu, cu_seqlens, *, wg_slot=None, wu_slot=None, split=None,
-                  row_scale=None, save_gate_up=True, out=None, g_begin=0, grid=0, dispatch=None):
+                  row_scale=None, save_gate_up=True, out=None, g_begin=0, grid=0, dispatch=None,
+                  pads=None):
     """``act[rows,H'] = silu(x Wg[g]) * (x Wu[g]) * row_scale``; also returns bf16 gate / up.
 
     ``x`` [rows, H]; ``wg``/``wu`` [G0, H, H'] (+ optional slot tensors for groups >= split).
@@ -200,7 +208,11 @@ def gateup_swiglu(x, wg, wu, cu_seqlens, *, wg_slot=None, wu_slot=None, split=No
     number of CTAs (to leave SMs to a concurrent communication kernel).  ``dispatch`` (from
     ``Buffer.dispatch_fused_begin``) makes this launch carry the dispatch all-to-all itself: ``x``
     must be the Buffer's row-buffer view, a seventh warp per CTA sends this rank's tokens, and
-    tiles are computed as their rows arrive (``dict(disp, mode=1)`` only waits for arrivals)."""
+    tiles are computed as their rows arrive (``dict(disp, mode=1)`` only waits for arrivals).
+
+    ``pads`` (a plan's ``zero_fill_ranges``), here and in the other grouped products: which rows of the
+    groups are padding.  Padding rows of the inputs are zero; the results are the same without it, but
+    rows and blocks of nothing but padding are then not computed."""
     rows, H = x.shape
     Hp = wg.shape[2]
     assert wg.shape[1] == H and wu.shape == wg.shape
@@ -213,11 +225,11 @@ def gateup_swiglu(x, wg, wu, cu_seqlens, *, wg_slot=None, wu_slot=None, split=No
     if row_scale is not None:
         assert row_scale.dtype == torch.float32 and row_scale.numel() >= rows
     _tokens_gemm([x], [wg, wu], [wg_slot, wu_slot], cu_seqlens, split, Hp, H, H, True, EPI_SWIGLU,
-                 [gate, up, act], Hp, row_scale, grid=grid, g_begin=g_begin, dispatch=dispatch)
+                 [gate, up, act], Hp, row_scale, grid=grid, g_begin=g_begin, dispatch=dispatch, pads=pads)
     return act, gate, up
 
 
-def down(act, wd, cu_seqlens, *, wd_slot=None, split=None, out=None, push=None):
+def down(act, wd, cu_seqlens, *, wd_slot=None, split=None, out=None, push=None, pads=None):
     """``y[rows,H] = act[rows,H'] Wd[g]^T`` with ``wd`` [G0, H, H'].
 
     With ``push`` (``Buffer.push_target(plan)``) nothing is written locally: every result row goes
@@ -227,14 +239,16 @@ def down(act, wd, cu_seqlens, *, wd_slot=None, split=None, out=None, push=None):
     H = wd.shape[1]
     assert wd.shape[2] == Hp
     if push is not None:
-        _tokens_gemm([act], [wd], [wd_slot], cu_seqlens, split, H, Hp, H, False, EPI_BF16, [], H, push=push)
+        _tokens_gemm([act], [wd], [wd_slot], cu_seqlens, split, H, Hp, H, False, EPI_BF16, [], H, push=push,
+                     pads=pads)
         return None
     y = torch.empty(rows, H, dtype=torch.bfloat16, device=act.device) if out is None else out
-    _tokens_gemm([act], [wd], [wd_slot], cu_seqlens, split, H, Hp, H, False, EPI_BF16, [y], y.stride(0))
+    _tokens_gemm([act], [wd], [wd_slot], cu_seqlens, split, H, Hp, H, False, EPI_BF16, [y], y.stride(0),
+                 pads=pads)
     return y
 
 
-def down_dgrad(dy, wd, cu_seqlens, *, wd_slot=None, split=None, out=None, g_begin=0, grid=0, dispatch=None):
+def down_dgrad(dy, wd, cu_seqlens, *, wd_slot=None, split=None, out=None, g_begin=0, grid=0, dispatch=None, pads=None):
     """``dact[rows,H'] = dy[rows,H] Wd[g]``.  ``out`` / ``g_begin`` / ``grid`` / ``dispatch`` as in
     :func:`gateup_swiglu`: the local experts and the prefetch slots may be two launches, and the
     launch may carry the dispatch of ``dy`` itself."""
@@ -243,28 +257,28 @@ def down_dgrad(dy, wd, cu_seqlens, *, wd_slot=None, split=None, out=None, g_begi
     if out is None:
         out = torch.empty(rows, Hp, dtype=torch.bfloat16, device=dy.device)
     _tokens_gemm([dy], [wd], [wd_slot], cu_seqlens, split, Hp, H, H, True, EPI_BF16, [out], Hp,
-                 grid=grid, g_begin=g_begin, dispatch=dispatch)
+                 grid=grid, g_begin=g_begin, dispatch=dispatch, pads=pads)
     return out
 
 
 def gateup_dgrad(dg, du, wg, wu, cu_seqlens, *, wg_slot=None, wu_slot=None, split=None, out=None,
-                 push=None, grid=0):
+                 push=None, grid=0, pads=None):
     """``dx[rows,H] = dg Wg[g]^T + du Wu[g]^T`` (two K segments into one accumulator); ``push`` as
     in :func:`down`."""
     rows, Hp = dg.shape
     H = wg.shape[1]
     if push is not None:
         _tokens_gemm([dg, du], [wg, wu], [wg_slot, wu_slot], cu_seqlens, split, H, Hp, H, False,
-                     EPI_BF16, [], H, push=push, grid=grid)
+                     EPI_BF16, [], H, push=push, grid=grid, pads=pads)
         return None
     dx = torch.empty(rows, H, dtype=torch.bfloat16, device=dg.device) if out is None else out
     _tokens_gemm([dg, du], [wg, wu], [wg_slot, wu_slot], cu_seqlens, split, H, Hp, H, False,
-                 EPI_BF16, [dx], dx.stride(0), grid=grid)
+                 EPI_BF16, [dx], dx.stride(0), grid=grid, pads=pads)
     return dx
 
 
 def wgrad(a, b, cu_seqlens, grad_local, *, grad_slot=None, split=None, accumulate=False, sgd=None,
-          grid=0, select=0):
+          grid=0, select=0, pads=None):
     """``grad[g] (+)= a[rows of g]^T b[rows of g]``; ``a`` [rows, M], ``b`` [rows, N], fp32 grads
     ``[G0, M, N]`` (+ slot grads for groups >= split).  Group sizes must be multiples of 64
     (padding rows must be zero in ``a`` or ``b``).  Empty groups below ``split`` are zeroed
@@ -306,6 +320,7 @@ def wgrad(a, b, cu_seqlens, grad_local, *, grad_slot=None, split=None, accumulat
         assert d.split >= ngroups
     d.ldc = N
     d.grid = grid
+    d.pads = _pads(pads, cu_seqlens)
     assert select in (0, 1, 2) and (select == 0 or sgd is not None), "select splits a fused-SGD weight grad"
     if sgd is not None:
         w, lr, keep = sgd
