@@ -56,8 +56,8 @@ nat.declare("mep_launch_push_reduce", I, [P, P, L, P, L, P, P, P, P, P, I, P])
 nat.declare("mep_launch_expand", I, [P, P, P, I, P])
 nat.declare("mep_launch_combine_prologue", I, [P, P, P, P])
 nat.declare("mep_launch_combine", I, [P, P, P, P, I, P])
-nat.declare("mep_launch_prefetch", I, [P, P, I, P, P, P, P, P])
-nat.declare("mep_launch_grad_reduce", I, [P, P, I, P, P, P, P, I, I, I, P])
+nat.declare("mep_launch_prefetch", I, [P, P, I, P, P, P, P, I, P])
+nat.declare("mep_launch_grad_reduce", I, [P, P, I, P, P, P, P, I, I, I, I, P])
 nat.declare("mep_launch_sync", I, [P, P])
 
 _KERNEL_NAMES = {1: "sync", 2: "plan", 3: "dispatch", 4: "expand", 5: "combine_prologue",
@@ -658,7 +658,7 @@ class Buffer:
 
         def run():
             self._rc(nat.call("mep_launch_prefetch", self._ctx, plan.experts_to_copy.data_ptr(), n,
-                              lp, pp, eb, rs, self._stream()), "prefetch_weight")
+                              lp, pp, eb, rs, int(self._one_device), self._stream()), "prefetch_weight")
             self._stats["prefetch_weight"] += 1
             self._maybe_check()
 
@@ -705,7 +705,8 @@ class Buffer:
 
         def run():
             self._rc(nat.call("mep_launch_grad_reduce", self._ctx, plan.experts_to_copy.data_ptr(), n,
-                              lp, pp, eb, rs, int(entry_sync), int(zero_consumed), int(num_sms), self._stream()), "reduce_grad")
+                              lp, pp, eb, rs, int(entry_sync), int(zero_consumed), int(num_sms),
+                              int(self._one_device), self._stream()), "reduce_grad")
             self._stats["reduce_grad"] += 1
             self._maybe_check()
 

@@ -31,6 +31,11 @@ constexpr int GR_THREADS = 32 + GR_ACC_THREADS;
 struct GradReduceParams {
   SyncCtx sync;
   int epn, n_tensors, entry_barrier, zero_consumed;
+  // Every rank's tensors are memory of this device.  All CTAs then share ONE list of all ranks' work
+  // (with one list a rank, the owners of popular experts work and the other ranks' CTAs idle), a
+  // consumed chunk is cleared by the CTA that has just read it, and nothing is left to wait for.
+  // 8 ranks x 16 experts of 2048 x 768, skewed: 279 -> 95 us (with the prefetch 122, where the bytes need 106).
+  int one_device;
   const int32_t* etc;                     // [Rv][R*epn]
   float* local[GR_MAX_TENSORS];           // [Rv][epn][expert_elems]
   float* pool[GR_MAX_TENSORS];            // slot (d,b) at pool + d*rank_stride + b*expert_elems
@@ -47,14 +52,18 @@ __global__ void __launch_bounds__(GR_THREADS, 1) ep_grad_reduce_kernel(const Gra
   __shared__ int n_active;
   const SyncCtx& sc = p.sync;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int vr = blockIdx.y, rank = sc.rank_base + vr;
-  const int G = gridDim.x, c = blockIdx.x;
-  const int R = sc.R, epn = p.epn;
+  const bool one = p.one_device != 0;
+  const int vr = one ? 0 : (int)blockIdx.y, rank = one ? 0 : sc.rank_base + vr;
+  const int G = one ? (int)(gridDim.x * gridDim.y) : (int)gridDim.x;
+  const int c = one ? (int)(blockIdx.y * gridDim.x + blockIdx.x) : (int)blockIdx.x;
+  const int R = one ? 1 : sc.R, epn = one ? p.epn * sc.R : p.epn;   // one list: as one rank with all experts
+  const int slots = sc.R * p.epn;
   uint8_t* ring = smem_raw;
-  int32_t* cnt = reinterpret_cast<int32_t*>(smem_raw + (size_t)ST * GR_CHUNK);  // [epn]
-  int32_t* start = cnt + epn;                                                   // [epn]
-  int32_t* active = start + epn;                                                // [epn]
-  int32_t* srcs = active + epn;                                                 // [R*epn] CSR
+  int32_t* cnt = reinterpret_cast<int32_t*>(smem_raw + (size_t)(ST + one) * GR_CHUNK);  // [epn]
+  int32_t* start = cnt + epn;                                                         // [epn]
+  int32_t* active = start + epn;                                                      // [epn]
+  int32_t* srcs = active + epn;                                                       // [slots] CSR
+  uint8_t* zeros = one ? ring + (size_t)ST * GR_CHUNK : ring;   // (several devices: once the ring is empty)
 
   if (tid == 0) {
     for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], GR_ACC_THREADS / 32); }
@@ -62,9 +71,14 @@ __global__ void __launch_bounds__(GR_THREADS, 1) ep_grad_reduce_kernel(const Gra
     n_active = 0;
   }
   for (int i = tid; i < epn; i += GR_THREADS) cnt[i] = 0;
+  if (one) {
+    for (uint32_t i = (uint32_t)tid * 16u; i < GR_CHUNK; i += GR_THREADS * 16u)
+      *reinterpret_cast<uint4*>(zeros + i) = make_uint4(0, 0, 0, 0);
+    fence_proxy_async_smem();
+  }
   __syncthreads();
-  const int32_t* etc = p.etc + (size_t)vr * R * epn;
-  for (int i = tid; i < R * epn; i += GR_THREADS) {
+  const int32_t* etc = p.etc + (size_t)vr * slots;
+  for (int i = tid; i < slots; i += GR_THREADS) {
     int e = etc[i];
     if (e >= 0 && e / epn == rank) atomicAdd(&cnt[e - rank * epn], 1);
   }
@@ -93,11 +107,11 @@ __global__ void __launch_bounds__(GR_THREADS, 1) ep_grad_reduce_kernel(const Gra
   // walks the whole table in order (deterministic; the table is small)
   for (int a = tid; a < n_active; a += GR_THREADS) {
     int le = active[a], want = rank * epn + le, pos = start[le];
-    for (int i = 0; i < R * epn; ++i)
+    for (int i = 0; i < slots; ++i)
       if (etc[i] == want) srcs[pos++] = i;
   }
   __syncthreads();
-  if (p.entry_barrier) cross_rank_barrier(sc, 1);
+  if (p.entry_barrier && !one) cross_rank_barrier(sc, 1);
   const int na = n_active;
 
   int64_t items_before[GR_MAX_TENSORS + 1];
@@ -139,7 +153,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) ep_grad_reduce_kernel(const Gra
             src = p.local[t] + ((size_t)vr * epn + le) * p.expert_elems[t] + off;
           } else {
             int slot = srcs[start[le] + q];
-            int d = slot / epn, b = slot - d * epn;
+            int d = slot / p.epn, b = slot - d * p.epn;
             src = p.pool[t] + (size_t)d * p.rank_stride[t] + (size_t)b * p.expert_elems[t] + off;
           }
           mbar_expect_tx(&full[s], bytes);
@@ -175,6 +189,12 @@ __global__ void __launch_bounds__(GR_THREADS, 1) ep_grad_reduce_kernel(const Gra
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
+        if (one && p.zero_consumed && ta == 0 && q >= 0) {      // the chunk has landed: clear it where it came from
+          const int slot = srcs[start[le] + q];
+          const int d = slot / p.epn, b = slot - d * p.epn;
+          bulk_s2g(p.pool[t] + (size_t)d * p.rank_stride[t] + (size_t)b * p.expert_elems[t] + off, zeros, bytes);
+          bulk_commit();
+        }
       }
 #pragma unroll
       for (int i = 0; i < GR_VEC_PER_THREAD; ++i) {
@@ -183,6 +203,10 @@ __global__ void __launch_bounds__(GR_THREADS, 1) ep_grad_reduce_kernel(const Gra
       }
     }
   }
+  if (one) {
+    if (tid == 32) bulk_wait<0>();
+    return;
+  }
   // every home rank has read what it needs before anyone clears
   cross_rank_barrier(sc, 2);
   if (!p.zero_consumed) return;
@@ -190,7 +214,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) ep_grad_reduce_kernel(const Gra
   // thread per CTA bulk-stores over this CTA's share of every consumed slot (the copy engine
   // writes full lines at a rate that per-thread 16-byte stores of 160 threads do not reach)
   for (uint32_t i = (uint32_t)tid * 16u; i < GR_CHUNK; i += GR_THREADS * 16u)
-    *reinterpret_cast<uint4*>(ring + i) = make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(zeros + i) = make_uint4(0, 0, 0, 0);
   fence_proxy_async_smem();
   __syncthreads();
   if (tid == 0) {
@@ -203,7 +227,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) ep_grad_reduce_kernel(const Gra
         const int64_t bytes = p.expert_elems[t] * 4;
         for (int64_t off = (int64_t)c * GR_CHUNK; off < bytes; off += (int64_t)G * GR_CHUNK) {
           const int64_t n = bytes - off < (int64_t)GR_CHUNK ? bytes - off : (int64_t)GR_CHUNK;
-          bulk_s2g(z + off, ring, (uint32_t)n);
+          bulk_s2g(z + off, zeros, (uint32_t)n);
           if (++pending == 8) { bulk_commit(); pending = 0; }
         }
       }
@@ -215,11 +239,17 @@ __global__ void __launch_bounds__(GR_THREADS, 1) ep_grad_reduce_kernel(const Gra
 
 template <int ST, uint32_t GR_CHUNK>
 static int launch_gr_t(const BufferCtx& c, GradReduceParams& p, int grid_x, cudaStream_t stream) {
-  size_t smem = (size_t)ST * GR_CHUNK + sizeof(int32_t) * ((size_t)3 * c.epn + (size_t)c.epn * c.R);
+  const size_t lists = p.one_device ? (size_t)3 * c.E : (size_t)3 * c.epn;
+  size_t smem = (size_t)(ST + p.one_device) * GR_CHUNK + sizeof(int32_t) * (lists + (size_t)c.E);
   if (smem > 220 * 1024) return fail(-2, "reduce_grad: E=%d is too large for the slot lists", c.E);
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_grad_reduce_kernel<ST, GR_CHUNK>, raised));
   dim3 grid(grid_x > 0 ? grid_x : c.num_sms_weights, c.Rv());
+  if (p.one_device) {      // no barrier inside: nothing has to be resident at once
+    ep_grad_reduce_kernel<ST, GR_CHUNK><<<grid, GR_THREADS, smem, stream>>>(p);
+    MEP_CUDA_OK(cudaGetLastError());
+    return 0;
+  }
   MEP_CUDA_OK(launch_coop_paired((const void*)ep_grad_reduce_kernel<ST, GR_CHUNK>, grid, dim3(GR_THREADS), smem, stream, p));
   return 0;
 }
@@ -239,16 +269,17 @@ extern "C" {
 // etc [Rv][R*epn]; per tensor: local grad [Rv][epn][elems] fp32, pool base, elements per expert
 // (multiple of 4), element stride between ranks' pools.  grid_x > 0 overrides the number of CTAs
 // (the Buffer's num_sms_weights): a reduce that runs next to nothing may take more SMs.
+// one_device != 0 (only where every rank's tensors are on this device): see GradReduceParams.
 int mep_launch_grad_reduce(const void* ctx_, const int32_t* etc, int n, void* const* local,
                            void* const* pool, const int64_t* expert_elems,
                            const int64_t* rank_stride, int entry_barrier, int zero_consumed,
-                           int grid_x, cudaStream_t stream) {
+                           int grid_x, int one_device, cudaStream_t stream) {
   const BufferCtx& c = *(const BufferCtx*)ctx_;
   if (n < 1 || n > GR_MAX_TENSORS) return fail(-1, "reduce_grad: %d tensors (1..%d)", n, GR_MAX_TENSORS);
   GradReduceParams p;
   p.sync = c.sync(KID_REDUCE, /*channel=*/1);
   p.epn = c.epn; p.n_tensors = n; p.etc = etc; p.entry_barrier = entry_barrier;
-  p.zero_consumed = zero_consumed;
+  p.zero_consumed = zero_consumed; p.one_device = one_device && c.one_device() && c.E <= 4096;   // (longer lists do not fit beside the ring)
   for (int t = 0; t < n; ++t) {
     if (expert_elems[t] % 4 != 0 || rank_stride[t] % 4 != 0 ||
         ((uintptr_t)local[t] | (uintptr_t)pool[t]) % 16 != 0)
@@ -256,6 +287,7 @@ int mep_launch_grad_reduce(const void* ctx_, const int32_t* etc, int n, void* co
     p.local[t] = (float*)local[t]; p.pool[t] = (float*)pool[t];
     p.expert_elems[t] = expert_elems[t]; p.rank_stride[t] = rank_stride[t];
   }
+  if (p.one_device) return launch_gr_t<8, 16 * 1024>(c, p, grid_x, stream);
   if (c.virt) return launch_gr_t<4, 16 * 1024>(c, p, grid_x, stream);
   // ring geometry: MOONEP_B200_GR_RING = <stages>x<KB> selects one of the built variants (tuning)
   static int cfg = -1;

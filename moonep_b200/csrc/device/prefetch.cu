@@ -26,6 +26,10 @@ constexpr int PF_THREADS = 64;
 struct PrefetchParams {
   SyncCtx sync;
   int epn, n_tensors;
+  // Every rank's tensors are memory of this device: all CTAs share one list of all ranks' work (the
+  // owners of popular experts would work alone otherwise) and the launch boundary orders the writes.
+  // 8 ranks x 16 experts of 2048 x 768, skewed: 77 -> 27 us.
+  int one_device;
   const int32_t* etc;                       // [Rv][R*epn]
   const uint8_t* local[PF_MAX_TENSORS];     // [Rv][epn][expert_bytes]
   uint8_t* pool[PF_MAX_TENSORS];            // slot (d, b) at pool + d*rank_stride + b*expert_bytes
@@ -40,15 +44,18 @@ __global__ void __launch_bounds__(PF_THREADS, 1) ep_prefetch_kernel(const Prefet
   __shared__ __align__(8) uint64_t full[ST];
   const SyncCtx& sc = p.sync;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int vr = blockIdx.y, rank = sc.rank_base + vr;
-  const int G = gridDim.x, c = blockIdx.x;
-  const int R = sc.R, epn = p.epn;
+  const bool one = p.one_device != 0;
+  const int vr = one ? 0 : (int)blockIdx.y, rank = one ? 0 : sc.rank_base + vr;
+  const int G = one ? (int)(gridDim.x * gridDim.y) : (int)gridDim.x;
+  const int c = one ? (int)(blockIdx.y * gridDim.x + blockIdx.x) : (int)blockIdx.x;
+  const int epn = one ? p.epn * sc.R : p.epn;        // one list: as one rank with all experts
+  const int slots = sc.R * p.epn;
   uint8_t* ring = smem_raw;
   int32_t* cnt = reinterpret_cast<int32_t*>(smem_raw + (size_t)ST * PF_CHUNK);  // [epn]
   int32_t* start = cnt + epn;                                                   // [epn]
   int32_t* cursor = start + epn;                                                // [epn]
   int32_t* active = cursor + epn;                                               // [epn]
-  int32_t* dests = active + epn;                                                // [R*epn] CSR
+  int32_t* dests = active + epn;                                                // [slots] CSR
   __shared__ int n_active;
 
   if (tid == 0) {
@@ -59,8 +66,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) ep_prefetch_kernel(const Prefet
   for (int i = tid; i < epn; i += PF_THREADS) { cnt[i] = 0; cursor[i] = 0; }
   __syncthreads();
   // which of my experts go where: count, prefix, fill (slot id = d*epn + b)
-  const int32_t* etc = p.etc + (size_t)vr * R * epn;
-  for (int i = tid; i < R * epn; i += PF_THREADS) {
+  const int32_t* etc = p.etc + (size_t)vr * slots;
+  for (int i = tid; i < slots; i += PF_THREADS) {
     int e = etc[i];
     if (e >= 0 && e / epn == rank) atomicAdd(&cnt[e - rank * epn], 1);
   }
@@ -85,7 +92,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) ep_prefetch_kernel(const Prefet
     if (lane == 0) n_active = base;
   }
   __syncthreads();
-  for (int i = tid; i < R * epn; i += PF_THREADS) {
+  for (int i = tid; i < slots; i += PF_THREADS) {
     int e = etc[i];
     if (e >= 0 && e / epn == rank) {
       int le = e - rank * epn;
@@ -138,7 +145,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) ep_prefetch_kernel(const Prefet
       const int nd = cnt[le];
       for (int q = lane; q < nd; q += 32) {
         int slot = dests[start[le] + q];
-        int d = slot / epn, b = slot - d * epn;
+        int d = slot / p.epn, b = slot - d * p.epn;
         bulk_s2g(p.pool[t] + (size_t)d * p.rank_stride[t] + (size_t)b * p.expert_bytes[t] + off,
                  ring + (size_t)s * PF_CHUNK, bytes);
       }
@@ -158,17 +165,23 @@ __global__ void __launch_bounds__(PF_THREADS, 1) ep_prefetch_kernel(const Prefet
     bulk_wait<0>();
     fence_proxy_async();
   }
+  if (one) return;
   fence_sys();
   cross_rank_barrier(sc, 2);  // prefetched weights are visible on every rank
 }
 
 template <int ST, uint32_t PF_CHUNK>
 static int launch_prefetch_t(const BufferCtx& c, PrefetchParams& p, cudaStream_t stream) {
-  size_t smem = (size_t)ST * PF_CHUNK + sizeof(int32_t) * ((size_t)4 * c.epn + (size_t)c.epn * c.R);
+  size_t smem = (size_t)ST * PF_CHUNK + sizeof(int32_t) * ((size_t)4 * (p.one_device ? c.E : c.epn) + (size_t)c.E);
   if (smem > 220 * 1024) return fail(-2, "prefetch: E=%d is too large for the slot lists", c.E);
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_prefetch_kernel<ST, PF_CHUNK>, raised));
   dim3 grid(c.num_sms_weights, c.Rv());
+  if (p.one_device) {      // no barrier inside: nothing has to be resident at once
+    ep_prefetch_kernel<ST, PF_CHUNK><<<grid, PF_THREADS, smem, stream>>>(p);
+    MEP_CUDA_OK(cudaGetLastError());
+    return 0;
+  }
   MEP_CUDA_OK(launch_coop_paired((const void*)ep_prefetch_kernel<ST, PF_CHUNK>, grid, dim3(PF_THREADS), smem, stream, p));
   return 0;
 }
@@ -180,15 +193,16 @@ using namespace mep;
 extern "C" {
 
 // etc [Rv][R*epn]; for each of n tensors: local [Rv][epn][expert_bytes], pool base, bytes per
-// expert (multiple of 16) and the byte stride between ranks' pools.
+// expert (multiple of 16) and the byte stride between ranks' pools.  one_device != 0 (only where every
+// rank's tensors are on this device): see PrefetchParams.
 int mep_launch_prefetch(const void* ctx_, const int32_t* etc, int n, const void* const* local,
                         void* const* pool, const int64_t* expert_bytes, const int64_t* rank_stride,
-                        cudaStream_t stream) {
+                        int one_device, cudaStream_t stream) {
   const BufferCtx& c = *(const BufferCtx*)ctx_;
   if (n < 1 || n > PF_MAX_TENSORS) return fail(-1, "prefetch: %d tensors (1..%d)", n, PF_MAX_TENSORS);
   PrefetchParams p;
   p.sync = c.sync(KID_PREFETCH, /*channel=*/1);
-  p.epn = c.epn; p.n_tensors = n; p.etc = etc;
+  p.epn = c.epn; p.n_tensors = n; p.etc = etc; p.one_device = one_device && c.one_device() && c.E <= 4096;   // (longer lists do not fit beside the ring)
   for (int t = 0; t < n; ++t) {
     if (expert_bytes[t] % 16 != 0 || rank_stride[t] % 16 != 0 ||
         ((uintptr_t)local[t] | (uintptr_t)pool[t]) % 16 != 0)
@@ -196,7 +210,8 @@ int mep_launch_prefetch(const void* ctx_, const int32_t* etc, int n, const void*
     p.local[t] = (const uint8_t*)local[t]; p.pool[t] = (uint8_t*)pool[t];
     p.expert_bytes[t] = expert_bytes[t]; p.rank_stride[t] = rank_stride[t];
   }
-  if (c.virt) return launch_prefetch_t<4, 16 * 1024>(c, p, stream);
+  if (p.one_device && c.E > 1024) return launch_prefetch_t<4, 32 * 1024>(c, p, stream);
+  if (c.virt && !p.one_device) return launch_prefetch_t<4, 16 * 1024>(c, p, stream);
   return launch_prefetch_t<6, 32 * 1024>(c, p, stream);
 }
 

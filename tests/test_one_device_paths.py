@@ -45,3 +45,40 @@ def test_duplicates_moved_directly_match_the_separate_kernels(R, S, K, E, H, tp,
         assert torch.equal(a, b)
     assert torch.equal(direct[-3], w)
     buf.destroy()
+
+
+# (R, experts a rank, elements an expert): one chunk, ragged last chunks, several chunks; CTAs a rank
+WEIGHT_CASES = [(2, 1, 8, 1), (2, 3, 4096, 2), (4, 8, 20000, 5), (8, 16, 70008, 18), (3, 5, 4104, 32)]
+
+
+@pytest.mark.parametrize("R,epn,n,sms", WEIGHT_CASES)
+@pytest.mark.parametrize("zero", [True, False])
+def test_weights_moved_from_one_list_match_one_list_a_rank(R, epn, n, sms, zero):
+    """``prefetch_weight`` / ``reduce_grad`` share one work list between all ranks' CTAs within one device;
+    same bytes, same order of the additions."""
+    from moonep_b200 import Buffer, CommPlan
+    buf = Buffer(16, 64, 1, R * epn, R, num_sms=sms, token_padding=8, virtual=True, timeout_s=2.0)
+    g = torch.Generator().manual_seed(n + R)
+    etc = torch.where(torch.rand(R, epn, generator=g) < 0.6, torch.randint(0, R * epn, (R, epn), generator=g),
+                      torch.full((R, epn), -1)).to(torch.int32).cuda()[None].expand(R, R, epn).contiguous()
+    z = lambda *s: torch.zeros(*s, dtype=torch.int32, device="cuda")
+    plan = CommPlan(dst=z(R, buf.N), experts_to_copy=etc, zero_fill_ranges=z(R, 2 * epn, 2), remote_stats=z(R, 2),
+                    cu_seqlens=z(R, 2 * epn), link=z(R, buf.NvS), N=buf.N, R=R, E=buf.E, NvS=buf.NvS, K=buf.K)
+    rnd = lambda: torch.randn(R, epn, n, generator=g).cuda()
+    w, grads, slots = [rnd().bfloat16() for _ in range(3)], [rnd() for _ in range(3)], [rnd() for _ in range(3)]
+    names = ("gate", "up", "down")
+
+    def both(one):
+        buf._one_device = one
+        pool = [torch.full_like(t, 7.0) for t in w]
+        buf.prefetch_weight(plan, **{f"local_{a}_weight": t for a, t in zip(names, w)},
+                            **{f"{a}_prefetch_buffer": t for a, t in zip(names, pool)})
+        gr, sl = [t.clone() for t in grads], [t.clone() for t in slots]
+        buf.reduce_grad(plan, zero_consumed=zero, **{f"local_{a}_grad": t for a, t in zip(names, gr)},
+                        **{f"{a}_reduce_buffer": t for a, t in zip(names, sl)})
+        buf.check()
+        return pool + gr + sl
+
+    for a, b in zip(both(True), both(False)):
+        assert torch.equal(a, b)
+    buf.destroy()
