@@ -78,6 +78,7 @@ class _MoEFn(torch.autograd.Function):
             logits = gemm.dense(x, layer.w_router)                         # [S, E] fp32
             topk, w, tpe = ew.router_topk(logits, buf.K, layer.router_bias)
         fused = layer.fused_dispatch
+        keep = ctx.needs_input_grad[0]         # a backward pass may follow
         disp = None
         with tr.span("f.dispatch"):
             shard = 1 if layer.hidden_in_place else 0
@@ -89,7 +90,9 @@ class _MoEFn(torch.autograd.Function):
             elif layer.hidden_in_place:
                 hidden, w_nvs, cu, plan = buf.dispatch(x, w, topk, tpe, zero_copy=True, shard=1)
             else:
-                hidden, w_nvs, cu, plan = buf.dispatch(x, w, topk, tpe)
+                # a pass without a backward pass reads the rows where they landed; else they are kept
+                hidden, w_nvs, cu, plan = buf.dispatch(x, w, topk, tpe, zero_copy=not keep,
+                                                       router_weights_zero_copy=not keep)
         wait_only = None if disp is None else dict(disp, mode=1)
         pools = layer.pools
         if pools is not None and pools.prefetch:
@@ -101,25 +104,25 @@ class _MoEFn(torch.autograd.Function):
             split, cu_use = epn, cu
             with tr.span("f.gateup_local"):
                 outs = gemm.gateup_swiglu(hidden, layer.w_gate, layer.w_up, cu[:epn], row_scale=w_nvs,
-                                          save_gate_up=layer.training, grid=layer.overlap_grid(), dispatch=disp,
+                                          save_gate_up=layer.training and keep, grid=layer.overlap_grid(), dispatch=disp,
                                           pads=plan.zero_fill_ranges)
             with tr.span("f.wait_prefetch"):
                 torch.cuda.current_stream().wait_event(ev)
             with tr.span("f.gateup_slots"):
                 act, gate, up = gemm.gateup_swiglu(hidden, layer.w_gate, layer.w_up, cu, wg_slot=slots["g"],
                                                    wu_slot=slots["u"], split=epn, row_scale=w_nvs,
-                                                   save_gate_up=layer.training, out=outs, g_begin=epn,
+                                                   save_gate_up=layer.training and keep, out=outs, g_begin=epn,
                                                    dispatch=wait_only, pads=plan.zero_fill_ranges)
         else:
             slots = dict(g=None, u=None, d=None)
             split, cu_use = None, cu[:epn]
             with tr.span("f.gateup"):
                 act, gate, up = gemm.gateup_swiglu(hidden, layer.w_gate, layer.w_up, cu_use, row_scale=w_nvs,
-                                                   save_gate_up=layer.training, dispatch=disp,
+                                                   save_gate_up=layer.training and keep, dispatch=disp,
                                                    pads=plan.zero_fill_ranges)
         if fused:
-            w_nvs = buf.dispatch_fused_end(plan, disp)     # plan records + a private copy of the weights
-            if not layer.hidden_in_place:
+            w_nvs = buf.dispatch_fused_end(plan, disp, clone_weights=keep)   # plan records, the weights
+            if keep and not layer.hidden_in_place:
                 hidden = hidden.clone()
         if layer.fused_combine:
             # down GEMM fused with the combine all-to-all: the epilogue stores every result row
@@ -302,10 +305,13 @@ class MoELayer:
         self.fused_combine = fused_combine
         # dispatch all-to-all inside the consuming GEMM launch (forward: gate/up, backward: down
         # dgrad) instead of a kernel of its own followed by a barrier; default: whenever the
-        # Buffer's shape allows it
+        # Buffer's shape allows it and rows cross NVLink.  A lone rank's dispatch is a local copy:
+        # there the stand-alone kernel and the GEMM with its full operand ring are shorter than
+        # the fused launch (128 experts, 4096 tokens x 2048: 88 + 408 us against 611; 16 tokens x
+        # 7168, 32 experts: 25 + 301 against 342).
         ok = buf.fused_dispatch_supported()
         assert not fused_dispatch or ok, "this Buffer's shape cannot use the fused dispatch"
-        self.fused_dispatch = ok if fused_dispatch is None else bool(fused_dispatch)
+        self.fused_dispatch = (ok and buf.R > 1) if fused_dispatch is None else bool(fused_dispatch)
         # set to a learning rate to run the SGD step of the expert weights inside the weight-grad
         # epilogues of the next backward pass (see ``fuse_sgd``)
         self.fused_sgd_lr: Optional[float] = None
