@@ -10,9 +10,8 @@
 // main loop through the second accumulator.  Kernels:
 //   ep_token_gemm_kernel (token_gemm.cuh): token-major products with bf16 output -- gate/up with
 //        SwiGLU, down, both dgrads, the pushed combine, the fused dispatch.
-//   ep_grouped_gemm_kernel (this file):
-//     token-major with fp32 output (router logits; 128 x 256 tiles, plain transposed stores)
-//     weight-grad (groups partition the REDUCTION dimension):
+//   ep_dense_f32_kernel (dense_f32.cuh): one product with fp32 output (router logits).
+//   ep_grouped_gemm_kernel (this file): weight-grad (groups partition the REDUCTION dimension):
 //        D[g] (+)= A[rows of g]^T * B[rows of g]   both operands MN-major, fp32 output by TMA
 //        store / reduce-add; or (template SGD) the optimizer step fused in: the accumulator is
 //        applied straight to the bf16 weights, w = bf16(w - lr * acc), through a per-warp TMA
@@ -113,9 +112,9 @@ struct Tile {
 
 // CLUSTER: the barrier also receives plain arrivals from the pair's other CTA, so the wait
 // acquires at cluster scope.  Barriers completed by TMA byte counts or tcgen05.commit do not need it.
-template <bool CLUSTER = false>
+template <bool CLUSTER = false, class Params>
 __device__ __forceinline__ bool gemm_wait(uint64_t* bar, uint32_t parity, volatile int* s_abort,
-                                          const GemmKParams& p, int where) {
+                                          const Params& p, int where) {
   auto ready = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
   if (ready()) return true;
   unsigned long long t0 = globaltimer_ns();
@@ -174,53 +173,31 @@ __device__ __forceinline__ int group_valid(const GemmKParams& p, int g, int star
   return (n > 0 && first >= start && first < end) ? max(1, first - start) : end - start;
 }
 
-template <bool WGRAD, bool TWO = false>
+template <bool TWO>
 __device__ __forceinline__ Tile get_tile(const GemmKParams& p, int id, const int* s_end, const int* s_valid,
-                                         const int* s_prefix, int n_tiles_n, int crank = 0) {
+                                         int n_tiles_n, int crank = 0) {
   Tile t;
   t.valid = true;
-  if constexpr (WGRAD) {
-    constexpr int TMW = TWO ? 2 * BM : BM;       // a pair owns 256 rows of the weight matrix
-    const int mt = p.Mw / TMW;
-    const int tpg = mt * n_tiles_n;
-    t.g = id / tpg;
-    int local = id - t.g * tpg;
-    int ni = local / mt, mi = local - ni * mt;
-    t.row0 = t.g == 0 ? 0 : s_end[t.g - 1];
-    t.rows = s_valid[t.g];                       // padding rows are zero: blocks of nothing else are skipped
-    t.m0 = mi * TMW + crank * BM;
-    t.n0 = ni * BN;
-    t.num_kb = (t.rows + BK - 1) / BK;
-    if (t.rows <= 0 && t.g >= p.zero_empty_below) t.valid = false;
-    if (t.rows <= 0 && p.sgd_w != nullptr && t.g < p.split &&
-        (p.sgd_keep == nullptr || p.sgd_keep[t.g] == 0)) t.valid = false;   // zero grad: nothing to apply
-    if (t.g < p.g_begin) t.valid = false;
-  } else {
-    // largest g with prefix[g] * n_tiles_n <= id
-    int lo = 0, hi = p.ngroups - 1;
-    while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if ((long long)s_prefix[mid] * n_tiles_n <= id) lo = mid; else hi = mid - 1;
-    }
-    t.g = lo;
-    int start = t.g == 0 ? 0 : s_end[t.g - 1];
-    int len = s_end[t.g] - start;
-    int mt = max(1, (len + BM - 1) / BM);
-    int local = id - s_prefix[t.g] * n_tiles_n;
-    int ni = local / mt, mi = local - ni * mt;
-    t.row0 = start + mi * BM;
-    t.rows = max(0, min(BM, s_end[t.g] - t.row0));
-    t.m0 = 0;
-    t.n0 = ni * BN;
-    t.num_kb = p.nseg * ((p.K + BK - 1) / BK);
-  }
+  constexpr int TMW = TWO ? 2 * BM : BM;       // a pair owns 256 rows of the weight matrix
+  const int mt = p.Mw / TMW;
+  const int tpg = mt * n_tiles_n;
+  t.g = id / tpg;
+  int local = id - t.g * tpg;
+  int mi = local / n_tiles_n, ni = local - mi * n_tiles_n;
+  t.row0 = t.g == 0 ? 0 : s_end[t.g - 1];
+  t.rows = s_valid[t.g];                       // padding rows are zero: blocks of nothing else are skipped
+  t.m0 = mi * TMW + crank * BM;
+  t.n0 = ni * BN;
+  t.num_kb = (t.rows + BK - 1) / BK;
+  if (t.rows <= 0 && t.g >= p.zero_empty_below) t.valid = false;
+  if (t.rows <= 0 && p.sgd_w != nullptr && t.g < p.split &&
+      (p.sgd_keep == nullptr || p.sgd_keep[t.g] == 0)) t.valid = false;   // zero grad: nothing to apply
+  if (t.g < p.g_begin) t.valid = false;
   t.alloc = t.g >= p.split ? 1 : 0;
   t.g_local = t.alloc ? t.g - p.split : t.g;
-  if constexpr (WGRAD) {
-    if (p.wg_select != 0 && p.sgd_w != nullptr) {
-      const bool applied = t.alloc == 0 && (p.sgd_keep == nullptr || p.sgd_keep[t.g_local] == 0);
-      if ((p.wg_select == 2) != applied) t.valid = false;
-    }
+  if (p.wg_select != 0 && p.sgd_w != nullptr) {
+    const bool applied = t.alloc == 0 && (p.sgd_keep == nullptr || p.sgd_keep[t.g_local] == 0);
+    if ((p.wg_select == 2) != applied) t.valid = false;
   }
   return t;
 }
@@ -235,12 +212,9 @@ template <bool TWO> __host__ __device__ constexpr int gemm_smem() {   // dynamic
   return gemm_stages<TWO>() * (TWO ? STAGE_BYTES2 : STAGE_BYTES) + 1024;
 }
 
-// WGRAD: the weight grads.  Otherwise the token-major kernel with fp32 output (router logits), tokens on
-// the M side; the other token-major products are in token_gemm.cuh.
-template <bool WGRAD, bool A_MN, bool B_MN, bool TWO = false, bool SGD = false>
+template <bool TWO, bool SGD>
 __global__ void __launch_bounds__(SGD ? GEMM_THREADS_SGD : GEMM_THREADS, 1)
 ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
-  static_assert(WGRAD || (!TWO && !SGD), "pairs and the fused SGD step belong to the weight grad");
   // operand stages: a constant, except in the SGD kernels (upper bound; p.stages are used)
   constexpr int GEMM_STAGES = gemm_stages<TWO>();
   const int nst = SGD ? p.stages : GEMM_STAGES;
@@ -258,11 +232,8 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   __shared__ int s_end[MAX_GROUPS];
-  __shared__ int s_valid[WGRAD ? MAX_GROUPS : 1];
-  __shared__ int s_prefix[WGRAD ? 1 : MAX_GROUPS + 1];
-  // per-warp staging of the fp32 epilogues: 32 x 33 floats token-major, a 4 KB swizzled block for
-  // the weight grad
-  __shared__ __align__(1024) float s_epi[4 * 32 * 33];
+  __shared__ int s_valid[MAX_GROUPS];
+  __shared__ __align__(1024) float s_epi[4 * 32 * 32];      // per-warp staging of stored tiles: a swizzled 4 KB block
   // fused SGD: per epilogue warp a ring of WB 32 x 32 bf16 weight blocks (in dynamic shared
   // memory, behind the operand stages) and their "landed" barriers
   __shared__ __align__(8) uint64_t wbar[SGD ? 8 : 4][WB_MAX];
@@ -284,29 +255,8 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
   for (int g = tid; g < p.ngroups; g += (int)blockDim.x)
     s_end[g] = p.cu_seqlens != nullptr ? p.cu_seqlens[g] : p.total_rows;
   __syncthreads();
-  if constexpr (WGRAD) {
-    for (int g = tid; g < p.ngroups; g += (int)blockDim.x)
-      s_valid[g] = group_valid(p, g, g == 0 ? 0 : s_end[g - 1], s_end[g]);
-  }
-  if (!WGRAD && warp == 0) {
-    // exclusive prefix of M tiles per group (token-major); cheap serial-by-chunks scan
-    int run = 0;
-    for (int g0 = 0; g0 < p.ngroups; g0 += 32) {
-      int g = g0 + lane;
-      int len = 0;
-      if (g < p.ngroups) len = s_end[g] - (g == 0 ? 0 : s_end[g - 1]);
-      int mt = (len > 0 && g >= p.g_begin) ? (len + BM - 1) / BM : 0;
-      int incl = mt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      if (g < p.ngroups) s_prefix[g] = run + incl - mt;
-      run += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) s_prefix[p.ngroups] = run;
-  }
+  for (int g = tid; g < p.ngroups; g += (int)blockDim.x)
+    s_valid[g] = group_valid(p, g, g == 0 ? 0 : s_end[g - 1], s_end[g]);
   if (warp == 1) {
     if constexpr (TWO) { tmem_alloc2(&s_tmem, 512); tmem_relinquish2(); }
     else { tmem_alloc(&s_tmem, 512); tmem_relinquish(); }
@@ -318,9 +268,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
   const uint32_t tmem_base = s_tmem;
 
   const int n_tiles_n = (p.N + BN - 1) / BN;
-  long long total_tiles;
-  if constexpr (WGRAD) total_tiles = (long long)p.ngroups * (p.Mw / (TWO ? 2 * BM : BM)) * n_tiles_n;
-  else total_tiles = (long long)s_prefix[p.ngroups] * n_tiles_n;
+  const long long total_tiles = (long long)p.ngroups * (p.Mw / (TWO ? 2 * BM : BM)) * n_tiles_n;
 
   if (warp == 0) {
     // ================= TMA producer =================
@@ -330,9 +278,8 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
       int it = 0;
       bool ok = true;
       for (long long id = work_id0; id < total_tiles && ok; id += work_stride) {
-        Tile t = get_tile<WGRAD, TWO>(p, (int)id, s_end, s_valid, s_prefix, n_tiles_n, crank);
+        Tile t = get_tile<TWO>(p, (int)id, s_end, s_valid, n_tiles_n, crank);
         if (!t.valid) continue;
-        const int kb_per_seg = WGRAD ? t.num_kb : (p.K + BK - 1) / BK;
         for (int kb = 0; kb < t.num_kb; ++kb, ++it) {
           const int s = it % nst;
           if (it >= nst &&
@@ -346,9 +293,8 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
           if constexpr (TWO) lead_bar = mapa_u32(&full[s], 0);
           // the peer's bytes may land before this arrival: the pending count keeps the phase open
           if (crank == 0) mbar_expect_tx(&full[s], TWO ? 2 * STAGE_BYTES : STAGE_BYTES);
-          const int seg = kb / kb_per_seg;
-          const int k0 = (kb - seg * kb_per_seg) * BK;
-          if constexpr (WGRAD && TWO) {
+          const int k0 = kb * BK;
+          if constexpr (TWO) {
             // this CTA's 128 columns of A (t.m0 is already its half) and its half of the B tile
 #pragma unroll
             for (int j = 0; j < 2; ++j)
@@ -356,7 +302,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
 #pragma unroll
             for (int j = 0; j < 2; ++j)
               tma_load_2d_pair(sb + j * 8192, &p.b[0][0], t.n0 + 128 * crank + 64 * j, t.row0 + k0, lead_bar);
-          } else if constexpr (WGRAD) {
+          } else {
             // A: [token rows][Mw cols], two 64-column blocks; B: [token rows][N cols], four
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
@@ -364,16 +310,6 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
               tma_load_2d(sb + j * 8192, &p.b[0][0], t.n0 + 64 * j, t.row0 + k0, &full[s]);
-          } else {
-            tma_load_2d(sa, &p.a[seg], k0, t.row0, &full[s]);
-            const int erow = t.g_local * p.rows_per_expert;
-            if constexpr (B_MN) {
-#pragma unroll
-              for (int j = 0; j < BN / 64; ++j)
-                tma_load_2d(sb + j * 8192, &p.b[seg][t.alloc], t.n0 + 64 * j, erow + k0, &full[s]);
-            } else {
-              tma_load_2d(sb, &p.b[seg][t.alloc], k0, erow + t.n0, &full[s]);
-            }
           }
         }
       }
@@ -383,11 +319,11 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
     if (lane == 0 && TWO && crank != 0) {
       // peer CTA of a pair: the leader issues the MMAs for both
     } else if (lane == 0) {
-      constexpr uint32_t idesc = make_instr_desc_bf16(TWO ? 2 * BM : BM, BN, A_MN, B_MN);
+      constexpr uint32_t idesc = make_instr_desc_bf16(TWO ? 2 * BM : BM, BN, true, true);
       int it = 0, tile_n = 0;
       bool ok = true;
       for (long long id = work_id0; id < total_tiles && ok; id += work_stride) {
-        Tile t = get_tile<WGRAD, TWO>(p, (int)id, s_end, s_valid, s_prefix, n_tiles_n, crank);
+        Tile t = get_tile<TWO>(p, (int)id, s_end, s_valid, n_tiles_n, crank);
         if (!t.valid) continue;
         const int acc = tile_n & 1;
         if (tile_n >= 2 &&
@@ -402,10 +338,8 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
           const uint32_t sb = sa + A_TILE_BYTES;
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = A_MN ? make_smem_desc(sa + kk * 2048, 8192, 1024)
-                                     : make_smem_desc(sa + kk * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc(sb + kk * 2048, 8192, 1024)
-                                     : make_smem_desc(sb + kk * 32, 16, 1024);
+            const uint64_t da = make_smem_desc(sa + kk * 2048, 8192, 1024);
+            const uint64_t db = make_smem_desc(sb + kk * 2048, 8192, 1024);
             if constexpr (TWO) umma_bf16_2cta(tacc, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
             else umma_bf16(tacc, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
           }
@@ -446,7 +380,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
     auto cursor_settle = [&]() {           // move to the next existing block at or after (lid, lc)
       while (lid < total_tiles) {
         if (!l_have) {
-          const Tile u = get_tile<WGRAD, TWO>(p, (int)lid, s_end, s_valid, s_prefix, n_tiles_n, crank);
+          const Tile u = get_tile<TWO>(p, (int)lid, s_end, s_valid, n_tiles_n, crank);
           if (sgd_tile(u)) { l_have = true; l_y0 = u.g_local * p.Mw + u.m0 + q * 32; l_n0 = u.n0; lc = 0; }
         }
         if (l_have && lc < CB && l_n0 + cofs + lc * WCOLS < p.N) return;
@@ -471,7 +405,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
       issue_loads();
     }
     for (long long id = work_id0; id < total_tiles; id += work_stride) {
-      Tile t = get_tile<WGRAD, TWO>(p, (int)id, s_end, s_valid, s_prefix, n_tiles_n, crank);
+      Tile t = get_tile<TWO>(p, (int)id, s_end, s_valid, n_tiles_n, crank);
       if (!t.valid) continue;
       const int acc = tile_n & 1;
       bool sgd_fuse = false;
@@ -481,8 +415,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
       const uint32_t tacc = tmem_base + (uint32_t)acc * BN + ((uint32_t)(q * 32) << 16);
       const bool have_acc = t.num_kb > 0;
       {
-        const int col_base = t.n0;
-        if constexpr (WGRAD) {
+          const int col_base = t.n0;
           // fp32 weight-grad tiles are 128 KB each and the main loop is short (one group's
           // tokens), so the epilogue must move ~30 GB/s per SM.  Four warps of plain stores
           // cannot (measured: ~14 B/clk/SM), so each warp stages 32x32 blocks in shared memory
@@ -563,42 +496,6 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
               bulk_commit();
             }
           }
-        } else {
-          // token-major fp32 output (router logits): rows of a tile may belong to the next
-          // group, so stores stay row-masked; each warp transposes through a padded pad so
-          // that every store instruction writes one full 128-byte line.
-          float* pad = s_epi + q * (32 * 33);
-          const long long row_stride = p.ldc;
-          const long long off_warp = ((long long)t.row0 + q * 32) * p.ldc;
-          const int rows_ok = min(32, t.rows - q * 32);
-#pragma unroll 1
-          for (int c = 0; c < BN / 32; ++c) {
-            uint32_t r[32];
-            if (have_acc) {
-              tmem_ld_32x32(tacc + c * 32, r);
-              tmem_ld_wait();
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = 0u;
-            }
-            const int col = col_base + c * 32 + lane;
-#pragma unroll
-            for (int i = 0; i < 32; ++i) pad[lane * 33 + i] = __uint_as_float(r[i]);
-            __syncwarp();
-            if (col < p.N) {
-              float* o = (float*)p.out[0] + off_warp + col;
-#pragma unroll 8
-              for (int rr = 0; rr < 32; ++rr) {
-                if (rr < rows_ok) {
-                  float v = pad[rr * 33 + lane];
-                  if (p.accumulate) v += o[rr * row_stride];
-                  o[rr * row_stride] = v;
-                }
-              }
-            }
-            __syncwarp();
-          }
-        }
       }
       tc_fence_before();
       __syncwarp();
@@ -627,6 +524,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
 
 }  // namespace mep
 
+#include "device/dense_f32.cuh"
 #include "device/token_gemm.cuh"
 
 namespace mep {
@@ -813,8 +711,8 @@ static int launch_single(const void* kern, std::atomic<unsigned long long>& rais
 
 template <bool SGD>
 static int launch_wgrad(const GemmKParams& kp, bool pair, int grid, cudaStream_t stream) {
-  const void* kern = pair ? (const void*)ep_grouped_gemm_kernel<true, true, true, true, SGD>
-                          : (const void*)ep_grouped_gemm_kernel<true, true, true, false, SGD>;
+  const void* kern = pair ? (const void*)ep_grouped_gemm_kernel<true, SGD>
+                          : (const void*)ep_grouped_gemm_kernel<false, SGD>;
   const int smem = SGD ? sgd_smem(kp, pair) : (pair ? gemm_smem<true>() : gemm_smem<false>());
   if (SGD && smem > sgd_smem_limit(kern))
     return fail(-3, "gemm: %d operand stages + %d weight blocks do not fit in shared memory", kp.stages, kp.wb);
@@ -827,11 +725,37 @@ static int launch_wgrad(const GemmKParams& kp, bool pair, int grid, cudaStream_t
   return launch_single(kern, raised, kp, grid, threads, smem, false, stream);
 }
 
+// CTAs that share one tile's reduction: as many as the SMs allow beside the other tiles, at most
+// eight (a portable cluster), with at least four k-blocks each.
+static int dense_parts(int tiles, int num_kb, int ctas) {
+  int parts = 1;
+  while (parts < 8 && tiles * parts * 2 <= ctas && num_kb >= parts * 2 * 4) parts *= 2;
+  return parts;
+}
 template <bool B_MN>
-static int launch_dense_f32(const GemmKParams& kp, int grid, cudaStream_t stream) {
+static int launch_dense_f32(const DenseParams& dp, int ctas, cudaStream_t stream) {
+  const void* kern = (const void*)ep_dense_f32_kernel<B_MN>;
   static std::atomic<unsigned long long> raised{0};
-  return launch_single((const void*)ep_grouped_gemm_kernel<false, false, B_MN>, raised, kp, grid, GEMM_THREADS,
-                       gemm_smem<false>(), false, stream);
+  MEP_CUDA_OK(raise_smem_limit(kern, raised));
+  const int mt = (dp.S + BM - 1) / BM, nt = (dp.N + dp.tile_n - 1) / dp.tile_n;
+  const int parts = dense_parts(mt * nt, dp.num_kb, ctas);
+  const int stage = A_TILE_BYTES + (dp.tile_n + 63) / 64 * 8192;
+  const int partial = BM * (((dp.tile_n + 15) & ~15) + 4) * 4;
+  const int ring = dp.stages * stage;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)parts, (unsigned)mt, (unsigned)nt);
+  cfg.blockDim = dim3(DN_THREADS);
+  cfg.dynamicSmemBytes = (size_t)((ring > partial ? ring : partial) + 1024);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)parts; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* args[] = {(void*)&dp};
+  MEP_CUDA_OK(cudaLaunchKernelExC(&cfg, kern, args));
+  return 0;
 }
 
 template <bool A_MN, int EPI, bool DISP>
@@ -911,19 +835,37 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
       return launch_wgrad<true>(kp, pair, grid, stream);
     return launch_wgrad<false>(kp, pair, grid, stream);
   }
+  if (d->epi == EPI_F32) {
+    // router logits: one group, one segment
+    if (d->ngroups != 1 || d->cu_seqlens != nullptr || d->nseg != 1 || d->accumulate)
+      return fail(-15, "gemm: fp32 output is one dense product");
+    if (d->K % 8 != 0) return fail(-4, "gemm: K=%d must be a multiple of 8", d->K);
+    DenseParams dp;
+    std::memset(&dp, 0, sizeof(dp));
+    dp.out = (float*)d->out[0]; dp.ldc = d->ldc; dp.S = d->total_rows; dp.N = d->N;
+    dp.num_kb = (d->K + BK - 1) / BK;
+    dp.tile_n = d->N < 256 ? d->N : 256;
+    const int stage = A_TILE_BYTES + (dp.tile_n + 63) / 64 * 8192;
+    dp.stages = DN_RING / stage < DN_MAX_STAGES ? DN_RING / stage : DN_MAX_STAGES;
+    dp.status = kp.status; dp.timeout_ns = kp.timeout_ns;
+    if (dp.S < 1) return 0;
+    if (dp.S > 65535 * BM) return fail(-16, "gemm: %d rows are too many for the dense product", dp.S);
+    if ((rc = make_map(&dp.a, d->a[0], d->a_rows, d->K, d->lda[0], BK, BM))) return rc;
+    if (d->b_mn) {
+      if ((rc = make_map(&dp.b, d->b[0][0], d->b_rows[0], d->N, d->ldb, 64, BK))) return rc;
+      return launch_dense_f32<true>(dp, grid, stream);
+    }
+    if ((rc = make_map(&dp.b, d->b[0][0], d->b_rows[0], d->K, d->ldb, BK, 64))) return rc;
+    return launch_dense_f32<false>(dp, grid, stream);
+  }
   // A reduction tail is legal: the TMA loads zero-fill A beyond K, which also cancels whatever
   // a MN-major B tile picks up from the next expert's rows.
   if (d->K % 8 != 0) return fail(-4, "gemm: K=%d must be a multiple of 8", d->K);
   if (d->nseg < 1 || d->nseg > 2) return fail(-5, "gemm: nseg=%d", d->nseg);
   for (int s = 0; s < d->nseg; ++s) {
-    if (d->epi == EPI_F32) {
-      if ((rc = make_map(&kp.a[s], d->a[s], d->a_rows, d->K, d->lda[s], BK, BM))) return rc;
-      continue;
-    }
     for (int b = 0; b < TG_BOXES; ++b)
       if ((rc = make_map(&kp.tok[s][b], d->a[s], d->a_rows, d->K, d->lda[s], BK, 32 * (b + 1)))) return rc;
   }
-  if (d->nseg == 1) kp.a[1] = kp.a[0];
   const int nsel = (d->epi == EPI_SWIGLU) ? 2 : d->nseg;
   for (int s = 0; s < 2; ++s)
     for (int al = 0; al < 2; ++al) {
@@ -933,13 +875,12 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
         if ((rc = make_map(&kp.b[s][al], base, rows, d->N, d->ldb, 64, BK))) return rc;
         kp.b2[s][al] = kp.b[s][al];
       } else {         // [N rows][K cols] per expert
-        if (d->epi == EPI_F32 && (rc = make_map(&kp.b[s][al], base, rows, d->K, d->ldb, BK, BN))) return rc;
         if ((rc = make_map(&kp.b2[s][al], base, rows, d->K, d->ldb, BK, BN / 2))) return rc;
       }
     }
   kp.tma_out = d->ldc % 8 == 0 && (((uintptr_t)d->out[0] | (uintptr_t)d->out[1] | (uintptr_t)d->out[2] |
                                     (uintptr_t)d->push_base) & 15) == 0 && d->push_rank_stride % 8 == 0;
-  const bool two = d->two_cta != 0 && grid >= 2;     // (fp32 output: single CTAs)
+  const bool two = d->two_cta != 0 && grid >= 2;
   if (d->disp_mode != 0) {
     // ---- fused dispatch: the A operand is a row buffer of the Buffer behind disp_ctx ----------
     if (d->disp_ctx == nullptr) return fail(-20, "gemm: the fused dispatch needs the Buffer's context");
@@ -985,8 +926,6 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
   if (d->epi == EPI_BF16)
     return d->b_mn ? launch_token<true, EPI_BF16, false>(kp, two, grid, stream)
                    : launch_token<false, EPI_BF16, false>(kp, two, grid, stream);
-  if (d->epi == EPI_F32)
-    return d->b_mn ? launch_dense_f32<true>(kp, grid, stream) : launch_dense_f32<false>(kp, grid, stream);
   if (d->epi == EPI_PUSH) {
     if (d->src_info == nullptr || d->push_base == nullptr || d->push_entries <= 0)
       return fail(-9, "gemm: the push epilogue needs src_info and a staging buffer");

@@ -1,0 +1,25 @@
+"""Dense product with fp32 output (router logits): tiles whose reduction a cluster shares, ragged rows,
+columns and reduction lengths, both layouts of the weights, against fp64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# rows around a tile and many tiles (one CTA a tile), reductions of one k-block (with a tail) up to 112 (eight CTAs
+# share them), columns around a 64-column block, one tile of 256 and more than one
+@pytest.mark.parametrize("S,K,N", [(1, 64, 8), (16, 7168, 32), (127, 520, 64), (128, 256, 72), (129, 2048, 128),
+                                   (300, 8, 200), (1531, 1024, 256), (40, 4096, 264), (4096, 512, 1000), (20000, 64, 16)])
+def test_dense_matches_fp64(S, K, N):
+    from moonep_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(S + K + N)
+    a = torch.randn(S, K, device="cuda", generator=g).bfloat16()
+    b = torch.randn(K, N, device="cuda", generator=g).bfloat16()
+    want = a.double() @ b.double()
+    # fp32 sums of K exact products: K/2 roundings of at most 2^-24 of the partial sum's size, sqrt(K) here
+    bound = 2.0 ** -24 * K * (a.double().abs() @ b.double().abs()) / K ** 0.5 + 1e-30
+    for got in (gemm.dense(a, b), gemm.dense(a, b.t().contiguous(), b_is_kn=False)):
+        assert got.dtype == torch.float32 and got.shape == (S, N)
+        assert bool(((got.double() - want).abs() <= bound).all())
+        assert torch.equal(got, gemm.dense(a, b)), "the order of the sums is fixed"
+    gemm.check_status()
