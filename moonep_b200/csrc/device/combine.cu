@@ -223,7 +223,9 @@ struct CombineParams {
 };
 
 constexpr int COMBINE_ACC_THREADS = ACC_THREADS;
-constexpr int COMBINE_THREADS = 32 + COMBINE_ACC_THREADS + 32;  // loader, accumulator warps, weights
+// loader, accumulator warps (two sets within one device), weights
+constexpr int combine_sets(bool direct, int nv) { return direct && nv <= 4 ? 2 : 1; }   // (registers)
+constexpr int combine_threads(bool direct, int nv) { return 32 + combine_sets(direct, nv) * COMBINE_ACC_THREADS + 32; }
 
 // What the accumulators do with a staged row.
 enum : int { ROW_STARTS_GROUP = 1, ROW_ENDS_GROUP = 2, ROW_ENDS_TOKEN = 4 };
@@ -246,9 +248,13 @@ __device__ __forceinline__ void fold_group(unsigned long long (&tot)[NV][4], con
 // in the order of the primaries' k, and the accumulators sum a group in registers, round it to
 // bf16 once and add it to the token's sum: the same additions and roundings, in the same order, as
 // pre-reduction + pull, without the pass that reads every duplicate group and writes its primary back,
-// and without the barriers, since launches of one stream already order the rows.
+// and without the barriers, since launches of one stream already order the rows.  Two sets of
+// accumulator warps take the tokens in turn: a row costs a set ~0.3 us of latencies (landed, read,
+// added, stage released) however short it is, which with one set was the kernel (4096 tokens x
+// 7168, top-8, 96 CTAs: 146 us, with two sets 117; eight ranks in 144 CTAs 760 -> 631, of 636 at the copy rate).
 template <int ST, int NV, bool DIRECT>
-__global__ void __launch_bounds__(COMBINE_THREADS, 1) ep_combine_kernel(const CombineParams p) {
+__global__ void __launch_bounds__(combine_threads(DIRECT, NV), 1) ep_combine_kernel(const CombineParams p) {
+  constexpr int SETS = combine_sets(DIRECT, NV);
   extern __shared__ __align__(128) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full[ST];
   __shared__ __align__(8) uint64_t empty[ST];
@@ -262,7 +268,7 @@ __global__ void __launch_bounds__(COMBINE_THREADS, 1) ep_combine_kernel(const Co
   uint8_t* ring = smem_raw;
 
   if (tid == 0) {
-    for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], COMBINE_ACC_THREADS / 32); }
+    for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], SETS * ACC_WARPS); }
     mbar_fence_init();
   }
   __syncthreads();
@@ -336,12 +342,24 @@ __global__ void __launch_bounds__(COMBINE_THREADS, 1) ep_combine_kernel(const Co
         ++prod;
       }
     }
-  } else if (warp <= COMBINE_ACC_THREADS / 32) {
+  } else if (warp <= SETS * ACC_WARPS) {
     // ---- accumulators ----------------------------------------------------------------------
-    const int ta = tid - 32;
+    const int set = SETS == 1 ? 0 : (warp - 1) / ACC_WARPS;
+    const int ta = tid - 32 - set * COMBINE_ACC_THREADS;
     __nv_bfloat16* out = p.out + (size_t)vr * p.S * p.H;
     int cons = 0;
     for (int j = 0; j < n_tok; ++j) {
+      if (SETS > 1 && (j & 1) != set) {
+        // The other set's token: every row is waited for and released by both sets.  A barrier's parity
+        // names a phase only to a thread that has seen the phase before it and none after, so a set
+        // may neither run ahead of rows that it has not seen nor be overtaken by a stage's next row.
+        for (int i = 0; i < p.K; ++i, ++cons) {
+          mbar_wait(sc, &full[cons % ST], (uint32_t)(cons / ST) & 1u, 30);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&empty[cons % ST]);
+        }
+        continue;
+      }
       unsigned long long acc[NV][4];
       [[maybe_unused]] unsigned long long grp[DIRECT ? NV : 1][4];
       bool first = true;
@@ -486,7 +504,7 @@ static int launch_combine_t(const BufferCtx& c, CombineParams& p, size_t smem, c
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_combine_kernel<ST, NV, DIRECT>, raised));
   dim3 grid(c.num_sms, c.Rv());
   // (DIRECT follows no kernel of its own chain and has no barrier inside)
-  MEP_CUDA_OK(launch_chained((const void*)ep_combine_kernel<ST, NV, DIRECT>, grid, dim3(COMBINE_THREADS), smem,
+  MEP_CUDA_OK(launch_chained((const void*)ep_combine_kernel<ST, NV, DIRECT>, grid, dim3(combine_threads(DIRECT, NV)), smem,
                              stream, p, /*coop=*/!DIRECT, c.pdl && !DIRECT));
   return 0;
 }
@@ -495,6 +513,8 @@ template <int NV, bool DIRECT>
 static int launch_combine_nv(const BufferCtx& c, CombineParams& p, cudaStream_t stream) {
   const size_t row = (size_t)c.H * 2;
   const size_t budget = c.ring_budget(210 * 1024);
+  // short rows: as many in flight as two tokens and more have
+  if (DIRECT && 28 * row <= budget) return launch_combine_t<DIRECT ? 28 : 14, NV, DIRECT>(c, p, 28 * row, stream);
   if (14 * row <= budget) return launch_combine_t<14, NV, DIRECT>(c, p, 14 * row, stream);
   if (10 * row <= budget) return launch_combine_t<10, NV, DIRECT>(c, p, 10 * row, stream);
   if (6 * row <= budget) return launch_combine_t<6, NV, DIRECT>(c, p, 6 * row, stream);
