@@ -11,6 +11,8 @@ import ctypes
 import os
 import threading
 
+import torch
+
 from . import _build
 
 _lock = threading.Lock()
@@ -57,7 +59,7 @@ def lib() -> ctypes.CDLL:
 # Number of native calls that launch at least one of this library's kernels (benchmarks read and
 # reset it to report how many launches a step takes).
 LAUNCHES = 0
-_LAUNCH_PREFIXES = ("mep_launch_", "mep_gemm_launch", "mep_router_", "mep_swiglu_", "mep_sgd_")
+_LAUNCH_PREFIXES = ("mep_launch_", "mep_gemm_launch", "mep_router_", "mep_swiglu_", "mep_sgd_", "mep_ce_")
 
 
 def call(name: str, *args):
@@ -78,6 +80,12 @@ def call(name: str, *args):
 def ptr(t) -> int:
     """``data_ptr`` of a tensor, or 0 for ``None``."""
     return 0 if t is None else t.data_ptr()
+
+
+def stream() -> int:
+    """Handle of the current device's current stream.  (``torch.cuda.current_stream()`` builds a Stream
+    object around it, ~5 us a call, which at 20 launches was an eighth of a small step's time.)"""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def last_error() -> str:

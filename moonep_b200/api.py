@@ -315,7 +315,7 @@ class Buffer:
 
     @staticmethod
     def _stream() -> int:
-        return torch.cuda.current_stream().cuda_stream
+        return nat.stream()
 
     def inter_rank_sync(self) -> None:
         """Device-side cross-rank barrier on the current stream (moonep/inter_rank_sync.py:119)."""

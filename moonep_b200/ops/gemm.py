@@ -111,7 +111,7 @@ def _launch(d: _GemmDesc) -> None:
     if not _checked_layout:
         assert nat.call("mep_gemm_desc_bytes") == ctypes.sizeof(_GemmDesc), "GemmDesc layout mismatch"
         _checked_layout = True
-    rc = nat.call("mep_gemm_launch", ctypes.byref(d), torch.cuda.current_stream().cuda_stream)
+    rc = nat.call("mep_gemm_launch", ctypes.byref(d), nat.stream())
     if rc != 0:
         raise RuntimeError(f"grouped GEMM launch failed: {nat.last_error()} (code {rc})")
 
