@@ -1,11 +1,12 @@
 // Memory-bound MoE ops that have no counterpart in the reference (it is a pure communication
 // library): router top-k + softmax + tokens-per-expert histogram and its backward, the SwiGLU
-// backward (the forward is fused into the gate/up GEMM epilogue), and the fused SGD update of
-// bf16 weights from fp32 grads.  All are bandwidth kernels: 16-byte vector accesses, one pass.
+// backward (the forward is fused into the gate/up GEMM epilogue), the decoder's cross-entropy, and the
+// fused SGD update of bf16 weights from fp32 grads.  All are bandwidth kernels: 16-byte vector accesses, one pass.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <cmath>
 #include <cstdint>
 
 #include "host/ctx.h"
@@ -177,6 +178,125 @@ ep_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bfloat16
   }
 }
 
+// ---- cross-entropy over bf16 logits ---------------------------------------------------------------
+// Forward: one block a row, one pass: every thread keeps a running maximum and the sum of exp(x - max)
+// (fp32; rescaled when the maximum grows), the block combines them into the row's log-sum-exp.
+// Backward: one pass, d logits = (exp(x - lse) - [x is the target]) * g / rows, rounded to bf16 once.
+// The logits are read once each way and nothing of their size is written but the gradient; as
+// cross_entropy(logits.float()) the same took an fp32 copy, two more fp32 tensors of their size and a
+// copy back.  Bound by HBM: 4096 x 32000 logits are 262 MB, 39 us a pass at the copy rate.
+constexpr int CE_THREADS = 512;
+
+__device__ __forceinline__ void ce_add(float& m, float& s, float x) {
+  if (x > m) { s = s * expf(m - x) + 1.f; m = x; }        // (m = -inf: s is 0 and exp(-inf) is 0)
+  else if (!(x == -INFINITY && m == -INFINITY)) s += expf(x - m);
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(CE_THREADS)
+ep_ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets, long long ignore,
+                 int V, float* __restrict__ lse, float* __restrict__ loss) {
+  __shared__ float sm[CE_THREADS / 32], ss[CE_THREADS / 32];
+  const long long r = blockIdx.x;
+  const __nv_bfloat16* row = logits + r * V;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float m = -INFINITY, s = 0.f;
+  if constexpr (VEC) {
+    const uint4* row4 = reinterpret_cast<const uint4*>(row);
+    for (int v = threadIdx.x; v < V / 8; v += CE_THREADS) {
+      const uint4 q = row4[v];
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+      float x[8], top = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); x[2 * i] = f.x; x[2 * i + 1] = f.y; }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) top = fmaxf(top, x[i]);
+      if (top > m) { s *= expf(m - top); m = top; }
+      if (m != -INFINITY) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s += expf(x[i] - m);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) if (x[i] != x[i]) s = x[i];      // a NaN among nothing but -inf
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < V; i += CE_THREADS) ce_add(m, s, __bfloat162float(row[i]));
+  }
+  auto join = [](float& m1, float& s1, float m2, float s2) {
+    const float top = fmaxf(m1, m2);
+    s1 = (s1 != 0.f ? s1 * (m1 == top ? 1.f : expf(m1 - top)) : 0.f) + (s2 != 0.f ? s2 * (m2 == top ? 1.f : expf(m2 - top)) : 0.f);
+    m1 = top;
+  };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) join(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
+  if (lane == 0) { sm[warp] = m; ss[warp] = s; }
+  __syncthreads();
+  if (warp == 0) {
+    m = lane < CE_THREADS / 32 ? sm[lane] : -INFINITY;
+    s = lane < CE_THREADS / 32 ? ss[lane] : 0.f;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) join(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
+    if (lane == 0) {
+      const float l = m + logf(s);
+      const long long t = targets[r];
+      lse[r] = l;
+      // (a target that is no class has no loss to report)
+      loss[r] = t == ignore ? 0.f : (t >= 0 && t < V ? l - __bfloat162float(row[t]) : NAN);
+    }
+  }
+}
+
+// out[0] = mean loss of the rows that count, out[1] = their number; summed in a fixed order
+__global__ void __launch_bounds__(1024) ep_ce_mean_kernel(const float* __restrict__ loss, const long long* __restrict__ targets,
+                                                         long long ignore, int S, float* __restrict__ out) {
+  __shared__ double sl[32];
+  __shared__ int sn[32];
+  double l = 0.0;
+  int n = 0;
+  for (int r = threadIdx.x; r < S; r += 1024) {
+    l += loss[r];
+    n += targets[r] != ignore;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) { l += __shfl_xor_sync(0xffffffffu, l, o); n += __shfl_xor_sync(0xffffffffu, n, o); }
+  if ((threadIdx.x & 31) == 0) { sl[threadIdx.x >> 5] = l; sn[threadIdx.x >> 5] = n; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 32; ++i) { l += sl[i]; n += sn[i]; }
+    out[0] = (float)(l / n);             // (no row counts: 0 / 0, NaN)
+    out[1] = (float)n;
+  }
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(CE_THREADS)
+ep_ce_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets, long long ignore,
+                 int V, const float* __restrict__ lse, const float* __restrict__ mean_n, const float* __restrict__ g,
+                 __nv_bfloat16* __restrict__ grad) {
+  const long long r = blockIdx.x;
+  const __nv_bfloat16* row = logits + r * V;
+  __nv_bfloat16* out = grad + r * V;
+  const long long t = targets[r];
+  const bool counts = t != ignore;
+  const float l = lse[r], scale = counts ? g[0] / mean_n[1] : 0.f;
+  auto d = [&](float x, int i) { return counts ? (expf(x - l) - (i == t ? 1.f : 0.f)) * scale : 0.f; };
+  if constexpr (VEC) {
+    for (int v = threadIdx.x; v < V / 8; v += CE_THREADS) {
+      uint4 q = reinterpret_cast<const uint4*>(row)[v];
+      __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(h[i]);
+        h[i] = __floats2bfloat162_rn(d(f.x, 8 * v + 2 * i), d(f.y, 8 * v + 2 * i + 1));
+      }
+      reinterpret_cast<uint4*>(out)[v] = q;
+    }
+  } else {
+    for (int i = threadIdx.x; i < V; i += CE_THREADS) out[i] = __float2bfloat16(d(__bfloat162float(row[i]), i));
+  }
+}
+
 // ---- SGD: w(bf16) -= lr * g(fp32) ----------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 ep_sgd_kernel(__nv_bfloat16* __restrict__ w, const float* __restrict__ g, long long n, float lr,
@@ -254,6 +374,37 @@ int mep_swiglu_bwd(const void* dact, const void* gate, const void* up, const flo
   ep_swiglu_bwd_kernel<<<blocks, 256, 0, stream>>>(
       (const __nv_bfloat16*)dact, (const __nv_bfloat16*)gate, (const __nv_bfloat16*)up, row_scale,
       rows_ptr, max_rows, Hp, (__nv_bfloat16*)dgate, (__nv_bfloat16*)dup, dscale);
+  MEP_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// logits [S][V] bf16, targets [S] int64; lse, loss [S] and mean_n [2] (mean, rows that count) fp32.
+int mep_ce_fwd(const void* logits, const long long* targets, long long ignore, int S, int V, float* lse, float* loss,
+               float* mean_n, cudaStream_t stream) {
+  if (V < 1 || S < 0) return fail(-1, "cross entropy: %d x %d logits", S, V);
+  const __nv_bfloat16* x = (const __nv_bfloat16*)logits;
+  if (S > 0) {
+    if (V % 8 == 0 && (uintptr_t)logits % 16 == 0)
+      ep_ce_fwd_kernel<true><<<S, CE_THREADS, 0, stream>>>(x, targets, ignore, V, lse, loss);
+    else
+      ep_ce_fwd_kernel<false><<<S, CE_THREADS, 0, stream>>>(x, targets, ignore, V, lse, loss);
+  }
+  ep_ce_mean_kernel<<<1, 1024, 0, stream>>>(loss, targets, ignore, S, mean_n);
+  MEP_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// grad [S][V] bf16 of g[0] * mean loss
+int mep_ce_bwd(const void* logits, const long long* targets, long long ignore, int S, int V, const float* lse,
+               const float* mean_n, const float* g, void* grad, cudaStream_t stream) {
+  if (V < 1 || S < 0) return fail(-1, "cross entropy: %d x %d logits", S, V);
+  if (S == 0) return 0;
+  const __nv_bfloat16* x = (const __nv_bfloat16*)logits;
+  __nv_bfloat16* out = (__nv_bfloat16*)grad;
+  if (V % 8 == 0 && (((uintptr_t)logits | (uintptr_t)grad) % 16) == 0)
+    ep_ce_bwd_kernel<true><<<S, CE_THREADS, 0, stream>>>(x, targets, ignore, V, lse, mean_n, g, out);
+  else
+    ep_ce_bwd_kernel<false><<<S, CE_THREADS, 0, stream>>>(x, targets, ignore, V, lse, mean_n, g, out);
   MEP_CUDA_OK(cudaGetLastError());
   return 0;
 }

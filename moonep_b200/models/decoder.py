@@ -5,8 +5,8 @@ The reference contains no model (it is a communication library; its README only 
 normalised end-to-end figure from a harness that is not in the repository,
 figure/e2e_vs_deepep.png).  This stack exists so that the expert-parallel path can be timed inside
 a real training step against the conventional NCCL all-to-all path with no redundant experts.
-Attention, norms, embedding and the loss are ordinary PyTorch (they are not part of the MoE
-path); the MoE FFN is ``MoELayer`` (peer-memory dispatch/combine + tcgen05 grouped GEMM) or
+Attention, norms and embedding are ordinary PyTorch (they are not part of the MoE path), the loss is
+one kernel each way over the bf16 logits; the MoE FFN is ``MoELayer`` (peer-memory dispatch/combine + tcgen05 grouped GEMM) or
 ``NcclMoELayer`` (all_to_all_single + permute around the same GEMM kernels).
 
 Parallelism: EP for the experts; everything else is replicated, so dense gradients are averaged
@@ -177,7 +177,7 @@ class MoEDecoder(nn.Module):
         for b in self.blocks:
             x = b(x)
         logits = self.head(self.norm(x))
-        return F.cross_entropy(logits.float(), targets)
+        return ew.cross_entropy(logits, targets)
 
     def moe_layers(self):
         return [b.moe for b in self.blocks]

@@ -1,5 +1,5 @@
 """Wrappers of the bandwidth kernels in ``csrc/device/elementwise.cu`` (router top-k / softmax /
-histogram and its backward, SwiGLU backward, fused SGD).  None of these exist in the reference,
+histogram and its backward, SwiGLU backward, cross-entropy, fused SGD).  None of these exist in the reference,
 which stops at communication; they are the remaining hot ops of the MoE layer."""
 from __future__ import annotations
 
@@ -11,12 +11,14 @@ from .._native import F, I, L, P
 nat.declare("mep_router_topk", I, [P, P, I, I, I, P, P, P, P])
 nat.declare("mep_router_topk_bwd", I, [P, P, P, I, I, I, P, P])
 nat.declare("mep_swiglu_bwd", I, [P, P, P, P, P, I, I, P, P, P, P])
+nat.declare("mep_ce_fwd", I, [P, P, L, I, I, P, P, P, P])
+nat.declare("mep_ce_bwd", I, [P, P, L, I, I, P, P, P, P, P])
 nat.declare("mep_sgd_update", I, [P, P, L, F, P])
 nat.declare("mep_sgd_update_masked", I, [P, P, L, L, P, F, P])
 
 
 def _st():
-    return torch.cuda.current_stream().cuda_stream
+    return nat.stream()
 
 
 def _rc(rc, what):
@@ -75,3 +77,38 @@ def sgd_update_(w: torch.Tensor, g: torch.Tensor, lr: float, only: torch.Tensor 
     assert only.dtype == torch.int32 and only.is_cuda and only.numel() >= w.shape[0]
     _rc(nat.call("mep_sgd_update_masked", w.data_ptr(), g.data_ptr(), w.shape[0], w[0].numel(),
                  only.data_ptr(), float(lr), _st()), "sgd_update")
+
+
+class _CrossEntropy(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, logits, targets, ignore_index):
+        S, V = logits.shape
+        f32 = dict(dtype=torch.float32, device=logits.device)
+        lse, loss, mean_n = torch.empty(S, **f32), torch.empty(S, **f32), torch.empty(2, **f32)
+        _rc(nat.call("mep_ce_fwd", logits.data_ptr(), targets.data_ptr(), ignore_index, S, V, lse.data_ptr(),
+                     loss.data_ptr(), mean_n.data_ptr(), _st()), "cross_entropy")
+        ctx.ignore_index = ignore_index
+        ctx.save_for_backward(logits, targets, lse, mean_n)
+        return mean_n[0].clone()
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, g):
+        logits, targets, lse, mean_n = ctx.saved_tensors
+        S, V = logits.shape
+        grad = torch.empty_like(logits)
+        _rc(nat.call("mep_ce_bwd", logits.data_ptr(), targets.data_ptr(), ctx.ignore_index, S, V, lse.data_ptr(),
+                     mean_n.data_ptr(), g.contiguous().data_ptr(), grad.data_ptr(), _st()), "cross_entropy backward")
+        return grad, None, None
+
+
+def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int = -100) -> torch.Tensor:
+    """``F.cross_entropy(logits.float(), targets)`` (mean over the rows whose target is not
+    ``ignore_index``) for bf16 ``logits [S, V]`` and int64 ``targets [S]`` on the GPU, without the
+    fp32 copies; the gradient is rounded to bf16 once, as there.  Other forms of the arguments go
+    to ``F.cross_entropy``."""
+    if (logits.is_cuda and logits.dtype == torch.bfloat16 and logits.dim() == 2 and logits.is_contiguous()
+            and targets.device == logits.device and targets.dtype == torch.int64
+            and tuple(targets.shape) == (logits.shape[0],) and targets.is_contiguous()):
+        return _CrossEntropy.apply(logits, targets, ignore_index)
+    return torch.nn.functional.cross_entropy(logits.float(), targets, ignore_index=ignore_index)

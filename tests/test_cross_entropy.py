@@ -1,0 +1,53 @@
+"""Cross-entropy over bf16 logits against PyTorch's, in fp64."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+# one class, rows below and above a block's stride, vector and scalar rows (odd classes, odd start)
+@pytest.mark.parametrize("S,V,offset", [(1, 1, 0), (3, 8, 0), (5, 33, 0), (7, 4096, 0), (64, 4104, 0), (16, 32000, 0),
+                                        (9, 50257, 0), (4, 64, 3)])
+@pytest.mark.parametrize("ignored", [0, 2])
+def test_matches_fp64(S, V, offset, ignored):
+    from moonep_b200.ops import elementwise as ew
+    g = torch.Generator(device="cuda").manual_seed(S + V)
+    flat = (torch.randn(S * V + offset, device="cuda", generator=g) * 4).bfloat16()
+    logits = flat[offset:].view(S, V)
+    targets = torch.randint(0, V, (S,), device="cuda", generator=g)
+    if ignored:
+        targets[-1:] = -100
+    if V > 4:
+        logits[0, 1:4] = float("-inf")
+        targets[0] = 0
+    a = logits.detach().requires_grad_(True)
+    loss = ew.cross_entropy(a, targets)
+    (loss * 3.0).backward()
+    b = logits.detach().double().requires_grad_(True)
+    want = F.cross_entropy(b, targets)
+    (want * 3.0).backward()
+    assert loss.dtype == torch.float32
+    if S == 1 and ignored:
+        assert bool(torch.isnan(loss)) and bool(torch.isnan(want))
+        return
+    # fp32 sum of up to 5e4 terms: 1e-5; the gradient is bf16: half an ulp of 2^-8, and the exponential's 1e-5
+    assert abs(float(loss) - float(want)) <= 1e-5 * (1 + abs(float(want)))
+    assert bool(((a.grad.double() - b.grad).abs() <= b.grad.abs() * (2.0 ** -8) + 1e-7).all())
+
+
+def test_odd_values_and_other_forms():
+    from moonep_b200.ops import elementwise as ew
+    x = torch.randn(4, 48, device="cuda").bfloat16()
+    x[0] = float("-inf")
+    x[1, 5] = float("nan")
+    x[2, 7] = float("inf")
+    t = torch.tensor([1, 2, 3, 4], device="cuda")
+    for r in range(4):
+        got, want = ew.cross_entropy(x[r:r + 1].contiguous(), t[r:r + 1]), F.cross_entropy(x[r:r + 1].float(), t[r:r + 1])
+        assert bool(torch.isnan(got)) == bool(torch.isnan(want)) == (r < 3)
+    # fp32 logits, strided logits and class probabilities take the general path
+    y = torch.randn(4, 96, device="cuda").bfloat16()
+    p = torch.softmax(torch.randn(4, 96, device="cuda"), 1)
+    for a, b in ((y.float(), t), (y[:, ::2], t), (y, p)):
+        assert torch.equal(ew.cross_entropy(a, b), F.cross_entropy(a.float(), b))
