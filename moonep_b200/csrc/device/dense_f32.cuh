@@ -1,31 +1,32 @@
 // C[S][N] = A[S][K] * B[K][N] (or B[N][K]) with fp32 output: the router logits.
 //
-// The output is small (S x experts) and the reduction long, so 128-row tiles alone leave most SMs
-// idle: 4096 tokens are 32 CTAs walking 112 k-blocks one after the other (65 us at K = 7168), 16
-// tokens are one (47 us).  A cluster of up to eight CTAs therefore shares a tile: each takes a
-// contiguous part of the k-blocks, leaves its fp32 partial tile in its shared memory (over the spent
-// operand ring), and after a cluster barrier every CTA sums its share of the tile's rows over the
-// cluster's partials through distributed shared memory, in rank order, so the result does not depend
-// on timing.  Bound by reading A once (59 MB, 9 us at 4096 x 7168).
-// A stage holds 128 rows of A and only as many 64-column blocks of B as the tile has.
+// The output is small (S x experts) and the reduction long: a CTA walks up to 112 k-blocks one after
+// the other, ~0.4 us each, bound by that chain and not by bytes.  The experts take the M side (128 a
+// tile) and the tokens the N side, in as small a tile as fills the SMs once (4096 tokens are 128 CTAs
+// of 32), with up to sixteen stages in flight.  Against tokens on M (32 CTAs, 256-column tiles):
+// 4096 x 2048 -> 128 experts 23.4 -> 17.7 us, 509 x 1024 -> 32 12.6 -> 10.2; at K = 7168 the same
+// (48 us for 16 tokens).  The reduction is NOT split, which would take those 48 us to 10: routing compares
+// these sums, and another order of the additions sends tokens at a tie elsewhere.
 #pragma once
 
 namespace mep {
 
-constexpr int DN_MAX_STAGES = 8;
+constexpr int DN_MAX_STAGES = 16;
 constexpr int DN_THREADS = 192;
 constexpr int DN_RING = 200 * 1024;
+constexpr int DN_MAX_TOK = 128;
 
 struct DenseParams {
-  CUtensorMap a, b;      // A: 128 x 64 boxes; B: 64 x 64 boxes (either layout)
+  CUtensorMap x, w;      // tokens: tok x 64 boxes; weights: 64 x 64 (B [K][N]) or m_rows x 64 boxes (B [N][K])
   float* out;
   long long ldc;
-  int S, N, num_kb, tile_n, stages;
+  int S, N, num_kb, tok, m_rows, stages;
   int32_t* status;
   unsigned long long timeout_ns;
 };
+__host__ __device__ constexpr int dense_stage_bytes(int m_rows, int tok) { return (m_rows + tok) * BK * 2; }
 
-template <bool B_MN>
+template <bool W_MN>
 __global__ void __launch_bounds__(DN_THREADS, 1) ep_dense_f32_kernel(const __grid_constant__ DenseParams p) {
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t full[DN_MAX_STAGES];
@@ -34,14 +35,11 @@ __global__ void __launch_bounds__(DN_THREADS, 1) ep_dense_f32_kernel(const __gri
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int parts = (int)gridDim.x, part = (int)blockIdx.x;      // one cluster spans grid.x
   uint8_t* ring = (uint8_t*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   volatile int* abortp = &s_abort;
-  const int row0 = (int)blockIdx.y * BM, n0 = (int)blockIdx.z * p.tile_n;
-  const int n_here = min(p.tile_n, p.N - n0);
-  const int mma_n = (n_here + 15) & ~15, blocks = (n_here + 63) / 64;
-  const int stage_bytes = A_TILE_BYTES + (p.tile_n + 63) / 64 * 8192;
-  const int kb0 = (int)((long long)p.num_kb * part / parts), kb1 = (int)((long long)p.num_kb * (part + 1) / parts);
+  const int row0 = (int)blockIdx.x * p.tok, m0 = (int)blockIdx.y * BM;
+  // (with at most 64 experts only half of the M side is loaded; what the other lanes compute is not stored)
+  const int w_bytes = p.m_rows * BK * 2, stage_bytes = dense_stage_bytes(p.m_rows, p.tok);
 
   if (tid == 0) {
     for (int s = 0; s < p.stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -49,96 +47,76 @@ __global__ void __launch_bounds__(DN_THREADS, 1) ep_dense_f32_kernel(const __gri
     mbar_fence_init();
     s_abort = 0;
   }
-  if (warp == 1) { tmem_alloc(&s_tmem, 256); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(&s_tmem, DN_MAX_TOK); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = s_tmem;
 
-  if (warp == 0 && lane == 0) {
-    for (int kb = kb0; kb < kb1; ++kb) {
-      const int it = kb - kb0, s = it % p.stages;
-      if (it >= p.stages && !gemm_wait(&empty[s], ((uint32_t)(it / p.stages) & 1u) ^ 1u, abortp, p, 1)) break;
-      uint8_t* sa = ring + (size_t)s * stage_bytes;
-      mbar_expect_tx(&full[s], (uint32_t)(A_TILE_BYTES + blocks * 8192));
-      tma_load_2d(sa, &p.a, kb * BK, row0, &full[s]);
-      for (int j = 0; j < blocks; ++j) {
-        if constexpr (B_MN) tma_load_2d(sa + A_TILE_BYTES + j * 8192, &p.b, n0 + 64 * j, kb * BK, &full[s]);
-        else tma_load_2d(sa + A_TILE_BYTES + j * 8192, &p.b, kb * BK, n0 + 64 * j, &full[s]);
+  if (warp == 0) {
+    if (lane == 0) {
+      tma_prefetch_desc(&p.x);
+      tma_prefetch_desc(&p.w);
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        const int s = kb % p.stages;
+        if (kb >= p.stages && !gemm_wait(&empty[s], ((uint32_t)(kb / p.stages) & 1u) ^ 1u, abortp, p, 1)) break;
+        uint8_t* sw = ring + (size_t)s * stage_bytes;
+        mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
+        if constexpr (W_MN) {
+          for (int j = 0; j < p.m_rows / 64; ++j) tma_load_2d(sw + j * 8192, &p.w, m0 + 64 * j, kb * BK, &full[s]);
+        } else {
+          tma_load_2d(sw, &p.w, kb * BK, m0, &full[s]);
+        }
+        tma_load_2d(sw + w_bytes, &p.x, kb * BK, row0, &full[s]);
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    const uint32_t idesc = make_instr_desc_bf16(BM, mma_n, false, B_MN);
-    bool ok = true;
-    for (int kb = kb0; kb < kb1; ++kb) {
-      const int it = kb - kb0, s = it % p.stages;
-      if (!gemm_wait(&full[s], (uint32_t)(it / p.stages) & 1u, abortp, p, 3)) { ok = false; break; }
-      tc_fence_after();
-      const uint32_t sa = smem_u32(ring + (size_t)s * stage_bytes), sb = sa + A_TILE_BYTES;
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = make_instr_desc_bf16(BM, p.tok, W_MN, false);
+      bool ok = true;
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        const int s = kb % p.stages;
+        if (!gemm_wait(&full[s], (uint32_t)(kb / p.stages) & 1u, abortp, p, 3)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sw = smem_u32(ring + (size_t)s * stage_bytes), sx = sw + (uint32_t)w_bytes;
 #pragma unroll
-      for (int kk = 0; kk < BK / 16; ++kk) {
-        const uint64_t da = make_smem_desc(sa + kk * 32, 16, 1024);
-        const uint64_t db = B_MN ? make_smem_desc(sb + kk * 2048, 8192, 1024) : make_smem_desc(sb + kk * 32, 16, 1024);
-        umma_bf16(tmem_base, da, db, idesc, (it > 0 || kk > 0) ? 1u : 0u);
+        for (int kk = 0; kk < BK / 16; ++kk) {
+          // (64 experts: the descriptor's second block of columns / rows is the token part of the stage)
+          const uint64_t dw = W_MN ? make_smem_desc(sw + kk * 2048, 8192, 1024) : make_smem_desc(sw + kk * 32, 16, 1024);
+          umma_bf16(tmem_base, dw, make_smem_desc(sx + kk * 32, 16, 1024), idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+        }
+        umma_commit(&empty[s]);
       }
-      umma_commit(&empty[s]);
+      if (ok) umma_commit(&acc_full);
     }
-    if (ok) umma_commit(&acc_full);
-  }
-  __syncwarp();
-  // ---- partial tile into shared memory: every MMA has read the ring by now --------------------------
-  const int pitch = mma_n + 4;       // floats; consecutive rows start 4 banks (mod 16-byte steps) apart
-  float* mine = reinterpret_cast<float*>(ring);
-  if (warp >= 2) {
+  } else {
+    // thread = expert: a token's 32 logits of a warp leave as one 128-byte line
     const int q = warp & 3;
-    bool have = kb1 > kb0;
-    if (have) have = gemm_wait(&acc_full, 0, abortp, p, 4);
+    const bool have = gemm_wait(&acc_full, 0, abortp, p, 4);
     __syncwarp();
     tc_fence_after();
-    float* row = mine + (size_t)(q * 32 + lane) * pitch;
-    for (int c = 0; c < mma_n; c += 16) {
-      uint32_t r[16];
-      __syncwarp();
-      tmem_ld_32x16(tmem_base + ((uint32_t)(q * 32) << 16) + c, r);
-      tmem_ld_wait();
+    const int col = m0 + q * 32 + lane;
+    if (__all_sync(0xffffffffu, have)) {
+      for (int c = 0; c < p.tok && row0 + c < p.S; c += 16) {
+        uint32_t r[16];
+        __syncwarp();
+        tmem_ld_32x16(tmem_base + ((uint32_t)(q * 32) << 16) + c, r);
+        tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 16; i += 4)
-        *reinterpret_cast<float4*>(row + c + i) = kb1 > kb0
-            ? make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]))
-            : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    tc_fence_before();
-  }
-  cluster_sync_all();
-  // ---- rows [128 part / parts, ..): the sum of the cluster's partials, in rank order -----------------
-  const int r_lo = BM * part / parts, r_hi = min(BM * (part + 1) / parts, p.S - row0);
-  const int vecs = mma_n / 4;
-  const uint32_t base = smem_u32(mine);
-  const bool vec_ok = p.ldc % 4 == 0 && n0 % 4 == 0 && ((uintptr_t)p.out & 15) == 0;
-  for (int i = tid; i < (r_hi - r_lo) * vecs; i += DN_THREADS) {
-    const int r = r_lo + i / vecs, c = (i - (r - r_lo) * vecs) * 4;
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = 0; k < parts; ++k) {
-      const float4 v = ld_cluster_f4(base + (uint32_t)(r * pitch + c) * 4u, (uint32_t)k);
-      if (k == 0) sum = v;
-      else { sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w; }
-    }
-    float* o = p.out + (long long)(row0 + r) * p.ldc + n0 + c;
-    if (vec_ok && c + 4 <= n_here) {
-      *reinterpret_cast<float4*>(o) = sum;
-    } else {
-      const float e[4] = {sum.x, sum.y, sum.z, sum.w};
-      for (int j = 0; j < 4 && c + j < n_here; ++j) o[j] = e[j];
+        for (int i = 0; i < 16; ++i)
+          if (row0 + c + i < p.S && col < p.N) p.out[(long long)(row0 + c + i) * p.ldc + col] = __uint_as_float(r[i]);
+      }
     }
   }
+  tc_fence_before();
+  __syncthreads();
   if (s_abort) {       // in-flight loads are given time to land
     unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) { }
   }
-  cluster_sync_all();  // no CTA leaves while a peer may still read its partial
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 256);
+    tmem_dealloc(tmem_base, DN_MAX_TOK);
   }
 }
 

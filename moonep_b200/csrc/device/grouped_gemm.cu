@@ -725,36 +725,16 @@ static int launch_wgrad(const GemmKParams& kp, bool pair, int grid, cudaStream_t
   return launch_single(kern, raised, kp, grid, threads, smem, false, stream);
 }
 
-// CTAs that share one tile's reduction: as many as the SMs allow beside the other tiles, at most
-// eight (a portable cluster), with at least four k-blocks each.
-static int dense_parts(int tiles, int num_kb, int ctas) {
-  int parts = 1;
-  while (parts < 8 && tiles * parts * 2 <= ctas && num_kb >= parts * 2 * 4) parts *= 2;
-  return parts;
-}
-template <bool B_MN>
-static int launch_dense_f32(const DenseParams& dp, int ctas, cudaStream_t stream) {
-  const void* kern = (const void*)ep_dense_f32_kernel<B_MN>;
+template <bool W_MN>
+static int launch_dense_f32(const DenseParams& dp, cudaStream_t stream) {
+  const void* kern = (const void*)ep_dense_f32_kernel<W_MN>;
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit(kern, raised));
-  const int mt = (dp.S + BM - 1) / BM, nt = (dp.N + dp.tile_n - 1) / dp.tile_n;
-  const int parts = dense_parts(mt * nt, dp.num_kb, ctas);
-  const int stage = A_TILE_BYTES + (dp.tile_n + 63) / 64 * 8192;
-  const int partial = BM * (((dp.tile_n + 15) & ~15) + 4) * 4;
-  const int ring = dp.stages * stage;
-  cudaLaunchConfig_t cfg;
-  std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)parts, (unsigned)mt, (unsigned)nt);
-  cfg.blockDim = dim3(DN_THREADS);
-  cfg.dynamicSmemBytes = (size_t)((ring > partial ? ring : partial) + 1024);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)parts; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  const dim3 grid((unsigned)((dp.S + dp.tok - 1) / dp.tok), (unsigned)((dp.N + BM - 1) / BM));
+  // (the MMA reads 128 rows of the weights' part whatever was loaded: 8 KB beyond the last stage may be read)
+  const size_t smem = (size_t)dp.stages * dense_stage_bytes(dp.m_rows, dp.tok) + 1024 + 8192;
   void* args[] = {(void*)&dp};
-  MEP_CUDA_OK(cudaLaunchKernelExC(&cfg, kern, args));
+  MEP_CUDA_OK(cudaLaunchKernel(kern, grid, dim3(DN_THREADS), args, smem, stream));
   return 0;
 }
 
@@ -844,19 +824,23 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
     std::memset(&dp, 0, sizeof(dp));
     dp.out = (float*)d->out[0]; dp.ldc = d->ldc; dp.S = d->total_rows; dp.N = d->N;
     dp.num_kb = (d->K + BK - 1) / BK;
-    dp.tile_n = d->N < 256 ? d->N : 256;
-    const int stage = A_TILE_BYTES + (dp.tile_n + 63) / 64 * 8192;
-    dp.stages = DN_RING / stage < DN_MAX_STAGES ? DN_RING / stage : DN_MAX_STAGES;
     dp.status = kp.status; dp.timeout_ns = kp.timeout_ns;
     if (dp.S < 1) return 0;
-    if (dp.S > 65535 * BM) return fail(-16, "gemm: %d rows are too many for the dense product", dp.S);
-    if ((rc = make_map(&dp.a, d->a[0], d->a_rows, d->K, d->lda[0], BK, BM))) return rc;
+    // token tile: as small as fills the CTAs once, in steps of 16
+    const int mt = (dp.N + BM - 1) / BM;
+    if (mt > 65535) return fail(-16, "gemm: %d columns are too many for the dense product", dp.N);
+    const long long want = ((long long)dp.S * mt + grid - 1) / grid;
+    dp.tok = want >= DN_MAX_TOK ? DN_MAX_TOK : ((int)want + 15) / 16 * 16;
+    dp.m_rows = dp.N <= 64 ? 64 : 128;
+    const int stage = dense_stage_bytes(dp.m_rows, dp.tok);
+    dp.stages = DN_RING / stage < DN_MAX_STAGES ? DN_RING / stage : DN_MAX_STAGES;
+    if ((rc = make_map(&dp.x, d->a[0], d->a_rows, d->K, d->lda[0], BK, dp.tok))) return rc;
     if (d->b_mn) {
-      if ((rc = make_map(&dp.b, d->b[0][0], d->b_rows[0], d->N, d->ldb, 64, BK))) return rc;
-      return launch_dense_f32<true>(dp, grid, stream);
+      if ((rc = make_map(&dp.w, d->b[0][0], d->b_rows[0], d->N, d->ldb, 64, BK))) return rc;
+      return launch_dense_f32<true>(dp, stream);
     }
-    if ((rc = make_map(&dp.b, d->b[0][0], d->b_rows[0], d->K, d->ldb, BK, 64))) return rc;
-    return launch_dense_f32<false>(dp, grid, stream);
+    if ((rc = make_map(&dp.w, d->b[0][0], d->b_rows[0], d->K, d->ldb, BK, dp.m_rows))) return rc;
+    return launch_dense_f32<false>(dp, stream);
   }
   // A reduction tail is legal: the TMA loads zero-fill A beyond K, which also cancels whatever
   // a MN-major B tile picks up from the next expert's rows.
@@ -867,15 +851,14 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
       if ((rc = make_map(&kp.tok[s][b], d->a[s], d->a_rows, d->K, d->lda[s], BK, 32 * (b + 1)))) return rc;
   }
   const int nsel = (d->epi == EPI_SWIGLU) ? 2 : d->nseg;
-  for (int s = 0; s < 2; ++s)
+  // (maps of operands that a launch does not have stay unset: no tile refers to them)
+  for (int s = 0; s < nsel; ++s)
     for (int al = 0; al < 2; ++al) {
-      const void* base = d->b[s < nsel ? s : 0][al] ? d->b[s < nsel ? s : 0][al] : d->b[s < nsel ? s : 0][0];
-      const int64_t rows = d->b[s < nsel ? s : 0][al] ? d->b_rows[al] : d->b_rows[0];
+      if (d->b[s][al] == nullptr) continue;
       if (d->b_mn) {   // [K rows][N cols] per expert
-        if ((rc = make_map(&kp.b[s][al], base, rows, d->N, d->ldb, 64, BK))) return rc;
-        kp.b2[s][al] = kp.b[s][al];
+        if ((rc = make_map(&kp.b[s][al], d->b[s][al], d->b_rows[al], d->N, d->ldb, 64, BK))) return rc;
       } else {         // [N rows][K cols] per expert
-        if ((rc = make_map(&kp.b2[s][al], base, rows, d->K, d->ldb, BK, BN / 2))) return rc;
+        if ((rc = make_map(&kp.b2[s][al], d->b[s][al], d->b_rows[al], d->K, d->ldb, BK, BN / 2))) return rc;
       }
     }
   kp.tma_out = d->ldc % 8 == 0 && (((uintptr_t)d->out[0] | (uintptr_t)d->out[1] | (uintptr_t)d->out[2] |

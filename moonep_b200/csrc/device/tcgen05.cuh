@@ -195,18 +195,6 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
-// Four floats of the variable at `smem_addr` in CTA `cta_rank` of this cluster.
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t smem_addr, uint32_t cta_rank) {
-  float4 v;
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\t"
-      "mapa.shared::cluster.u32 ra, %4, %5;\n\t"
-      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "r"(smem_addr), "r"(cta_rank)
-      : "memory");
-  return v;
-}
 // 16 lanes x 32 consecutive fp32 columns as matrix fragments: for the 8-column block j, thread t gets
 // rows t / 4 (r[4j], r[4j+1]) and t / 4 + 8 (r[4j+2], r[4j+3]), columns 8j + 2 (t % 4) and the next.
 __device__ __forceinline__ void tmem_ld_16x256_x4(uint32_t taddr, uint32_t* r) {

@@ -1,13 +1,13 @@
-"""Dense product with fp32 output (router logits): tiles whose reduction a cluster shares, ragged rows,
-columns and reduction lengths, both layouts of the weights, against fp64."""
+"""Dense product with fp32 output (router logits): token tiles of all sizes, ragged rows, columns and
+reduction lengths, both layouts of the weights, against fp64."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-# rows around a tile and many tiles (one CTA a tile), reductions of one k-block (with a tail) up to 112 (eight CTAs
-# share them), columns around a 64-column block, one tile of 256 and more than one
+# rows around a tile of 16 and of 128, many tiles; reductions of one k-block (with a tail) up to 112, below and
+# above the stages in flight; columns around half a tile, one tile and several
 @pytest.mark.parametrize("S,K,N", [(1, 64, 8), (16, 7168, 32), (127, 520, 64), (128, 256, 72), (129, 2048, 128),
                                    (300, 8, 200), (1531, 1024, 256), (40, 4096, 264), (4096, 512, 1000), (20000, 64, 16)])
 def test_dense_matches_fp64(S, K, N):
