@@ -31,6 +31,7 @@ struct PlanParams {
   int32_t* send_order;
   int64_t arrive_off;       // ARRIVE counters in the meta chunk, cleared before the exchange
   int n_arrive;
+  int rank_warps, rank_counts;   // warps that number the entries, and where their counters start in shared memory
 };
 
 // Position of expert e in the sending order of `rank` (see PlanParams::send_order).
