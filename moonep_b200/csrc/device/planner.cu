@@ -247,9 +247,12 @@ int mep_launch_plan(const void* ctx_, const int32_t* topk, const int32_t* tpe, i
   p.scratch = c.plan_scratch; p.scratch_ints = c.plan_scratch_ints;
   p.send_order = send_order; p.arrive_off = c.ml.arrive_off; p.n_arrive = (int)(c.NvS / 128 + 1);
   size_t smem = (size_t)mep_plan_smem_bytes(c.R, c.E);
-  // counters of the ranking warps: sixteen warps' up to 1024 experts, at least one warp's
+  // ranking warps: one per 128 entries of a CTA (clearing and summing their counters costs more than a
+  // few steps of 32 entries: with sixteen for 8 entries 27 -> 31 us), as many as have room for counters
   p.rank_counts = (int)(smem / sizeof(int32_t));
+  const int entries = (c.S + c.num_sms - 1) / c.num_sms * c.K;
   p.rank_warps = 64 * 1024 / (int)(sizeof(int32_t) * c.E);
+  if (p.rank_warps > entries / 128) p.rank_warps = entries / 128;
   p.rank_warps = p.rank_warps < 1 ? 1 : (p.rank_warps > PLAN_WARPS ? PLAN_WARPS : p.rank_warps);
   const size_t counters = sizeof(int32_t) * (size_t)p.rank_warps * c.E;
   if (p.rank_warps > 1) smem += counters;
