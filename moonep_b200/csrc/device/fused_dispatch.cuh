@@ -79,8 +79,10 @@ __device__ __forceinline__ void fused_dispatch_copy_warp(const FusedDispatch& d,
   // Done in slices between the batches of entries below: the padding of local group j is needed
   // when the GEMM reaches group j, which is when the senders reach round j of the sending order,
   // and doing all of it up front would only delay the first groups.
-  // The rows of up to 32 groups are zeroed first and announced together behind ONE system fence:
-  // a release per row drained the warp's stores each time (~2 us a row).
+  // The rows of up to 32 groups are zeroed first and announced together behind one system fence:
+  // a release per row drained the warp's stores each time (~2 us a row).  The fence is executed by every
+  // lane that announces: only a fence in the announcing thread's own order makes its relaxed reductions
+  // a release (of the other lanes' zeros too, which the warp barrier before it put in its past).
   auto do_pads = [&](int g_from, int g_to) {
     for (int g0 = g_from; g0 < g_to; g0 += 32) {
       const int g = g0 + lane;
@@ -102,10 +104,11 @@ __device__ __forceinline__ void fused_dispatch_copy_warp(const FusedDispatch& d,
         }
       }
       __syncwarp();
-      if (lane == 0) fence_sys();
-      __syncwarp();
-      for (int r = first_l + cta; r < first_l + n_l; r += n_cta)
-        red_relaxed_sys_add(my_meta + d.arrive_off + (r >> 7), d.nsplit);
+      if (cta < n_l) {
+        fence_sys();
+        for (int r = first_l + cta; r < first_l + n_l; r += n_cta)
+          red_relaxed_sys_add(my_meta + d.arrive_off + (r >> 7), d.nsplit);
+      }
     }
   };
 
@@ -159,15 +162,15 @@ __device__ __forceinline__ void fused_dispatch_copy_warp(const FusedDispatch& d,
         }
       }
     }
-    // The route weights above are plain stores to the peers; ONE system-scope fence per batch (by
-    // lane 0, made cumulative over the warp by the barriers around it) orders them before every
-    // arrival signal of this batch.  The rows themselves need no fence: a signal is only issued
+    // The route weights above are plain stores to the peers; one system-scope fence per batch, in
+    // every lane that announces (lanes < NST), orders them before every arrival signal of this batch;
+    // the warp barrier before it makes it cumulative over the other lanes' stores.
+    // The rows themselves need no fence: a signal is only issued  The rows themselves need no fence: a signal is only issued
     // after cp.async.bulk.wait_group has reported the row's copy complete, so a relaxed reduction
     // is enough per round.  (A release per round cost a full drain of the SM's stores each time
     // and made the copy warp, not NVLink, the limit.)
     __syncwarp();
-    if (lane == 0) fence_sys();
-    __syncwarp();
+    if (lane < NST) fence_sys();
     // ---- rounds of NST units: lane i < NST moves unit u0 + r0 + i through stage i ---------------
     for (int r0 = 0; r0 < PER_BATCH && u0 + r0 < n_units; r0 += NST) {
       const int from = r0 + (lane < NST ? lane : 0);
