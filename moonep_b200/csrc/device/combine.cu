@@ -436,11 +436,19 @@ struct PushReduceParams {
   int one_device;                  // every rank's staging is memory of this device
 };
 
-// 1024 threads, eight 16-byte loads each in flight: one CTA an SM with 256 threads kept 32 KB in
-// flight and ran at 3.4 TB/s (4096 tokens x 7168, top-8: 154 us).
-constexpr int PUSH_REDUCE_THREADS = 1024;
+// Within one device: 1024 threads, eight 16-byte loads each in flight (one CTA an SM with 256 threads
+// kept 32 KB in flight and ran at 3.4 TB/s, 4096 tokens x 7168, top-8: 154 us, with 1024 103).  Such
+// a CTA takes every register of its SM.
+// Several devices: 256 threads and at most a third of the registers.  Both this kernel and reduce_grad
+// wait for other ranks while they hold their SMs, and a backward pass starts the two together on two
+// streams: on one rank this kernel may be placed first, on another reduce_grad, and then each has to fit
+// beside the other (reduce_grad: 160 threads of at most 255 registers) or both ranks wait until the
+// time limit.  The same geometry serves a virtual group that wants more CTAs than the device has SMs.
+constexpr int PUSH_REDUCE_THREADS_ONE = 1024, PUSH_REDUCE_THREADS = 256;
 
-__global__ void __launch_bounds__(PUSH_REDUCE_THREADS, 1) ep_push_reduce_kernel(const PushReduceParams p) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == PUSH_REDUCE_THREADS ? 3 : 1)
+ep_push_reduce_kernel(const PushReduceParams p) {
   const SyncCtx& sc = p.sync;
   const int tid = threadIdx.x;
   const int vr = blockIdx.y, rank = sc.rank_base + vr;
@@ -450,7 +458,7 @@ __global__ void __launch_bounds__(PUSH_REDUCE_THREADS, 1) ep_push_reduce_kernel(
     const float* rs = p.row_scalar + (size_t)vr * p.NvS;
     int64_t rows = p.cu_seqlens[(size_t)vr * 2 * p.epn + 2 * p.epn - 1];
     if (rows > p.NvS) rows = p.NvS;
-    for (int64_t r = (int64_t)c * PUSH_REDUCE_THREADS + tid; r < rows; r += (int64_t)G * PUSH_REDUCE_THREADS) {
+    for (int64_t r = (int64_t)c * THREADS + tid; r < rows; r += (int64_t)G * THREADS) {
       const int v = si[r];
       if (v < 0) continue;
       const int64_t sr = v / p.N, ent = v - sr * p.N;
@@ -465,8 +473,8 @@ __global__ void __launch_bounds__(PUSH_REDUCE_THREADS, 1) ep_push_reduce_kernel(
   uint4* out = reinterpret_cast<uint4*>(p.out + (size_t)vr * p.S * p.H);
   // one 16-byte vector v of one token s per thread and step; (s, v) advance without a division
   const int nvec = p.H / 8;
-  const int step_s = G * PUSH_REDUCE_THREADS / nvec, step_v = G * PUSH_REDUCE_THREADS - step_s * nvec;
-  int s = (c * PUSH_REDUCE_THREADS + tid) / nvec, v = c * PUSH_REDUCE_THREADS + tid - s * nvec;
+  const int step_s = G * THREADS / nvec, step_v = G * THREADS - step_s * nvec;
+  int s = (c * THREADS + tid) / nvec, v = c * THREADS + tid - s * nvec;
   while (s < p.S) {
     const uint4* base = mine + (size_t)s * p.K * nvec + v;
     float acc[8];
@@ -493,7 +501,7 @@ __global__ void __launch_bounds__(PUSH_REDUCE_THREADS, 1) ep_push_reduce_kernel(
   if (p.w_out != nullptr) {
     const float* wm = p.wpush + (size_t)rank * p.wpush_stride;
     float* wo = p.w_out + (size_t)vr * p.N;
-    for (int64_t i = (int64_t)c * PUSH_REDUCE_THREADS + tid; i < p.N; i += (int64_t)G * PUSH_REDUCE_THREADS)
+    for (int64_t i = (int64_t)c * THREADS + tid; i < p.N; i += (int64_t)G * THREADS)
       wo[i] = wm[i];
   }
 }
@@ -588,8 +596,17 @@ int mep_launch_push_reduce(const void* ctx_, const void* push, int64_t push_stri
   p.row_scalar = row_scalar; p.cu_seqlens = cu_seqlens; p.out = (__nv_bfloat16*)out; p.w_out = w_out;
   p.one_device = c.one_device();
   dim3 grid(grid_x > 0 ? grid_x : c.num_sms, c.Rv());
-  MEP_CUDA_OK(launch_coop((const void*)ep_push_reduce_kernel, grid, dim3(PUSH_REDUCE_THREADS), 0, stream, p));
+  const bool one = c.one_device() && (int)(grid.x * grid.y) <= c.sm_count;
+  MEP_CUDA_OK(launch_coop(one ? (const void*)ep_push_reduce_kernel<PUSH_REDUCE_THREADS_ONE>
+                              : (const void*)ep_push_reduce_kernel<PUSH_REDUCE_THREADS>,
+                          grid, dim3(one ? PUSH_REDUCE_THREADS_ONE : PUSH_REDUCE_THREADS), 0, stream, p));
   return 0;
+}
+
+// Registers and shared memory that a CTA of the push-reduce kernel for several devices takes of its SM;
+// 0, or an error.
+int mep_push_reduce_footprint(int* regs, int* smem) {
+  return cta_footprint((const void*)ep_push_reduce_kernel<PUSH_REDUCE_THREADS>, PUSH_REDUCE_THREADS, 0, regs, smem);
 }
 
 // dst [Rv][N], out [Rv][S][H] bf16, w_out [Rv][S][K] fp32 or null.  direct != 0 (only where every

@@ -309,6 +309,24 @@ int mep_launch_grad_reduce(const void* ctx_, const int32_t* etc, int n, void* co
   }
 }
 
+// The most registers and shared memory that a CTA takes of its SM in a launch over several devices, over
+// all ring geometries, for a Buffer of E experts on R ranks; 0, or an error.
+int mep_grad_reduce_footprint(int R, int E, int* regs, int* smem) {
+  *regs = *smem = 0;
+  const size_t lists = sizeof(int32_t) * ((size_t)3 * (E / R) + (size_t)E);
+  const struct { const void* kernel; int ring; } all[] = {
+      {(const void*)ep_grad_reduce_kernel<4, 16 * 1024>, 4 * 16}, {(const void*)ep_grad_reduce_kernel<8, 16 * 1024>, 8 * 16},
+      {(const void*)ep_grad_reduce_kernel<12, 16 * 1024>, 12 * 16}, {(const void*)ep_grad_reduce_kernel<16, 8 * 1024>, 16 * 8},
+      {(const void*)ep_grad_reduce_kernel<4, 32 * 1024>, 4 * 32}, {(const void*)ep_grad_reduce_kernel<6, 32 * 1024>, 6 * 32}};
+  for (const auto& k : all) {
+    int r = 0, s = 0;
+    if (int rc = cta_footprint(k.kernel, GR_THREADS, (size_t)k.ring * 1024 + lists, &r, &s)) return rc;
+    *regs = r > *regs ? r : *regs;
+    *smem = s > *smem ? s : *smem;
+  }
+  return 0;
+}
+
 // Pure cross-rank barrier (one CTA per rank).
 int mep_launch_sync(const void* ctx_, cudaStream_t stream) {
   const BufferCtx& c = *(const BufferCtx*)ctx_;

@@ -14,6 +14,7 @@
 
 #include "common/layout.h"
 #include "device/sync.cuh"
+#include "host/errors.h"
 
 namespace mep {
 
@@ -90,6 +91,16 @@ inline cudaError_t raise_smem_limit(const void* kernel, std::atomic<unsigned lon
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
   if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
   return e;
+}
+
+// What one CTA of a kernel takes of its SM: registers (handed out to warps in units of 256, so of 8 a
+// thread) and shared memory (with the 1 KB that the system keeps for each CTA).
+inline int cta_footprint(const void* kernel, int threads, size_t dyn_smem, int* regs, int* smem) {
+  cudaFuncAttributes fa;
+  MEP_CUDA_OK(cudaFuncGetAttributes(&fa, kernel));
+  *regs = (fa.numRegs + 7) / 8 * 8 * threads;
+  *smem = (int)(fa.sharedSizeBytes + dyn_smem) + 1024;
+  return 0;
 }
 
 // Cooperative launch helper: all CTAs of grid (gx, gy) must be co-resident.
