@@ -316,6 +316,18 @@ __global__ void __launch_bounds__(256) ep_plan_snapshot_kernel(const SnapshotPar
   }
 }
 
+// Token rows that a dispatch CTA keeps staged (one more holds the zero row); 0 if not even two fit.
+// Sixteen only within one device: over several, dispatch and the weight ops wait for other ranks while
+// they hold their SMs, on two streams.  Where they share SMs, dispatch takes no more than eight rows need,
+// beside which reduce_grad's ring fits up to rows of 10 KB; with sixteen only up to 5 KB.
+static int dispatch_ring(const BufferCtx& c) {
+  const size_t row = (size_t)c.H * 2, budget = c.ring_budget(200 * 1024);
+  if (c.one_device() && 17 * row <= budget) return 16;
+  if (9 * row <= budget) return 8;
+  if (5 * row <= budget) return 4;
+  return 3 * row <= 220 * 1024 ? 2 : 0;
+}
+
 template <int ST>
 static int launch_dispatch_t(const BufferCtx& c, DispatchParams& p, size_t smem,
                              cudaStream_t stream) {
@@ -354,12 +366,19 @@ int mep_launch_dispatch(const void* ctx_, const void* x, const float* w, const i
   p.hidden = (__nv_bfloat16*)c.shard_base(shard); p.link_out = link_out; p.src_out = src_out;
   p.entry_barrier = entry_barrier; p.fresh = fresh; p.direct = direct;
   const size_t row = (size_t)c.H * 2;
-  const size_t budget = c.ring_budget(200 * 1024);
-  if (17 * row <= budget) return launch_dispatch_t<16>(c, p, 17 * row, stream);
-  if (9 * row <= budget) return launch_dispatch_t<8>(c, p, 9 * row, stream);
-  if (5 * row <= budget) return launch_dispatch_t<4>(c, p, 5 * row, stream);
-  if (3 * row <= 220 * 1024) return launch_dispatch_t<2>(c, p, 3 * row, stream);
+  switch (dispatch_ring(c)) {
+    case 16: return launch_dispatch_t<16>(c, p, 17 * row, stream);
+    case 8: return launch_dispatch_t<8>(c, p, 9 * row, stream);
+    case 4: return launch_dispatch_t<4>(c, p, 5 * row, stream);
+    case 2: return launch_dispatch_t<2>(c, p, 3 * row, stream);
+  }
   return fail(-2, "dispatch: H=%d does not fit a 2-stage ring", c.H);
+}
+
+// Dynamic shared memory of a dispatch launch of this Buffer.
+int64_t mep_dispatch_smem_bytes(const void* ctx_) {
+  const BufferCtx& c = *(const BufferCtx*)ctx_;
+  return (int64_t)(dispatch_ring(c) + 1) * c.H * 2;
 }
 
 // Copy every primary row to its duplicates inside this rank's shard.

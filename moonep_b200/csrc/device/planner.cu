@@ -229,6 +229,24 @@ int64_t mep_plan_smem_bytes(int R, int E) {
   return (int64_t)sizeof(int32_t) * (2 * (int64_t)E + 4 * R + (int64_t)PLAN_WARPS * R);
 }
 
+// Ranking warps of a planner launch: one per 128 entries of a CTA (clearing and summing their counters costs
+// more than a few steps of 32 entries: with sixteen for 8 entries 27 -> 31 us), as many as have room for
+// counters.  Over several devices that is 8 KB: the planner and the weight ops wait for other ranks while
+// they hold their SMs, on two streams, and beside prefetch_weight's ring (192 KB and its lists) 64 KB do not fit.
+static int plan_rank_warps(const BufferCtx& c) {
+  const int64_t entries = (int64_t)((c.S + c.num_sms - 1) / c.num_sms) * c.K;
+  int64_t w = (c.one_device() ? 64 * 1024 : 8 * 1024) / (int64_t)(sizeof(int32_t) * c.E);
+  if (w > entries / 128) w = entries / 128;
+  return w < 1 ? 1 : (w > PLAN_WARPS ? PLAN_WARPS : (int)w);
+}
+
+// Dynamic shared memory of a planner launch of this Buffer.
+int64_t mep_plan_launch_smem_bytes(const void* ctx_) {
+  const BufferCtx& c = *(const BufferCtx*)ctx_;
+  const int w = plan_rank_warps(c);            // (a lone warp counts in place)
+  return mep_plan_smem_bytes(c.R, c.E) + (w > 1 ? (int64_t)sizeof(int32_t) * w * c.E : 0);
+}
+
 // Fresh plan for this rank (or for all virtual ranks).  send_order [Rv][N] may be null (it is
 // only needed by the fused dispatch -> GEMM path).  Leaves the chain links in the peers'
 // meta chunks; they become visible with the next cross-rank barrier (the dispatch kernel's
@@ -246,17 +264,9 @@ int mep_launch_plan(const void* ctx_, const int32_t* topk, const int32_t* tpe, i
   p.etc = etc; p.remote_stats = remote_stats;
   p.scratch = c.plan_scratch; p.scratch_ints = c.plan_scratch_ints;
   p.send_order = send_order; p.arrive_off = c.ml.arrive_off; p.n_arrive = (int)(c.NvS / 128 + 1);
-  size_t smem = (size_t)mep_plan_smem_bytes(c.R, c.E);
-  // ranking warps: one per 128 entries of a CTA (clearing and summing their counters costs more than a
-  // few steps of 32 entries: with sixteen for 8 entries 27 -> 31 us), as many as have room for counters
-  p.rank_counts = (int)(smem / sizeof(int32_t));
-  const int entries = (c.S + c.num_sms - 1) / c.num_sms * c.K;
-  p.rank_warps = 64 * 1024 / (int)(sizeof(int32_t) * c.E);
-  if (p.rank_warps > entries / 128) p.rank_warps = entries / 128;
-  p.rank_warps = p.rank_warps < 1 ? 1 : (p.rank_warps > PLAN_WARPS ? PLAN_WARPS : p.rank_warps);
-  const size_t counters = sizeof(int32_t) * (size_t)p.rank_warps * c.E;
-  if (p.rank_warps > 1) smem += counters;
-  else p.rank_counts = 0;              // the one warp's counters are cnt itself
+  const size_t smem = (size_t)mep_plan_launch_smem_bytes(ctx_);
+  p.rank_warps = plan_rank_warps(c);
+  p.rank_counts = p.rank_warps > 1 ? (int)(mep_plan_smem_bytes(c.R, c.E) / sizeof(int32_t)) : 0;
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_plan_kernel, raised));
   dim3 grid(c.num_sms, c.Rv());

@@ -1,0 +1,42 @@
+"""Shared memory of the dispatch and planner launches of a group over several devices: they and the weight
+ops wait for other ranks on two streams, so where they can share an SM they have to keep room for one another."""
+import pytest
+
+from moonep_b200 import _native as nat
+import moonep_b200.api  # noqa: F401  (declares the entries)
+
+SM_SHARED, PER_CTA = 228 * 1024, 1024 + 1024      # what the system keeps for a CTA, and static parts
+
+
+@pytest.fixture
+def ctx():
+    made = []
+
+    def make(R, E, S, K, H, num_sms=32, virt=0):
+        c = nat.call("mep_ctx_create", 0, R, virt, E, S, K, H, 128, num_sms, 148, num_sms, 0, 0, 0, 0, 0, 0, 0, 10 ** 9)
+        assert c, nat.last_error()
+        made.append(c)
+        return c
+
+    yield make
+    for c in made:
+        nat.call("mep_ctx_destroy", c)
+
+
+@pytest.mark.parametrize("R", [2, 8])
+@pytest.mark.parametrize("H", [256, 1024, 2048, 2560, 4096, 5120])
+def test_dispatch_beside_reduce_grad(ctx, R, H):
+    E = 256
+    smem = nat.call("mep_dispatch_smem_bytes", ctx(R, E, 4096, 8, H))
+    lists = 4 * (3 * (E // R) + E)
+    assert smem + (128 * 1024 + lists) + 2 * PER_CTA <= SM_SHARED
+    assert nat.call("mep_dispatch_smem_bytes", ctx(1, E, 4096, 8, H)) == 17 * 2 * H      # one device: the deep ring
+
+
+@pytest.mark.parametrize("R", [2, 8])
+@pytest.mark.parametrize("E", [64, 256, 1024])
+@pytest.mark.parametrize("S,num_sms", [(16, 32), (4096, 32), (8192, 8)])
+def test_planner_beside_prefetch_weight(ctx, R, E, S, num_sms):
+    smem = nat.call("mep_plan_launch_smem_bytes", ctx(R, E, S, 8, 1024, num_sms))
+    lists = 4 * (4 * (E // R) + E)
+    assert smem + (192 * 1024 + lists) + 2 * PER_CTA <= SM_SHARED
