@@ -241,31 +241,45 @@ ep_ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __re
       const float l = m + logf(s);
       const long long t = targets[r];
       lse[r] = l;
-      // (a target that is no class has no loss to report)
+      // (a target that is no class: ep_ce_mean_kernel reports it)
       loss[r] = t == ignore ? 0.f : (t >= 0 && t < V ? l - __bfloat162float(row[t]) : NAN);
     }
   }
 }
 
-// out[0] = mean loss of the rows that count, out[1] = their number; summed in a fixed order
+// out[0] = mean loss of the rows that count, out[1] = their number; summed in a fixed order.  A target that is
+// no class makes both NaN, so that every gradient is too, and the first such row is recorded in `status`.
 __global__ void __launch_bounds__(1024) ep_ce_mean_kernel(const float* __restrict__ loss, const long long* __restrict__ targets,
-                                                         long long ignore, int S, float* __restrict__ out) {
+                                                         long long ignore, int S, int V, float* __restrict__ out,
+                                                         int32_t* __restrict__ status) {
   __shared__ double sl[32];
-  __shared__ int sn[32];
+  __shared__ int sn[32], sb[32];
   double l = 0.0;
-  int n = 0;
+  int n = 0, bad = S;
   for (int r = threadIdx.x; r < S; r += 1024) {
+    const long long t = targets[r];
     l += loss[r];
-    n += targets[r] != ignore;
+    n += t != ignore;
+    if (t != ignore && (t < 0 || t >= V)) bad = min(bad, r);
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) { l += __shfl_xor_sync(0xffffffffu, l, o); n += __shfl_xor_sync(0xffffffffu, n, o); }
-  if ((threadIdx.x & 31) == 0) { sl[threadIdx.x >> 5] = l; sn[threadIdx.x >> 5] = n; }
+  for (int o = 16; o > 0; o >>= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, o);
+    n += __shfl_xor_sync(0xffffffffu, n, o);
+    bad = min(bad, __shfl_xor_sync(0xffffffffu, bad, o));
+  }
+  if ((threadIdx.x & 31) == 0) { sl[threadIdx.x >> 5] = l; sn[threadIdx.x >> 5] = n; sb[threadIdx.x >> 5] = bad; }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int i = 1; i < 32; ++i) { l += sl[i]; n += sn[i]; }
+    for (int i = 1; i < 32; ++i) { l += sl[i]; n += sn[i]; bad = min(bad, sb[i]); }
     out[0] = (float)(l / n);             // (no row counts: 0 / 0, NaN)
-    out[1] = (float)n;
+    out[1] = bad < S ? NAN : (float)n;
+    if (bad < S && atomicCAS(status, 0, (int)ST_BAD_INDEX) == 0) {
+      status[1] = KID_CROSS_ENTROPY;
+      status[4] = bad;
+      status[5] = (int)targets[bad];
+      status[6] = V;
+    }
   }
 }
 
@@ -378,9 +392,10 @@ int mep_swiglu_bwd(const void* dact, const void* gate, const void* up, const flo
   return 0;
 }
 
-// logits [S][V] bf16, targets [S] int64; lse, loss [S] and mean_n [2] (mean, rows that count) fp32.
+// logits [S][V] bf16, targets [S] int64; lse, loss [S] and mean_n [2] (mean, rows that count) fp32; status
+// int32 [8], where a target that is neither `ignore` nor a class is recorded.
 int mep_ce_fwd(const void* logits, const long long* targets, long long ignore, int S, int V, float* lse, float* loss,
-               float* mean_n, cudaStream_t stream) {
+               float* mean_n, int32_t* status, cudaStream_t stream) {
   if (V < 1 || S < 0) return fail(-1, "cross entropy: %d x %d logits", S, V);
   const __nv_bfloat16* x = (const __nv_bfloat16*)logits;
   if (S > 0) {
@@ -389,7 +404,7 @@ int mep_ce_fwd(const void* logits, const long long* targets, long long ignore, i
     else
       ep_ce_fwd_kernel<false><<<S, CE_THREADS, 0, stream>>>(x, targets, ignore, V, lse, loss);
   }
-  ep_ce_mean_kernel<<<1, 1024, 0, stream>>>(loss, targets, ignore, S, mean_n);
+  ep_ce_mean_kernel<<<1, 1024, 0, stream>>>(loss, targets, ignore, S, V, mean_n, status);
   MEP_CUDA_OK(cudaGetLastError());
   return 0;
 }

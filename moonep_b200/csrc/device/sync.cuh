@@ -32,6 +32,7 @@ enum StatusCode : int {
 enum KernelId : int {
   KID_SYNC = 1, KID_PLAN = 2, KID_DISPATCH = 3, KID_EXPAND = 4, KID_PROLOGUE = 5,
   KID_COMBINE = 6, KID_PREFETCH = 7, KID_REDUCE = 8, KID_GEMM = 9,
+  KID_CROSS_ENTROPY = 10,
 };
 
 // Per-(virtual-)rank local synchronisation state, 8 int32:

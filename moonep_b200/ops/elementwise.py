@@ -7,11 +7,12 @@ import torch
 
 from .. import _native as nat
 from .._native import F, I, L, P
+from .gemm import status_word
 
 nat.declare("mep_router_topk", I, [P, P, I, I, I, P, P, P, P])
 nat.declare("mep_router_topk_bwd", I, [P, P, P, I, I, I, P, P])
 nat.declare("mep_swiglu_bwd", I, [P, P, P, P, P, I, I, P, P, P, P])
-nat.declare("mep_ce_fwd", I, [P, P, L, I, I, P, P, P, P])
+nat.declare("mep_ce_fwd", I, [P, P, L, I, I, P, P, P, P, P])
 nat.declare("mep_ce_bwd", I, [P, P, L, I, I, P, P, P, P, P])
 nat.declare("mep_sgd_update", I, [P, P, L, F, P])
 nat.declare("mep_sgd_update_masked", I, [P, P, L, L, P, F, P])
@@ -86,7 +87,7 @@ class _CrossEntropy(torch.autograd.Function):
         f32 = dict(dtype=torch.float32, device=logits.device)
         lse, loss, mean_n = torch.empty(S, **f32), torch.empty(S, **f32), torch.empty(2, **f32)
         _rc(nat.call("mep_ce_fwd", logits.data_ptr(), targets.data_ptr(), ignore_index, S, V, lse.data_ptr(),
-                     loss.data_ptr(), mean_n.data_ptr(), _st()), "cross_entropy")
+                     loss.data_ptr(), mean_n.data_ptr(), status_word(logits.device).data_ptr(), _st()), "cross_entropy")
         ctx.ignore_index = ignore_index
         ctx.save_for_backward(logits, targets, lse, mean_n)
         return mean_n[0].clone()
@@ -106,7 +107,9 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int
     """``F.cross_entropy(logits.float(), targets)`` (mean over the rows whose target is not
     ``ignore_index``) for bf16 ``logits [S, V]`` and int64 ``targets [S]`` on the GPU, without the
     fp32 copies; the gradient is rounded to bf16 once, as there.  Other forms of the arguments go
-    to ``F.cross_entropy``."""
+    to ``F.cross_entropy``.  A target that is neither ``ignore_index`` nor a class, for which that function
+    stops the device with an assertion, makes the loss and all gradients NaN, and
+    ``gemm.check_status`` raises."""
     if (logits.is_cuda and logits.dtype == torch.bfloat16 and logits.dim() == 2 and logits.is_contiguous()
             and targets.device == logits.device and targets.dtype == torch.int64
             and tuple(targets.shape) == (logits.shape[0],) and targets.is_contiguous()):

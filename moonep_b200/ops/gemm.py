@@ -64,7 +64,8 @@ _checked_layout = False
 
 
 def status_word(device) -> torch.Tensor:
-    """Per-device int32[8] that GEMM kernels flag on a bounded-wait expiry (0 = healthy)."""
+    """Per-device int32[8] that GEMM kernels flag on a bounded-wait expiry, and the cross-entropy on a
+    target that is no class (0 = healthy)."""
     idx = torch.device(device).index or 0
     if idx not in _status:
         _status[idx] = torch.zeros(8, dtype=torch.int32, device=f"cuda:{idx}")
@@ -73,6 +74,8 @@ def status_word(device) -> torch.Tensor:
 
 def check_status(device="cuda") -> None:
     st = status_word(device).tolist()
+    if st[0] == 4:
+        raise RuntimeError(f"cross entropy: target {st[5]} of row {st[4]} is not one of {st[6]} classes")
     if st[0] == 5:
         raise RuntimeError(f"grouped GEMM with fused dispatch: the rows of block {st[4]} never arrived "
                            f"(CTA {st[3]} saw {st[5]} of {st[6]} row parts)")

@@ -51,3 +51,19 @@ def test_odd_values_and_other_forms():
     p = torch.softmax(torch.randn(4, 96, device="cuda"), 1)
     for a, b in ((y.float(), t), (y[:, ::2], t), (y, p)):
         assert torch.equal(ew.cross_entropy(a, b), F.cross_entropy(a.float(), b))
+
+
+@pytest.mark.parametrize("V", [48, 49])
+@pytest.mark.parametrize("bad", [-1, 49, 1 << 40])
+def test_target_that_is_no_class(V, bad):
+    from moonep_b200.ops import elementwise as ew, gemm
+    gemm.check_status()
+    x = torch.randn(5, V, device="cuda").bfloat16().requires_grad_(True)
+    t = torch.tensor([1, -100, 2, bad, 3], device="cuda")
+    loss = ew.cross_entropy(x, t)
+    loss.backward()
+    assert bool(torch.isnan(loss))
+    assert bool(torch.isnan(x.grad[[0, 2, 3, 4]]).all()) and bool((x.grad[1] == 0).all())
+    with pytest.raises(RuntimeError, match="row 3 is not one of"):
+        gemm.check_status()
+    gemm.reset_status()
