@@ -93,9 +93,11 @@ class _CrossEntropy(torch.autograd.Function):
         return mean_n[0].clone()
 
     @staticmethod
-    @torch.autograd.function.once_differentiable
     def backward(ctx, g):
         logits, targets, lse, mean_n = ctx.saved_tensors
+        if torch.is_grad_enabled():        # create_graph: a gradient that can be differentiated again
+            loss = torch.nn.functional.cross_entropy(logits.float(), targets, ignore_index=ctx.ignore_index)
+            return torch.autograd.grad(loss, logits, g, create_graph=True)[0], None, None
         S, V = logits.shape
         grad = torch.empty_like(logits)
         _rc(nat.call("mep_ce_bwd", logits.data_ptr(), targets.data_ptr(), ctx.ignore_index, S, V, lse.data_ptr(),
@@ -103,14 +105,25 @@ class _CrossEntropy(torch.autograd.Function):
         return grad, None, None
 
 
+def _eager(*tensors) -> bool:
+    """True if nothing stands between these tensors and their memory: no tracer, dispatch mode, subclass,
+    functorch transform or forward-mode tangent, which a kernel of our own would pass by."""
+    return (not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+            and torch._C._len_torch_dispatch_stack() == 0
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+                    and torch.autograd.forward_ad.unpack_dual(t).tangent is None for t in tensors))
+
+
 def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int = -100) -> torch.Tensor:
     """``F.cross_entropy(logits.float(), targets)`` (mean over the rows whose target is not
     ``ignore_index``) for bf16 ``logits [S, V]`` and int64 ``targets [S]`` on the GPU, without the
-    fp32 copies; the gradient is rounded to bf16 once, as there.  Other forms of the arguments go
-    to ``F.cross_entropy``.  A target that is neither ``ignore_index`` nor a class, for which that function
+    fp32 copies; the gradient is rounded to bf16 once, as there.  Other forms of the arguments, other
+    devices than the current one, tracing, ``vmap``, forward-mode and second derivatives go to
+    ``F.cross_entropy``.  A target that is neither ``ignore_index`` nor a class, for which that function
     stops the device with an assertion, makes the loss and all gradients NaN, and
     ``gemm.check_status`` raises."""
-    if (logits.is_cuda and logits.dtype == torch.bfloat16 and logits.dim() == 2 and logits.is_contiguous()
+    if (logits.is_cuda and logits.dtype == torch.bfloat16 and logits.dim() == 2 and _eager(logits, targets)
+            and logits.device.index == torch.cuda.current_device() and logits.is_contiguous()
             and targets.device == logits.device and targets.dtype == torch.int64
             and tuple(targets.shape) == (logits.shape[0],) and targets.is_contiguous()):
         return _CrossEntropy.apply(logits, targets, ignore_index)

@@ -67,3 +67,34 @@ def test_target_that_is_no_class(V, bad):
     with pytest.raises(RuntimeError, match="row 3 is not one of"):
         gemm.check_status()
     gemm.reset_status()
+
+
+def test_derivatives_and_transforms():
+    """Whatever ``F.cross_entropy`` can be put through: second derivatives, forward mode, vmap, tracing."""
+    from moonep_b200.ops import elementwise as ew
+    from torch.autograd import forward_ad
+    ref = lambda a, b: F.cross_entropy(a.float(), b)
+    x = torch.randn(6, 40, device="cuda").bfloat16()
+    t = torch.randint(0, 40, (6,), device="cuda")
+
+    def second(fn):
+        a = x.clone().requires_grad_(True)
+        g, = torch.autograd.grad(fn(a, t), a, create_graph=True)
+        return torch.autograd.grad((g.float() ** 2).sum(), a)[0]
+
+    def forward(fn):
+        with forward_ad.dual_level():
+            return forward_ad.unpack_dual(fn(forward_ad.make_dual(x, torch.ones_like(x) * 0.5 + x), t)).tangent
+
+    for case in (second, forward, lambda fn: torch.func.grad(lambda a: fn(a, t))(x),
+                 lambda fn: torch.func.vmap(fn)(x.view(2, 3, 40), t.view(2, 3)),
+                 lambda fn: torch.jit.trace(lambda a: fn(a, t), (x,))(-x)):
+        got, want = case(ew.cross_entropy), case(ref)
+        assert got is not None and torch.equal(got, want)
+    # a plain first derivative beside a hook on the saved tensors
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda v: packed.append(v) or v.clone(), lambda v: v):
+        a = x.clone().requires_grad_(True)
+        loss = ew.cross_entropy(a, t)
+    loss.backward()
+    assert packed and bool(torch.isfinite(a.grad).all())
