@@ -188,7 +188,8 @@ ep_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bfloat16
 constexpr int CE_THREADS = 512;
 
 __device__ __forceinline__ void ce_add(float& m, float& s, float x) {
-  if (x > m) { s = s * expf(m - x) + 1.f; m = x; }        // (m = -inf: s is 0 and exp(-inf) is 0)
+  // (m = -inf: s is 0 and exp(-inf) is 0; x - x is 0, or NaN for an infinite logit, as its loss is)
+  if (x > m) { s = s * expf(m - x) + (1.f + (x - x)); m = x; }
   else if (!(x == -INFINITY && m == -INFINITY)) s += expf(x - m);
 }
 

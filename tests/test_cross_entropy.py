@@ -98,3 +98,28 @@ def test_derivatives_and_transforms():
         loss = ew.cross_entropy(a, t)
     loss.backward()
     assert packed and bool(torch.isfinite(a.grad).all())
+
+
+# scalar rows (odd classes, odd start) answer infinities and NaN as vector rows do
+@pytest.mark.parametrize("V,offset", [(49, 0), (48, 3), (48, 0), (600, 1)])
+def test_odd_values_in_scalar_rows(V, offset):
+    from moonep_b200.ops import elementwise as ew
+    inf = float("inf")
+    rows = torch.randn(6, V, device="cuda")
+    rows[0] = -inf
+    rows[1, 5] = float("nan")
+    rows[2, 7] = inf
+    rows[3, V - 1] = inf
+    rows[4, ::2] = -inf
+    t = torch.tensor([1, 2, 7, 3, 5, 4], device="cuda")
+    for r in range(6):
+        flat = torch.zeros(V + offset, device="cuda", dtype=torch.bfloat16)
+        flat[offset:] = rows[r].bfloat16()
+        a, b = flat[offset:].view(1, V).detach().requires_grad_(True), rows[r:r + 1].bfloat16().double().requires_grad_(True)
+        got, want = ew.cross_entropy(a, t[r:r + 1]), F.cross_entropy(b, t[r:r + 1])
+        got.backward()
+        want.backward()
+        assert bool(torch.isnan(got)) == bool(torch.isnan(want)) == (r < 4)
+        assert torch.equal(torch.isnan(a.grad), torch.isnan(b.grad))
+        if r >= 4:
+            assert abs(float(got.detach()) - float(want.detach())) <= 1e-5 * (1 + abs(float(want.detach())))
