@@ -28,6 +28,7 @@ constexpr int ROUTER_VPL = 8;                 // keys per lane kept in registers
 __device__ __forceinline__ uint32_t router_key(float x) {
   const uint32_t b = __float_as_uint(x);
   if ((b & 0x7FFFFFFFu) > 0x7F800000u) return 1u;                 // NaN; 0 marks "already selected"
+  if (b == 0x80000000u) return b;                                 // -0 ties with +0
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);              // (-inf maps to 0x007FFFFF)
 }
 

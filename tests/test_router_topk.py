@@ -32,3 +32,15 @@ def test_not_a_number_and_infinities(E):
     topk, _, tpe = ew.router_topk(logits, K)
     assert topk.cpu().tolist() == [[0, 1, 2, 3], [0, 1, 2, 3], [7, 1, 3, 5], [5, 0, 1, 2]]
     assert int(tpe.sum()) == 4 * K
+
+
+@pytest.mark.parametrize("E", [40, 300])
+def test_zeros_of_either_sign_tie(E):
+    """A bias of -0.0 (no popularity at all) beside logits of -0.0: equal values go by the expert's index."""
+    from moonep_b200.ops import elementwise as ew
+    logits = torch.zeros(3, E, device="cuda")
+    logits[0, ::2] = -0.0
+    logits[1] = -0.0
+    logits[2, 3] = -1.0
+    topk, _, _ = ew.router_topk(logits, 4, -torch.zeros(E, device="cuda"))
+    assert topk.cpu().tolist() == [[0, 1, 2, 3], [0, 1, 2, 3], [0, 1, 2, 4]]
