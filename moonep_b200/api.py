@@ -48,6 +48,7 @@ nat.declare("mep_phase_stamps_compiled", I, [])
 nat.declare("mep_trace_ints64", L, [])
 nat.declare("mep_trace_dims", None, [ctypes.POINTER(ctypes.c_int)])
 nat.declare("mep_ctx_set_trace", None, [P, P])
+nat.declare("mep_ctx_direct_ctas", I, [P])
 nat.declare("mep_launch_plan", I, [P, P, P, P, P, P, P, P, P, P])
 nat.declare("mep_launch_arrive_reset", I, [P, P])
 nat.declare("mep_launch_plan_snapshot", I, [P, P, P, P])

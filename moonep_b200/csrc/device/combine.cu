@@ -510,7 +510,7 @@ template <int ST, int NV, bool DIRECT>
 static int launch_combine_t(const BufferCtx& c, CombineParams& p, size_t smem, cudaStream_t stream) {
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_combine_kernel<ST, NV, DIRECT>, raised));
-  dim3 grid(c.num_sms, c.Rv());
+  dim3 grid(DIRECT ? c.direct_ctas() : c.num_sms, c.Rv());
   // (DIRECT follows no kernel of its own chain and has no barrier inside)
   MEP_CUDA_OK(launch_chained((const void*)ep_combine_kernel<ST, NV, DIRECT>, grid, dim3(combine_threads(DIRECT, NV)), smem,
                              stream, p, /*coop=*/!DIRECT, c.pdl && !DIRECT));

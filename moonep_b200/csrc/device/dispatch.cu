@@ -333,7 +333,7 @@ static int launch_dispatch_t(const BufferCtx& c, DispatchParams& p, size_t smem,
                              cudaStream_t stream) {
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_dispatch_kernel<ST>, raised));
-  dim3 grid(c.num_sms, c.Rv());
+  dim3 grid(p.direct ? c.direct_ctas() : c.num_sms, c.Rv());
   MEP_CUDA_OK(launch_chained((const void*)ep_dispatch_kernel<ST>, grid, dim3(DISPATCH_THREADS), smem,
                              stream, p, /*coop=*/1, c.pdl && p.fresh));
   return 0;

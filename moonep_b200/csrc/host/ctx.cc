@@ -55,6 +55,8 @@ void* mep_ctx_create(int rank, int R, int virt, int E, int S, int K, int H, int 
   return c;
 }
 
+int mep_ctx_direct_ctas(const void* ctx) { return ((const BufferCtx*)ctx)->direct_ctas(); }
+
 void mep_ctx_destroy(void* ctx) { delete (BufferCtx*)ctx; }
 
 // Phase stamps: 1 when the library was built with -DMEP_PHASE_STAMPS; the buffer holds

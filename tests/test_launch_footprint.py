@@ -1,4 +1,4 @@
-"""Shared memory of the dispatch and planner launches of a group over several devices: they and the weight
+"""Launches by Buffer.  Shared memory of dispatch and planner over several devices: they and the weight
 ops wait for other ranks on two streams, so where they can share an SM they have to keep room for one another."""
 import pytest
 
@@ -12,8 +12,8 @@ SM_SHARED, PER_CTA = 228 * 1024, 1024 + 1024      # what the system keeps for a 
 def ctx():
     made = []
 
-    def make(R, E, S, K, H, num_sms=32, virt=0):
-        c = nat.call("mep_ctx_create", 0, R, virt, E, S, K, H, 128, num_sms, 148, num_sms, 0, 0, 0, 0, 0, 0, 0, 10 ** 9)
+    def make(R, E, S, K, H, num_sms=32, virt=0, local=148):
+        c = nat.call("mep_ctx_create", 0, R, virt, E, S, K, H, 128, num_sms, local, num_sms, 0, 0, 0, 0, 0, 0, 0, 10 ** 9)
         assert c, nat.last_error()
         made.append(c)
         return c
@@ -40,3 +40,11 @@ def test_planner_beside_prefetch_weight(ctx, R, E, S, num_sms):
     smem = nat.call("mep_plan_launch_smem_bytes", ctx(R, E, S, 8, 1024, num_sms))
     lists = 4 * (4 * (E // R) + E)
     assert smem + (192 * 1024 + lists) + 2 * PER_CTA <= SM_SHARED
+
+
+# ranks on the device, num_sms, local SMs -> CTAs a rank
+@pytest.mark.parametrize("R,num_sms,local,want", [(1, 8, 148, 148), (1, 32, 148, 148), (1, 148, 148, 148), (1, 32, 16, 32),
+                                                  (8, 2, 148, 18), (8, 18, 148, 18), (8, 32, 148, 32), (2, 8, 148, 74)])
+def test_few_communication_sms_on_one_device(ctx, R, num_sms, local, want):
+    """Dispatch and combine that move all rows themselves run on no fewer SMs than the local kernels they replace."""
+    assert nat.call("mep_ctx_direct_ctas", ctx(R, 64, 512, 8, 1024, num_sms, int(R > 1), local)) == want
