@@ -77,19 +77,19 @@ __device__ __forceinline__ uint4 f32x2_to_bf16x8(const unsigned long long* f) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 // acc (+)= one staged row; `first` is uniform over the CTA's accumulator threads
-template <int NV>
+template <int NV, int THREADS = ACC_THREADS>
 __device__ __forceinline__ void accumulate_row(unsigned long long (&acc)[NV][4], const uint4* src, int ta,
                                                int nvec, bool first) {
   if (first) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int v = ta + i * ACC_THREADS;
+      const int v = ta + i * THREADS;
       if (v < nvec) bf16x8_to_f32x2(src[v], acc[i]);
     }
   } else {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int v = ta + i * ACC_THREADS;
+      const int v = ta + i * THREADS;
       if (v < nvec) {
         unsigned long long t[4];
         bf16x8_to_f32x2(src[v], t);
@@ -222,10 +222,10 @@ struct CombineParams {
   float* w_out;                  // [Rv][S][K] or null
 };
 
-constexpr int COMBINE_ACC_THREADS = ACC_THREADS;
-// loader, accumulator warps (two sets within one device), weights
-constexpr int combine_sets(bool direct, int nv) { return direct && nv <= 4 ? 2 : 1; }   // (registers)
-constexpr int combine_threads(bool direct, int nv) { return 32 + combine_sets(direct, nv) * COMBINE_ACC_THREADS + 32; }
+// accumulator warps of a set; within one device two sets, or one of twice the warps
+constexpr int combine_sets(bool direct, int aw) { return direct && aw == ACC_WARPS ? 2 : 1; }
+// loader, accumulator warps, weights
+constexpr int combine_threads(bool direct, int aw) { return 32 + combine_sets(direct, aw) * aw * 32 + 32; }
 
 // What the accumulators do with a staged row.
 enum : int { ROW_STARTS_GROUP = 1, ROW_ENDS_GROUP = 2, ROW_ENDS_TOKEN = 4 };
@@ -243,7 +243,7 @@ __device__ __forceinline__ void fold_group(unsigned long long (&tot)[NV][4], con
   }
 }
 
-// NV: 16-byte vectors per accumulator thread (H <= NV * 128 * 8).
+// NV: 16-byte vectors per accumulator thread (H <= NV * AW * 32 * 8, AW warps a set).
 // DIRECT (every shard is memory of this device): the loader also reads the duplicates, group by group
 // in the order of the primaries' k, and the accumulators sum a group in registers, round it to
 // bf16 once and add it to the token's sum: the same additions and roundings, in the same order, as
@@ -252,9 +252,13 @@ __device__ __forceinline__ void fold_group(unsigned long long (&tot)[NV][4], con
 // accumulator warps take the tokens in turn: a row costs a set ~0.3 us of latencies (landed, read,
 // added, stage released) however short it is, which with one set was the kernel (4096 tokens x
 // 7168, top-8, 96 CTAs: 146 us, with two sets 117; eight ranks in 144 CTAs 760 -> 631, of 636 at the copy rate).
-template <int ST, int NV, bool DIRECT>
-__global__ void __launch_bounds__(combine_threads(DIRECT, NV), 1) ep_combine_kernel(const CombineParams p) {
-  constexpr int SETS = combine_sets(DIRECT, NV);
+// Rows of more than 4 vectors a thread (7168 elements) are summed by all the warps as one set: a set of seven
+// warps needed ten vectors a thread, whose two sums spilled (8 ranks x 512 tokens x 10240, top-8, 144 CTAs: 375
+// us, where the separate kernels take 258 and one set of fourteen warps 127).
+template <int ST, int NV, bool DIRECT, int AW>
+__global__ void __launch_bounds__(combine_threads(DIRECT, AW), 1) ep_combine_kernel(const CombineParams p) {
+  constexpr int SETS = combine_sets(DIRECT, AW);
+  constexpr int SET_THREADS = AW * 32;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full[ST];
   __shared__ __align__(8) uint64_t empty[ST];
@@ -268,7 +272,7 @@ __global__ void __launch_bounds__(combine_threads(DIRECT, NV), 1) ep_combine_ker
   uint8_t* ring = smem_raw;
 
   if (tid == 0) {
-    for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], SETS * ACC_WARPS); }
+    for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], SETS * AW); }
     mbar_fence_init();
   }
   __syncthreads();
@@ -342,10 +346,10 @@ __global__ void __launch_bounds__(combine_threads(DIRECT, NV), 1) ep_combine_ker
         ++prod;
       }
     }
-  } else if (warp <= SETS * ACC_WARPS) {
+  } else if (warp <= SETS * AW) {
     // ---- accumulators ----------------------------------------------------------------------
-    const int set = SETS == 1 ? 0 : (warp - 1) / ACC_WARPS;
-    const int ta = tid - 32 - set * COMBINE_ACC_THREADS;
+    const int set = SETS == 1 ? 0 : (warp - 1) / AW;
+    const int ta = tid - 32 - set * SET_THREADS;
     __nv_bfloat16* out = p.out + (size_t)vr * p.S * p.H;
     int cons = 0;
     for (int j = 0; j < n_tok; ++j) {
@@ -372,15 +376,15 @@ __global__ void __launch_bounds__(combine_threads(DIRECT, NV), 1) ep_combine_ker
           const int f = ok ? last_flag[s] : (ROW_STARTS_GROUP | ROW_ENDS_GROUP | ROW_ENDS_TOKEN);
           is_last = (f & ROW_ENDS_TOKEN) != 0;
           if ((f & ROW_STARTS_GROUP) && (f & ROW_ENDS_GROUP)) {
-            accumulate_row<NV>(acc, src, ta, nvec, first);      // a lone row is its own rounded sum
+            accumulate_row<NV, SET_THREADS>(acc, src, ta, nvec, first);      // a lone row is its own rounded sum
             first = false;
           } else {
-            accumulate_row<NV>(grp, src, ta, nvec, (f & ROW_STARTS_GROUP) != 0);
+            accumulate_row<NV, SET_THREADS>(grp, src, ta, nvec, (f & ROW_STARTS_GROUP) != 0);
             if (f & ROW_ENDS_GROUP) { fold_group<NV>(acc, grp, first); first = false; }
           }
         } else {
           is_last = !ok || last_flag[s] != 0;
-          accumulate_row<NV>(acc, src, ta, nvec, first);
+          accumulate_row<NV, SET_THREADS>(acc, src, ta, nvec, first);
           first = false;
         }
         __syncwarp();
@@ -395,7 +399,7 @@ __global__ void __launch_bounds__(combine_threads(DIRECT, NV), 1) ep_combine_ker
       uint4* orow = reinterpret_cast<uint4*>(out + (size_t)(c + (int64_t)j * G) * p.H);
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        int v = ta + i * COMBINE_ACC_THREADS;
+        int v = ta + i * SET_THREADS;
         if (v < nvec) orow[v] = f32x2_to_bf16x8(acc[i]);
       }
     }
@@ -506,27 +510,28 @@ ep_push_reduce_kernel(const PushReduceParams p) {
   }
 }
 
-template <int ST, int NV, bool DIRECT>
+template <int ST, int NV, bool DIRECT, int AW>
 static int launch_combine_t(const BufferCtx& c, CombineParams& p, size_t smem, cudaStream_t stream) {
   static std::atomic<unsigned long long> raised{0};
-  MEP_CUDA_OK(raise_smem_limit((const void*)ep_combine_kernel<ST, NV, DIRECT>, raised));
+  MEP_CUDA_OK(raise_smem_limit((const void*)ep_combine_kernel<ST, NV, DIRECT, AW>, raised));
   dim3 grid(DIRECT ? c.direct_ctas() : c.num_sms, c.Rv());
   // (DIRECT follows no kernel of its own chain and has no barrier inside)
-  MEP_CUDA_OK(launch_chained((const void*)ep_combine_kernel<ST, NV, DIRECT>, grid, dim3(combine_threads(DIRECT, NV)), smem,
+  MEP_CUDA_OK(launch_chained((const void*)ep_combine_kernel<ST, NV, DIRECT, AW>, grid, dim3(combine_threads(DIRECT, AW)), smem,
                              stream, p, /*coop=*/!DIRECT, c.pdl && !DIRECT));
   return 0;
 }
 
-template <int NV, bool DIRECT>
+template <int NV, bool DIRECT, int AW = ACC_WARPS>
 static int launch_combine_nv(const BufferCtx& c, CombineParams& p, cudaStream_t stream) {
   const size_t row = (size_t)c.H * 2;
   const size_t budget = c.ring_budget(210 * 1024);
   // short rows: as many in flight as two tokens and more have
-  if (DIRECT && 28 * row <= budget) return launch_combine_t<DIRECT ? 28 : 14, NV, DIRECT>(c, p, 28 * row, stream);
-  if (14 * row <= budget) return launch_combine_t<14, NV, DIRECT>(c, p, 14 * row, stream);
-  if (10 * row <= budget) return launch_combine_t<10, NV, DIRECT>(c, p, 10 * row, stream);
-  if (6 * row <= budget) return launch_combine_t<6, NV, DIRECT>(c, p, 6 * row, stream);
-  if (3 * row <= 220 * 1024) return launch_combine_t<3, NV, DIRECT>(c, p, 3 * row, stream);
+  constexpr bool SHORT = DIRECT && AW == ACC_WARPS;
+  if (SHORT && 28 * row <= budget) return launch_combine_t<SHORT ? 28 : 14, NV, DIRECT, AW>(c, p, 28 * row, stream);
+  if (14 * row <= budget) return launch_combine_t<14, NV, DIRECT, AW>(c, p, 14 * row, stream);
+  if (10 * row <= budget) return launch_combine_t<10, NV, DIRECT, AW>(c, p, 10 * row, stream);
+  if (6 * row <= budget) return launch_combine_t<6, NV, DIRECT, AW>(c, p, 6 * row, stream);
+  if (3 * row <= 220 * 1024) return launch_combine_t<3, NV, DIRECT, AW>(c, p, 3 * row, stream);
   return fail(-2, "combine: H=%d does not fit a 2-stage ring", c.H);
 }
 
@@ -623,11 +628,13 @@ int mep_launch_combine(const void* ctx_, const int32_t* dst, void* out, float* w
   p.dst = dst; p.hidden = (const __nv_bfloat16*)c.hidden;
   p.out = (__nv_bfloat16*)out; p.w_out = w_out;
   const int nvec = c.H / 8;
-  const int nv = (nvec + COMBINE_ACC_THREADS - 1) / COMBINE_ACC_THREADS;
+  const int nv = (nvec + ACC_THREADS - 1) / ACC_THREADS;
   if (nv <= 1) return launch_combine_d<1>(c, p, direct, stream);
   if (nv <= 2) return launch_combine_d<2>(c, p, direct, stream);
   if (nv <= 4) return launch_combine_d<4>(c, p, direct, stream);
-  if (nv <= 10) return launch_combine_d<10>(c, p, direct, stream);
+  if (direct && nv <= 8) return launch_combine_nv<4, true, 2 * ACC_WARPS>(c, p, stream);
+  if (direct && nv <= 10) return launch_combine_nv<5, true, 2 * ACC_WARPS>(c, p, stream);
+  if (nv <= 10) return launch_combine_nv<10, false>(c, p, stream);
   return fail(-3, "combine: H=%d is larger than 16384", c.H);
 }
 

@@ -11,7 +11,10 @@ pytestmark = pytest.mark.gpu
 # row; every expert on one rank; rings of 16 / 8 / 3 rows
 CASES = [(1, 1, 1, 1, 8, 8, 1), (1, 37, 8, 64, 7168, 128, 16), (1, 200, 5, 16, 1024, 16, 32),
          (2, 33, 3, 8, 2560, 64, 4), (4, 19, 8, 64, 512, 16, 32), (8, 17, 8, 128, 2560, 16, 18),
-         (8, 65, 1, 16, 256, 8, 2), (2, 9, 32, 64, 16384, 8, 3), (3, 50, 12, 96, 4096, 32, 49)]
+         (8, 65, 1, 16, 256, 8, 2), (2, 9, 32, 64, 16384, 8, 3), (3, 50, 12, 96, 4096, 32, 49),
+         # rows summed by all warps: just above 7168 elements, around 14336, several tokens a CTA
+         (1, 300, 6, 16, 7176, 16, 8), (2, 160, 8, 32, 10240, 16, 8), (1, 170, 3, 8, 14336, 8, 4), (2, 90, 4, 16, 14344, 8, 2),
+         (1, 200, 8, 8, 16384, 8, 32)]
 
 
 @pytest.mark.parametrize("R,S,K,E,H,tp,sms", CASES)
