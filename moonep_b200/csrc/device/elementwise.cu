@@ -352,16 +352,20 @@ extern "C" {
 int mep_router_topk(const float* logits, const float* bias, int S, int E, int K, int32_t* topk,
                     float* weights, int32_t* tpe, cudaStream_t stream) {
   if (K > 32 || K < 1 || E < K) return fail(-1, "router: need 1 <= K <= min(32, E)");
-  int blocks = (S + ROUTER_WARPS - 1) / ROUTER_WARPS;
-  if (blocks > 148 * 2) blocks = 148 * 2;
+  // as many warps a block as its keys leave room for (up to 256 experts they are in registers)
+  int warps = ROUTER_WARPS;
+  if (E > 32 * ROUTER_VPL) {
+    const int room = (int)(200 * 1024 / (sizeof(uint32_t) * (size_t)E)) - 1;
+    if (room < 1) return fail(-2, "router: E=%d too large", E);
+    if (room < warps) warps = room;
+  }
+  int blocks = (S + warps - 1) / warps;
+  const int most = 148 * (E <= 32 * ROUTER_VPL ? 2 : (E <= 1536 ? 4 : (E <= 2816 ? 2 : 1)));
+  if (blocks > most) blocks = most;
   MEP_CUDA_OK(cudaMemsetAsync(tpe, 0, sizeof(int32_t) * E, stream));
   if (E <= 32 * ROUTER_VPL) {
     ep_router_topk_kernel<true><<<blocks, ROUTER_WARPS * 32, E * sizeof(uint32_t), stream>>>(logits, bias, S, E, K, topk, weights, tpe);
   } else {
-    // as many warps as the keys leave room for
-    int warps = (int)(200 * 1024 / (sizeof(uint32_t) * (size_t)E)) - 1;
-    if (warps < 1) return fail(-2, "router: E=%d too large", E);
-    if (warps > ROUTER_WARPS) warps = ROUTER_WARPS;
     const size_t smem = (size_t)(warps + 1) * E * sizeof(uint32_t);
     static std::atomic<unsigned long long> raised{0};
     MEP_CUDA_OK(raise_smem_limit((const void*)ep_router_topk_kernel<false>, raised));
