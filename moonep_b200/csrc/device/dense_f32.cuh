@@ -1,4 +1,5 @@
-// C[S][N] = A[S][K] * B[K][N] (or B[N][K]) with fp32 output: the router logits.
+// C[S][N] = A[S][K] * B[K][N] (or B[N][K]) with fp32 output: the router logits.  (Outputs of more tiles than the
+// CTAs hold at once go to the token-major kernel.)
 //
 // The output is small (S x experts) and the reduction long: a CTA walks up to 112 k-blocks one after
 // the other, ~0.4 us each, bound by that chain and not by bytes.  The experts take the M side (128 a

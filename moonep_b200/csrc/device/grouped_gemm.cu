@@ -10,6 +10,7 @@
 // main loop through the second accumulator.  Kernels:
 //   ep_token_gemm_kernel (token_gemm.cuh): token-major products with bf16 output -- gate/up with
 //        SwiGLU, down, both dgrads, the pushed combine, the fused dispatch.
+//        Also large products with fp32 output.
 //   ep_dense_f32_kernel (dense_f32.cuh): one product with fp32 output (router logits).
 //   ep_grouped_gemm_kernel (this file): weight-grad (groups partition the REDUCTION dimension):
 //        D[g] (+)= A[rows of g]^T * B[rows of g]   both operands MN-major, fp32 output by TMA
@@ -820,17 +821,21 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
     if (d->ngroups != 1 || d->cu_seqlens != nullptr || d->nseg != 1 || d->accumulate)
       return fail(-15, "gemm: fp32 output is one dense product");
     if (d->K % 8 != 0) return fail(-4, "gemm: K=%d must be a multiple of 8", d->K);
+    if (d->total_rows < 1) return 0;
+  }
+  // Router logits: a dense product with fp32 output whose tiles fill the CTAs at most once.  Larger ones take the
+  // token-major kernel (same order of the sums), whose CTAs compute on across tiles: 4096 x 4096 -> 4096
+  // columns 237 -> 110 us, 16384 x 2048 -> 512 86 -> 46.  Up to 128 columns half of a pair's tile would be empty:
+  // single CTAs, from twice as many tiles on (65536 x 512 -> 128 49 -> 34; 32768 x 2048 -> 128 48 either way).
+  const long long dn_rows = ((long long)d->total_rows * ((d->N + BM - 1) / BM) + grid - 1) / grid;
+  if (d->epi == EPI_F32 && (dn_rows <= DN_MAX_TOK || (d->N <= BM && dn_rows <= 2 * DN_MAX_TOK))) {
     DenseParams dp;
     std::memset(&dp, 0, sizeof(dp));
     dp.out = (float*)d->out[0]; dp.ldc = d->ldc; dp.S = d->total_rows; dp.N = d->N;
     dp.num_kb = (d->K + BK - 1) / BK;
     dp.status = kp.status; dp.timeout_ns = kp.timeout_ns;
-    if (dp.S < 1) return 0;
     // token tile: as small as fills the CTAs once, in steps of 16
-    const int mt = (dp.N + BM - 1) / BM;
-    if (mt > 65535) return fail(-16, "gemm: %d columns are too many for the dense product", dp.N);
-    const long long want = ((long long)dp.S * mt + grid - 1) / grid;
-    dp.tok = want >= DN_MAX_TOK ? DN_MAX_TOK : ((int)want + 15) / 16 * 16;
+    dp.tok = dn_rows >= DN_MAX_TOK ? DN_MAX_TOK : ((int)dn_rows + 15) / 16 * 16;
     dp.m_rows = dp.N <= 64 ? 64 : 128;
     const int stage = dense_stage_bytes(dp.m_rows, dp.tok);
     dp.stages = DN_RING / stage < DN_MAX_STAGES ? DN_RING / stage : DN_MAX_STAGES;
@@ -909,6 +914,9 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
   if (d->epi == EPI_BF16)
     return d->b_mn ? launch_token<true, EPI_BF16, false>(kp, two, grid, stream)
                    : launch_token<false, EPI_BF16, false>(kp, two, grid, stream);
+  if (d->epi == EPI_F32)
+    return d->b_mn ? launch_token<true, EPI_F32, false>(kp, two && d->N > BM, grid, stream)
+                   : launch_token<false, EPI_F32, false>(kp, two && d->N > BM, grid, stream);
   if (d->epi == EPI_PUSH) {
     if (d->src_info == nullptr || d->push_base == nullptr || d->push_entries <= 0)
       return fail(-9, "gemm: the push epilogue needs src_info and a staging buffer");

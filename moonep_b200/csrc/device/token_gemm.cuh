@@ -95,7 +95,7 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
   __shared__ int s_groups_ready;
   __shared__ int s_end[MAX_GROUPS];
   __shared__ int s_prefix[MAX_GROUPS + 1];
-  __shared__ __align__(128) uint8_t s_stage[2][TG_CHUNK * TG_STAGE_ROW];
+  __shared__ __align__(128) uint8_t s_stage[2][EPI == EPI_F32 ? 16 : TG_CHUNK * TG_STAGE_ROW];
   // per token of a tile: address of its row at the home rank (PUSH) or its scale (SwiGLU); two tiles
   __shared__ unsigned long long s_ptr[EPI == EPI_PUSH ? 2 : 1][EPI == EPI_PUSH ? TG_MAX_N : 1];
   __shared__ float s_scale[EPI == EPI_SWIGLU ? 2 : 1][EPI == EPI_SWIGLU ? TG_MAX_N : 1];
@@ -339,6 +339,30 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
       tc_fence_after();
       const uint32_t tacc = tmem_base + (uint32_t)acc * TG_MAX_N + ((uint32_t)(q * 32) << 16);
       uint32_t r[32];
+      auto release_acc = [&] {           // the accumulator has been read: the next tile but one may overwrite it
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (TWO && crank != 0) mbar_arrive_remote(&acc_empty[acc], 0);
+          else mbar_arrive(&acc_empty[acc]);
+        }
+      };
+      if constexpr (EPI == EPI_F32) {
+        // thread = output column: a warp's 32 columns of a token leave as one 128-byte line
+        const int col = t.m0 + 128 * crank + q * 32 + lane;
+#pragma unroll 1
+        for (int c = 0; c < t.n; c += TG_CHUNK) {
+          __syncwarp();
+          tmem_ld_32x32(tacc + c, r);
+          tmem_ld_wait();
+          if (c + TG_CHUNK >= t.n) release_acc();
+          float* o = (float*)p.out[0] + (long long)(t.row0 + c) * p.ldc + col;
+#pragma unroll
+          for (int i = 0; i < TG_CHUNK; ++i)
+            if (c + i < t.rows && col < p.N) o[i * p.ldc] = __uint_as_float(r[i]);
+        }
+        continue;
+      }
       tmem_ld_16x256_x4(tacc, r);
       tmem_ld_16x256_x4(tacc + (16u << 16), r + 16);
       if constexpr (EPI == EPI_SWIGLU) {
@@ -360,13 +384,8 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
         if (c + TG_CHUNK < t.n) {        // the next 32 tokens travel while these leave
           tmem_ld_16x256_x4(tacc + c + TG_CHUNK, r);
           tmem_ld_16x256_x4(tacc + c + TG_CHUNK + (16u << 16), r + 16);
-        } else {                         // the accumulator has been read: the next tile but one may overwrite it
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (TWO && crank != 0) mbar_arrive_remote(&acc_empty[acc], 0);
-            else mbar_arrive(&acc_empty[acc]);
-          }
+        } else {
+          release_acc();
         }
         uint8_t* sb = s_stage[buf];
         __syncwarp();

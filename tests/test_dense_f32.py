@@ -23,3 +23,21 @@ def test_dense_matches_fp64(S, K, N):
         assert bool(((got.double() - want).abs() <= bound).all())
         assert torch.equal(got, gemm.dense(a, b)), "the order of the sums is fixed"
     gemm.check_status()
+
+
+# more tiles than CTAs: the token-major kernel takes them, with the same sums
+@pytest.mark.parametrize("S,K,N", [(4096, 264, 1000), (20000, 512, 264), (2500, 1024, 4104), (40000, 64, 72)])
+def test_large_products(S, K, N):
+    from moonep_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(S + K + N)
+    a = torch.randn(S, K, device="cuda", generator=g).bfloat16()
+    b = torch.randn(K, N, device="cuda", generator=g).bfloat16()
+    bt = b.t().contiguous()
+    want = a.double() @ b.double()
+    bound = 2.0 ** -24 * K ** 0.5 * (a.double().abs() @ b.double().abs()) + 1e-30
+    got = gemm.dense(a, b)
+    assert bool(((got.double() - want).abs() <= bound).all())
+    assert torch.equal(gemm.dense(a, bt, b_is_kn=False), got)
+    for r in (0, S // 2, S - 100):       # a few of its rows alone fit the other kernel
+        assert torch.equal(gemm.dense(a[r:r + 100].contiguous(), b), got[r:r + 100])
+    gemm.check_status()
