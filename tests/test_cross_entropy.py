@@ -6,6 +6,13 @@ import torch.nn.functional as F
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def _kernel_at_all_sizes(monkeypatch):
+    from moonep_b200.ops import elementwise as ew
+    monkeypatch.setattr(ew, "CE_MIN_CLASSES", 0)
+    monkeypatch.setattr(ew, "CE_MIN_LOGITS", 0)
+
+
 # one class, rows below and above a block's stride, vector and scalar rows (odd classes, odd start)
 @pytest.mark.parametrize("S,V,offset", [(1, 1, 0), (3, 8, 0), (5, 33, 0), (7, 4096, 0), (64, 4104, 0), (16, 32000, 0),
                                         (9, 50257, 0), (4, 64, 3)])
@@ -123,3 +130,16 @@ def test_odd_values_in_scalar_rows(V, offset):
         assert torch.equal(torch.isnan(a.grad), torch.isnan(b.grad))
         if r >= 4:
             assert abs(float(got.detach()) - float(want.detach())) <= 1e-5 * (1 + abs(float(want.detach())))
+
+
+def test_small_logits_take_the_general_path(monkeypatch):
+    from moonep_b200 import _native as nat
+    from moonep_b200.ops import elementwise as ew
+    monkeypatch.setattr(ew, "CE_MIN_CLASSES", 1000)
+    monkeypatch.setattr(ew, "CE_MIN_LOGITS", 1 << 23)
+    for S, V, kernel in ((16384, 512, False), (100, 32000, False), (263, 32000, True), (8389, 1000, True)):
+        x, t = torch.randn(S, V, device="cuda").bfloat16(), torch.randint(0, V, (S,), device="cuda")
+        before = nat.LAUNCHES
+        got, want = ew.cross_entropy(x, t), F.cross_entropy(x.float(), t)
+        assert (nat.LAUNCHES > before) == kernel
+        assert abs(float(got) - float(want)) <= 1e-5 * (1 + abs(float(want)))
