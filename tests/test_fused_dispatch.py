@@ -66,6 +66,52 @@ def test_fused_dispatch_gateup_matches_unfused(H, Hp):
     buf.destroy()
 
 
+@pytest.mark.parametrize("two", [0, 1])
+@pytest.mark.parametrize("S,H,Hp", [(384, 512, 256), (40, 2048, 192)])
+def test_padding_ranges_beside_the_fused_dispatch(S, H, Hp, two, monkeypatch):
+    """As the layer launches it: the rows still travel while the tiles are cut by the plan's padding ranges, and a
+    second launch takes the groups behind the first ones."""
+    from moonep_b200 import Buffer
+    from moonep_b200.ops import gemm
+    monkeypatch.setattr(gemm, "TWO_CTA", two)
+    K, E, first = 4, 12, 5
+    buf = Buffer(S, H, K, E, 1, num_sms=8, token_padding=128, timeout_s=5.0)
+    topk, w, tpe = _routing(S, K, E, 17)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, dy = (torch.randn(S, H, device="cuda", generator=g).bfloat16() for _ in range(2))
+    wg, wu, wd = ((torch.randn(E, H, Hp, device="cuda", generator=g) * 0.05).bfloat16() for _ in range(3))
+    hid0, w0, cu0, plan0 = buf.dispatch(x, w, topk, tpe)
+    rows = int(cu0[-1])
+    want = gemm.gateup_swiglu(hid0, wg, wu, cu0[:E], row_scale=w0)                # nothing told about padding
+    want_d = gemm.down_dgrad(buf.dispatch(dy, plan=plan0)[0], wd, cu0[:E])
+    torch.cuda.synchronize()
+    new = lambda: torch.full((buf.NvS, Hp), float("nan"), dtype=torch.bfloat16, device="cuda")
+    for cut in (E, first):
+        buf.hidden_nvsh_buffer_view.fill_(7.0)
+        hid, wv, cu, plan, disp = buf.dispatch_fused_begin(x, w, topk, tpe)
+        out, kw = (new(), new(), new()), dict(row_scale=wv, pads=plan.zero_fill_ranges)
+        got = gemm.gateup_swiglu(hid, wg, wu, cu[:cut], out=out, dispatch=disp, **kw)
+        if cut < E:
+            got = gemm.gateup_swiglu(hid, wg, wu, cu[:E], out=out, g_begin=cut, dispatch=dict(disp, mode=1), **kw)
+        buf.dispatch_fused_end(plan, disp)
+        buf.check()
+        gemm.check_status()
+        assert torch.equal(hid[:rows], hid0[:rows])
+        for a, b in zip(got, want):
+            assert torch.equal(a[:rows], b[:rows])
+        buf.hidden_nvsh_buffer_view.fill_(-3.0)
+        d, _, _, _, disp = buf.dispatch_fused_begin(dy, plan=plan)
+        out = new()
+        gemm.down_dgrad(d, wd, cu0[:cut], out=out, dispatch=disp, pads=plan.zero_fill_ranges)
+        if cut < E:
+            gemm.down_dgrad(d, wd, cu0[:E], out=out, g_begin=cut, dispatch=dict(disp, mode=1), pads=plan.zero_fill_ranges)
+        buf.dispatch_fused_end(plan, disp)
+        buf.check()
+        gemm.check_status()
+        assert torch.equal(out[:rows], want_d[:rows])
+    buf.destroy()
+
+
 def test_send_order_is_the_documented_permutation():
     from moonep_b200 import Buffer
     S, H, K, R = 128, 256, 4, 4

@@ -81,3 +81,49 @@ def test_ragged_groups(H, Hp, pad, with_pads, two, monkeypatch):
         gemm.wgrad(x, a, cu, l1, grad_slot=s1, split=split, pads=pads)
         assert torch.equal(l0, l1) and torch.equal(s0, s1)
     gemm.check_status()
+
+
+@pytest.mark.parametrize("two", [0, 1])
+@pytest.mark.parametrize("pad,with_pads", [(64, True), (128, False), (1, False)])
+@pytest.mark.parametrize("H,Hp", [(256, 192), (640, 64), (328, 128)])
+def test_pushed_rows_of_ragged_groups(H, Hp, pad, with_pads, two, monkeypatch):
+    """The push epilogue stores what the plain one stores, each real row at its entry's slot, and nothing else."""
+    from moonep_b200.ops import gemm
+    monkeypatch.setattr(gemm, "TWO_CTA", two)
+    g = torch.Generator(device="cuda").manual_seed(H + pad)
+    G, split, ranks = len(VALID), 9, 3
+    padded = torch.tensor([(v + pad - 1) // pad * pad for v in VALID])
+    ends = padded.cumsum(0)
+    starts, rows, n_real = (ends - padded).tolist(), int(ends[-1]), sum(VALID)
+    cu = ends.to(torch.int32).cuda()
+    pads = torch.tensor([[s + v, n - v] if n > v else [0, 0] for s, v, n in zip(starts, VALID, padded.tolist())],
+                        dtype=torch.int32).cuda()
+    real = torch.cat([torch.arange(s, s + v) for s, v in zip(starts, VALID)]).cuda()
+    entries = n_real // ranks + 40                        # (of which some get no row)
+    slots = torch.randperm(ranks * entries, device="cuda", generator=g)[:n_real]
+    src = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+    src[real] = slots.to(torch.int32)
+    stride = entries * H + 64                             # elements between the ranks' staging buffers
+
+    def mk(*shape, std=1.0):
+        return (torch.randn(*shape, device="cuda", generator=g) * std).bfloat16()
+
+    a, dg, du = mk(rows, Hp), mk(rows, Hp), mk(rows, Hp)
+    for t in (a, dg, du):
+        t[src < 0] = 0
+    wd, wg, wu = (mk(G, H, Hp, std=0.05) for _ in range(3))
+    sl = lambda w: (w[:split].contiguous(), w[split:].contiguous())
+    (wd0, wd1), (wg0, wg1), (wu0, wu1) = sl(wd), sl(wg), sl(wu)
+    kw = dict(split=split, pads=pads if with_pads else None)
+    down = lambda **k: gemm.down(a, wd0, cu, wd_slot=wd1, **kw, **k)
+    dgrad = lambda **k: gemm.gateup_dgrad(dg, du, wg0, wu0, cu, wg_slot=wg1, wu_slot=wu1, **kw, **k)
+    for op in (down, dgrad):
+        staging = torch.full((ranks, stride), float("nan"), dtype=torch.bfloat16, device="cuda")
+        assert op(push=dict(src_info=src, push_base=staging, push_rank_stride=stride, push_entries=entries,
+                            push_ranks=ranks)) is None
+        want = torch.full((ranks * entries, H), float("nan"), dtype=torch.bfloat16, device="cuda")
+        want[slots] = op()[real]
+        bits = lambda t: t.contiguous().view(torch.int16)
+        assert torch.equal(bits(staging[:, :entries * H]), bits(want.view(ranks, -1)))
+        assert torch.isnan(staging[:, entries * H:].float()).all()
+    gemm.check_status()
