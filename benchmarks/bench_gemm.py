@@ -42,9 +42,9 @@ def main():
     ap.add_argument("--iters", type=int, default=10)
     ap.add_argument("--only", default="")
     ap.add_argument("--ab", action="store_true",
-                    help="interleaved A/B of the kernel variants (single CTA / CTA pair, TMA-store / plain "
-                         "epilogue, weight grad with and without the fused SGD step): best of 6 rounds each, "
-                         "run back to back so that all variants see the same clocks")
+                    help="interleaved A/B of the kernel variants (single CTA / CTA pair, weight grad with and "
+                         "without the fused SGD step): best of 6 rounds each, run back to back so that all "
+                         "variants see the same clocks")
     args = ap.parse_args()
     G, rpg, H, Hp = args.groups, args.rows_per_group, args.H, args.Hp
     rows = G * rpg

@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(combine_threads(DIRECT, AW), 1) ep_combine_ker
 }
 
 // ---- pushed combine: barrier, then every rank sums the K rows its peers pushed per token -------
-// Counterpart of the pull combine for the fused path: the GEMM epilogue (grouped_gemm.cu, PUSH)
+// Counterpart of the pull combine for the fused path: the GEMM epilogue (token_gemm.cuh, PUSH)
 // already stored every result row into staging[home rank][token*K + k], so what is left is one
 // cross-rank barrier and a local, bandwidth-bound K-way fp32 sum in ascending k.  Route-weight
 // grads (backward of dispatch) ride along: each rank first pushes its per-row scalars to the

@@ -185,7 +185,8 @@ ep_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bfloat16
 // Backward: one pass, d logits = (exp(x - lse) - [x is the target]) * g / rows, rounded to bf16 once.
 // The logits are read once each way and nothing of their size is written but the gradient; as
 // cross_entropy(logits.float()) the same took an fp32 copy, two more fp32 tensors of their size and a
-// copy back.  Bound by HBM: 4096 x 32000 logits are 262 MB, 39 us a pass at the copy rate.
+// copy back.  Bound by HBM: 4096 x 32000 logits are 262 MB, 40 us forward (read) and 80 us backward (read, and as
+// much gradient written) at the copy rate.
 constexpr int CE_THREADS = 512;
 
 __device__ __forceinline__ void ce_add(float& m, float& s, float x) {

@@ -65,7 +65,7 @@ enum { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_F32 = 2, EPI_PUSH = 3 };
 constexpr int TG_BOXES = 4;
 
 struct GemmKParams {
-  CUtensorMap a[2];        // 128-row boxes (weight grad: 64 x 64)
+  CUtensorMap a;           // weight grad: token rows of A in 64 x 64 boxes
   CUtensorMap tok[2][TG_BOXES];   // token rows in boxes of 32, 64, 96 and 128 rows (token_gemm.cuh)
   CUtensorMap b[2][2];
   CUtensorMap c[2];        // weight-grad output (fp32), per allocation
@@ -79,7 +79,7 @@ struct GemmKParams {
   // travel be computed first, so that their reduce runs beside the rest of the weight grad.
   int wg_select;
   int g_begin; // groups below this index are skipped (a launch may cover a suffix of the groups)
-  int tma_out; // outputs allow 16-byte stores
+  int vec_out; // outputs allow 16-byte stores
   // weight grad fused with the SGD step: a local expert's tile is applied straight to its bf16
   // weights, w = bf16(w - lr * acc), instead of being stored as an fp32 grad.  Experts whose
   // sgd_keep flag is set (they have replicas elsewhere, whose grads must be added first) and the
@@ -274,7 +274,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
   if (warp == 0) {
     // ================= TMA producer =================
     if (lane == 0) {
-      tma_prefetch_desc(&p.a[0]);
+      tma_prefetch_desc(&p.a);
       tma_prefetch_desc(&p.b[0][0]);
       int it = 0;
       bool ok = true;
@@ -299,7 +299,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
             // this CTA's 128 columns of A (t.m0 is already its half) and its half of the B tile
 #pragma unroll
             for (int j = 0; j < 2; ++j)
-              tma_load_2d_pair(sa + j * 8192, &p.a[0], t.m0 + 64 * j, t.row0 + k0, lead_bar);
+              tma_load_2d_pair(sa + j * 8192, &p.a, t.m0 + 64 * j, t.row0 + k0, lead_bar);
 #pragma unroll
             for (int j = 0; j < 2; ++j)
               tma_load_2d_pair(sb + j * 8192, &p.b[0][0], t.n0 + 128 * crank + 64 * j, t.row0 + k0, lead_bar);
@@ -307,7 +307,7 @@ ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
             // A: [token rows][Mw cols], two 64-column blocks; B: [token rows][N cols], four
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
-              tma_load_2d(sa + j * 8192, &p.a[0], t.m0 + 64 * j, t.row0 + k0, &full[s]);
+              tma_load_2d(sa + j * 8192, &p.a, t.m0 + 64 * j, t.row0 + k0, &full[s]);
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
               tma_load_2d(sb + j * 8192, &p.b[0][0], t.n0 + 64 * j, t.row0 + k0, &full[s]);
@@ -790,9 +790,8 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
   if (d->mode == 1) {
     // weight grad: A [a_rows][Mw] and B [a_rows][N], both read as MN-major 64x64 boxes
     if (d->Mw % BM != 0) return fail(-2, "wgrad: Mw=%d must be a multiple of %d", d->Mw, BM);
-    if ((rc = make_map(&kp.a[0], d->a[0], d->a_rows, d->Mw, d->lda[0], 64, BK))) return rc;
+    if ((rc = make_map(&kp.a, d->a[0], d->a_rows, d->Mw, d->lda[0], 64, BK))) return rc;
     if ((rc = make_map(&kp.b[0][0], d->b[0][0], d->a_rows, d->N, d->ldb, 64, BK))) return rc;
-    kp.a[1] = kp.a[0]; kp.b[0][1] = kp.b[1][0] = kp.b[1][1] = kp.b[0][0];
     if (d->epi != EPI_F32) return fail(-3, "wgrad writes fp32");
     if (d->sgd_w != nullptr) {
       if (d->accumulate) return fail(-13, "wgrad: the fused SGD step cannot accumulate into existing grads");
@@ -866,7 +865,7 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
         if ((rc = make_map(&kp.b2[s][al], d->b[s][al], d->b_rows[al], d->K, d->ldb, BK, BN / 2))) return rc;
       }
     }
-  kp.tma_out = d->ldc % 8 == 0 && (((uintptr_t)d->out[0] | (uintptr_t)d->out[1] | (uintptr_t)d->out[2] |
+  kp.vec_out = d->ldc % 8 == 0 && (((uintptr_t)d->out[0] | (uintptr_t)d->out[1] | (uintptr_t)d->out[2] |
                                     (uintptr_t)d->push_base) & 15) == 0 && d->push_rank_stride % 8 == 0;
   const bool two = d->two_cta != 0 && grid >= 2;
   if (d->disp_mode != 0) {

@@ -315,7 +315,7 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
     // 8 (lane / 8 % 2) of the warp's quarter
     const uint32_t st_addr = smem_u32(&s_stage[0][0]) +
                              (uint32_t)((8 * (lane >> 4) + (lane & 7)) * TG_STAGE_ROW + q * 64 + ((lane >> 3) & 1) * 16);
-    const bool vec_ok = p.tma_out != 0;                     // outputs allow 16-byte stores
+    const bool vec_ok = p.vec_out != 0;                     // outputs allow 16-byte stores
     for (long long id = work_id0; id < total_tiles; id += work_stride, ++tile_n) {
       const TokenTile t = get((int)id);
       const int acc = tile_n & 1;
