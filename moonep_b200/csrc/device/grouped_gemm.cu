@@ -54,7 +54,6 @@ constexpr int GEMM_THREADS = 192;
 // half of the tile's columns (the read-modify-write stream of a warp is a chain of latencies:
 // accumulator load, weight block landed, update, store read; twice the warps run twice the chains)
 constexpr int GEMM_THREADS_SGD = 320;
-constexpr int GEMM_THREADS_DISP = 224;      // + the copy warp of the fused dispatch
 constexpr int MAX_GROUPS = 1024;
 // CTA-pair variant: each CTA stages A (16 KB) and half of B (16 KB) per k-block, six stages.
 constexpr int GEMM_STAGES2 = 6;
@@ -741,7 +740,7 @@ static int launch_dense_f32(const DenseParams& dp, cudaStream_t stream) {
 
 template <bool A_MN, int EPI, bool DISP>
 static int launch_token(const GemmKParams& kp, bool pair, int grid, cudaStream_t stream) {
-  const int threads = DISP ? GEMM_THREADS_DISP : GEMM_THREADS;
+  const int threads = TG_THREADS + (DISP ? 32 : 0);
   const bool coop = DISP && fused_dispatch_cooperative();
   if (pair) {
     static PairLaunch once;

@@ -15,10 +15,13 @@
 // the tokens (up to 16 KB) in one of six stages (five beside the fused dispatch's copy ring).
 //   warp 0  TMA producer (and, with the fused dispatch, 31 arrival watchers)
 //   warp 1  MMA issuer   (two 256-column TMEM accumulators)
-//   warps 2..5 epilogue: 32 tokens at a time are read as matrix fragments, rounded to bf16 and
-//           transposed by stmatrix into token rows in shared memory (double-buffered, one barrier
-//           of the four warps per 32 tokens), then leave as 256-byte (SwiGLU: 128-byte) row segments
-//   warp 6  copy warp of the fused dispatch
+//   warps 2..5, 6..9 epilogue, two sets of four that take 32 tokens in turn: they are read as matrix
+//           fragments, rounded to bf16 and transposed by stmatrix into token rows in shared memory,
+//           then leave as 256-byte (SwiGLU: 128-byte) row segments.  A step is a chain of latencies
+//           (~0.6 us for 32 tokens), which with one set was a tile's time where the reduction is short:
+//           128 groups x 256 rows, H = 1024, H' = 512, gate/up 127 -> 99 us; 280 rows, down 78 -> 68;
+//           H' = 64, 53 -> 47; long reductions the same
+//   warp 10 copy warp of the fused dispatch
 // SwiGLU: a CTA's 128 columns are 64 gate and the same 64 up columns, which meet in the staged rows.
 //
 // Measured against tokens on M (pairs; isolated launches, 32 groups, H = 7168, H' = 2048), gate/up:
@@ -31,6 +34,8 @@ namespace mep {
 
 constexpr int TG_MAX_N = 256;
 constexpr int TG_CHUNK = 32;                                  // tokens per epilogue step
+constexpr int TG_SETS = 2;                                    // sets of four epilogue warps
+constexpr int TG_THREADS = 64 + TG_SETS * 128;                // and one more warp with the fused dispatch
 constexpr int TG_STAGE_ROW = 256 + 16;                        // bytes of a staged token row: 128 columns; the rows
                                                               // of an 8x8 matrix fall into different banks
 constexpr int TG_W_BYTES = BM * BK * 2;                       // weights of a k-block, one CTA: 16 KB
@@ -61,20 +66,21 @@ __device__ __forceinline__ void store8(__nv_bfloat16* dst, const uint4& v, int l
     for (int i = 0; i < 8 && i < left; ++i) dst[i] = e[i];
   }
 }
-// Barrier of the four epilogue warps that also agrees on a condition: true if it held for all of them.
-__device__ __forceinline__ bool epilogue_all(bool mine) {
+// Barrier of a set's four epilogue warps, and one that also agrees on a condition: true if it held for all of them.
+__device__ __forceinline__ void epilogue_sync(int set) { asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory"); }
+__device__ __forceinline__ bool epilogue_all(int set, bool mine) {
   uint32_t all;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
-      "barrier.cta.red.and.aligned.pred q, 1, 128, p;\n\t"
+      "barrier.cta.red.and.aligned.pred q, %2, 128, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(all) : "r"((uint32_t)mine) : "memory");
+      : "=r"(all) : "r"((uint32_t)mine), "r"(1 + set) : "memory");
   return all != 0;
 }
 
 template <bool A_MN, int EPI, bool TWO, bool DISP>
-__global__ void __launch_bounds__(DISP ? GEMM_THREADS_DISP : GEMM_THREADS, 1)
+__global__ void __launch_bounds__(TG_THREADS + (DISP ? 32 : 0), 1)
 ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
   constexpr int NST = tg_stages<TWO, DISP>();
   constexpr int STAGE = tg_stage_bytes<TWO>();
@@ -95,7 +101,7 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
   __shared__ int s_groups_ready;
   __shared__ int s_end[MAX_GROUPS];
   __shared__ int s_prefix[MAX_GROUPS + 1];
-  __shared__ __align__(128) uint8_t s_stage[2][EPI == EPI_F32 ? 16 : TG_CHUNK * TG_STAGE_ROW];
+  __shared__ __align__(128) uint8_t s_stage[TG_SETS][EPI == EPI_F32 ? 16 : TG_CHUNK * TG_STAGE_ROW];
   // per token of a tile: address of its row at the home rank (PUSH) or its scale (SwiGLU); two tiles
   __shared__ unsigned long long s_ptr[EPI == EPI_PUSH ? 2 : 1][EPI == EPI_PUSH ? TG_MAX_N : 1];
   __shared__ float s_scale[EPI == EPI_SWIGLU ? 2 : 1][EPI == EPI_SWIGLU ? TG_MAX_N : 1];
@@ -107,7 +113,7 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
   if (tid == 0) {
     // both CTAs' loads count on the LEADER's full barrier, on which only its producer arrives
     for (int s = 0; s < NST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], TWO ? 8 : 4); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], (TWO ? 8 : 4) * TG_SETS); }
     if constexpr (DISP) for (int a = 0; a < FD_NST; ++a) mbar_init(&fd_full[a], 1);
     mbar_fence_init();
     s_abort = 0;
@@ -294,7 +300,7 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
         else umma_commit(&acc_full[acc]);
       }
     }
-  } else if (DISP && warp >= 6) {
+  } else if (DISP && warp >= 2 + 4 * TG_SETS) {
     // ================= fused dispatch: this CTA's share of the all-to-all =================
     if constexpr (DISP) {
       if (p.disp.x != nullptr) {
@@ -307,13 +313,18 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
       }
     }
   } else {
-    // ================= epilogue: four warps, one quarter of the tile's columns each =================
+    // ========= epilogue: two sets of four warps, each warp one quarter of the tile's columns =========
     const int q = warp & 3;
-    const int te = tid - 64;                                // 0..127
-    int tile_n = 0, buf = 0;
+    const int set = (warp - 2) >> 2;
+    const int te = tid - 64 - set * 128;                    // 0..127
+    // this set's chunks start at tokens first, first + step, ...; the thread's own token in one of them
+    const int first = set * TG_CHUNK, step = TG_SETS * TG_CHUNK;
+    const int my_tok = (te >> 5) * step + first + (te & 31);
+    int tile_n = 0;
     // this thread's row of the matrices that its warp stores: token 8 (lane / 16) + lane % 8, columns
     // 8 (lane / 8 % 2) of the warp's quarter
-    const uint32_t st_addr = smem_u32(&s_stage[0][0]) +
+    uint8_t* const sb = s_stage[set];
+    const uint32_t st_addr = smem_u32(sb) +
                              (uint32_t)((8 * (lane >> 4) + (lane & 7)) * TG_STAGE_ROW + q * 64 + ((lane >> 3) & 1) * 16);
     const bool vec_ok = p.vec_out != 0;                     // outputs allow 16-byte stores
     for (long long id = work_id0; id < total_tiles; id += work_stride, ++tile_n) {
@@ -321,7 +332,7 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
       const int acc = tile_n & 1;
       // home rows of this tile's tokens, looked up while the tile is still being computed
       if constexpr (EPI == EPI_PUSH) {
-        for (int i = te; i < t.n; i += 128) {
+        for (int i = my_tok; i < t.n; i += 4 * step) {
           const int si = i < t.rows ? p.src_info[t.row0 + i] : -1;
           unsigned long long dptr = 0ull;
           if (si >= 0) {
@@ -335,7 +346,7 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
       }
       const bool have = gemm_wait(&acc_full[acc], (uint32_t)(tile_n >> 1) & 1u, abortp, p, 4);
       __syncwarp();
-      if (!epilogue_all(have)) break;      // the four warps leave together: they share barriers below
+      if (!epilogue_all(set, have)) break;      // a set's four warps leave together: they share barriers below
       tc_fence_after();
       const uint32_t tacc = tmem_base + (uint32_t)acc * TG_MAX_N + ((uint32_t)(q * 32) << 16);
       uint32_t r[32];
@@ -351,28 +362,33 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
         // thread = output column: a warp's 32 columns of a token leave as one 128-byte line
         const int col = t.m0 + 128 * crank + q * 32 + lane;
 #pragma unroll 1
-        for (int c = 0; c < t.n; c += TG_CHUNK) {
+        for (int c = first; c < t.n; c += step) {
           __syncwarp();
           tmem_ld_32x32(tacc + c, r);
           tmem_ld_wait();
-          if (c + TG_CHUNK >= t.n) release_acc();
+          if (c + step >= t.n) release_acc();
           float* o = (float*)p.out[0] + (long long)(t.row0 + c) * p.ldc + col;
 #pragma unroll
           for (int i = 0; i < TG_CHUNK; ++i)
             if (c + i < t.rows && col < p.N) o[i * p.ldc] = __uint_as_float(r[i]);
         }
+        if (first >= t.n) release_acc();
         continue;
       }
-      tmem_ld_16x256_x4(tacc, r);
-      tmem_ld_16x256_x4(tacc + (16u << 16), r + 16);
+      if (first < t.n) {
+        tmem_ld_16x256_x4(tacc + first, r);
+        tmem_ld_16x256_x4(tacc + first + (16u << 16), r + 16);
+      } else {
+        release_acc();
+      }
       if constexpr (EPI == EPI_SWIGLU) {
         // (read past L1, and only now: with the fused dispatch another rank wrote the scale along with the
         // row; the first barrier below publishes it)
-        for (int i = te; i < t.n; i += 128)
+        for (int i = my_tok; i < t.n; i += 4 * step)
           s_scale[acc][i] = i < t.rows && p.row_scale != nullptr ? __ldcg(p.row_scale + t.row0 + i) : 1.f;
       }
 #pragma unroll 1
-      for (int c = 0; c < t.n; c += TG_CHUNK, buf ^= 1) {
+      for (int c = first; c < t.n; c += step) {
         __syncwarp();
         tmem_ld_wait();
         uint32_t pk[16];       // [16-column half][token block][lower, upper 8 columns]
@@ -381,24 +397,21 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
           const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
           pk[i] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        if (c + TG_CHUNK < t.n) {        // the next 32 tokens travel while these leave
-          tmem_ld_16x256_x4(tacc + c + TG_CHUNK, r);
-          tmem_ld_16x256_x4(tacc + c + TG_CHUNK + (16u << 16), r + 16);
+        if (c + step < t.n) {            // the next 32 tokens travel while these leave
+          tmem_ld_16x256_x4(tacc + c + step, r);
+          tmem_ld_16x256_x4(tacc + c + step + (16u << 16), r + 16);
         } else {
           release_acc();
         }
-        uint8_t* sb = s_stage[buf];
         __syncwarp();
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
           for (int j = 0; j < 4; j += 2)
-            stmatrix_x4_trans(st_addr + (uint32_t)(buf * (TG_CHUNK * TG_STAGE_ROW) + j * 8 * TG_STAGE_ROW + h * 32),
+            stmatrix_x4_trans(st_addr + (uint32_t)(j * 8 * TG_STAGE_ROW + h * 32),
                               pk[8 * h + 2 * j], pk[8 * h + 2 * j + 1], pk[8 * h + 2 * j + 2], pk[8 * h + 2 * j + 3]);
-        // One barrier per step: a thread that fills this buffer again (two steps on) has passed the
-        // barrier in between, which every reader of this step reaches only after its reads.
         __syncwarp();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        epilogue_sync(set);
         if constexpr (EPI == EPI_SWIGLU) {
           const int f = (te & 7) * 8, col0 = t.m0 + 64 * crank + f;
 #pragma unroll
@@ -440,12 +453,13 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
             }
           }
         }
+        epilogue_sync(set);              // every row of the set's buffer has been read: it may be filled again
       }
       if constexpr (EPI != EPI_PUSH) {      // padding rows that no tile computes
         constexpr int V = EPI == EPI_SWIGLU ? 8 : 16;      // vectors of this CTA's columns in a row
         const int f = (te & (V - 1)) * 8, col0 = t.m0 + V * 8 * crank + f;
         if (col0 < p.N)
-          for (int r = t.row0 + t.rows + te / V; r < t.zero_to; r += 128 / V) {
+          for (int r = t.row0 + t.rows + (te + 128 * set) / V; r < t.zero_to; r += 128 * TG_SETS / V) {
             const long long off = (long long)r * p.ldc + col0;
 #pragma unroll
             for (int o = 0; o < (EPI == EPI_SWIGLU ? 3 : 1); ++o)
