@@ -11,6 +11,22 @@
 
 namespace mep {
 
+// True in one lane of a converged warp (the same one each time).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+
+// Position in a ring of slots, and the parity of its round.
+struct RingSlot {
+  int slot = 0;
+  uint32_t parity = 0;
+  __device__ __forceinline__ void next(int slots) {
+    if (++slot == slots) { slot = 0; parity ^= 1u; }
+  }
+};
+
 // ---- TMEM ------------------------------------------------------------------------------------
 // One full warp allocates `ncols` (power of two, 32..512) columns; the base address lands in
 // shared memory.  The same warp must free them before the CTA exits.

@@ -106,7 +106,7 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
   __shared__ unsigned long long s_ptr[EPI == EPI_PUSH ? 2 : 1][EPI == EPI_PUSH ? TG_MAX_N : 1];
   __shared__ float s_scale[EPI == EPI_SWIGLU ? 2 : 1][EPI == EPI_SWIGLU ? TG_MAX_N : 1];
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   uint8_t* stages = (uint8_t*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   volatile int* abortp = &s_abort;
 
@@ -177,20 +177,40 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
     return t;
   };
   const int kb_per_seg = (p.K + BK - 1) / BK;
-  const int num_kb = p.nseg * kb_per_seg;
+  // The producer's and the issuer's warps walk their loops as a whole and one lane issues: loop state and
+  // descriptors then live in uniform registers.  With the loops in a single lane's branch, the issuer took
+  // longer for a k-block than the tensor cores and set the rate.  Isolated launches, H = 7168, H' = 2048, us:
+  // 128 groups of 256 rows on average, gate/up 1980 -> 1765, down 1165 -> 1070; 32 groups of 1024, 1530 -> 1440
+  // and 850 -> 750; 16 tokens on 32 experts (a stream of the weights) 344 -> 304 and 178 -> 172.
+  // A wait has the same outcome in every lane, so that the warp leaves its loops together.  (Beside the
+  // arrival watchers of the fused dispatch the producer is one lane.)
+  auto warp_wait = [&](uint64_t* bar, uint32_t parity, int where) {
+    return __all_sync(0xffffffffu, gemm_wait(bar, parity, abortp, p, where)) != 0;
+  };
 
   if (warp == 0) {
     // ================= TMA producer =================
-    if (lane == 0) {
-      tma_prefetch_desc(&p.tok[0][TG_BOXES - 1]);
-      tma_prefetch_desc(A_MN ? &p.b[0][0] : &p.b2[0][0]);
-      int it = 0;
+    if (!DISP || lane == 0) {
+      const bool issue = DISP || elect_one();
+      if (issue) {
+        tma_prefetch_desc(&p.tok[0][TG_BOXES - 1]);
+        tma_prefetch_desc(A_MN ? &p.b[0][0] : &p.b2[0][0]);
+      }
+      RingSlot st;
       bool ok = true;
       int groups_ready = 0;
       if constexpr (DISP) phase_stamp(p.trace, 2, (int)blockIdx.x, 0);
       bool stamped_first = false;
       for (long long id = work_id0; id < total_tiles && ok; id += work_stride) {
-        const TokenTile t = get((int)id);
+        TokenTile t = get((int)id);
+        if constexpr (!DISP) {
+          // (the same in every lane: said so)
+          t.alloc = __shfl_sync(0xffffffffu, t.alloc, 0);
+          t.g_local = __shfl_sync(0xffffffffu, t.g_local, 0);
+          t.row0 = __shfl_sync(0xffffffffu, t.row0, 0);
+          t.n = __shfl_sync(0xffffffffu, t.n, 0);
+          t.m0 = __shfl_sync(0xffffffffu, t.m0, 0);
+        }
         if constexpr (DISP) {
           // wait for the tile's whole GROUP, published by the watchers below: CTAs then enter a group
           // together and share its rows and weights in L2
@@ -218,11 +238,15 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
         const CUtensorMap* tmap = &p.tok[0][0] + (box - 1);
         const uint32_t bytes = (uint32_t)(TG_W_BYTES + box * (!TWO && tok > 128 ? 64 : 32) * BK * 2) * (TWO ? 2u : 1u);
         const int erow = t.g_local * p.rows_per_expert;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % NST;
-          if (it >= NST && !gemm_wait(&empty[s], ((uint32_t)(it / NST) & 1u) ^ 1u, abortp, p, 1)) { ok = false; break; }
+        for (int seg = 0; seg < p.nseg && ok; ++seg)
+        for (int k0 = 0; k0 < p.K; k0 += BK, st.next(NST)) {
+          const int s = st.slot;
+          if constexpr (DISP) ok = gemm_wait(&empty[s], st.parity ^ 1u, abortp, p, 1);
+          else ok = warp_wait(&empty[s], st.parity ^ 1u, 1);
+          if (!ok) break;
+          if (!issue) continue;
           uint8_t* sw = stages + (size_t)s * STAGE;
-          uint8_t* st = sw + TG_W_BYTES;
+          uint8_t* stok = sw + TG_W_BYTES;
           uint32_t lead_bar = 0;
           if constexpr (TWO) lead_bar = mapa_u32(&full[s], 0);
           if (crank == 0) mbar_expect_tx(&full[s], bytes);
@@ -230,8 +254,6 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
             if constexpr (TWO) tma_load_2d_pair(dst, map, x, y, lead_bar);
             else tma_load_2d(dst, map, x, y, &full[s]);
           };
-          const int seg = kb / kb_per_seg;
-          const int k0 = (kb - seg * kb_per_seg) * BK;
           if constexpr (A_MN) {            // weights [K rows][N columns]: two blocks of 64 columns
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -243,8 +265,8 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
           } else {                         // weights [N rows][K columns]: 128 rows
             load(sw, &p.b2[seg][t.alloc], k0, erow + t.m0 + 128 * crank);
           }
-          load(st, tmap + seg * TG_BOXES, k0, trow);
-          if (!TWO && tok > 128) load(st + 128 * 128, tmap + seg * TG_BOXES, k0, trow + 128);
+          load(stok, tmap + seg * TG_BOXES, k0, trow);
+          if (!TWO && tok > 128) load(stok + 128 * 128, tmap + seg * TG_BOXES, k0, trow + 128);
         }
       }
       if constexpr (DISP) phase_stamp(p.trace, 2, (int)blockIdx.x, 2);
@@ -267,37 +289,46 @@ ep_token_gemm_kernel(const __grid_constant__ GemmKParams p) {
     }
   } else if (warp == 1) {
     // ================= MMA issuer (the leader issues for both CTAs of a pair) =================
-    if (lane == 0 && crank == 0) {
-      int it = 0, tile_n = 0;
+    if (crank == 0) {
+      const bool issue = elect_one();
+      const int num_kb = p.nseg * kb_per_seg;
+      // descriptors of slot 0; a slot further, and a k-step of 16, add to the address field
+      const uint64_t desc_w = A_MN ? make_smem_desc(smem_u32(stages), 8192, 1024) : make_smem_desc(smem_u32(stages), 16, 1024);
+      const uint64_t desc_t = make_smem_desc(smem_u32(stages) + TG_W_BYTES, 16, 1024);
+      constexpr int W_STEP = (A_MN ? 2048 : 32) >> 4, T_STEP = 32 >> 4;
+      RingSlot st;
+      int tile_n = 0;
       bool ok = true;
+      auto tokens = [&](long long id) { return __shfl_sync(0xffffffffu, id < total_tiles ? get((int)id).n : 0, 0); };
+      int n = tokens(work_id0);
       for (long long id = work_id0; id < total_tiles && ok; id += work_stride, ++tile_n) {
-        const TokenTile t = get((int)id);
-        const uint32_t idesc = make_instr_desc_bf16(TM, t.n, A_MN, false);
+        const uint32_t idesc = make_instr_desc_bf16(TM, n, A_MN, false);
         const int acc = tile_n & 1;
-        if (tile_n >= 2 &&
-            !gemm_wait<TWO>(&acc_empty[acc], ((uint32_t)(tile_n >> 1) & 1u) ^ 1u, abortp, p, 2)) break;
+        if (!warp_wait(&acc_empty[acc], ((uint32_t)(tile_n >> 1) & 1u) ^ 1u, 2)) break;
         tc_fence_after();
         const uint32_t tacc = tmem_base + (uint32_t)acc * TG_MAX_N;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % NST;
-          if (!gemm_wait(&full[s], (uint32_t)(it / NST) & 1u, abortp, p, 3)) { ok = false; break; }
+        for (int kb = 0; kb < num_kb; ++kb, st.next(NST)) {
+          const int s = st.slot;
+          ok = warp_wait(&full[s], st.parity, 3);
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t sw = smem_u32(stages + (size_t)s * STAGE);
-          const uint32_t st = sw + TG_W_BYTES;
+          if (issue) {
+            const uint64_t da = desc_w + (uint32_t)(s * (STAGE >> 4)), db = desc_t + (uint32_t)(s * (STAGE >> 4));
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = A_MN ? make_smem_desc(sw + kk * 2048, 8192, 1024)
-                                     : make_smem_desc(sw + kk * 32, 16, 1024);
-            const uint64_t db = make_smem_desc(st + kk * 32, 16, 1024);
-            if constexpr (TWO) umma_bf16_2cta(tacc, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-            else umma_bf16(tacc, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < BK / 16; ++kk) {
+              if constexpr (TWO) umma_bf16_2cta(tacc, da + kk * W_STEP, db + kk * T_STEP, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+              else umma_bf16(tacc, da + kk * W_STEP, db + kk * T_STEP, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            }
+            if constexpr (TWO) umma_commit_2cta(&empty[s], 3);
+            else umma_commit(&empty[s]);
           }
-          if constexpr (TWO) umma_commit_2cta(&empty[s], 3);
-          else umma_commit(&empty[s]);
+          if (kb == 0) n = tokens(id + work_stride);       // (looked up while the tile is being computed)
         }
         if (!ok) break;
-        if constexpr (TWO) umma_commit_2cta(&acc_full[acc], 3);
-        else umma_commit(&acc_full[acc]);
+        if (issue) {
+          if constexpr (TWO) umma_commit_2cta(&acc_full[acc], 3);
+          else umma_commit(&acc_full[acc]);
+        }
       }
     }
   } else if (DISP && warp >= 2 + 4 * TG_SETS) {
