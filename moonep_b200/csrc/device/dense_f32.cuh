@@ -2,12 +2,12 @@
 // CTAs hold at once go to the token-major kernel.)
 //
 // The output is small (S x experts) and the reduction long: a CTA walks up to 112 k-blocks one after
-// the other, ~0.4 us each, bound by that chain and not by bytes.  The experts take the M side (128 a
+// the other, ~0.2 us each, bound by that chain and not by bytes.  The experts take the M side (128 a
 // tile) and the tokens the N side, in as small a tile as fills the SMs once (4096 tokens are 128 CTAs
-// of 32), with up to sixteen stages in flight.  Against tokens on M (32 CTAs, 256-column tiles):
-// 4096 x 2048 -> 128 experts 23.4 -> 17.7 us, 509 x 1024 -> 32 12.6 -> 10.2; at K = 7168 the same
-// (48 us for 16 tokens).  The reduction is NOT split, which would take those 48 us to 10: routing compares
-// these sums, and another order of the additions sends tokens at a tie elsewhere.
+// of 32), with up to sixteen stages in flight.  Loads and MMAs are issued by one lane of a converged warp,
+// which halved the chain: K = 7168 50 -> 25 us for 16 tokens and 52 -> 27 for 4096, 4096 x 2048 -> 128
+// experts 18.8 -> 15.2.  The reduction is NOT split: routing compares these sums, and another order of the
+// additions sends tokens at a tie elsewhere.
 #pragma once
 
 namespace mep {
@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) ep_dense_f32_kernel(const __gri
   __shared__ __align__(8) uint64_t acc_full;
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   uint8_t* ring = (uint8_t*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   volatile int* abortp = &s_abort;
   const int row0 = (int)blockIdx.x * p.tok, m0 = (int)blockIdx.y * BM;
@@ -54,42 +54,52 @@ __global__ void __launch_bounds__(DN_THREADS, 1) ep_dense_f32_kernel(const __gri
   tc_fence_after();
   const uint32_t tmem_base = s_tmem;
 
+  // a wait has the same outcome in every lane: a warp walks its loop as a whole, one lane issues
+  auto warp_wait = [&](uint64_t* bar, uint32_t parity, int where) {
+    return __all_sync(0xffffffffu, gemm_wait(bar, parity, abortp, p, where)) != 0;
+  };
   if (warp == 0) {
-    if (lane == 0) {
+    const bool issue = elect_one();
+    if (issue) {
       tma_prefetch_desc(&p.x);
       tma_prefetch_desc(&p.w);
-      for (int kb = 0; kb < p.num_kb; ++kb) {
-        const int s = kb % p.stages;
-        if (kb >= p.stages && !gemm_wait(&empty[s], ((uint32_t)(kb / p.stages) & 1u) ^ 1u, abortp, p, 1)) break;
-        uint8_t* sw = ring + (size_t)s * stage_bytes;
-        mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
-        if constexpr (W_MN) {
-          for (int j = 0; j < p.m_rows / 64; ++j) tma_load_2d(sw + j * 8192, &p.w, m0 + 64 * j, kb * BK, &full[s]);
-        } else {
-          tma_load_2d(sw, &p.w, kb * BK, m0, &full[s]);
-        }
-        tma_load_2d(sw + w_bytes, &p.x, kb * BK, row0, &full[s]);
+    }
+    RingSlot st;
+    for (int kb = 0; kb < p.num_kb; ++kb, st.next(p.stages)) {
+      const int s = st.slot;
+      if (!warp_wait(&empty[s], st.parity ^ 1u, 1)) break;
+      if (!issue) continue;
+      uint8_t* sw = ring + s * stage_bytes;
+      mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
+      if constexpr (W_MN) {
+        for (int j = 0; j < p.m_rows / 64; ++j) tma_load_2d(sw + j * 8192, &p.w, m0 + 64 * j, kb * BK, &full[s]);
+      } else {
+        tma_load_2d(sw, &p.w, kb * BK, m0, &full[s]);
       }
+      tma_load_2d(sw + w_bytes, &p.x, kb * BK, row0, &full[s]);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = make_instr_desc_bf16(BM, p.tok, W_MN, false);
-      bool ok = true;
-      for (int kb = 0; kb < p.num_kb; ++kb) {
-        const int s = kb % p.stages;
-        if (!gemm_wait(&full[s], (uint32_t)(kb / p.stages) & 1u, abortp, p, 3)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t sw = smem_u32(ring + (size_t)s * stage_bytes), sx = sw + (uint32_t)w_bytes;
+    const bool issue = elect_one();
+    const uint32_t idesc = make_instr_desc_bf16(BM, p.tok, W_MN, false);
+    // (64 experts: the descriptor's second block of columns / rows is the token part of the stage)
+    const uint64_t desc_w = W_MN ? make_smem_desc(smem_u32(ring), 8192, 1024) : make_smem_desc(smem_u32(ring), 16, 1024);
+    const uint64_t desc_x = make_smem_desc(smem_u32(ring) + w_bytes, 16, 1024);
+    constexpr int W_STEP = (W_MN ? 2048 : 32) >> 4, X_STEP = 32 >> 4;
+    RingSlot st;
+    bool ok = true;
+    for (int kb = 0; kb < p.num_kb; ++kb, st.next(p.stages)) {
+      ok = warp_wait(&full[st.slot], st.parity, 3);
+      if (!ok) break;
+      tc_fence_after();
+      if (issue) {
+        const uint64_t dw = desc_w + (uint32_t)(st.slot * (stage_bytes >> 4)), dx = desc_x + (uint32_t)(st.slot * (stage_bytes >> 4));
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk) {
-          // (64 experts: the descriptor's second block of columns / rows is the token part of the stage)
-          const uint64_t dw = W_MN ? make_smem_desc(sw + kk * 2048, 8192, 1024) : make_smem_desc(sw + kk * 32, 16, 1024);
-          umma_bf16(tmem_base, dw, make_smem_desc(sx + kk * 32, 16, 1024), idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-        }
-        umma_commit(&empty[s]);
+        for (int kk = 0; kk < BK / 16; ++kk)
+          umma_bf16(tmem_base, dw + kk * W_STEP, dx + kk * X_STEP, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(&empty[st.slot]);
       }
-      if (ok) umma_commit(&acc_full);
     }
+    if (ok && issue) umma_commit(&acc_full);
   } else {
     // thread = expert: a token's 32 logits of a warp leave as one 128-byte line
     const int q = warp & 3;
