@@ -12,22 +12,15 @@
 //        SwiGLU, down, both dgrads, the pushed combine, the fused dispatch.
 //        Also large products with fp32 output.
 //   ep_dense_f32_kernel (dense_f32.cuh): one product with fp32 output (router logits).
-//   ep_grouped_gemm_kernel (this file): weight-grad (groups partition the REDUCTION dimension):
-//        D[g] (+)= A[rows of g]^T * B[rows of g]   both operands MN-major, fp32 output by TMA
-//        store / reduce-add; or (template SGD) the optimizer step fused in: the accumulator is
-//        applied straight to the bf16 weights, w = bf16(w - lr * acc), through a per-warp TMA
-//        ring of weight blocks, for every local expert that has no replica this step.  Those
-//        kernels run eight epilogue warps (two per quarter of the accumulator's lanes, one half
-//        of the columns each) and take their split of the shared memory at launch.
+//   ep_weight_grad_kernel (weight_grad.cuh): weight grads, fp32 output or with the SGD step in the epilogue.
 // Group g < split reads/writes allocation 0 (local experts), g >= split allocation 1 (this
 // rank's prefetch / reduce slots): the [2*epn] compute view never has to be contiguous.
 // CTA pairs (template TWO, clusters of two CTAs, tcgen05 cta_group::2): the leader issues
 // 256-row MMAs over both CTAs' shared memory; each CTA stages its own 128 rows of A and half
-// of the B tile (32 KB per k-block instead of 48 KB, six stages), which lifts the single-CTA
-// kernel's limit of 12 KB of operand reads per MMA.  Both CTAs' loads count on the LEADER's full
+// of the B tile (32 KB per k-block instead of 48 KB), which lifts the single-CTA kernel's limit of
+// 12 KB of operand reads per MMA.  Both CTAs' loads count on the LEADER's full
 // barrier, on which only the leader's producer arrives (expecting the bytes of both): a per-stage
-// arrival from the peer over the cluster network measured 2x slower overall.  Weight-grad pairs
-// cover 256 rows of the weight matrix (+24% over single CTAs, 32 groups x 1024 rows, H=7168, H'=2048).
+// arrival from the peer over the cluster network measured 2x slower overall.
 // Every mbarrier wait is bounded; on expiry the CTA records an error, drains and frees TMEM.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -45,34 +38,25 @@
 namespace mep {
 void* driver_tensor_map_encode();
 
-constexpr int BM = 128, BN = 256, BK = 64, GEMM_STAGES = 4;
-constexpr int A_TILE_BYTES = BM * BK * 2;   // 16 KB
-constexpr int B_TILE_BYTES = BN * BK * 2;   // 32 KB
-constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
-constexpr int GEMM_THREADS = 192;
-// SGD kernels: eight epilogue warps, two per quarter of the accumulator's lanes, each with one
-// half of the tile's columns (the read-modify-write stream of a warp is a chain of latencies:
-// accumulator load, weight block landed, update, store read; twice the warps run twice the chains)
-constexpr int GEMM_THREADS_SGD = 320;
+constexpr int BM = 128, BN = 256, BK = 64;
 constexpr int MAX_GROUPS = 1024;
-// CTA-pair variant: each CTA stages A (16 KB) and half of B (16 KB) per k-block, six stages.
-constexpr int GEMM_STAGES2 = 6;
-constexpr int STAGE_BYTES2 = A_TILE_BYTES + B_TILE_BYTES / 2;
 
 enum { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_F32 = 2, EPI_PUSH = 3 };
 
 constexpr int TG_BOXES = 4;
 
 struct GemmKParams {
-  CUtensorMap a;           // weight grad: token rows of A in 64 x 64 boxes
+  CUtensorMap a;           // weight grad: token rows of A in 64 x 64 boxes (and of B, in b)
   CUtensorMap tok[2][TG_BOXES];   // token rows in boxes of 32, 64, 96 and 128 rows (token_gemm.cuh)
   CUtensorMap b[2][2];
-  CUtensorMap c[2];        // weight-grad output (fp32), per allocation
   CUtensorMap b2[2][2];    // K-major B with a 128-row box
   const int32_t* cu_seqlens;
   const int32_t* pads;     // [ngroups][2] first padding row and their number, per group; or null
   int ngroups, split, total_rows, N, K, nseg, rows_per_expert, Mw, accumulate, zero_empty_below;
-  int stages, wb;   // SGD kernels: operand stages and weight blocks per epilogue warp of this launch
+  // weight grad: tiles of a unit; slots of the shared memory for k-blocks of rows and of columns, and for
+  // weight pieces of an epilogue warp (SGD)
+  int unit, row_slots, col_slots, pieces;
+  int vec32;   // weight grad: rows of the weights allow 32-byte accesses
   // SGD kernels: 1 = only the tiles whose grads are STORED (experts with replicas, slot groups),
   // 2 = only the tiles that are applied to the weights, 0 = all.  Lets the grads that have to
   // travel be computed first, so that their reduce runs beside the rest of the weight grad.
@@ -84,7 +68,7 @@ struct GemmKParams {
   // sgd_keep flag is set (they have replicas elsewhere, whose grads must be added first) and the
   // slot groups are still written as fp32 grads.
   __nv_bfloat16* sgd_w;
-  CUtensorMap wmap;        // the same weights as a [G0 * Mw][N] bf16 tensor, 32-row x 64-column boxes, 128B swizzle
+  CUtensorMap wmap;        // the same weights as a [G0 * Mw][N] bf16 tensor, 16-row x 64-column boxes
   const int32_t* sgd_keep;
   float sgd_lr;
   void* out[3];
@@ -105,21 +89,13 @@ struct GemmKParams {
   unsigned long long arrive_timeout_ns;
 };
 
-struct Tile {
-  int g, row0, rows, n0, num_kb, alloc, g_local, m0;
-  bool valid;
-};
-
-// CLUSTER: the barrier also receives plain arrivals from the pair's other CTA, so the wait
-// acquires at cluster scope.  Barriers completed by TMA byte counts or tcgen05.commit do not need it.
-template <bool CLUSTER = false, class Params>
+template <class Params>
 __device__ __forceinline__ bool gemm_wait(uint64_t* bar, uint32_t parity, volatile int* s_abort,
                                           const Params& p, int where) {
-  auto ready = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
-  if (ready()) return true;
+  if (mbar_try_wait(bar, parity)) return true;
   unsigned long long t0 = globaltimer_ns();
   unsigned spins = 0;
-  while (!ready()) {
+  while (!mbar_try_wait(bar, parity)) {
     if ((++spins & 255u) == 0) {
       if (*s_abort) return false;
       if (globaltimer_ns() - t0 > p.timeout_ns) {
@@ -173,359 +149,11 @@ __device__ __forceinline__ int group_valid(const GemmKParams& p, int g, int star
   return (n > 0 && first >= start && first < end) ? max(1, first - start) : end - start;
 }
 
-template <bool TWO>
-__device__ __forceinline__ Tile get_tile(const GemmKParams& p, int id, const int* s_end, const int* s_valid,
-                                         int n_tiles_n, int crank = 0) {
-  Tile t;
-  t.valid = true;
-  constexpr int TMW = TWO ? 2 * BM : BM;       // a pair owns 256 rows of the weight matrix
-  const int mt = p.Mw / TMW;
-  const int tpg = mt * n_tiles_n;
-  t.g = id / tpg;
-  int local = id - t.g * tpg;
-  int mi = local / n_tiles_n, ni = local - mi * n_tiles_n;
-  t.row0 = t.g == 0 ? 0 : s_end[t.g - 1];
-  t.rows = s_valid[t.g];                       // padding rows are zero: blocks of nothing else are skipped
-  t.m0 = mi * TMW + crank * BM;
-  t.n0 = ni * BN;
-  t.num_kb = (t.rows + BK - 1) / BK;
-  if (t.rows <= 0 && t.g >= p.zero_empty_below) t.valid = false;
-  if (t.rows <= 0 && p.sgd_w != nullptr && t.g < p.split &&
-      (p.sgd_keep == nullptr || p.sgd_keep[t.g] == 0)) t.valid = false;   // zero grad: nothing to apply
-  if (t.g < p.g_begin) t.valid = false;
-  t.alloc = t.g >= p.split ? 1 : 0;
-  t.g_local = t.alloc ? t.g - p.split : t.g;
-  if (p.wg_select != 0 && p.sgd_w != nullptr) {
-    const bool applied = t.alloc == 0 && (p.sgd_keep == nullptr || p.sgd_keep[t.g_local] == 0);
-    if ((p.wg_select == 2) != applied) t.valid = false;
-  }
-  return t;
-}
-
-// Operand stages of the kernels whose geometry is fixed at compile time.
-template <bool TWO> __host__ __device__ constexpr int gemm_stages() { return TWO ? GEMM_STAGES2 : GEMM_STAGES; }
-// The SGD kernels (weight grad with the optimizer step in the epilogue) take their geometry at
-// launch instead (GemmKParams::stages / wb, sgd_geometry() below): how the shared memory is best
-// split between operand stages and weight blocks depends on the group length.
-constexpr int SGD_RING_MAX = 8;      // 4 KB weight blocks per epilogue warp, at most
-template <bool TWO> __host__ __device__ constexpr int gemm_smem() {   // dynamic shared memory
-  return gemm_stages<TWO>() * (TWO ? STAGE_BYTES2 : STAGE_BYTES) + 1024;
-}
-
-template <bool TWO, bool SGD>
-__global__ void __launch_bounds__(SGD ? GEMM_THREADS_SGD : GEMM_THREADS, 1)
-ep_grouped_gemm_kernel(const __grid_constant__ GemmKParams p) {
-  // operand stages: a constant, except in the SGD kernels (upper bound; p.stages are used)
-  constexpr int GEMM_STAGES = gemm_stages<TWO>();
-  const int nst = SGD ? p.stages : GEMM_STAGES;
-  constexpr int STAGE_BYTES = TWO ? STAGE_BYTES2 : mep::STAGE_BYTES;
-  constexpr int WB_MAX = SGD ? SGD_RING_MAX : 1;
-  const int WB = SGD ? p.wb : 1;
-  const int crank = TWO ? (int)cluster_cta_rank() : 0;        // 0 = leader of the pair
-  const int work_id0 = TWO ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-  const int work_stride = TWO ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-  extern __shared__ uint8_t smem_dyn[];
-  __shared__ __align__(8) uint64_t full[GEMM_STAGES];
-  __shared__ __align__(8) uint64_t empty[GEMM_STAGES];
-  __shared__ __align__(8) uint64_t acc_full[2];
-  __shared__ __align__(8) uint64_t acc_empty[2];
-  __shared__ uint32_t s_tmem;
-  __shared__ int s_abort;
-  __shared__ int s_end[MAX_GROUPS];
-  __shared__ int s_valid[MAX_GROUPS];
-  __shared__ __align__(1024) float s_epi[4 * 32 * 32];      // per-warp staging of stored tiles: a swizzled 4 KB block
-  // fused SGD: per epilogue warp a ring of WB 32 x 32 bf16 weight blocks (in dynamic shared
-  // memory, behind the operand stages) and their "landed" barriers
-  __shared__ __align__(8) uint64_t wbar[SGD ? 8 : 4][WB_MAX];
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
-  volatile int* abortp = &s_abort;
-
-  if (tid == 0) {
-    // CTA pairs: both CTAs' loads are credited to the LEADER's full barrier, which only the
-    // leader's producer arrives on (expecting the bytes of both CTAs); no per-stage remote arrive
-    for (int s = 0; s < GEMM_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], (TWO ? 8 : 4) * (SGD ? 2 : 1)); }
-    for (int a = 0; a < (SGD ? 8 : 4) * WB_MAX; ++a) mbar_init(&wbar[a / WB_MAX][a % WB_MAX], 1);
-    mbar_fence_init();
-    s_abort = 0;
-  }
-  // group table
-  for (int g = tid; g < p.ngroups; g += (int)blockDim.x)
-    s_end[g] = p.cu_seqlens != nullptr ? p.cu_seqlens[g] : p.total_rows;
-  __syncthreads();
-  for (int g = tid; g < p.ngroups; g += (int)blockDim.x)
-    s_valid[g] = group_valid(p, g, g == 0 ? 0 : s_end[g - 1], s_end[g]);
-  if (warp == 1) {
-    if constexpr (TWO) { tmem_alloc2(&s_tmem, 512); tmem_relinquish2(); }
-    else { tmem_alloc(&s_tmem, 512); tmem_relinquish(); }
-  }
-  tc_fence_before();
-  if constexpr (TWO) cluster_sync_all();     // the peer's barriers exist before anyone arrives on them
-  else __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = s_tmem;
-
-  const int n_tiles_n = (p.N + BN - 1) / BN;
-  const long long total_tiles = (long long)p.ngroups * (p.Mw / (TWO ? 2 * BM : BM)) * n_tiles_n;
-
-  if (warp == 0) {
-    // ================= TMA producer =================
-    if (lane == 0) {
-      tma_prefetch_desc(&p.a);
-      tma_prefetch_desc(&p.b[0][0]);
-      int it = 0;
-      bool ok = true;
-      for (long long id = work_id0; id < total_tiles && ok; id += work_stride) {
-        Tile t = get_tile<TWO>(p, (int)id, s_end, s_valid, n_tiles_n, crank);
-        if (!t.valid) continue;
-        for (int kb = 0; kb < t.num_kb; ++kb, ++it) {
-          const int s = it % nst;
-          if (it >= nst &&
-              !gemm_wait(&empty[s], ((uint32_t)(it / nst) & 1u) ^ 1u, abortp, p, 1)) {
-            ok = false;
-            break;
-          }
-          uint8_t* sa = tiles + (size_t)s * STAGE_BYTES;
-          uint8_t* sb = sa + A_TILE_BYTES;
-          uint32_t lead_bar = 0;
-          if constexpr (TWO) lead_bar = mapa_u32(&full[s], 0);
-          // the peer's bytes may land before this arrival: the pending count keeps the phase open
-          if (crank == 0) mbar_expect_tx(&full[s], TWO ? 2 * STAGE_BYTES : STAGE_BYTES);
-          const int k0 = kb * BK;
-          if constexpr (TWO) {
-            // this CTA's 128 columns of A (t.m0 is already its half) and its half of the B tile
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-              tma_load_2d_pair(sa + j * 8192, &p.a, t.m0 + 64 * j, t.row0 + k0, lead_bar);
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-              tma_load_2d_pair(sb + j * 8192, &p.b[0][0], t.n0 + 128 * crank + 64 * j, t.row0 + k0, lead_bar);
-          } else {
-            // A: [token rows][Mw cols], two 64-column blocks; B: [token rows][N cols], four
-#pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
-              tma_load_2d(sa + j * 8192, &p.a, t.m0 + 64 * j, t.row0 + k0, &full[s]);
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(sb + j * 8192, &p.b[0][0], t.n0 + 64 * j, t.row0 + k0, &full[s]);
-          }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    // ================= MMA issuer =================
-    if (lane == 0 && TWO && crank != 0) {
-      // peer CTA of a pair: the leader issues the MMAs for both
-    } else if (lane == 0) {
-      constexpr uint32_t idesc = make_instr_desc_bf16(TWO ? 2 * BM : BM, BN, true, true);
-      int it = 0, tile_n = 0;
-      bool ok = true;
-      for (long long id = work_id0; id < total_tiles && ok; id += work_stride) {
-        Tile t = get_tile<TWO>(p, (int)id, s_end, s_valid, n_tiles_n, crank);
-        if (!t.valid) continue;
-        const int acc = tile_n & 1;
-        if (tile_n >= 2 &&
-            !gemm_wait<TWO>(&acc_empty[acc], ((uint32_t)(tile_n >> 1) & 1u) ^ 1u, abortp, p, 2)) break;
-        tc_fence_after();
-        const uint32_t tacc = tmem_base + (uint32_t)acc * BN;
-        for (int kb = 0; kb < t.num_kb; ++kb, ++it) {
-          const int s = it % nst;
-          if (!gemm_wait(&full[s], (uint32_t)(it / nst) & 1u, abortp, p, 3)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(tiles + (size_t)s * STAGE_BYTES);
-          const uint32_t sb = sa + A_TILE_BYTES;
-#pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = make_smem_desc(sa + kk * 2048, 8192, 1024);
-            const uint64_t db = make_smem_desc(sb + kk * 2048, 8192, 1024);
-            if constexpr (TWO) umma_bf16_2cta(tacc, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-            else umma_bf16(tacc, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-          }
-          // stage reusable (in both CTAs of a pair) once these MMAs have read it
-          if constexpr (TWO) umma_commit_2cta(&empty[s], 3);
-          else umma_commit(&empty[s]);
-        }
-        if (!ok) break;
-        if constexpr (TWO) umma_commit_2cta(&acc_full[acc], 3);   // accumulator complete, both halves
-        else umma_commit(&acc_full[acc]);
-        ++tile_n;
-      }
-    }
-  } else {
-    // ================= epilogue (4 warps, one TMEM lane quarter each) =================
-    const int q = warp & 3;
-    // SGD: warps 2..5 take the tile's first 128 columns, warps 6..9 the other 128
-    const int half = SGD ? (warp - 2) >> 2 : 0;
-    const int ew = q + 4 * half;
-    constexpr int CB = SGD ? BN / 64 / 2 : BN / 64;     // 64-column weight blocks per warp and tile
-    const int cofs = half * CB * 64;
-    int tile_n = 0;
-    // ---- fused SGD: weight blocks stream through this warp's ring, ahead of the tiles ----------
-    // Block k of the stream (the 32-row x 64-column blocks of this warp's rows, tile after tile,
-    // fused tiles only) lives in buffer k % WB.  The load cursor runs up to WB blocks ahead of the
-    // block being updated, across tile boundaries.  Blocks are as wide as the 128B swizzle
-    // allows: the TMA engine moves about one box row per 5 cycles per SM whatever its length
-    // (measured), so 64-byte rows cap this epilogue at half the HBM rate.
-    constexpr int WBLK = 4096, WCOLS = 64;
-    uint8_t* wring = tiles + (size_t)nst * STAGE_BYTES + ew * (WB * WBLK);
-    int wseq = 0, lseq = 0;                // blocks consumed / loads issued (a few thousand per launch)
-    long long lid = work_id0;              // cursor: tile id, block in tile, cached coordinates
-    int lc = 0, l_y0 = 0, l_n0 = 0;
-    bool l_have = false;
-    auto sgd_tile = [&](const Tile& u) {
-      return u.valid && u.alloc == 0 && (p.sgd_keep == nullptr || p.sgd_keep[u.g_local] == 0);
-    };
-    auto cursor_settle = [&]() {           // move to the next existing block at or after (lid, lc)
-      while (lid < total_tiles) {
-        if (!l_have) {
-          const Tile u = get_tile<TWO>(p, (int)lid, s_end, s_valid, n_tiles_n, crank);
-          if (sgd_tile(u)) { l_have = true; l_y0 = u.g_local * p.Mw + u.m0 + q * 32; l_n0 = u.n0; lc = 0; }
-        }
-        if (l_have && lc < CB && l_n0 + cofs + lc * WCOLS < p.N) return;
-        l_have = false;
-        lid += work_stride;
-      }
-    };
-    auto issue_loads = [&]() {             // lane 0 issues; every lane tracks the cursor
-      while (lid < total_tiles && lseq < wseq + WB) {
-        if (lane == 0) {
-          uint64_t* bar = &wbar[ew][lseq % WB];
-          mbar_expect_tx(bar, WBLK);
-          tma_load_2d(wring + (lseq % WB) * WBLK, &p.wmap, l_n0 + cofs + lc * WCOLS, l_y0, bar);
-        }
-        ++lseq;
-        ++lc;
-        cursor_settle();
-      }
-    };
-    if constexpr (SGD) {
-      cursor_settle();
-      issue_loads();
-    }
-    for (long long id = work_id0; id < total_tiles; id += work_stride) {
-      Tile t = get_tile<TWO>(p, (int)id, s_end, s_valid, n_tiles_n, crank);
-      if (!t.valid) continue;
-      const int acc = tile_n & 1;
-      bool sgd_fuse = false;
-      if constexpr (SGD) sgd_fuse = sgd_tile(t);
-      if (!gemm_wait(&acc_full[acc], (uint32_t)(tile_n >> 1) & 1u, abortp, p, 4)) break;
-      tc_fence_after();
-      const uint32_t tacc = tmem_base + (uint32_t)acc * BN + ((uint32_t)(q * 32) << 16);
-      const bool have_acc = t.num_kb > 0;
-      {
-          const int col_base = t.n0;
-          // fp32 weight-grad tiles are 128 KB each and the main loop is short (one group's
-          // tokens), so the epilogue must move ~30 GB/s per SM.  Four warps of plain stores
-          // cannot (measured: ~14 B/clk/SM), so each warp stages 32x32 blocks in shared memory
-          // (128-byte swizzle, conflict-free 16-byte stores) and hands them to the TMA engine:
-          // a tiled store, or a tiled reduce-add when accumulating into existing grads.
-          uint8_t* pad = reinterpret_cast<uint8_t*>(s_epi) + q * 4096;
-          const int y0 = t.g_local * p.Mw + t.m0 + q * 32;
-          const CUtensorMap* cmap = &p.c[t.alloc];
-          if (SGD && sgd_fuse) {
-            // Weights travel by TMA both ways: a block is 32 rows x 64 bf16 (128-byte rows, 128B
-            // swizzle); lane i owns row i of the block, exactly the accumulator row it reads from
-            // tensor memory, so no transposition is needed.  The block is updated in place,
-            // stored back, and its buffer handed to the load cursor.
-            const float nlr = -p.sgd_lr;
-            bool wok = true;
-#pragma unroll 1
-            for (int c = 0; c < CB; ++c) {
-              if (col_base + cofs + c * WCOLS >= p.N) break;
-              const int b = wseq % WB;
-              uint8_t* wbuf = wring + b * WBLK;
-              uint32_t ra[32], rb[32];
-              tmem_ld_32x32(tacc + cofs + c * WCOLS, ra);
-              tmem_ld_32x32(tacc + cofs + c * WCOLS + 32, rb);
-              if (!gemm_wait(&wbar[ew][b], (uint32_t)(wseq / WB) & 1u, abortp, p, 5)) {
-                tmem_ld_wait();
-                wok = false;
-                break;
-              }
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const uint32_t* g = j < 4 ? ra + 8 * j : rb + 8 * (j - 4);
-                uint4* slot = reinterpret_cast<uint4*>(wbuf + lane * 128 + ((j ^ (lane & 7)) << 4));
-                uint4 w4 = *slot;
-                __nv_bfloat162* w2 = reinterpret_cast<__nv_bfloat162*>(&w4);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const float2 x = __bfloat1622float2(w2[i]);
-                  w2[i] = __floats2bfloat162_rn(__fmaf_rn(nlr, __uint_as_float(g[2 * i]), x.x),
-                                                __fmaf_rn(nlr, __uint_as_float(g[2 * i + 1]), x.y));
-                }
-                *slot = w4;
-              }
-              fence_proxy_async_smem();
-              __syncwarp();
-              if (lane == 0) {
-                tma_store_2d(&p.wmap, col_base + cofs + c * WCOLS, y0, wbuf);
-                bulk_commit();
-                bulk_wait_read<0>();                // the store has read the buffer: it may be refilled
-              }
-              ++wseq;
-              issue_loads();
-            }
-            if (!wok) break;
-          } else if (half == 0)      // (SGD kernels: a tile that is not applied is stored by warps 2..5 alone)
-#pragma unroll 1
-          for (int c = 0; c < BN / 32; ++c) {
-            uint32_t r[32];
-            if (have_acc) {
-              tmem_ld_32x32(tacc + c * 32, r);
-              tmem_ld_wait();
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = 0u;
-            }
-            if (lane == 0) bulk_wait_read<0>();     // the previous block has left the pad
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              *reinterpret_cast<uint4*>(pad + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                  make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-            fence_proxy_async_smem();
-            __syncwarp();
-            const int x0 = col_base + c * 32;
-            if (lane == 0 && x0 < p.N) {
-              if (p.accumulate) tma_reduce_add_2d(cmap, x0, y0, pad);
-              else tma_store_2d(cmap, x0, y0, pad);
-              bulk_commit();
-            }
-          }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (TWO && crank != 0) mbar_arrive_remote(&acc_empty[acc], 0);   // the leader issues the MMAs
-        else mbar_arrive(&acc_empty[acc]);
-      }
-      ++tile_n;
-    }
-  }
-  // ---- teardown: everything joins, in-flight work is given time to land on an abort ----------
-  tc_fence_before();
-  __syncthreads();
-  if (s_abort) {
-    unsigned long long t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) { }
-  }
-  if (warp >= 2 && lane == 0) bulk_wait<0>();   // epilogue TMA stores have completed
-  if constexpr (TWO) cluster_sync_all();        // neither CTA leaves while its peer may still touch it
-  if (warp == 1) {
-    tc_fence_after();
-    if constexpr (TWO) tmem_dealloc2(tmem_base, 512);
-    else tmem_dealloc(tmem_base, 512);
-  }
-}
-
 }  // namespace mep
 
 #include "device/dense_f32.cuh"
 #include "device/token_gemm.cuh"
+#include "device/weight_grad.cuh"
 
 namespace mep {
 
@@ -573,23 +201,6 @@ typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void
                              CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                              CUtensorMapFloatOOBfill);
 
-// 2-D fp32 tensor [rows][cols], box 32 x 32 (128-byte rows), 128B swizzle: weight-grad output.
-static int make_map_f32(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int64_t ld) {
-  EncodeFn enc = (EncodeFn)driver_tensor_map_encode();
-  if (!enc) return fail(-10, "CUDA driver entry cuTensorMapEncodeTiled not available");
-  if (((uintptr_t)base & 15) != 0 || (ld * 4) % 16 != 0)
-    return fail(-11, "weight-grad output must be 16-byte aligned with a 16-byte multiple row stride");
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-  cuuint32_t box[2] = {32, 32};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides,
-                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(-12, "cuTensorMapEncodeTiled (fp32) failed with code %d", (int)r);
-  return 0;
-}
-
 // 2-D bf16 tensor [rows][cols] (row stride ld elements), box [box_rows][box_cols], 128B swizzle.
 static int make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int64_t ld,
                     int box_cols, int box_rows, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
@@ -619,37 +230,6 @@ static bool fused_dispatch_cooperative() {
     v = (e != nullptr && e[0] == '0') ? 0 : 1;
   }
   return v != 0;
-}
-
-// SGD kernels: dynamic shared memory of a launch (operand stages, alignment slack, four rings of
-// 4 KB weight blocks) and the most that the kernel may ask for next to its static part.
-static int sgd_smem(const GemmKParams& kp, bool two) {
-  return kp.stages * (two ? STAGE_BYTES2 : STAGE_BYTES) + 1024 + 8 * kp.wb * 4096;
-}
-// How an SGD launch splits its shared memory between operand stages and weight blocks (4 KB, per
-// epilogue warp).  Measured on the benchmark's shapes (32 x 1024, 64 x 512, 256 x 128 rows): the
-// depth of the weight ring hardly matters once eight warps run the read-modify-write chains (a
-// warp needs ~1.4 us per block whatever the depth), so the operand ring gets what is left after
-// two (pairs) or three (single CTA, whose stages are 48 KB) blocks per warp.
-// MOONEP_B200_SGD_RING="stages,blocks" overrides the choice (tuning).
-static void sgd_geometry(bool pair, GemmKParams* kp) {
-  if (pair) { kp->stages = 4; kp->wb = 2; }
-  else { kp->stages = 2; kp->wb = 3; }
-  if (const char* e = getenv("MOONEP_B200_SGD_RING")) {
-    int a = 0, b = 0;
-    if (sscanf(e, "%d,%d", &a, &b) == 2 && a >= 2 && a <= (pair ? GEMM_STAGES2 : GEMM_STAGES) && b >= 2 &&
-        b <= SGD_RING_MAX) {
-      kp->stages = a; kp->wb = b;
-    }
-  }
-}
-static int sgd_smem_limit(const void* kern) {
-  cudaFuncAttributes fa;
-  int dev = 0, optin = 0;
-  if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) { cudaGetLastError(); return 0; }
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return optin - (int)fa.sharedSizeBytes;
 }
 
 // CTA-pair launch: clusters of two CTAs, one pair per two SMs.  `coop`: the whole grid must be
@@ -709,20 +289,42 @@ static int launch_single(const void* kern, std::atomic<unsigned long long>& rais
   return 0;
 }
 
+// How a weight-grad launch splits its shared memory and its tiles, by the average group (which is all the host knows;
+// every choice computes every group).  SGD: up to eight k-blocks a group the stream of old weights needs two
+// pieces a warp in flight (128 groups x 256 rows, 7168 x 2048: 1790 us, 1810 with one and more operand slots); longer
+// ones the operand slots (32 x 1024: 866, 913 with two pieces).  Two tiles a unit share staged rows: SGD with more
+// than the five k-blocks that stay staged anyway (80 groups x 410 rows, 4096 x 2048: 717, 761 one by one; 32 x 1024 880,
+// 989); shorter groups lose by it (64 x 192, 4096 x 1024: 221 one by one, 252), stored grads gain nothing (32 x
+// 1024, 2048 x 1024: 159, 165), and an odd number of column tiles leaves units of unequal length (128 x 256, 2048 x 768:
+// 210, 294).
+static void wgrad_geometry(GemmKParams* kp, bool pair) {
+  const int local = kp->split < kp->ngroups ? kp->split : kp->ngroups;
+  const double kb = (double)kp->total_rows / (local > 0 ? local : 1) / BK;
+  const bool sgd = kp->sgd_w != nullptr, brief = kb <= 8;
+  kp->pieces = sgd ? (brief ? 2 : 1) : 0;
+  if (pair) {
+    kp->row_slots = sgd ? (brief ? 5 : 6) : 7;
+    kp->col_slots = sgd ? (brief ? 4 : 5) : 6;
+  } else {
+    kp->row_slots = sgd ? (brief ? 3 : 4) : 5;
+    kp->col_slots = sgd ? 3 : 4;
+  }
+  kp->unit = sgd && ((kp->N + BN - 1) / BN) % 2 == 0 && kb > 5 ? 2 : 1;
+}
+static int wgrad_smem(const GemmKParams& kp, bool pair) {
+  return kp.row_slots * WG_ROW_BYTES + kp.col_slots * (pair ? wg_col_bytes<true>() : wg_col_bytes<false>()) +
+         WG_EPI_WARPS * kp.pieces * WG_PIECE + 1024;
+}
+
 template <bool SGD>
 static int launch_wgrad(const GemmKParams& kp, bool pair, int grid, cudaStream_t stream) {
-  const void* kern = pair ? (const void*)ep_grouped_gemm_kernel<true, SGD>
-                          : (const void*)ep_grouped_gemm_kernel<false, SGD>;
-  const int smem = SGD ? sgd_smem(kp, pair) : (pair ? gemm_smem<true>() : gemm_smem<false>());
-  if (SGD && smem > sgd_smem_limit(kern))
-    return fail(-3, "gemm: %d operand stages + %d weight blocks do not fit in shared memory", kp.stages, kp.wb);
-  const int threads = SGD ? GEMM_THREADS_SGD : GEMM_THREADS;
+  const int smem = wgrad_smem(kp, pair);
   if (pair) {
     static PairLaunch once;
-    return launch_pair(kern, once, kp, grid, threads, smem, false, stream);
+    return launch_pair((const void*)ep_weight_grad_kernel<true, SGD>, once, kp, grid, WG_THREADS, smem, false, stream);
   }
   static std::atomic<unsigned long long> raised{0};
-  return launch_single(kern, raised, kp, grid, threads, smem, false, stream);
+  return launch_single((const void*)ep_weight_grad_kernel<false, SGD>, raised, kp, grid, WG_THREADS, smem, false, stream);
 }
 
 template <bool W_MN>
@@ -798,17 +400,14 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
         return fail(-14, "wgrad: the fused SGD step needs N %% 8 == 0 and 16-byte aligned weights");
       kp.sgd_w = (__nv_bfloat16*)d->sgd_w; kp.sgd_keep = d->sgd_keep; kp.sgd_lr = d->sgd_lr;
       const int n_w = d->split < d->ngroups ? d->split : d->ngroups;
-      if ((rc = make_map(&kp.wmap, d->sgd_w, (int64_t)n_w * d->Mw, d->N, d->ldc, 64, 32))) return rc;
+      if ((rc = make_map(&kp.wmap, d->sgd_w, (int64_t)n_w * d->Mw, d->N, d->ldc, 64, 16))) return rc;
     }
-    const int n_local = d->split < d->ngroups ? d->split : d->ngroups;
-    if ((rc = make_map_f32(&kp.c[0], d->out[0], (int64_t)n_local * d->Mw, d->N, d->ldc))) return rc;
-    kp.c[1] = kp.c[0];
-    if (d->ngroups > d->split) {
-      if (d->out[1] == nullptr) return fail(-8, "wgrad: groups >= split need a slot grad tensor");
-      if ((rc = make_map_f32(&kp.c[1], d->out[1], (int64_t)(d->ngroups - d->split) * d->Mw, d->N, d->ldc))) return rc;
-    }
-    const bool pair = d->two_cta != 0 && grid >= 2 && d->Mw % (2 * BM) == 0;
-    if (kp.sgd_w != nullptr) sgd_geometry(pair, &kp);
+    if (d->ngroups > d->split && d->out[1] == nullptr) return fail(-8, "wgrad: groups >= split need a slot grad tensor");
+    if ((((uintptr_t)d->out[0] | (uintptr_t)d->out[1]) & 15) != 0 || d->ldc % 4 != 0)
+      return fail(-11, "weight-grad output must be 16-byte aligned with a 16-byte multiple row stride");
+    kp.vec32 = ((uintptr_t)d->sgd_w & 31) == 0 && d->N % 16 == 0;
+    const bool pair = d->two_cta != 0 && grid >= 2;
+    wgrad_geometry(&kp, pair);
     kp.wg_select = kp.sgd_w != nullptr ? d->wg_select : 0;
     if (kp.sgd_w != nullptr)
       return launch_wgrad<true>(kp, pair, grid, stream);

@@ -94,12 +94,15 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrive on the barrier that sits at the same offset in CTA `cta_rank` of this cluster.
+// Arrive on the barrier that sits at the same offset in CTA `cta_rank` of this cluster.  Released at CTA scope (the
+// default): what the arrival hands over is tensor memory, ordered by tcgen05.fence, not memory.  A release at
+// cluster scope waits for the thread's earlier global stores: beside a stream of them 5000 cycles of a weight-grad
+// tile's 7700; the token GEMMs of 128 groups x 256 rows, H = 2048, H' = 768 lost 1 - 4 % to it.
 __device__ __forceinline__ void mbar_arrive_remote(uint64_t* local_bar, uint32_t cta_rank) {
   asm volatile(
       "{\n\t.reg .b32 ra;\n\t"
       "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}"
+      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}"
       ::"r"(smem_u32(local_bar)), "r"(cta_rank)
       : "memory");
 }
@@ -108,12 +111,6 @@ __device__ __forceinline__ uint32_t mapa_u32(const void* local_ptr, uint32_t cta
   uint32_t ra;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(local_ptr)), "r"(cta_rank));
   return ra;
-}
-// arrive + expect_tx on a barrier given by its cluster address (possibly in the peer CTA)
-__device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t bar_cluster_addr, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;"
-               ::"r"(bar_cluster_addr), "r"(bytes)
-               : "memory");
 }
 // Tiled TMA load of a CTA pair: the data lands in THIS CTA's shared memory, the byte count is
 // credited to a barrier that may live in the pair's other CTA (the leader's).  No multicast.
@@ -125,19 +122,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(bar_cluster_addr)
       : "memory");
 }
-// try_wait with cluster-scope acquire, for barriers that receive remote arrivals.
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // ---- descriptors -------------------------------------------------------------------------------
 // Shared-memory matrix descriptor, 128-byte swizzle, tile base 1024-byte aligned:
 //   bits  0..13  start address >> 4          bits 16..29  leading-dimension byte offset >> 4
@@ -223,12 +207,32 @@ __device__ __forceinline__ void tmem_ld_16x256_x4(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
+// Four 8x8 matrices of 16-bit elements from shared memory: thread 8i + k gives the address of row k of matrix i (16
+// bytes) and gets, of each, columns 2 (t % 4) and the next of row t / 4.
+__device__ __forceinline__ void ldmatrix_x4(uint32_t smem_addr, uint32_t* r) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr) : "memory");
+}
 // Four 8x8 matrices of 16-bit elements, held as fragments (thread t: row t / 4, columns 2 (t % 4) and the
 // next), stored transposed: thread 8i + k gives the address of the 16 bytes of column k of matrix i.
 __device__ __forceinline__ void stmatrix_x4_trans(uint32_t smem_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
                ::"r"(smem_addr), "r"(a), "r"(b), "r"(c), "r"(d)
                : "memory");
+}
+// The same with 64 columns: column blocks j = 0..7.
+__device__ __forceinline__ void tmem_ld_16x256_x8(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -243,19 +247,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       "[%0], [%1, {%2, %3}], [%4];"
       ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
-}
-// tiled TMA store / reduce-add (2-D) from this CTA's shared memory, tracked by the thread's bulk
-// async-group.  x * element size must be a multiple of 16 bytes and coordinates non-negative.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, const void* smem_src) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
-               ::"l"(map), "r"(x), "r"(y), "r"(smem_u32(smem_src))
-               : "memory");
-}
-__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, int x, int y,
-                                                  const void* smem_src) {
-  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%1, %2}], [%3];"
-               ::"l"(map), "r"(x), "r"(y), "r"(smem_u32(smem_src))
-               : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");

@@ -88,27 +88,20 @@ def reset_status(device="cuda") -> None:
 
 
 # CTA pairs (tcgen05 cta_group::2: clusters of two CTAs issue one 256-row MMA and each stages only
-# half of the second operand's tile).  ``MOONEP_B200_TWO_CTA``: ``auto`` (default) uses pairs for the
-# token-major products always and for the weight grads when the groups are long enough on average
-# (see ``_launch``); ``1`` always, ``0`` never.  A launch with a CTA limit (one that runs next to a
+# half of the second operand's tile).  ``MOONEP_B200_TWO_CTA``: ``auto`` (default) uses pairs unless the
+# CTA limit is odd; ``1`` always, ``0`` never.  A launch with a CTA limit (one that runs next to a
 # copy kernel) needs an even limit; the copy kernels are placed as SM pairs too, so the SMs they
 # leave free can all be paired.
 _two = __import__("os").environ.get("MOONEP_B200_TWO_CTA", "auto").strip().lower()
 TWO_CTA = {"auto": 2, "": 2}.get(_two, None)
 if TWO_CTA is None:
     TWO_CTA = int(_two)
-PAIR_MIN_AVG_ROWS_WGRAD = 512   # 64 groups x 512 rows, fused SGD: pairs 1.16 ms, single CTAs 1.44 ms
 
 
 def _launch(d: _GemmDesc) -> None:
     global _checked_layout
     if TWO_CTA == 2:
-        # Weight-grad tiles split the weight rows between the pair's CTAs; with short groups (a few
-        # k-blocks per tile) the pair's extra hand-shakes cost more than they save.  The host only
-        # knows the average (over the local groups, the slot groups hold rows taken from those).
-        local_groups = max(1, min(d.ngroups, d.split))
-        least = PAIR_MIN_AVG_ROWS_WGRAD if d.mode == 1 else 0
-        d.two_cta = int(d.grid % 2 == 0 and d.total_rows >= least * local_groups)
+        d.two_cta = int(d.grid % 2 == 0)
     else:
         d.two_cta = TWO_CTA
     if not _checked_layout:

@@ -1,0 +1,54 @@
+"""Weight-grad kernel at the edges of its tiles: weight rows that end inside a CTA pair's 256, columns that end
+inside a tile (and where rows allow 16-byte stores only), reductions shorter than, as long as and longer than the
+row slots, one and two tiles a unit, groups without rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(groups, M, N, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    ends = torch.tensor(groups, device="cuda").cumsum(0).to(torch.int32)
+    rows = sum(groups)
+    a = torch.randn(rows, M, device="cuda", generator=g).bfloat16()
+    b = torch.randn(rows, N, device="cuda", generator=g).bfloat16()
+    return g, ends, a, b
+
+
+@pytest.mark.parametrize("two", [0, 1])
+@pytest.mark.parametrize("M, N", [(128, 8), (384, 40), (256, 264), (640, 512), (256, 1032)])
+@pytest.mark.parametrize("groups", [[64, 0, 128], [320, 384, 0, 448, 512], [1152, 64, 832]])
+def test_edges(groups, M, N, two, monkeypatch):
+    from moonep_b200.ops import elementwise as ew
+    from moonep_b200.ops import gemm
+    monkeypatch.setattr(gemm, "TWO_CTA", two)
+    gen, ends, a, b = _inputs(groups, M, N, M + N)
+    G, lr = len(groups), 0.25
+    grad = torch.full((G, M, N), float("nan"), device="cuda")
+    gemm.wgrad(a, b, ends, grad)
+    start = 0
+    for g, n in enumerate(groups):
+        want = a[start:start + n].double().t() @ b[start:start + n].double()
+        # products are exact in fp32; n additions, each off by at most one unit of the running sum (truncated), which
+        # stays below sum |a b|
+        bound = 2.0 ** -23 * max(n, 1) * (a[start:start + n].double().abs().t() @ b[start:start + n].double().abs())
+        assert bool(((grad[g].double() - want).abs() <= bound).all()), g
+        start += n
+    # accumulating adds the same sums
+    base = torch.randn(G, M, N, device="cuda", generator=gen)
+    acc = base.clone()
+    gemm.wgrad(a, b, ends, acc, accumulate=True)
+    assert torch.equal(acc, base + grad)
+    # the SGD step in the epilogue: bit for bit the update by the stored grads
+    w = torch.randn(G, M, N, device="cuda", generator=gen).bfloat16()
+    want = w.clone()
+    ew.sgd_update_(want, grad, lr)
+    keep = torch.zeros(G, dtype=torch.int32, device="cuda")
+    keep[G - 1] = 1
+    want[G - 1] = w[G - 1]
+    kept = torch.zeros(G, M, N, device="cuda")
+    gemm.wgrad(a, b, ends, kept, sgd=(w, lr, keep))
+    assert torch.equal(w, want)
+    assert torch.equal(kept[G - 1], grad[G - 1]) and not bool(kept[:G - 1].any())
+    gemm.check_status()
