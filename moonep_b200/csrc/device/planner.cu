@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) ep_plan_kernel(const PlanPara
   const int tok0 = min(p.S, c * tpc), tok1 = min(p.S, tok0 + tpc);
   const int64_t i0 = (int64_t)tok0 * K, i1 = (int64_t)tok1 * K;
 
-  if (c == 0) {
+  if (c == 0 && !p.one_device) {
     // all-gather of tpe by peer stores: my row into everyone's table
     const int32_t* my_tpe = p.tpe + (size_t)vr * E;
     for (int64_t i = tid; i < (int64_t)R * E; i += PLAN_THREADS) {
@@ -68,8 +68,9 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) ep_plan_kernel(const PlanPara
     // the exchange orders the clear before every peer's first increment of this step
     int32_t* arrive = sc.meta + (size_t)rank * sc.meta_stride + p.arrive_off;
     for (int i = tid; i < p.n_arrive; i += PLAN_THREADS) arrive[i] = 0;
-    cta_cross_rank_exchange(sc, 1);
-    plan_solve(p, rank, sc.meta + (size_t)rank * sc.meta_stride + tbl_off, smem);
+    if (!p.one_device) cta_cross_rank_exchange(sc, 1);
+    plan_solve(p, rank, p.one_device ? p.tpe : sc.meta + (size_t)rank * sc.meta_stride + tbl_off, smem,
+               p.tables != 0 ? smem + p.tables : nullptr);
   }
   grid_sync(sc, 2);
   if (c == 0 && tid == 0) st[3] = parity ^ 1;
@@ -86,17 +87,27 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) ep_plan_kernel(const PlanPara
   for (int i = tid; i < E * shares; i += PLAN_THREADS) {
     const int e = i % E;
     int sum = 0;
-    for (int c0 = i / E; c0 < c; c0 += 8 * shares) {
-      int n[8];
+    for (int c0 = i / E; c0 < c; c0 += 16 * shares) {
+      int n[16];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < 16; ++u) {
         const int cc = c0 + u * shares;
         n[u] = cc < c ? hist_g[(size_t)cc * E + e] : 0;
       }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) sum += n[u];
+      for (int u = 0; u < 16; ++u) sum += n[u];
     }
     if (sum != 0) atomicAdd(&cnt[e], sum);
+  }
+  // the tables that every entry looks up, in shared memory where the solver's had room there
+  if (p.tables != 0) {
+    int32_t* at = smem + p.tables + (p.rank_warps > 1 ? p.rank_warps * E : 0);
+    for (int i = tid; i < R * E; i += PLAN_THREADS) {
+      at[i] = alloc_cumsum[i];
+      at[R * E + i] = expert_off[i];
+    }
+    alloc_cumsum = at;
+    expert_off = at + R * E;
   }
   // sending order: exclusive prefix of my per-expert counts in the permuted expert order
   int32_t* pperm = smem + E;
@@ -229,22 +240,47 @@ int64_t mep_plan_smem_bytes(int R, int E) {
   return (int64_t)sizeof(int32_t) * (2 * (int64_t)E + 4 * R + (int64_t)PLAN_WARPS * R);
 }
 
-// Ranking warps of a planner launch: one per 128 entries of a CTA (clearing and summing their counters costs
-// more than a few steps of 32 entries: with sixteen for 8 entries 27 -> 31 us), as many as have room for
-// counters.  Over several devices that is 8 KB: the planner and the weight ops wait for other ranks while
-// they hold their SMs, on two streams, and beside prefetch_weight's ring (192 KB and its lists) 64 KB do not fit.
+// CTAs a rank.  Within one device no more than have 256 entries each: the grid's barrier and the sums over the
+// CTAs before one's own cost more than the entries of the smallest calls.
+static int plan_ctas(const BufferCtx& c) {
+  if (!c.one_device()) return c.num_sms;
+  const int64_t useful = (c.N + 255) / 256;
+  return useful < c.num_sms ? (int)useful : c.num_sms;
+}
+
+// Ranking warps of a planner launch: one per 64 entries of a CTA within one device (4096 tokens on 256 experts
+// 21.6 us, 22.4 with one per 128), per 128 over several (clearing and summing their counters costs more than a few steps of 32
+// entries: with sixteen for 8 entries 27 -> 31 us), as many as have room for counters.  Over several devices
+// that is 8 KB: the planner and the weight ops wait for other ranks while they hold their SMs, on two
+// streams, and beside prefetch_weight's ring (192 KB and its lists) 64 KB do not fit.
 static int plan_rank_warps(const BufferCtx& c) {
-  const int64_t entries = (int64_t)((c.S + c.num_sms - 1) / c.num_sms) * c.K;
+  const int ctas = plan_ctas(c);
+  const int64_t entries = (int64_t)((c.S + ctas - 1) / ctas) * c.K;
   int64_t w = (c.one_device() ? 64 * 1024 : 8 * 1024) / (int64_t)(sizeof(int32_t) * c.E);
-  if (w > entries / 128) w = entries / 128;
+  const int64_t least = c.one_device() ? 64 : 128;
+  if (w > entries / least) w = entries / least;
   return w < 1 ? 1 : (w > PLAN_WARPS ? PLAN_WARPS : (int)w);
+}
+
+// Where the solver's tables start in shared memory: behind its other arrays, over the ranking warps' counters, which
+// are used later.  0 (none) over several devices, where the planner shares SMs (see above), and when they are
+// too large.  Tables in shared memory, no exchange within one device, the layout split over all warps: 16 tokens on
+// 32 experts 17 -> 15 us, 4096 on 256 28 -> 22, 8 ranks x 17 tokens on 128 experts 29 -> 19, 8 x 4096 on 256 42 -> 35.
+static int64_t plan_tables(const BufferCtx& c) {
+  const int64_t at = mep_plan_smem_bytes(c.R, c.E);
+  return c.one_device() && at + (int64_t)sizeof(int32_t) * solve_table_ints(c.R, c.E) <= 160 * 1024 ? at : 0;
 }
 
 // Dynamic shared memory of a planner launch of this Buffer.
 int64_t mep_plan_launch_smem_bytes(const void* ctx_) {
   const BufferCtx& c = *(const BufferCtx*)ctx_;
   const int w = plan_rank_warps(c);            // (a lone warp counts in place)
-  return mep_plan_smem_bytes(c.R, c.E) + (w > 1 ? (int64_t)sizeof(int32_t) * w * c.E : 0);
+  int64_t more = w > 1 ? (int64_t)w * c.E : 0;
+  if (plan_tables(c) != 0) {
+    more += 2 * (int64_t)c.R * c.E;            // the tables that are looked up, behind the counters
+    if (more < solve_table_ints(c.R, c.E)) more = solve_table_ints(c.R, c.E);
+  }
+  return mep_plan_smem_bytes(c.R, c.E) + (int64_t)sizeof(int32_t) * more;
 }
 
 // Fresh plan for this rank (or for all virtual ranks).  send_order [Rv][N] may be null (it is
@@ -266,10 +302,12 @@ int mep_launch_plan(const void* ctx_, const int32_t* topk, const int32_t* tpe, i
   p.send_order = send_order; p.arrive_off = c.ml.arrive_off; p.n_arrive = (int)(c.NvS / 128 + 1);
   const size_t smem = (size_t)mep_plan_launch_smem_bytes(ctx_);
   p.rank_warps = plan_rank_warps(c);
+  p.one_device = c.one_device();
+  p.tables = (int)(plan_tables(c) / sizeof(int32_t));
   p.rank_counts = p.rank_warps > 1 ? (int)(mep_plan_smem_bytes(c.R, c.E) / sizeof(int32_t)) : 0;
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_plan_kernel, raised));
-  dim3 grid(c.num_sms, c.Rv());
+  dim3 grid(plan_ctas(c), c.Rv());
   MEP_CUDA_OK(launch_coop((const void*)ep_plan_kernel, grid, dim3(PLAN_THREADS), smem, stream, p));
   return 0;
 }

@@ -32,6 +32,8 @@ struct PlanParams {
   int64_t arrive_off;       // ARRIVE counters in the meta chunk, cleared before the exchange
   int n_arrive;
   int rank_warps, rank_counts;   // warps that number the entries, and where their counters start in shared memory
+  int one_device;           // every rank's counts are in `tpe`, and stream order separates launches
+  int tables;               // where the solver's tables start in shared memory; 0: they stay in the scratch
 };
 
 // Position of expert e in the sending order of `rank` (see PlanParams::send_order).
@@ -47,34 +49,39 @@ constexpr int PLAN_WARPS = PLAN_THREADS / 32;
 
 // (value, index) arg-max with ties to the smaller index, across a warp.
 __device__ __forceinline__ void warp_argmax(int& v, int& i) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    int ov = __shfl_xor_sync(0xffffffffu, v, o);
-    int oi = __shfl_xor_sync(0xffffffffu, i, o);
-    if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
-  }
+  const int best = __reduce_max_sync(0xffffffffu, v);
+  i = __reduce_min_sync(0xffffffffu, v == best ? i : INT32_MAX);
+  v = best;
 }
 __device__ __forceinline__ void warp_argmin(int& v, int& i) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    int ov = __shfl_xor_sync(0xffffffffu, v, o);
-    int oi = __shfl_xor_sync(0xffffffffu, i, o);
-    if (ov < v || (ov == v && oi < i)) { v = ov; i = oi; }
-  }
+  const int best = __reduce_min_sync(0xffffffffu, v);
+  i = __reduce_min_sync(0xffffffffu, v == best ? i : INT32_MAX);
+  v = best;
 }
 
-// Steps 1-4 of the algorithm, executed by CTA 0 of every rank.
+// Ints of shared memory that the solver's tables take: the counts, four [R][E] tables, the experts to copy.
+MEP_HD int64_t solve_table_ints(int R, int E) { return 5 * (int64_t)R * E + E; }
+
+// Steps 1-4 of the algorithm, executed by CTA 0 of every rank.  `work` (solve_table_ints) holds the tables while they
+// are made, where there is room for it: the steps are chains of dependent accesses, ~30 cycles each in shared
+// memory and ~600 in the scratch.  What other CTAs read is in the scratch in the end either way.
 static __device__ void plan_solve(const PlanParams& p, int rank, const int32_t* tbl /*[R][E]*/,
-                           int32_t* smem) {
+                           int32_t* smem, int32_t* work = nullptr) {
   const int R = p.sync.R, E = p.E, epn = p.epn;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int vr = blockIdx.y;
   int32_t* scratch = p.scratch + (size_t)vr * p.scratch_ints;
-  int32_t* tpe_cumsum = scratch;
-  int32_t* alloc = scratch + (size_t)R * E;
-  int32_t* alloc_cumsum = scratch + (size_t)2 * R * E;
-  int32_t* expert_off = scratch + (size_t)3 * R * E;
-  int32_t* etc = p.etc + (size_t)vr * R * epn;
+  int32_t* const tables = work != nullptr ? work + (size_t)R * E : scratch;
+  int32_t* tpe_cumsum = tables;
+  int32_t* alloc = tables + (size_t)R * E;
+  int32_t* alloc_cumsum = tables + (size_t)2 * R * E;
+  int32_t* expert_off = tables + (size_t)3 * R * E;
+  int32_t* etc = work != nullptr ? tables + (size_t)4 * R * E : p.etc + (size_t)vr * R * epn;
+  if (work != nullptr) {
+    for (int i = tid; i < R * E; i += PLAN_THREADS) work[i] = tbl[i];
+    __syncthreads();
+    tbl = work;
+  }
 
   int32_t* count = smem;                 // [E]
   int32_t* remaining = smem + E;         // [E]
@@ -96,7 +103,7 @@ static __device__ void plan_solve(const PlanParams& p, int rank, const int32_t* 
   }
   for (int i = tid; i < R; i += PLAN_THREADS) { recv_from[i] = -1; recv_amt[i] = 0; stat1[i] = 0; }
   for (int i = tid; i < R * epn; i += PLAN_THREADS) etc[i] = -1;
-  for (size_t i = tid; i < (size_t)R * E; i += PLAN_THREADS) expert_off[i] = 0;
+  for (int i = tid; i < R * E; i += PLAN_THREADS) expert_off[i] = 0;
   __syncthreads();
   const int CAP = (int)p.N;
   for (int h = warp; h < R; h += PLAN_WARPS) {
@@ -106,8 +113,8 @@ static __device__ void plan_solve(const PlanParams& p, int rank, const int32_t* 
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) balance[h] = s - CAP;
   }
-  for (size_t i = tid; i < (size_t)E * R; i += PLAN_THREADS) {
-    int e = (int)(i / R), d = (int)(i % R);
+  for (int i = tid; i < E * R; i += PLAN_THREADS) {
+    const int e = i / R, d = i - e * R;
     alloc[i] = (d == e / epn) ? count[e] : 0;
   }
   __syncthreads();
@@ -175,59 +182,87 @@ static __device__ void plan_solve(const PlanParams& p, int rank, const int32_t* 
       alloc_cumsum[(size_t)e * R + d] = run;
     }
   }
-  // 4b. layout of every destination rank, one warp per rank
-  const int tp = p.token_padding;
+  // 4b. experts that every destination rank gets from elsewhere, one warp per rank
+  int32_t* nremote = recv_amt;           // (the amounts have been moved)
   for (int d = warp; d < R; d += PLAN_WARPS) {
     const int h = recv_from[d];
-    int nremote = 0;
+    int n = 0;
     if (h >= 0) {
       for (int j0 = 0; j0 < epn; j0 += 32) {
         int j = j0 + lane;
         bool has = j < epn && alloc[(size_t)(h * epn + j) * R + d] > 0;
         unsigned m = __ballot_sync(0xffffffffu, has);
-        if (has) etc[d * epn + nremote + __popc(m & ((1u << lane) - 1))] = h * epn + j;
-        nremote += __popc(m);
+        if (has) etc[d * epn + n + __popc(m & ((1u << lane) - 1))] = h * epn + j;
+        n += __popc(m);
       }
     }
-    __syncwarp();
     if (lane == 0) {
-      if (h >= 0) atomicAdd(&stat1[h], nremote);
-      if (d == rank) p.remote_stats[(size_t)vr * 2] = nremote;
+      nremote[d] = n;
+      if (h >= 0) atomicAdd(&stat1[h], n);
+      if (d == rank) p.remote_stats[(size_t)vr * 2] = n;
     }
+  }
+  __syncthreads();
+  // 4c. layout of every destination rank: its groups in as many parts as there are warps for, whose sizes are summed
+  // first (one warp a rank took 6 us of 17 for a lone rank's 256 experts)
+  const int tp = p.token_padding;
+  const bool pow2 = (tp & (tp - 1)) == 0;
+  const int parts = R < PLAN_WARPS ? PLAN_WARPS / R : 1;
+  const int part = ((2 * epn + parts - 1) / parts + 31) / 32 * 32;      // groups of a part
+  int32_t* part_rows = quotas;           // [R][parts]: no more than it had
+  auto group = [&](int d, int g, int& eid, int& cnt) {                  // padded size of a group
+    eid = -1;
+    if (g < epn) eid = d * epn + g;
+    else if (g < 2 * epn && g - epn < nremote[d]) eid = etc[d * epn + (g - epn)];
+    cnt = eid >= 0 ? alloc[(size_t)eid * R + d] : 0;
+    return pow2 ? (cnt + tp - 1) & -tp : (cnt + tp - 1) / tp * tp;
+  };
+  for (int job = warp; job < R * parts; job += PLAN_WARPS) {
+    const int d = job / parts, first = (job - d * parts) * part;
+    int sum = 0, eid, cnt;
+    for (int g = first + lane; g < min(first + part, 2 * epn); g += 32) sum += group(d, g, eid, cnt);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) part_rows[job] = sum;
+  }
+  __syncthreads();
+  for (int job = warp; job < R * parts; job += PLAN_WARPS) {
+    const int d = job / parts, first = (job - d * parts) * part;
     int carry = 0;
-    for (int g0 = 0; g0 < 2 * epn; g0 += 32) {
-      int g = g0 + lane;
-      int eid = -1, cnt = 0;
-      if (g < epn) {
-        eid = d * epn + g;
-      } else if (g < 2 * epn && g - epn < nremote) {
-        eid = etc[d * epn + (g - epn)];
-      }
-      if (eid >= 0) cnt = alloc[(size_t)eid * R + d];
-      int padded = cnt > 0 ? (cnt + tp - 1) / tp * tp : 0;
+    for (int k = d * parts; k < job; ++k) carry += part_rows[k];
+    for (int g0 = first; g0 < min(first + part, 2 * epn); g0 += 32) {
+      const int g = g0 + lane;
+      int eid, cnt;
+      const int padded = group(d, g, eid, cnt);
       int incl = padded;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         int v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
       }
-      int end = carry + incl, start = end - padded;
+      const int end = carry + incl, start = end - padded, npad = padded - cnt;
       if (g < 2 * epn) {
         if (cnt > 0) expert_off[(size_t)d * E + eid] = start;
         if (d == rank) {
           p.cu_seqlens[(size_t)vr * 2 * epn + g] = end;
-          int npad = padded - cnt;
-          p.zero_fill[((size_t)vr * 2 * epn + g) * 2 + 0] = (cnt > 0 && npad > 0) ? start + cnt : 0;
-          p.zero_fill[((size_t)vr * 2 * epn + g) * 2 + 1] = (cnt > 0 && npad > 0) ? npad : 0;
+          p.zero_fill[((size_t)vr * 2 * epn + g) * 2 + 0] = npad > 0 ? start + cnt : 0;
+          p.zero_fill[((size_t)vr * 2 * epn + g) * 2 + 1] = npad;
         }
       }
       carry = __shfl_sync(0xffffffffu, end, 31);
     }
-    if (lane == 0 && (int64_t)carry > p.NvS)
+    if (job == d * parts + parts - 1 && lane == 0 && (int64_t)carry > p.NvS)
       report_failure(p.sync, ST_BAD_INDEX, 40, d, carry, (int)p.NvS);
   }
   __syncthreads();
   if (tid == 0) p.remote_stats[(size_t)vr * 2 + 1] = stat1[rank];
+  if (work != nullptr) {
+    for (int i = tid; i < R * E; i += PLAN_THREADS) {
+      scratch[i] = tpe_cumsum[i];
+      scratch[2 * R * E + i] = alloc_cumsum[i];
+      scratch[3 * R * E + i] = expert_off[i];
+    }
+    for (int i = tid; i < R * epn; i += PLAN_THREADS) p.etc[(size_t)vr * R * epn + i] = etc[i];
+  }
 }
 
 }  // namespace mep
