@@ -25,10 +25,13 @@ F = ctypes.c_float
 
 # name -> (restype, [argtypes]).  Filled by the modules that own the entry points.
 _SIGNATURES: dict[str, tuple] = {}
+# name -> (function, launches a call counts for), once called
+_RESOLVED: dict[str, tuple] = {}
 
 
 def declare(name: str, restype, argtypes) -> None:
     _SIGNATURES[name] = (restype, list(argtypes))
+    _RESOLVED.pop(name, None)
     if _lib is not None and hasattr(_lib, name):
         fn = getattr(_lib, name)
         fn.restype = restype
@@ -65,8 +68,12 @@ _LAUNCH_PREFIXES = ("mep_launch_", "mep_gemm_launch", "mep_router_", "mep_swiglu
 def call(name: str, *args):
     """Call a declared entry point; raises if the symbol is missing (no silent fallback)."""
     global LAUNCHES
-    if name.startswith(_LAUNCH_PREFIXES):
-        LAUNCHES += 1
+    fn, launches = _RESOLVED.get(name) or _resolve(name)
+    LAUNCHES += launches
+    return fn(*args)
+
+
+def _resolve(name: str) -> tuple:
     handle = lib()
     try:
         fn = getattr(handle, name)
@@ -74,7 +81,8 @@ def call(name: str, *args):
         raise RuntimeError(f"native symbol {name} missing from {_build.LIB_PATH}") from exc
     if name in _SIGNATURES and fn.argtypes is None:
         fn.restype, fn.argtypes = _SIGNATURES[name][0], _SIGNATURES[name][1]
-    return fn(*args)
+    _RESOLVED[name] = entry = (fn, int(name.startswith(_LAUNCH_PREFIXES)))
+    return entry
 
 
 def ptr(t) -> int:
@@ -84,8 +92,9 @@ def ptr(t) -> int:
 
 def stream() -> int:
     """Handle of the current device's current stream.  (``torch.cuda.current_stream()`` builds a Stream
-    object around it, a few us a call: with ~25 launches a tenth of a small step.)"""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    object around it, a few us a call: with ~25 launches a tenth of a small step.  CUDA is initialised: whoever
+    launches something has device memory, so ``torch.cuda.current_device()``'s check for it is left out.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def last_error() -> str:

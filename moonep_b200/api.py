@@ -171,6 +171,7 @@ class Buffer:
                 (meta_ints,), torch.int32, group=self.group, device=self.device)
         self.hidden_stride = self.hidden_buf.shape[0] // R
         self.hidden_buf2 = None
+        self._own_views: dict = {}
         self.meta_stride = self.meta_buf.shape[0] // R
         offs = (ctypes.c_int64 * 6)()
         nat.call("mep_meta_offsets", self.NvS, R, E, offs)
@@ -229,6 +230,22 @@ class Buffer:
         hb = buf.view(self.R, self.hidden_stride, self.H)
         return hb[:, : self.NvS] if self.virtual else hb[self.rank: self.rank + 1, : self.NvS]
 
+    def _own_view(self, name, make) -> torch.Tensor:
+        """A view of this Buffer's memory, made once.  For looking at only: what a caller gets is an alias of its own
+        (``detach``), so that nothing it does to the tensor object stays behind here."""
+        v = self._own_views.get(name)
+        if v is None:
+            v = make()
+            self._own_views[name] = v = v if self.virtual else v[0]
+        return v
+
+    def _hidden_own(self, shard: int = 0) -> torch.Tensor:
+        return self._own_view(shard, lambda: self._shards(shard))
+
+    def _weights_own(self) -> torch.Tensor:
+        return self._own_view("weights", lambda: self._meta_rows()[:, self.weights_off: self.weights_off + self.NvS]
+                              .view(torch.float32))
+
     def enable_second_shard(self) -> None:
         """Allocates a second symmetric ``[NvS, H]`` row buffer (collective, once).  ``dispatch(...,
         zero_copy=True, shard=1)`` then lands a forward pass's rows there and returns them in
@@ -264,8 +281,7 @@ class Buffer:
     def hidden_view(self, shard: int = 0) -> torch.Tensor:
         """``hidden_nvsh_buffer_view`` of the given shard."""
         self._require()
-        v = self._shards(shard)
-        return v if self.virtual else v[0]
+        return self._hidden_own(shard).detach()
 
     def _meta_rows(self) -> torch.Tensor:
         mb = self.meta_buf.view(self.R, self.meta_stride)
@@ -275,15 +291,13 @@ class Buffer:
     def hidden_nvsh_buffer_view(self) -> torch.Tensor:
         """``[NvS, H]`` bf16 view of this rank's dispatch shard (``[R, NvS, H]`` when virtual)."""
         self._require()
-        v = self._shards()
-        return v if self.virtual else v[0]
+        return self._hidden_own().detach()
 
     @property
     def router_weight_buffer_view(self) -> torch.Tensor:
         """``[NvS]`` fp32 view of this rank's route-weight slots."""
         self._require()
-        v = self._meta_rows()[:, self.weights_off: self.weights_off + self.NvS].view(torch.float32)
-        return v if self.virtual else v[0]
+        return self._weights_own().detach()
 
     def check(self) -> None:
         """Synchronise and raise ``CommTimeoutError`` if any device-side wait ran out."""
@@ -396,7 +410,6 @@ class Buffer:
         dev = x.device
         st = self._stream()
         fresh = plan is None
-        i32 = dict(dtype=torch.int32, device=dev)
         if fresh:
             plan = self._fresh_plan(topk, tpe, dev, st)
         self._rc(nat.call("mep_launch_dispatch", self._ctx, x.data_ptr(), nat.ptr(w),
@@ -408,27 +421,27 @@ class Buffer:
         if not self._one_device:
             self._rc(nat.call("mep_launch_expand", self._ctx, plan.link.data_ptr(),
                               plan.cu_seqlens.data_ptr(), shard, st), "dispatch expand")
-        view = self.hidden_view(shard)
-        hidden = view if zero_copy else view.clone()
+        view = self._hidden_own(shard)
+        hidden = view.detach() if zero_copy else view.clone()
         weights = None
         if w is not None:
-            wv = self.router_weight_buffer_view
-            weights = wv if w_zero_copy else wv.clone()
+            wv = self._weights_own()
+            weights = wv.detach() if w_zero_copy else wv.clone()
         self._stats["dispatch"] += 1
         self._stats["bytes_dispatch"] += self.N * self.H * 2 * self.Rv
         self._maybe_check()
         return hidden, weights, (plan.cu_seqlens if fresh else None), plan
 
     def _fresh_plan(self, topk, tpe, dev, st) -> CommPlan:
-        i32 = dict(dtype=torch.int32, device=dev)
-        dst = torch.empty(self._shape(self.N), **i32)
-        cu = torch.empty(self._shape(2 * self.epn), **i32)
-        zf = torch.empty(self._shape(2 * self.epn, 2), **i32)
-        etc = torch.empty(self._shape(self.R, self.epn), **i32)
-        rs = torch.empty(self._shape(2), **i32)
-        link = torch.empty(self._shape(self.NvS), **i32)
-        src = torch.empty(self._shape(self.NvS), **i32)
-        order = torch.empty(self._shape(self.N), **i32)
+        empty = tpe.new_empty                  # int32 on this device, with less to parse than torch.empty
+        dst = empty(self._shape(self.N))
+        cu = empty(self._shape(2 * self.epn))
+        zf = empty(self._shape(2 * self.epn, 2))
+        etc = empty(self._shape(self.R, self.epn))
+        rs = empty(self._shape(2))
+        link = empty(self._shape(self.NvS))
+        src = empty(self._shape(self.NvS))
+        order = empty(self._shape(self.N))
         self._rc(nat.call("mep_launch_plan", self._ctx, topk.data_ptr(), tpe.data_ptr(),
                           dst.data_ptr(), cu.data_ptr(), zf.data_ptr(), etc.data_ptr(),
                           rs.data_ptr(), order.data_ptr(), st), "plan")
@@ -515,7 +528,7 @@ class Buffer:
         assert tuple(hidden_nvsh.shape) == self._shape(self.NvS, self.H)
         assert plan.N == self.N and plan.NvS == self.NvS and plan.R == self.R
         if zero_copy:
-            assert hidden_nvsh.data_ptr() == self.hidden_nvsh_buffer_view.data_ptr(), \
+            assert hidden_nvsh.data_ptr() == self._hidden_own().data_ptr(), \
                 "zero_copy combine needs hidden_nvsh to alias the Buffer's dispatch view"
         else:
             assert hidden_nvsh.is_contiguous()
@@ -523,7 +536,7 @@ class Buffer:
             assert route_weights_nvs.dtype == torch.float32
             assert tuple(route_weights_nvs.shape) == self._shape(self.NvS)
             if router_weights_zero_copy:
-                assert route_weights_nvs.data_ptr() == self.router_weight_buffer_view.data_ptr(), \
+                assert route_weights_nvs.data_ptr() == self._weights_own().data_ptr(), \
                     "router_weights_zero_copy needs route_weights_nvs to alias the Buffer's weight view"
 
         def run():
@@ -545,9 +558,9 @@ class Buffer:
         if inter_rank_sync and not self._one_device:
             self._rc(nat.call("mep_launch_sync", self._ctx, st), "inter_rank_sync")
         if not zero_copy:
-            self.hidden_nvsh_buffer_view.copy_(hidden_nvsh)
+            self._hidden_own().copy_(hidden_nvsh)
         if w_nvs is not None and not w_zero_copy:
-            self.router_weight_buffer_view.copy_(w_nvs)
+            self._weights_own().copy_(w_nvs)
         if not self._one_device:
             self._rc(nat.call("mep_launch_combine_prologue", self._ctx, plan.link.data_ptr(),
                               plan.cu_seqlens.data_ptr(), st), "combine prologue")
@@ -788,6 +801,7 @@ class Buffer:
         if self._destroyed:
             return
         self._destroyed = True
+        self._own_views.clear()
         if self in _LIVE_BUFFERS:
             _LIVE_BUFFERS.remove(self)
         try:

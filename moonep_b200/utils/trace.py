@@ -18,17 +18,31 @@ from collections import OrderedDict
 import torch
 
 
+class _NoSpan(contextlib.ContextDecorator):
+    """The span of a tracer that is off: one object for all of them (a generator-based context manager a span
+    was 1.2 us, fourteen times a training step)."""
+
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NO_SPAN = _NoSpan()
+
+
 class Tracer:
     def __init__(self, enabled: bool = False, nvtx: bool = True):
         self.enabled = enabled
         self.nvtx = nvtx
         self._spans: list[tuple[str, torch.cuda.Event, torch.cuda.Event]] = []
 
-    @contextlib.contextmanager
     def span(self, name: str):
-        if not self.enabled:
-            yield
-            return
+        return self._timed(name) if self.enabled else _NO_SPAN
+
+    @contextlib.contextmanager
+    def _timed(self, name: str):
         if self.nvtx:
             torch.cuda.nvtx.range_push(name)
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
