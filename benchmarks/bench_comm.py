@@ -134,11 +134,11 @@ class OursArm:
         r["k_plan_us"] = timed(lambda: (nat.call(
             "mep_launch_plan", buf._ctx, self.topk.data_ptr(), self.tpe.data_ptr(), plan.dst.data_ptr(),
             plan.cu_seqlens.data_ptr(), plan.zero_fill_ranges.data_ptr(), plan.experts_to_copy.data_ptr(),
-            plan.remote_stats.data_ptr(), plan.send_order.data_ptr(), st()),
+            plan.remote_stats.data_ptr(), plan.send_order.data_ptr(), 0, 0, st()),
             nat.call("mep_launch_sync", buf._ctx, st())))
         r["k_dispatch_us"] = timed(lambda: nat.call(
             "mep_launch_dispatch", buf._ctx, x.data_ptr(), 0, plan.dst.data_ptr(),
-            plan.zero_fill_ranges.data_ptr(), 0, 0, 1, 0, 0, 0, st()))
+            plan.zero_fill_ranges.data_ptr(), 0, 0, 1, 0, 0, 0, 0, 0, 0, 0, st()))
         r["k_expand_us"] = timed(lambda: nat.call(
             "mep_launch_expand", buf._ctx, plan.link.data_ptr(), plan.cu_seqlens.data_ptr(), 0, st()))
         r["k_prologue_us"] = timed(lambda: nat.call(

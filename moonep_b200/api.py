@@ -49,10 +49,10 @@ nat.declare("mep_trace_ints64", L, [])
 nat.declare("mep_trace_dims", None, [ctypes.POINTER(ctypes.c_int)])
 nat.declare("mep_ctx_set_trace", None, [P, P])
 nat.declare("mep_ctx_direct_ctas", I, [P])
-nat.declare("mep_launch_plan", I, [P, P, P, P, P, P, P, P, P, P])
+nat.declare("mep_launch_plan", I, [P, P, P, P, P, P, P, P, P, P, P, P])
 nat.declare("mep_launch_arrive_reset", I, [P, P])
 nat.declare("mep_launch_plan_snapshot", I, [P, P, P, P])
-nat.declare("mep_launch_dispatch", I, [P, P, P, P, P, P, P, I, I, I, I, P])
+nat.declare("mep_launch_dispatch", I, [P, P, P, P, P, P, P, I, I, I, I, I, P, P, I, P])
 nat.declare("mep_launch_push_reduce", I, [P, P, L, P, L, P, P, P, P, P, I, P])
 nat.declare("mep_launch_expand", I, [P, P, P, I, P])
 nat.declare("mep_launch_combine_prologue", I, [P, P, P, P])
@@ -411,13 +411,8 @@ class Buffer:
         st = self._stream()
         fresh = plan is None
         if fresh:
-            plan = self._fresh_plan(topk, tpe, dev, st)
-        self._rc(nat.call("mep_launch_dispatch", self._ctx, x.data_ptr(), nat.ptr(w),
-                          plan.dst.data_ptr(), plan.zero_fill_ranges.data_ptr(),
-                          plan.link.data_ptr() if fresh else 0,
-                          plan.src_info.data_ptr() if fresh else 0,
-                          int(bool(inter_rank_sync) and not fresh), int(fresh), shard,
-                          int(self._one_device), st), "dispatch")
+            plan = self._fresh_plan(topk, tpe, dev, st, records=self._one_device)
+        self._launch_dispatch(x, w, plan, st, fresh, shard, int(bool(inter_rank_sync) and not fresh))
         if not self._one_device:
             self._rc(nat.call("mep_launch_expand", self._ctx, plan.link.data_ptr(),
                               plan.cu_seqlens.data_ptr(), shard, st), "dispatch expand")
@@ -432,7 +427,39 @@ class Buffer:
         self._maybe_check()
         return hidden, weights, (plan.cu_seqlens if fresh else None), plan
 
-    def _fresh_plan(self, topk, tpe, dev, st) -> CommPlan:
+    def _launch_dispatch(self, x, w, plan, st, fresh, shard, entry_barrier, rows=0, w_rows=0, keep_padding=0):
+        self._rc(nat.call("mep_launch_dispatch", self._ctx, x.data_ptr(), nat.ptr(w),
+                          plan.dst.data_ptr(), plan.zero_fill_ranges.data_ptr(),
+                          plan.link.data_ptr() if fresh else 0,
+                          plan.src_info.data_ptr() if fresh else 0,
+                          entry_barrier, int(fresh), shard, int(self._one_device),
+                          int(fresh and self._one_device), rows, w_rows, keep_padding, st), "dispatch")
+
+    def _dispatch_lone(self, x, w, topk, tpe, *, keep: bool, shard: int):
+        """A lone rank's dispatch with a fresh plan for a layer of its own: ``(rows, weights, cu_seqlens, plan)``.
+        With ``keep`` (a backward pass will read them again) the weights, and unless ``shard`` is 1 the
+        rows, are received in tensors of their own: what ``dispatch`` copies out of the Buffer afterwards is
+        written once.  Without ``keep`` they stay in the Buffer, and padding rows keep whatever they hold: products
+        are row by row, and no row of padding leaves a GEMM that is given the plan's padding ranges."""
+        self._require()
+        assert self._one_device and not self.virtual
+        assert x.dtype == torch.bfloat16 and x.is_cuda and x.is_contiguous() and tuple(x.shape) == (self.S, self.H)
+        assert x.data_ptr() % 16 == 0
+        assert w.dtype == torch.float32 and w.is_contiguous() and tuple(w.shape) == (self.S, self.K)
+        st = self._stream()
+        plan = self._fresh_plan(topk, tpe, x.device, st, records=True)
+        own = keep and shard == 0
+        rows = x.new_empty((self.NvS, self.H)) if own else self._hidden_own(shard).detach()
+        weights = w.new_empty((self.NvS,)) if keep else self._weights_own().detach()
+        self._launch_dispatch(x, w, plan, st, True, shard, 0, rows.data_ptr() if own else 0,
+                              weights.data_ptr() if keep else 0, int(not keep))
+        self._stats["dispatch"] += 1
+        self._stats["bytes_dispatch"] += self.N * self.H * 2
+        self._maybe_check()
+        return rows, weights, plan.cu_seqlens, plan
+
+    def _fresh_plan(self, topk, tpe, dev, st, records: bool = False) -> CommPlan:
+        """``records``: the planner writes links and source records into the plan itself (one device)."""
         empty = tpe.new_empty                  # int32 on this device, with less to parse than torch.empty
         dst = empty(self._shape(self.N))
         cu = empty(self._shape(2 * self.epn))
@@ -444,7 +471,8 @@ class Buffer:
         order = empty(self._shape(self.N))
         self._rc(nat.call("mep_launch_plan", self._ctx, topk.data_ptr(), tpe.data_ptr(),
                           dst.data_ptr(), cu.data_ptr(), zf.data_ptr(), etc.data_ptr(),
-                          rs.data_ptr(), order.data_ptr(), st), "plan")
+                          rs.data_ptr(), order.data_ptr(), link.data_ptr() if records else 0,
+                          src.data_ptr() if records else 0, st), "plan")
         plan = CommPlan(dst=dst, experts_to_copy=etc, zero_fill_ranges=zf, remote_stats=rs,
                         cu_seqlens=cu, link=link, N=self.N, R=self.R, E=self.E, NvS=self.NvS,
                         K=self.K, src_info=src, send_order=order)

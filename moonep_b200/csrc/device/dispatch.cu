@@ -38,6 +38,11 @@ struct DispatchParams {
   int32_t* src_out;           // [Rv][NvS] or null
   int entry_barrier;
   int fresh;                  // plan made by the preceding planner launch
+  float* w_rows;              // where the route weights land instead of the meta chunk (a lone rank), or null
+  int keep_padding;           // the payload of padding rows is left as it is
+  // The planner has written the links and source records into link_out / src_out itself (one device): only those
+  // of padding rows are set here, and nothing is copied behind a barrier.
+  int records_written;
   // Every destination's row buffer is on this device: duplicates are stored from the staged row, and
   // launches of one stream order what the cross-rank entry barrier would.  8 ranks x 4096 tokens x
   // 7168, top-8: one launch of 0.59 ms and an expansion of 0.95 ms (which reads every primary row
@@ -131,8 +136,10 @@ __global__ void __launch_bounds__(DISPATCH_THREADS, 1) ep_dispatch_kernel(const 
         int d = dst[e];
         int64_t raw = d >= 0 ? d : -(int64_t)d - 1;
         int64_t dr = raw / p.NvS, row = raw - dr * p.NvS;
-        if (dr < sc.R)
-          sc.meta[(size_t)dr * sc.meta_stride + p.weights_off + row] = __float_as_int(w[e]);
+        if (dr < sc.R) {
+          if (p.w_rows != nullptr) p.w_rows[row] = w[e];
+          else sc.meta[(size_t)dr * sc.meta_stride + p.weights_off + row] = __float_as_int(w[e]);
+        }
       }
     }
   } else {
@@ -155,7 +162,7 @@ __global__ void __launch_bounds__(DISPATCH_THREADS, 1) ep_dispatch_kernel(const 
         const int c_rot = (int)((unsigned)(c + (g0 + i) * 7) % (unsigned)G);
         if (warp == 2) {
           // one elected thread issues the row stores of this CTA's share
-          if (lane == 0) {
+          if (lane == 0 && !p.keep_padding) {
             for (int r = first + c_rot; r < first + n; r += G) {
               bulk_s2g(my_shard + (size_t)r * p.H, zero_row, row_bytes);
               if (++pending == 16) { bulk_commit(); bulk_wait_read<4>(); pending = 0; }
@@ -163,8 +170,17 @@ __global__ void __launch_bounds__(DISPATCH_THREADS, 1) ep_dispatch_kernel(const 
           }
         } else {
           for (int r = first + c_rot * 32 + lane; r < first + n; r += G * 32) {
-            if (p.w != nullptr) my_meta[p.weights_off + r] = 0;
-            if (p.fresh) { my_meta[p.link_off + r] = LINK_NONE; my_meta[p.src_off + r] = -1; }
+            if (p.w != nullptr) {
+              if (p.w_rows != nullptr) p.w_rows[r] = 0.f;
+              else my_meta[p.weights_off + r] = 0;
+            }
+            if (p.records_written) {
+              p.link_out[(size_t)vr * p.NvS + r] = LINK_NONE;
+              p.src_out[(size_t)vr * p.NvS + r] = -1;
+            } else if (p.fresh) {
+              my_meta[p.link_off + r] = LINK_NONE;
+              my_meta[p.src_off + r] = -1;
+            }
           }
         }
       }
@@ -174,7 +190,7 @@ __global__ void __launch_bounds__(DISPATCH_THREADS, 1) ep_dispatch_kernel(const 
   if (tid == 0) phase_stamp(sc.trace, 0, c, 2);          // this CTA's rows, weights and padding issued
   // With everything on one device the end of the launch orders the rows; the barrier is then only
   // needed ahead of the snapshots below, which read what other CTAs wrote.
-  if (p.direct && p.link_out == nullptr && p.src_out == nullptr) return;
+  if (p.direct && (p.records_written || (p.link_out == nullptr && p.src_out == nullptr))) return;
   fence_sys();
   cross_rank_barrier(sc, 2);
   if (tid == 0) phase_stamp(sc.trace, 0, c, 3);          // past the exit barrier
@@ -334,8 +350,10 @@ static int launch_dispatch_t(const BufferCtx& c, DispatchParams& p, size_t smem,
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_dispatch_kernel<ST>, raised));
   dim3 grid(p.direct ? c.direct_ctas() : c.num_sms, c.Rv());
+  // (no barrier inside where everything is on one device and there is nothing to copy at the end)
+  const bool barrier = !p.direct || (p.link_out != nullptr && !p.records_written);
   MEP_CUDA_OK(launch_chained((const void*)ep_dispatch_kernel<ST>, grid, dim3(DISPATCH_THREADS), smem,
-                             stream, p, /*coop=*/1, c.pdl && p.fresh));
+                             stream, p, /*coop=*/barrier, c.pdl && p.fresh));
   return 0;
 }
 
@@ -350,20 +368,29 @@ extern "C" {
 // precedes this one on the stream (its barrier stands in for the entry sync).  shard selects
 // the row buffer the rows land in (0, or 1 once a second shard is registered).  direct != 0 (only
 // where every rank's buffer is on this device) also stores the duplicates; no expansion follows.
+// records_written != 0 (direct, fresh): the planner was given link_out and src_out.  A lone rank (direct) may
+// receive elsewhere than in a shard: rows [NvS][H] and w_rows [NvS] (null: the shard, the meta chunk); with
+// keep_padding padding rows are not cleared.
 int mep_launch_dispatch(const void* ctx_, const void* x, const float* w, const int32_t* dst,
                         const int32_t* zero_fill, int32_t* link_out, int32_t* src_out, int entry_barrier,
-                        int fresh, int shard, int direct, cudaStream_t stream) {
+                        int fresh, int shard, int direct, int records_written, void* rows, float* w_rows,
+                        int keep_padding, cudaStream_t stream) {
   const BufferCtx& c = *(const BufferCtx*)ctx_;
   if (c.H % 8 != 0) return fail(-1, "dispatch needs H %% 8 == 0 (got %d)", c.H);
   if (c.shard_base(shard) == nullptr) return fail(-4, "dispatch: shard %d does not exist", shard);
   if (direct && !c.one_device()) return fail(-5, "dispatch: duplicates travel only within one device");
+  if ((records_written || keep_padding) && !direct) return fail(-6, "dispatch: records and padding are handled here only within one device");
+  if ((rows != nullptr || w_rows != nullptr) && (!direct || c.R != 1)) return fail(-7, "dispatch: rows of a lone rank only go elsewhere");
+  if (records_written && (!fresh || link_out == nullptr || src_out == nullptr)) return fail(-8, "dispatch: no records to complete");
+  if (((uintptr_t)rows & 15) != 0) return fail(-9, "dispatch: rows must be 16-byte aligned");
   DispatchParams p;
   p.sync = c.sync(KID_DISPATCH);
   p.S = c.S; p.K = c.K; p.H = c.H; p.epn = c.epn;
   p.N = c.N; p.NvS = c.NvS; p.hidden_stride = c.hidden_stride;
   p.weights_off = c.ml.weights_off; p.link_off = c.ml.link_off; p.src_off = c.ml.src_off;
   p.x = (const __nv_bfloat16*)x; p.w = w; p.dst = dst; p.zero_fill = zero_fill;
-  p.hidden = (__nv_bfloat16*)c.shard_base(shard); p.link_out = link_out; p.src_out = src_out;
+  p.hidden = (__nv_bfloat16*)(rows != nullptr ? rows : c.shard_base(shard)); p.link_out = link_out; p.src_out = src_out;
+  p.w_rows = w_rows; p.keep_padding = keep_padding; p.records_written = records_written;
   p.entry_barrier = entry_barrier; p.fresh = fresh; p.direct = direct;
   const size_t row = (size_t)c.H * 2;
   switch (dispatch_ring(c)) {

@@ -128,6 +128,7 @@ extern "C" int mep_plan_local_noalloc(const int32_t* tpe_all, const int32_t* top
   p.etc = etc; p.remote_stats = remote_stats;
   p.scratch = scratch; p.scratch_ints = NOALLOC_INTS;
   p.send_order = nullptr; p.arrive_off = 0; p.n_arrive = 0; p.one_device = 0; p.tables = 0;
+  p.link_out = nullptr; p.src_out = nullptr;
   lp.tpe_all = tpe_all; lp.rank = rank; lp.status_out = status;
   const size_t smem = sizeof(int32_t) * (2 * (size_t)E + 4 * (size_t)R + (size_t)PLAN_WARPS * R);
   if (smem > 40 * 1024) {     // (beside the kernel's static part)

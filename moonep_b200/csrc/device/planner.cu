@@ -222,8 +222,10 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) ep_plan_kernel(const PlanPara
       const int next = above ? (int)(raw_next - (int64_t)dr * p.NvS) : LINK_NONE;
       const int64_t row = raw - (int64_t)dr * p.NvS;
       int32_t* peer = sc.meta + (size_t)dr * sc.meta_stride;
-      peer[p.link_off + row] = next | (dup ? LINK_DUP_BIT : 0);
-      peer[p.src_off + row] = (int32_t)((int64_t)rank * p.N + (int64_t)t * K + k);
+      int32_t* link = p.link_out != nullptr ? p.link_out + (size_t)dr * p.NvS : peer + p.link_off;
+      int32_t* src = p.src_out != nullptr ? p.src_out + (size_t)dr * p.NvS : peer + p.src_off;
+      link[row] = next | (dup ? LINK_DUP_BIT : 0);
+      src[row] = (int32_t)((int64_t)rank * p.N + (int64_t)t * K + k);
       if (dup) d[k] = -raw - 1;
     }
   }
@@ -286,11 +288,15 @@ int64_t mep_plan_launch_smem_bytes(const void* ctx_) {
 // Fresh plan for this rank (or for all virtual ranks).  send_order [Rv][N] may be null (it is
 // only needed by the fused dispatch -> GEMM path).  Leaves the chain links in the peers'
 // meta chunks; they become visible with the next cross-rank barrier (the dispatch kernel's
-// exit barrier, or an explicit mep_launch_sync).
+// exit barrier, or an explicit mep_launch_sync).  Within one device link_out and src_out [Rv][NvS] may take the
+// records of all real rows instead (the dispatch that follows sets those of padding rows): that saves
+// dispatch its exit barrier and the copies behind it, 6 - 9 us.
 int mep_launch_plan(const void* ctx_, const int32_t* topk, const int32_t* tpe, int32_t* dst,
                     int32_t* cu_seqlens, int32_t* zero_fill, int32_t* etc, int32_t* remote_stats,
-                    int32_t* send_order, cudaStream_t stream) {
+                    int32_t* send_order, int32_t* link_out, int32_t* src_out, cudaStream_t stream) {
   const BufferCtx& c = *(const BufferCtx*)ctx_;
+  if ((link_out != nullptr || src_out != nullptr) && !c.one_device())
+    return fail(-1, "plan: records go straight into the plan only within one device");
   PlanParams p;
   p.sync = c.sync(KID_PLAN);
   p.E = c.E; p.epn = c.epn; p.S = c.S; p.K = c.K; p.token_padding = c.token_padding;
@@ -303,6 +309,7 @@ int mep_launch_plan(const void* ctx_, const int32_t* topk, const int32_t* tpe, i
   const size_t smem = (size_t)mep_plan_launch_smem_bytes(ctx_);
   p.rank_warps = plan_rank_warps(c);
   p.one_device = c.one_device();
+  p.link_out = link_out; p.src_out = src_out;
   p.tables = (int)(plan_tables(c) / sizeof(int32_t));
   p.rank_counts = p.rank_warps > 1 ? (int)(mep_plan_smem_bytes(c.R, c.E) / sizeof(int32_t)) : 0;
   static std::atomic<unsigned long long> raised{0};

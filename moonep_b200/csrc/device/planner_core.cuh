@@ -32,6 +32,8 @@ struct PlanParams {
   int64_t arrive_off;       // ARRIVE counters in the meta chunk, cleared before the exchange
   int n_arrive;
   int rank_warps, rank_counts;   // warps that number the entries, and where their counters start in shared memory
+  int32_t* link_out;        // [Rv][NvS] each, one device: where links and source records go instead of the meta chunks
+  int32_t* src_out;
   int one_device;           // every rank's counts are in `tpe`, and stream order separates launches
   int tables;               // where the solver's tables start in shared memory; 0: they stay in the scratch
 };

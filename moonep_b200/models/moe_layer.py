@@ -87,6 +87,8 @@ class _MoEFn(torch.autograd.Function):
             if fused:
                 # only the plan is made here: the rows travel inside the gate/up GEMM launch below
                 hidden, w_nvs, cu, plan, disp = buf.dispatch_fused_begin(x, w, topk, tpe, shard=shard)
+            elif buf._one_device:
+                hidden, w_nvs, cu, plan = buf._dispatch_lone(x, w, topk, tpe, keep=keep, shard=shard)
             elif layer.hidden_in_place:
                 hidden, w_nvs, cu, plan = buf.dispatch(x, w, topk, tpe, zero_copy=True, shard=1)
             else:
