@@ -57,6 +57,7 @@ struct GemmKParams {
   // weight pieces of an epilogue warp (SGD)
   int unit, row_slots, col_slots, pieces;
   int vec32;   // weight grad: rows of the weights allow 32-byte accesses
+  int products; // weight grad: 2 = a second one with the same A (b[1], out + 2, sgd_w[1])
   // SGD kernels: 1 = only the tiles whose grads are STORED (experts with replicas, slot groups),
   // 2 = only the tiles that are applied to the weights, 0 = all.  Lets the grads that have to
   // travel be computed first, so that their reduce runs beside the rest of the weight grad.
@@ -67,11 +68,11 @@ struct GemmKParams {
   // weights, w = bf16(w - lr * acc), instead of being stored as an fp32 grad.  Experts whose
   // sgd_keep flag is set (they have replicas elsewhere, whose grads must be added first) and the
   // slot groups are still written as fp32 grads.
-  __nv_bfloat16* sgd_w;
-  CUtensorMap wmap;        // the same weights as a [G0 * Mw][N] bf16 tensor, 16-row x 64-column boxes
+  __nv_bfloat16* sgd_w[2];
+  CUtensorMap wmap[2];        // the same weights as a [G0 * Mw][N] bf16 tensor, 16-row x 64-column boxes
   const int32_t* sgd_keep;
   float sgd_lr;
-  void* out[3];
+  void* out[4];
   const float* row_scale;
   long long ldc;
   int32_t* status;
@@ -169,7 +170,7 @@ struct GemmDesc {
   int64_t b_rows[2];
   int64_t ldb;
   const int32_t* cu_seqlens;
-  void* out[3];
+  void* out[4];            // weight grad: local and slot grads, of the second product behind them
   int64_t ldc;
   const float* row_scale;
   int32_t* status;
@@ -179,7 +180,7 @@ struct GemmDesc {
   int64_t push_rank_stride;
   int32_t push_entries, push_ranks;
   int32_t two_cta, wg_select;
-  void* sgd_w;
+  void* sgd_w[2];
   const int32_t* sgd_keep;
   float sgd_lr;
   // Fused dispatch (0 = off): 1 = only wait for the rows of each tile to arrive, 2 = also send
@@ -300,7 +301,7 @@ static int launch_single(const void* kern, std::atomic<unsigned long long>& rais
 static void wgrad_geometry(GemmKParams* kp, bool pair) {
   const int local = kp->split < kp->ngroups ? kp->split : kp->ngroups;
   const double kb = (double)kp->total_rows / (local > 0 ? local : 1) / BK;
-  const bool sgd = kp->sgd_w != nullptr, brief = kb <= 8;
+  const bool sgd = kp->sgd_w[0] != nullptr, brief = kb <= 8;
   kp->pieces = sgd ? (brief ? 2 : 1) : 0;
   if (pair) {
     kp->row_slots = sgd ? (brief ? 5 : 6) : 7;
@@ -380,7 +381,7 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
   kp.g_begin = d->g_begin; kp.pads = d->pads;
   kp.src_info = d->src_info; kp.push_base = d->push_base; kp.push_rank_stride = d->push_rank_stride;
   kp.push_entries = d->push_entries; kp.push_ranks = d->push_ranks;
-  kp.out[0] = d->out[0]; kp.out[1] = d->out[1]; kp.out[2] = d->out[2];
+  kp.out[0] = d->out[0]; kp.out[1] = d->out[1]; kp.out[2] = d->out[2]; kp.out[3] = d->out[3];
   kp.row_scale = d->row_scale; kp.ldc = d->ldc; kp.status = d->status;
   kp.timeout_ns = (unsigned long long)(d->timeout_ns > 0 ? d->timeout_ns : 2000000000ll);
   int dev = 0, sms = 148;
@@ -392,24 +393,31 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
     // weight grad: A [a_rows][Mw] and B [a_rows][N], both read as MN-major 64x64 boxes
     if (d->Mw % BM != 0) return fail(-2, "wgrad: Mw=%d must be a multiple of %d", d->Mw, BM);
     if ((rc = make_map(&kp.a, d->a[0], d->a_rows, d->Mw, d->lda[0], 64, BK))) return rc;
-    if ((rc = make_map(&kp.b[0][0], d->b[0][0], d->a_rows, d->N, d->ldb, 64, BK))) return rc;
     if (d->epi != EPI_F32) return fail(-3, "wgrad writes fp32");
-    if (d->sgd_w != nullptr) {
+    kp.products = d->b[1][0] != nullptr ? 2 : 1;
+    if (d->sgd_w[0] != nullptr) {
       if (d->accumulate) return fail(-13, "wgrad: the fused SGD step cannot accumulate into existing grads");
-      if (d->N % 8 != 0 || ((uintptr_t)d->sgd_w & 15) != 0)
-        return fail(-14, "wgrad: the fused SGD step needs N %% 8 == 0 and 16-byte aligned weights");
-      kp.sgd_w = (__nv_bfloat16*)d->sgd_w; kp.sgd_keep = d->sgd_keep; kp.sgd_lr = d->sgd_lr;
-      const int n_w = d->split < d->ngroups ? d->split : d->ngroups;
-      if ((rc = make_map(&kp.wmap, d->sgd_w, (int64_t)n_w * d->Mw, d->N, d->ldc, 64, 16))) return rc;
+      kp.sgd_keep = d->sgd_keep; kp.sgd_lr = d->sgd_lr;
+      kp.vec32 = d->N % 16 == 0;
     }
-    if (d->ngroups > d->split && d->out[1] == nullptr) return fail(-8, "wgrad: groups >= split need a slot grad tensor");
-    if ((((uintptr_t)d->out[0] | (uintptr_t)d->out[1]) & 15) != 0 || d->ldc % 4 != 0)
-      return fail(-11, "weight-grad output must be 16-byte aligned with a 16-byte multiple row stride");
-    kp.vec32 = ((uintptr_t)d->sgd_w & 31) == 0 && d->N % 16 == 0;
+    for (int i = 0; i < kp.products; ++i) {
+      if ((rc = make_map(&kp.b[i][0], d->b[i][0], d->a_rows, d->N, d->ldb, 64, BK))) return rc;
+      if (d->sgd_w[0] != nullptr) {
+        if (d->N % 8 != 0 || d->sgd_w[i] == nullptr || ((uintptr_t)d->sgd_w[i] & 15) != 0)
+          return fail(-14, "wgrad: the fused SGD step needs N %% 8 == 0 and 16-byte aligned weights");
+        kp.sgd_w[i] = (__nv_bfloat16*)d->sgd_w[i];
+        kp.vec32 = kp.vec32 && ((uintptr_t)d->sgd_w[i] & 31) == 0;
+        const int n_w = d->split < d->ngroups ? d->split : d->ngroups;
+        if ((rc = make_map(&kp.wmap[i], d->sgd_w[i], (int64_t)n_w * d->Mw, d->N, d->ldc, 64, 16))) return rc;
+      }
+      if (d->ngroups > d->split && d->out[2 * i + 1] == nullptr) return fail(-8, "wgrad: groups >= split need a slot grad tensor");
+      if ((((uintptr_t)d->out[2 * i] | (uintptr_t)d->out[2 * i + 1]) & 15) != 0 || d->ldc % 4 != 0)
+        return fail(-11, "weight-grad output must be 16-byte aligned with a 16-byte multiple row stride");
+    }
     const bool pair = d->two_cta != 0 && grid >= 2;
     wgrad_geometry(&kp, pair);
-    kp.wg_select = kp.sgd_w != nullptr ? d->wg_select : 0;
-    if (kp.sgd_w != nullptr)
+    kp.wg_select = kp.sgd_w[0] != nullptr ? d->wg_select : 0;
+    if (kp.sgd_w[0] != nullptr)
       return launch_wgrad<true>(kp, pair, grid, stream);
     return launch_wgrad<false>(kp, pair, grid, stream);
   }

@@ -214,10 +214,8 @@ class _MoEFn(torch.autograd.Function):
         zc = layer.accumulate_grads            # the slots are overwritten next step otherwise
         if fused_lr is None:
             with tr.span("b.wgrad_gateup"):
-                gemm.wgrad(hidden, d_gate, cu, layer.g_gate, grad_slot=gslot("gate"), split=split, accumulate=acc,
-                           pads=pads)
-                gemm.wgrad(hidden, d_up, cu, layer.g_up, grad_slot=gslot("up"), split=split, accumulate=acc,
-                           pads=pads)
+                gemm.wgrad2(hidden, (d_gate, d_up), cu, (layer.g_gate, layer.g_up),
+                            grad_slot=(gslot("gate"), gslot("up")), split=split, accumulate=acc, pads=pads)
             if layer.hidden_in_place:  # the forward rows have had their last reader
                 buf.release_second_shard(layer)
             # the replicas' weight grads travel home on the comm stream while this stream computes dX
@@ -269,22 +267,25 @@ class _MoEFn(torch.autograd.Function):
                                               sgd=sgd(getattr(layer, "w_" + w)),
                                               pads=plan.zero_fill_ranges, **kw)
         with layer.tracer.span("b.wgrad_gateup"):
-            wg(d_gate, layer.g_gate, "gate")
-            if do_reduce:     # the gate grads travel home under the up projection's weight grad
+            if not do_reduce:
+                gemm.wgrad2(hidden, (d_gate, d_up), cu, (layer.g_gate, layer.g_up), grad_slot=(gslot("gate"), gslot("up")),
+                            split=split, sgd=((layer.w_gate, layer.w_up), *sgd(None)[1:]), pads=plan.zero_fill_ranges)
+            else:
+                wg(d_gate, layer.g_gate, "gate")
+                # the gate grads travel home under the up projection's weight grad
                 ev_r = layer.buf.reduce_grad_tensors(plan, [layer.g_gate], [pools.reduce["gate"]],
                                                      async_finish=True, zero_consumed=zc)
-            if do_reduce and layer.split_last_wgrad:
-                # The up grads are the last to be computed, and only the combine and the router
-                # backward are left to cover their way home.  So the grads that have to travel
-                # (experts with replicas elsewhere, this rank's slot groups) are computed first, in
-                # a short launch of their own, and leave while the rest is computed and applied.
-                wg(d_up, layer.g_up, "up", select=1, grid=layer.overlap_grid())
-                ev_r = layer.buf.reduce_grad_tensors(plan, [layer.g_up], [pools.reduce["up"]],
-                                                     async_finish=True, zero_consumed=zc)
-                wg(d_up, layer.g_up, "up", select=2, grid=layer.overlap_grid())
-            else:
-                wg(d_up, layer.g_up, "up", grid=layer.overlap_grid() if do_reduce else 0)
-                if do_reduce:
+                if layer.split_last_wgrad:
+                    # The up grads are the last to be computed, and only the combine and the router
+                    # backward are left to cover their way home.  So the grads that have to travel
+                    # (experts with replicas elsewhere, this rank's slot groups) are computed first, in
+                    # a short launch of their own, and leave while the rest is computed and applied.
+                    wg(d_up, layer.g_up, "up", select=1, grid=layer.overlap_grid())
+                    ev_r = layer.buf.reduce_grad_tensors(plan, [layer.g_up], [pools.reduce["up"]],
+                                                         async_finish=True, zero_consumed=zc)
+                    wg(d_up, layer.g_up, "up", select=2, grid=layer.overlap_grid())
+                else:
+                    wg(d_up, layer.g_up, "up", grid=layer.overlap_grid())
                     ev_r = layer.buf.reduce_grad_tensors(plan, [layer.g_up], [pools.reduce["up"]],
                                                          async_finish=True, zero_consumed=zc)
         if layer.hidden_in_place:      # the forward rows have had their last reader

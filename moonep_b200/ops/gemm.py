@@ -43,12 +43,12 @@ class _GemmDesc(ctypes.Structure):
         ("grid", ctypes.c_int32), ("g_begin", ctypes.c_int32),
         ("a_rows", ctypes.c_int64), ("lda", ctypes.c_int64 * 2), ("a", ctypes.c_void_p * 2),
         ("b", (ctypes.c_void_p * 2) * 2), ("b_rows", ctypes.c_int64 * 2), ("ldb", ctypes.c_int64),
-        ("cu_seqlens", ctypes.c_void_p), ("out", ctypes.c_void_p * 3), ("ldc", ctypes.c_int64),
+        ("cu_seqlens", ctypes.c_void_p), ("out", ctypes.c_void_p * 4), ("ldc", ctypes.c_int64),
         ("row_scale", ctypes.c_void_p), ("status", ctypes.c_void_p), ("timeout_ns", ctypes.c_int64),
         ("src_info", ctypes.c_void_p), ("push_base", ctypes.c_void_p),
         ("push_rank_stride", ctypes.c_int64), ("push_entries", ctypes.c_int32),
         ("push_ranks", ctypes.c_int32), ("two_cta", ctypes.c_int32), ("wg_select", ctypes.c_int32),
-        ("sgd_w", ctypes.c_void_p), ("sgd_keep", ctypes.c_void_p), ("sgd_lr", ctypes.c_float),
+        ("sgd_w", ctypes.c_void_p * 2), ("sgd_keep", ctypes.c_void_p), ("sgd_lr", ctypes.c_float),
         ("disp_mode", ctypes.c_int32), ("disp_ctx", ctypes.c_void_p), ("disp_x", ctypes.c_void_p),
         ("disp_w", ctypes.c_void_p), ("disp_dst", ctypes.c_void_p), ("disp_order", ctypes.c_void_p),
         ("disp_zero_fill", ctypes.c_void_p), ("disp_fresh", ctypes.c_int32), ("disp_shard", ctypes.c_int32),
@@ -291,11 +291,26 @@ def wgrad(a, b, cu_seqlens, grad_local, *, grad_slot=None, split=None, accumulat
     groups) and ``select=2`` only the ones that are applied; the two launches together equal one
     with ``select=0``.  The stored grads are the ones that ``reduce_grad`` has to move, so computing
     them first lets that transfer run beside the rest of the weight grad."""
-    _bf16(a, "a"), _bf16(b, "b")
+    assert select in (0, 1, 2) and (select == 0 or sgd is not None), "select splits a fused-SGD weight grad"
+    w, lr, keep = (None, None, None) if sgd is None else (sgd[0], float(sgd[1]), sgd[2])
+    _wgrads(a, ((b, grad_local, grad_slot, w),), cu_seqlens, split, accumulate, lr, keep, grid, select, pads)
+    return grad_local
+
+
+def wgrad2(a, b, cu_seqlens, grad_local, *, grad_slot=(None, None), split=None, accumulate=False, sgd=None,
+           grid=0, pads=None):
+    """Two weight grads that share ``a`` (gate and up projections) in one launch: :func:`wgrad` with pairs for
+    ``b``, ``grad_local``, ``grad_slot`` and the ``weights`` of ``sgd=(weights, lr, keep)``; same results."""
+    w, lr, keep = ((None, None), None, None) if sgd is None else (sgd[0], float(sgd[1]), sgd[2])
+    assert b[0].shape == b[1].shape and b[0].stride() == b[1].stride()
+    _wgrads(a, tuple(zip(b, grad_local, grad_slot, w)), cu_seqlens, split, accumulate, lr, keep, grid, 0, pads)
+    return grad_local
+
+
+def _wgrads(a, products, cu_seqlens, split, accumulate, lr, keep, grid, select, pads):
+    _bf16(a, "a")
     rows, M = a.shape
-    N = b.shape[1]
-    assert b.shape[0] == rows and grad_local.dtype == torch.float32 and grad_local.is_contiguous()
-    assert grad_local.shape[1:] == (M, N)
+    N = products[0][0].shape[1]
     d = _GemmDesc()
     d.mode, d.epi, d.b_mn, d.nseg = 1, EPI_F32, 1, 1
     cu_ptr, ngroups = _groups(cu_seqlens, rows)
@@ -306,30 +321,33 @@ def wgrad(a, b, cu_seqlens, grad_local, *, grad_slot=None, split=None, accumulat
     d.zero_empty_below = 0 if accumulate else d.split
     d.a_rows = rows
     d.a[0], d.lda[0] = a.data_ptr(), a.stride(0)
-    d.b[0][0], d.ldb = b.data_ptr(), b.stride(0)
     d.cu_seqlens = cu_ptr
-    d.out[0] = grad_local.data_ptr()
-    if grad_slot is not None:
-        assert grad_slot.dtype == torch.float32 and grad_slot.is_contiguous()
-        d.out[1] = grad_slot.data_ptr()
-    else:
-        assert d.split >= ngroups
-    d.ldc = N
-    d.grid = grid
-    d.pads = _pads(pads, cu_seqlens)
-    assert select in (0, 1, 2) and (select == 0 or sgd is not None), "select splits a fused-SGD weight grad"
-    if sgd is not None:
-        w, lr, keep = sgd
-        _bf16(w, "weights")
-        assert not accumulate and w.is_contiguous() and w.shape == grad_local.shape and N % 8 == 0
-        d.sgd_w, d.sgd_lr = w.data_ptr(), float(lr)
+    for i, (b, grad, slot, w) in enumerate(products):
+        _bf16(b, "b")
+        assert b.shape[0] == rows and grad.dtype == torch.float32 and grad.is_contiguous()
+        assert grad.shape[1:] == (M, N)
+        d.b[i][0], d.ldb = b.data_ptr(), b.stride(0)
+        d.out[2 * i] = grad.data_ptr()
+        if slot is not None:
+            assert slot.dtype == torch.float32 and slot.is_contiguous()
+            d.out[2 * i + 1] = slot.data_ptr()
+        else:
+            assert d.split >= ngroups
+        if lr is not None:
+            _bf16(w, "weights")
+            assert not accumulate and w.is_contiguous() and w.shape == grad.shape and N % 8 == 0
+            d.sgd_w[i] = w.data_ptr()
+    if lr is not None:
+        d.sgd_lr = lr
         d.wg_select = int(select)
         if keep is not None:
             assert keep.dtype == torch.int32 and keep.is_cuda and keep.numel() >= min(d.split, ngroups)
             d.sgd_keep = keep.data_ptr()
+    d.ldc = N
+    d.grid = grid
+    d.pads = _pads(pads, cu_seqlens)
     d.status = status_word(a.device).data_ptr()
     _launch(d)
-    return grad_local
 
 
 def dense(a, b, *, out_dtype=torch.float32, b_is_kn=True):

@@ -52,3 +52,32 @@ def test_edges(groups, M, N, two, monkeypatch):
     assert torch.equal(w, want)
     assert torch.equal(kept[G - 1], grad[G - 1]) and not bool(kept[:G - 1].any())
     gemm.check_status()
+
+
+@pytest.mark.parametrize("two", [0, 1])
+@pytest.mark.parametrize("M, N", [(128, 8), (384, 264), (640, 512)])
+def test_two_products_equal_one_each(M, N, two, monkeypatch):
+    """Bit for bit the two launches: stored, accumulated and applied grads, groups with slots and without rows."""
+    from moonep_b200.ops import gemm
+    monkeypatch.setattr(gemm, "TWO_CTA", two)
+    groups, split = [320, 0, 512, 64, 0, 128], 4
+    gen, ends, a, b0 = _inputs(groups, M, N, 3 * M + N)
+    b = (b0, torch.randn(a.shape[0], N, device="cuda", generator=gen).bfloat16())
+    rnd = lambda n: [torch.randn(n, M, N, device="cuda", generator=gen) for _ in range(2)]
+    copy = lambda ts: [t.clone() for t in ts]
+    local, slots = rnd(split), rnd(len(groups) - split)
+    w = [t.bfloat16() for t in rnd(split)]
+    keep = torch.tensor([0, 0, 1, 0], dtype=torch.int32, device="cuda")
+    for form in (dict(), dict(accumulate=True), dict(sgd=0.25)):
+        got, want = [], []
+        l, s, ws = copy(local), copy(slots), copy(w)
+        kw = dict(form, sgd=(ws, 0.25, keep)) if "sgd" in form else form
+        gemm.wgrad2(a, b, ends, l, grad_slot=s, split=split, **kw)
+        got += l + s + ws
+        l, s, ws = copy(local), copy(slots), copy(w)
+        for i in range(2):
+            kw = dict(form, sgd=(ws[i], 0.25, keep)) if "sgd" in form else form
+            gemm.wgrad(a, b[i], ends, l[i], grad_slot=s[i], split=split, **kw)
+        want += l + s + ws
+        assert all(torch.equal(x, y) for x, y in zip(got, want)), form
+    gemm.check_status()
