@@ -127,9 +127,10 @@ __global__ void ep_router_topk_bwd_kernel(const float* __restrict__ weights, con
 //                            dw = sum_h dact * silu(g) * u
 // One warp a row, whose lanes take its 16-byte vectors in turn, SB_DEPTH at once.  Bound by HBM (five bf16 tensors) and,
 // next to it, by issue.  A block a row left 160 of 256 threads idle at H' = 768 and met at two barriers a row: 36900
-// rows x 512 89 -> 46 us, x 2048 142 -> 134, 20000 x 1024 62 -> 48 (with the clearing of the sums in front).  More vectors
-// at once cost the registers of other warps (four: 185 us for x 2048).  A row's sum keeps the order that it had
-// there: eight partial sums, of the vectors with the same v / 32 % 8, each over the lanes first.
+// rows x 512 89 -> 46 us, x 2048 142 -> 134, 20000 x 1024 62 -> 48 (with the clearing of the sums in front, which the
+// kernel now does itself for the rows behind the last).  More vectors at once cost the registers of other warps (four:
+// 185 us for x 2048).  A row's sum keeps the order that it had there: eight partial sums, of the vectors with the
+// same v / 32 % 8, each over the lanes first.
 constexpr int SB_WARPS = 8, SB_DEPTH = 2;
 
 __global__ void __launch_bounds__(SB_WARPS * 32, 4)
@@ -201,6 +202,9 @@ ep_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bfloat16
       if (lane == 0) dscale[r] = part[0];
     }
   }
+  // rows that hold nothing
+  if (dscale)
+    for (int r = max(rows, 0) + blockIdx.x * SB_WARPS * 32 + threadIdx.x; r < max_rows; r += gridDim.x * SB_WARPS * 32) dscale[r] = 0.f;
 }
 
 // ---- cross-entropy over bf16 logits ---------------------------------------------------------------

@@ -60,7 +60,7 @@ def swiglu_bwd(dact, gate, up, row_scale=None, rows_ptr=None, want_dscale=True):
     for t in (dact, gate, up):
         assert t.dtype == torch.bfloat16 and t.is_contiguous()
     dgate, dup = torch.empty_like(dact), torch.empty_like(dact)
-    dscale = torch.zeros(rows, dtype=torch.float32, device=dact.device) if want_dscale else None
+    dscale = torch.empty(rows, dtype=torch.float32, device=dact.device) if want_dscale else None
     _rc(nat.call("mep_swiglu_bwd", dact.data_ptr(), gate.data_ptr(), up.data_ptr(),
                  nat.ptr(row_scale), nat.ptr(rows_ptr), rows, Hp, dgate.data_ptr(), dup.data_ptr(),
                  nat.ptr(dscale), _st()), "swiglu_bwd")

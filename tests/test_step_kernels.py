@@ -1,0 +1,54 @@
+"""Kernels around the layer's products at the edges of their ranges: SwiGLU backward by warps, a lone
+rank's dispatch straight into the tensors that are kept."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("Hp", [8, 264, 520, 2048, 2312])       # part of a warp, one block of 256 columns and a bit, ...
+@pytest.mark.parametrize("rows, valid", [(1, 1), (37, 0), (300, 261)])
+def test_swiglu_bwd_widths(rows, valid, Hp):
+    from moonep_b200.ops import elementwise as ew
+    gen = torch.Generator(device="cuda").manual_seed(Hp + rows)
+    d, g, u = [torch.randn(rows, Hp, device="cuda", generator=gen).bfloat16() for _ in range(3)]
+    w = torch.rand(rows, device="cuda", generator=gen) + 0.5
+    dg, du, ds = ew.swiglu_bwd(d, g, u, w, rows_ptr=torch.tensor([valid], dtype=torch.int32, device="cuda"))
+    assert not bool(ds[valid:].any())
+    d, g, u, w = d[:valid].double(), g[:valid].double(), u[:valid].double(), w[:valid].double()[:, None]
+    s = torch.sigmoid(g)
+    # |g| < 6: the exponential is off by at most 9 units of 2^-24, s and each product by one more; so 2^-19 of a
+    # term's size.  bf16 results add 2^-8 of themselves, the sum at most Hp additions.
+    factor = s * (1 + g * (1 - s))
+    size = (d * u * w).abs() * (1 + g.abs())
+    assert bool(((dg[:valid].double() - d * u * w * factor).abs() <= 2.0 ** -8 * (d * u * w * factor).abs() + 2.0 ** -19 * size).all())
+    want = d * g * s * w
+    assert bool(((du[:valid].double() - want).abs() <= (2.0 ** -8 + 2.0 ** -19) * want.abs()).all())
+    terms = d * g * s * u
+    assert bool(((ds[:valid].double() - terms.sum(1)).abs() <= (2.0 ** -19 + Hp * 2.0 ** -24) * terms.abs().sum(1)).all())
+
+
+@pytest.mark.parametrize("shard", [0, 1])
+@pytest.mark.parametrize("S, H, K, E, pad", [(1, 128, 1, 8, 64), (53, 1024, 4, 32, 64), (260, 7168, 8, 64, 128)])
+def test_lone_dispatch_equals_dispatch(S, H, K, E, pad, shard):
+    from moonep_b200 import Buffer
+    buf = Buffer(S, H, K, E, 1, num_sms=4, token_padding=pad, timeout_s=5.0)
+    if shard:
+        buf.enable_second_shard()
+    gen = torch.Generator(device="cuda").manual_seed(S)
+    x = torch.randn(S, H, device="cuda", generator=gen).bfloat16()
+    w = torch.rand(S, K, device="cuda", generator=gen)
+    topk = torch.stack([torch.randperm(E, device="cuda", generator=gen)[:K] for _ in range(S)]).to(torch.int32)
+    tpe = torch.bincount(topk.flatten().long(), minlength=E).to(torch.int32)
+    rows, wr, cu, plan = buf.dispatch(x, w, topk, tpe)
+    n = int(cu[-1])
+    for keep in (True, False):
+        rows2, wr2, cu2, plan2 = buf._dispatch_lone(x, w, topk, tpe, keep=keep, shard=shard)
+        for name in ("dst", "zero_fill_ranges", "cu_seqlens"):
+            assert torch.equal(getattr(plan, name), getattr(plan2, name)), name
+        for name in ("link", "src_info"):
+            assert torch.equal(getattr(plan, name)[:n], getattr(plan2, name)[:n]), name
+        real = plan.src_info[:n] >= 0 if not keep else slice(None)     # (padding rows keep what they hold)
+        assert torch.equal(rows[:n][real], rows2[:n][real])
+        assert torch.equal(wr[:n], wr2[:n])
+    buf.destroy()
