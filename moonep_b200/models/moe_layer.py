@@ -396,17 +396,16 @@ class MoELayer:
         """``w -= lr * grad`` on every parameter (the router grad is averaged over the group by
         the caller if it wants data-parallel semantics; experts are rank-private)."""
         with self.tracer.span("sgd"):
-            ew.sgd_update_(self.w_router, self.g_router[0], lr)
-            if self.fused_sgd_lr is not None:
-                assert float(lr) == self.fused_sgd_lr, "fuse_sgd() and sgd_step() disagree on the learning rate"
-                if self._sgd_keep is None:
-                    return                              # every expert was updated in backward
-                for w, g in ((self.w_gate, self.g_gate), (self.w_up, self.g_up), (self.w_down, self.g_down)):
-                    ew.sgd_update_(w, g, lr, only=self._sgd_keep)
+            router = (self.w_router, self.g_router[0])
+            experts = ((self.w_gate, self.g_gate), (self.w_up, self.g_up), (self.w_down, self.g_down))
+            if self.fused_sgd_lr is None:
+                ew.sgd_update_all_((router, *experts), lr)
                 return
-            ew.sgd_update_(self.w_gate, self.g_gate, lr)
-            ew.sgd_update_(self.w_up, self.g_up, lr)
-            ew.sgd_update_(self.w_down, self.g_down, lr)
+            ew.sgd_update_(*router, lr)
+            assert float(lr) == self.fused_sgd_lr, "fuse_sgd() and sgd_step() disagree on the learning rate"
+            if self._sgd_keep is not None:              # else every expert was updated in backward
+                for w, g in experts:
+                    ew.sgd_update_(w, g, lr, only=self._sgd_keep)
 
     def state_dict(self):
         """Home-layout weights only; prefetch slots are transient and never saved."""

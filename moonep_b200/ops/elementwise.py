@@ -14,7 +14,7 @@ nat.declare("mep_router_topk_bwd", I, [P, P, P, I, I, I, P, P])
 nat.declare("mep_swiglu_bwd", I, [P, P, P, P, P, I, I, P, P, P, P])
 nat.declare("mep_ce_fwd", I, [P, P, L, I, I, P, P, P, P, P])
 nat.declare("mep_ce_bwd", I, [P, P, L, I, I, P, P, P, P, P])
-nat.declare("mep_sgd_update", I, [P, P, L, F, P])
+nat.declare("mep_sgd_update", I, [P, P, P, I, F, P])
 nat.declare("mep_sgd_update_masked", I, [P, P, L, L, P, F, P])
 
 
@@ -67,14 +67,28 @@ def swiglu_bwd(dact, gate, up, row_scale=None, rows_ptr=None, want_dscale=True):
     return dgate, dup, dscale
 
 
+def _sgd_pair(w, g):
+    assert w.dtype == torch.bfloat16 and g.dtype == torch.float32 and w.numel() == g.numel()
+    assert w.is_contiguous() and g.is_contiguous()
+
+
+def sgd_update_all_(pairs, lr: float) -> None:
+    """:func:`sgd_update_` of up to eight ``(w, g)`` pairs in one launch."""
+    n = len(pairs)
+    w, g, size = (P * n)(), (P * n)(), (L * n)()
+    for i, (wi, gi) in enumerate(pairs):
+        _sgd_pair(wi, gi)
+        w[i], g[i], size[i] = wi.data_ptr(), gi.data_ptr(), wi.numel()
+    _rc(nat.call("mep_sgd_update", w, g, size, n, float(lr), _st()), "sgd_update")
+
+
 def sgd_update_(w: torch.Tensor, g: torch.Tensor, lr: float, only: torch.Tensor = None) -> None:
     """In place ``w(bf16) = bf16(w - lr * g(fp32))``.  ``only`` (int32 ``[experts]``, with ``w`` and
     ``g`` shaped ``[experts, ...]``) restricts the update to the experts whose flag is non-zero."""
-    assert w.dtype == torch.bfloat16 and g.dtype == torch.float32 and w.numel() == g.numel()
-    assert w.is_contiguous() and g.is_contiguous()
     if only is None:
-        _rc(nat.call("mep_sgd_update", w.data_ptr(), g.data_ptr(), w.numel(), float(lr), _st()), "sgd_update")
+        sgd_update_all_(((w, g),), lr)
         return
+    _sgd_pair(w, g)
     assert only.dtype == torch.int32 and only.is_cuda and only.numel() >= w.shape[0]
     _rc(nat.call("mep_sgd_update_masked", w.data_ptr(), g.data_ptr(), w.shape[0], w[0].numel(),
                  only.data_ptr(), float(lr), _st()), "sgd_update")

@@ -1,5 +1,5 @@
-"""Kernels around the layer's products at the edges of their ranges: SwiGLU backward by warps, a lone
-rank's dispatch straight into the tensors that are kept."""
+"""Kernels around the layer's products at the edges of their ranges: SwiGLU backward by warps, the update of several
+tensors in one launch, a lone rank's dispatch straight into the tensors that are kept."""
 import pytest
 import torch
 
@@ -26,6 +26,25 @@ def test_swiglu_bwd_widths(rows, valid, Hp):
     assert bool(((du[:valid].double() - want).abs() <= (2.0 ** -8 + 2.0 ** -19) * want.abs()).all())
     terms = d * g * s * u
     assert bool(((ds[:valid].double() - terms.sum(1)).abs() <= (2.0 ** -19 + Hp * 2.0 ** -24) * terms.abs().sum(1)).all())
+
+
+@pytest.mark.parametrize("sizes", [(5,), (8, 3, 4096), (1 << 20, 17, 8, 7, 300000, 1, 16, 2056)])
+def test_update_of_several_tensors(sizes):
+    from moonep_b200.ops import elementwise as ew
+    gen = torch.Generator(device="cuda").manual_seed(len(sizes))
+    w = [torch.randn(n, device="cuda", generator=gen).bfloat16() for n in sizes]
+    g = [torch.randn(n, device="cuda", generator=gen) for n in sizes]
+    # 0.25 g is exact, so the sum is rounded to fp32 once and then to bf16, as here
+    want = [(a.float() - 0.25 * b).bfloat16() for a, b in zip(w, g)]
+    ew.sgd_update_all_(list(zip(w, g)), 0.25)
+    assert all(torch.equal(a, b) for a, b in zip(w, want))
+
+
+def test_update_refuses_more_than_a_launch_takes():
+    from moonep_b200.ops import elementwise as ew
+    t = [(torch.zeros(8, device="cuda", dtype=torch.bfloat16), torch.zeros(8, device="cuda")) for _ in range(9)]
+    with pytest.raises(RuntimeError):
+        ew.sgd_update_all_(t, 1.0)
 
 
 @pytest.mark.parametrize("shard", [0, 1])
