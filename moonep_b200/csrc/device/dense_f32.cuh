@@ -2,11 +2,12 @@
 // CTAs hold at once go to the token-major kernel.)
 //
 // The output is small (S x experts) and the reduction long: a CTA walks up to 112 k-blocks one after
-// the other, ~0.2 us each, bound by that chain and not by bytes.  The experts take the M side (128 a
-// tile) and the tokens the N side, in as small a tile as fills the SMs once (4096 tokens are 128 CTAs
-// of 32), with up to sixteen stages in flight.  Loads and MMAs are issued by one lane of a converged warp,
-// which halved the chain: K = 7168 50 -> 25 us for 16 tokens and 52 -> 27 for 4096, 4096 x 2048 -> 128
-// experts 18.8 -> 15.2.  The reduction is NOT split: routing compares these sums, and another order of the
+// the other, bound by that chain and not by bytes or MMAs (25 us for 8 as for 128 experts; 21 with no MMA but the
+// first).  The experts take the M side (128 a tile) and the tokens the N side, in as small a tile as fills the SMs
+// once (4096 tokens are 128 CTAs of 32).  Loads and MMAs are issued by one lane of a converged warp, which halved the
+// chain (K = 7168 50 -> 25 us for 16 tokens), and one wait and one commit serve two or four k-blocks, which are
+// what remains of it: inputs out of L2, 16 x 7168 -> 32 experts 28.5 -> 19.4 us, 1531 29.5 -> 21.4, 4096 31.6 -> 27.6, 4096 ->
+// 128 experts 30.7 -> 28.7.  The reduction is NOT split: routing compares these sums, and another order of the
 // additions sends tokens at a tie elsewhere.
 #pragma once
 
@@ -16,16 +17,17 @@ constexpr int DN_MAX_STAGES = 16;
 constexpr int DN_THREADS = 192;
 constexpr int DN_RING = 200 * 1024;
 constexpr int DN_MAX_TOK = 128;
+constexpr int DN_MAX_BLOCKS = 4;       // k-blocks of a stage, at most
 
 struct DenseParams {
   CUtensorMap x, w;      // tokens: tok x 64 boxes; weights: 64 x 64 (B [K][N]) or m_rows x 64 boxes (B [N][K])
   float* out;
   long long ldc;
-  int S, N, num_kb, tok, m_rows, stages;
+  int S, N, num_kb, tok, m_rows, stages, blocks;
   int32_t* status;
   unsigned long long timeout_ns;
 };
-__host__ __device__ constexpr int dense_stage_bytes(int m_rows, int tok) { return (m_rows + tok) * BK * 2; }
+__host__ __device__ constexpr int dense_block_bytes(int m_rows, int tok) { return (m_rows + tok) * BK * 2; }
 
 template <bool W_MN>
 __global__ void __launch_bounds__(DN_THREADS, 1) ep_dense_f32_kernel(const __grid_constant__ DenseParams p) {
@@ -40,7 +42,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) ep_dense_f32_kernel(const __gri
   volatile int* abortp = &s_abort;
   const int row0 = (int)blockIdx.x * p.tok, m0 = (int)blockIdx.y * BM;
   // (with at most 64 experts only half of the M side is loaded; what the other lanes compute is not stored)
-  const int w_bytes = p.m_rows * BK * 2, stage_bytes = dense_stage_bytes(p.m_rows, p.tok);
+  const int w_bytes = p.m_rows * BK * 2, block_bytes = dense_block_bytes(p.m_rows, p.tok), stage_bytes = p.blocks * block_bytes;
 
   if (tid == 0) {
     for (int s = 0; s < p.stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -65,18 +67,21 @@ __global__ void __launch_bounds__(DN_THREADS, 1) ep_dense_f32_kernel(const __gri
       tma_prefetch_desc(&p.w);
     }
     RingSlot st;
-    for (int kb = 0; kb < p.num_kb; ++kb, st.next(p.stages)) {
-      const int s = st.slot;
+    for (int kb0 = 0; kb0 < p.num_kb; kb0 += p.blocks, st.next(p.stages)) {
+      const int s = st.slot, blocks = min(p.blocks, p.num_kb - kb0);
       if (!warp_wait(&empty[s], st.parity ^ 1u, 1)) break;
       if (!issue) continue;
-      uint8_t* sw = ring + s * stage_bytes;
-      mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
-      if constexpr (W_MN) {
-        for (int j = 0; j < p.m_rows / 64; ++j) tma_load_2d(sw + j * 8192, &p.w, m0 + 64 * j, kb * BK, &full[s]);
-      } else {
-        tma_load_2d(sw, &p.w, kb * BK, m0, &full[s]);
+      mbar_expect_tx(&full[s], (uint32_t)(blocks * block_bytes));
+      for (int b = 0; b < blocks; ++b) {
+        uint8_t* sw = ring + s * stage_bytes + b * block_bytes;
+        const int k = (kb0 + b) * BK;
+        if constexpr (W_MN) {
+          for (int j = 0; j < p.m_rows / 64; ++j) tma_load_2d(sw + j * 8192, &p.w, m0 + 64 * j, k, &full[s]);
+        } else {
+          tma_load_2d(sw, &p.w, k, m0, &full[s]);
+        }
+        tma_load_2d(sw + w_bytes, &p.x, k, row0, &full[s]);
       }
-      tma_load_2d(sw + w_bytes, &p.x, kb * BK, row0, &full[s]);
     }
   } else if (warp == 1) {
     const bool issue = elect_one();
@@ -87,15 +92,20 @@ __global__ void __launch_bounds__(DN_THREADS, 1) ep_dense_f32_kernel(const __gri
     constexpr int W_STEP = (W_MN ? 2048 : 32) >> 4, X_STEP = 32 >> 4;
     RingSlot st;
     bool ok = true;
-    for (int kb = 0; kb < p.num_kb; ++kb, st.next(p.stages)) {
+    for (int kb0 = 0; kb0 < p.num_kb; kb0 += p.blocks, st.next(p.stages)) {
       ok = warp_wait(&full[st.slot], st.parity, 3);
       if (!ok) break;
       tc_fence_after();
       if (issue) {
-        const uint64_t dw = desc_w + (uint32_t)(st.slot * (stage_bytes >> 4)), dx = desc_x + (uint32_t)(st.slot * (stage_bytes >> 4));
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk)
-          umma_bf16(tmem_base, dw + kk * W_STEP, dx + kk * X_STEP, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+        for (int b = 0; b < DN_MAX_BLOCKS; ++b) {
+          if (b >= p.blocks || kb0 + b >= p.num_kb) break;
+          const uint32_t at = (uint32_t)((st.slot * stage_bytes + b * block_bytes) >> 4);
+          const uint64_t dw = desc_w + at, dx = desc_x + at;
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk)
+            umma_bf16(tmem_base, dw + kk * W_STEP, dx + kk * X_STEP, idesc, (kb0 + b > 0 || kk > 0) ? 1u : 0u);
+        }
         umma_commit(&empty[st.slot]);
       }
     }

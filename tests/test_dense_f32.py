@@ -41,3 +41,19 @@ def test_large_products(S, K, N):
     for r in (0, S // 2, S - 100):       # a few of its rows alone fit the other kernel
         assert torch.equal(gemm.dense(a[r:r + 100].contiguous(), b), got[r:r + 100])
     gemm.check_status()
+
+
+# stages of four and of two k-blocks, the last one partly filled, reductions shorter and longer than the ring
+@pytest.mark.parametrize("N", [32, 128])
+@pytest.mark.parametrize("S", [5, 1000])
+@pytest.mark.parametrize("K", [8, 320, 1480, 5800])
+def test_last_stage(S, K, N):
+    from moonep_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(S + K + N)
+    a = torch.randn(S, K, device="cuda", generator=g).bfloat16()
+    b = torch.randn(K, N, device="cuda", generator=g).bfloat16()
+    # exact products, K additions that are each off by at most one unit of a running sum below sum |a b|
+    bound = 2.0 ** -23 * K * (a.double().abs() @ b.double().abs())
+    for got in (gemm.dense(a, b), gemm.dense(a, b.t().contiguous(), b_is_kn=False)):
+        assert bool(((got.double() - a.double() @ b.double()).abs() <= bound).all())
+    gemm.check_status()
