@@ -231,12 +231,15 @@ class Buffer:
         return hb[:, : self.NvS] if self.virtual else hb[self.rank: self.rank + 1, : self.NvS]
 
     def _own_view(self, name, make) -> torch.Tensor:
-        """A view of this Buffer's memory, made once.  For looking at only: what a caller gets is an alias of its own
-        (``detach``), so that nothing it does to the tensor object stays behind here."""
+        """A view of this Buffer's memory, made once.  What a caller gets is an alias of its own (``detach``), so that
+        nothing it does to the tensor object stays behind here.  Autograd knows nothing of the view or its base,
+        whatever mode it is made in: write into it from detached tensors only."""
         v = self._own_views.get(name)
         if v is None:
-            v = make()
-            self._own_views[name] = v = v if self.virtual else v[0]
+            with torch.inference_mode(False), torch.no_grad():
+                v = make()
+                v = (v if self.virtual else v[0]).detach()
+            self._own_views[name] = v
         return v
 
     def _hidden_own(self, shard: int = 0) -> torch.Tensor:
@@ -586,9 +589,9 @@ class Buffer:
         if inter_rank_sync and not self._one_device:
             self._rc(nat.call("mep_launch_sync", self._ctx, st), "inter_rank_sync")
         if not zero_copy:
-            self._hidden_own().copy_(hidden_nvsh)
+            self._hidden_own().copy_(hidden_nvsh.detach())
         if w_nvs is not None and not w_zero_copy:
-            self._weights_own().copy_(w_nvs)
+            self._weights_own().copy_(w_nvs.detach())
         if not self._one_device:
             self._rc(nat.call("mep_launch_combine_prologue", self._ctx, plan.link.data_ptr(),
                               plan.cu_seqlens.data_ptr(), st), "combine prologue")
