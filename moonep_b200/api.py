@@ -62,6 +62,7 @@ nat.declare("mep_launch_grad_reduce", I, [P, P, I, P, P, P, P, I, I, I, I, P])
 nat.declare("mep_launch_sync", I, [P, P])
 nat.declare("mep_dispatch_smem_bytes", L, [P])
 nat.declare("mep_plan_launch_smem_bytes", L, [P])
+nat.declare("mep_plan_launch_ctas", I, [P])
 nat.declare("mep_push_reduce_footprint", I, [P, P])
 nat.declare("mep_grad_reduce_footprint", I, [I, I, P, P])
 

@@ -243,11 +243,15 @@ int64_t mep_plan_smem_bytes(int R, int E) {
 }
 
 // CTAs a rank.  Within one device no more than have 256 entries each: the grid's barrier and the sums over the
-// CTAs before one's own cost more than the entries of the smallest calls.
+// CTAs before one's own cost more than the entries of the smallest calls.  All CTAs of a virtual group's ranks
+// are resident at once, and an SM holds one (512 threads of more than 64 registers): a group whose
+// num_sms * R is above the number of SMs, which the copy kernels fit twice, takes fewer here.
 static int plan_ctas(const BufferCtx& c) {
   if (!c.one_device()) return c.num_sms;
   const int64_t useful = (c.N + 255) / 256;
-  return useful < c.num_sms ? (int)useful : c.num_sms;
+  const int sms = c.sm_count > 0 ? c.sm_count : 148, fit = sms > c.Rv() ? sms / c.Rv() : 1;
+  const int most = c.num_sms < fit ? c.num_sms : fit;
+  return useful < most ? (int)useful : most;
 }
 
 // Ranking warps of a planner launch: one per 64 entries of a CTA within one device (4096 tokens on 256 experts
@@ -272,6 +276,9 @@ static int64_t plan_tables(const BufferCtx& c) {
   const int64_t at = mep_plan_smem_bytes(c.R, c.E);
   return c.one_device() && at + (int64_t)sizeof(int32_t) * solve_table_ints(c.R, c.E) <= 160 * 1024 ? at : 0;
 }
+
+// CTAs a rank of a planner launch of this Buffer.
+int mep_plan_launch_ctas(const void* ctx_) { return plan_ctas(*(const BufferCtx*)ctx_); }
 
 // Dynamic shared memory of a planner launch of this Buffer.
 int64_t mep_plan_launch_smem_bytes(const void* ctx_) {

@@ -48,3 +48,31 @@ def test_planner_beside_prefetch_weight(ctx, R, E, S, num_sms):
 def test_few_communication_sms_on_one_device(ctx, R, num_sms, local, want):
     """Dispatch and combine that move all rows themselves run on no fewer SMs than the local kernels they replace."""
     assert nat.call("mep_ctx_direct_ctas", ctx(R, 64, 512, 8, 1024, num_sms, int(R > 1), local)) == want
+
+
+# ranks of a virtual group, CTAs a rank for its copy kernels -> CTAs a rank of the planner
+@pytest.mark.parametrize("R,num_sms,S,want", [(8, 18, 4096, 18), (32, 8, 512, 4), (128, 2, 512, 1), (2, 148, 8192, 74),
+                                              (32, 8, 16, 1), (1, 96, 4096, 96)])
+def test_planner_of_a_virtual_group_fits_one_cta_an_sm(ctx, R, num_sms, S, want):
+    c = ctx(R, 6 * R, S, 8, 1024, num_sms, int(R > 1))
+    assert nat.call("mep_plan_launch_ctas", c) == want
+    assert want * R <= 148 and nat.call("mep_plan_launch_smem_bytes", c) <= 227 * 1024 - 1024
+
+
+@pytest.mark.gpu
+def test_virtual_group_of_more_ctas_than_sms():
+    """32 ranks x 8 CTAs: the copy kernels' CTAs share SMs, the planner's cannot."""
+    import torch
+    from moonep_b200 import Buffer, reference as ref
+    from moonep_b200.utils.routing import routing_for_maxvio, tokens_per_expert
+    R, S, H, K, E, tp = 32, 40, 256, 4, 96, 16
+    buf = Buffer(S, H, K, E, R, num_sms=8, token_padding=tp, virtual=True, timeout_s=5.0)
+    topk, w, _, _ = routing_for_maxvio(S, K, E, R, 1.0, seed=4)
+    tpe = torch.stack([tokens_per_expert(topk[r], E) for r in range(R)])
+    x = torch.randn(R, S, H, generator=torch.Generator().manual_seed(2)).bfloat16()
+    rows, wn, _, plan = buf.dispatch(x.cuda(), w.cuda(), topk.cuda(), tpe.cuda())
+    y, wb, _ = buf.combine(plan, rows, wn)
+    buf.check()
+    assert torch.equal(plan.dst.cpu(), ref.plan_all_ranks(topk, S, K, E, tp, tpe)[1])
+    assert torch.equal(y.cpu(), (x.float() * K).bfloat16()) and torch.equal(wb.cpu(), w)
+    buf.destroy()
