@@ -790,7 +790,8 @@ class Buffer:
 
     def phase_stamps(self) -> dict:
         """``{kernel: {phase: (min_us, max_us)}}`` of the LAST launch of each stamped kernel, in
-        microseconds after the kernel's earliest stamp, over the CTAs that ran (synchronises)."""
+        microseconds after the kernel's earliest stamp, over the CTAs that ran (synchronises).  A
+        phase that a launch has no barrier for (one device) is passed at once."""
         if getattr(self, "_trace", None) is None:
             return {}
         torch.cuda.synchronize(self.device)

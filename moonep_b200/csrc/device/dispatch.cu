@@ -48,6 +48,11 @@ struct DispatchParams {
   // 7168, top-8: one launch of 0.59 ms and an expansion of 0.95 ms (which reads every primary row
   // back from HBM) became one launch of 0.80 ms, bound by its stores (5.5 TB/s).
   int direct;
+  // Whether the launch ends in a barrier of all CTAs.  With everything on one device the end of the launch orders
+  // the rows; the barrier is then only needed ahead of snapshots, which read what other CTAs wrote.
+  __host__ __device__ bool exit_barrier() const {
+    return !direct || (!records_written && (link_out != nullptr || src_out != nullptr));
+  }
 };
 
 constexpr int DISPATCH_THREADS = 128;
@@ -188,12 +193,12 @@ __global__ void __launch_bounds__(DISPATCH_THREADS, 1) ep_dispatch_kernel(const 
     if (warp == 2 && lane == 0) { bulk_commit(); bulk_wait<0>(); fence_proxy_async(); }
   }
   if (tid == 0) phase_stamp(sc.trace, 0, c, 2);          // this CTA's rows, weights and padding issued
-  // With everything on one device the end of the launch orders the rows; the barrier is then only
-  // needed ahead of the snapshots below, which read what other CTAs wrote.
-  if (p.direct && (p.records_written || (p.link_out == nullptr && p.src_out == nullptr))) return;
-  fence_sys();
-  cross_rank_barrier(sc, 2);
-  if (tid == 0) phase_stamp(sc.trace, 0, c, 3);          // past the exit barrier
+  if (p.exit_barrier()) {
+    fence_sys();
+    cross_rank_barrier(sc, 2);
+  }
+  if (tid == 0) phase_stamp(sc.trace, 0, c, 3);          // past the exit barrier, or there is none
+  if (p.records_written) return;
 
   if (p.link_out != nullptr) {
     const int32_t* src = sc.meta + (size_t)rank * sc.meta_stride + p.link_off;
@@ -350,10 +355,8 @@ static int launch_dispatch_t(const BufferCtx& c, DispatchParams& p, size_t smem,
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_dispatch_kernel<ST>, raised));
   dim3 grid(p.direct ? c.direct_ctas() : c.num_sms, c.Rv());
-  // (no barrier inside where everything is on one device and there is nothing to copy at the end)
-  const bool barrier = !p.direct || (p.link_out != nullptr && !p.records_written);
   MEP_CUDA_OK(launch_chained((const void*)ep_dispatch_kernel<ST>, grid, dim3(DISPATCH_THREADS), smem,
-                             stream, p, /*coop=*/barrier, c.pdl && p.fresh));
+                             stream, p, /*coop=*/p.exit_barrier(), c.pdl && p.fresh));
   return 0;
 }
 
