@@ -134,7 +134,7 @@ class OursArm:
         r["k_plan_us"] = timed(lambda: (nat.call(
             "mep_launch_plan", buf._ctx, self.topk.data_ptr(), self.tpe.data_ptr(), plan.dst.data_ptr(),
             plan.cu_seqlens.data_ptr(), plan.zero_fill_ranges.data_ptr(), plan.experts_to_copy.data_ptr(),
-            plan.remote_stats.data_ptr(), plan.send_order.data_ptr(), 0, 0, st()),
+            plan.remote_stats.data_ptr(), plan.send_order.data_ptr(), 0, 0, int(buf._one_device), st()),
             nat.call("mep_launch_sync", buf._ctx, st())))
         r["k_dispatch_us"] = timed(lambda: nat.call(
             "mep_launch_dispatch", buf._ctx, x.data_ptr(), 0, plan.dst.data_ptr(),

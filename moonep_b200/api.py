@@ -49,7 +49,7 @@ nat.declare("mep_trace_ints64", L, [])
 nat.declare("mep_trace_dims", None, [ctypes.POINTER(ctypes.c_int)])
 nat.declare("mep_ctx_set_trace", None, [P, P])
 nat.declare("mep_ctx_direct_ctas", I, [P])
-nat.declare("mep_launch_plan", I, [P, P, P, P, P, P, P, P, P, P, P, P])
+nat.declare("mep_launch_plan", I, [P, P, P, P, P, P, P, P, P, P, P, I, P])
 nat.declare("mep_launch_arrive_reset", I, [P, P])
 nat.declare("mep_launch_plan_snapshot", I, [P, P, P, P])
 nat.declare("mep_launch_dispatch", I, [P, P, P, P, P, P, P, I, I, I, I, I, P, P, I, P])
@@ -476,7 +476,7 @@ class Buffer:
         self._rc(nat.call("mep_launch_plan", self._ctx, topk.data_ptr(), tpe.data_ptr(),
                           dst.data_ptr(), cu.data_ptr(), zf.data_ptr(), etc.data_ptr(),
                           rs.data_ptr(), order.data_ptr(), link.data_ptr() if records else 0,
-                          src.data_ptr() if records else 0, st), "plan")
+                          src.data_ptr() if records else 0, int(self._one_device), st), "plan")
         plan = CommPlan(dst=dst, experts_to_copy=etc, zero_fill_ranges=zf, remote_stats=rs,
                         cu_seqlens=cu, link=link, N=self.N, R=self.R, E=self.E, NvS=self.NvS,
                         K=self.K, src_info=src, send_order=order)

@@ -246,9 +246,8 @@ int64_t mep_plan_smem_bytes(int R, int E) {
 // CTAs before one's own cost more than the entries of the smallest calls.  All CTAs of a virtual group's ranks
 // are resident at once, and an SM holds one (512 threads of more than 64 registers): a group whose
 // num_sms * R is above the number of SMs, which the copy kernels fit twice, takes fewer here.
-static int plan_ctas(const BufferCtx& c) {
-  if (!c.one_device()) return c.num_sms;
-  const int64_t useful = (c.N + 255) / 256;
+static int plan_ctas(const BufferCtx& c, bool one_device) {
+  const int64_t useful = one_device ? (c.N + 255) / 256 : c.num_sms;
   const int sms = c.sm_count > 0 ? c.sm_count : 148, fit = sms > c.Rv() ? sms / c.Rv() : 1;
   const int most = c.num_sms < fit ? c.num_sms : fit;
   return useful < most ? (int)useful : most;
@@ -259,11 +258,11 @@ static int plan_ctas(const BufferCtx& c) {
 // entries: with sixteen for 8 entries 27 -> 31 us), as many as have room for counters.  Over several devices
 // that is 8 KB: the planner and the weight ops wait for other ranks while they hold their SMs, on two
 // streams, and beside prefetch_weight's ring (192 KB and its lists) 64 KB do not fit.
-static int plan_rank_warps(const BufferCtx& c) {
-  const int ctas = plan_ctas(c);
+static int plan_rank_warps(const BufferCtx& c, bool one_device) {
+  const int ctas = plan_ctas(c, one_device);
   const int64_t entries = (int64_t)((c.S + ctas - 1) / ctas) * c.K;
-  int64_t w = (c.one_device() ? 64 * 1024 : 8 * 1024) / (int64_t)(sizeof(int32_t) * c.E);
-  const int64_t least = c.one_device() ? 64 : 128;
+  int64_t w = (one_device ? 64 * 1024 : 8 * 1024) / (int64_t)(sizeof(int32_t) * c.E);
+  const int64_t least = one_device ? 64 : 128;
   if (w > entries / least) w = entries / least;
   return w < 1 ? 1 : (w > PLAN_WARPS ? PLAN_WARPS : (int)w);
 }
@@ -272,24 +271,29 @@ static int plan_rank_warps(const BufferCtx& c) {
 // are used later.  0 (none) over several devices, where the planner shares SMs (see above), and when they are
 // too large.  Tables in shared memory, no exchange within one device, the layout split over all warps: 16 tokens on
 // 32 experts 17 -> 15 us, 4096 on 256 28 -> 22, 8 ranks x 17 tokens on 128 experts 29 -> 19, 8 x 4096 on 256 42 -> 35.
-static int64_t plan_tables(const BufferCtx& c) {
+static int64_t plan_tables(const BufferCtx& c, bool one_device) {
   const int64_t at = mep_plan_smem_bytes(c.R, c.E);
-  return c.one_device() && at + (int64_t)sizeof(int32_t) * solve_table_ints(c.R, c.E) <= 160 * 1024 ? at : 0;
+  return one_device && at + (int64_t)sizeof(int32_t) * solve_table_ints(c.R, c.E) <= 160 * 1024 ? at : 0;
 }
 
-// CTAs a rank of a planner launch of this Buffer.
-int mep_plan_launch_ctas(const void* ctx_) { return plan_ctas(*(const BufferCtx*)ctx_); }
-
-// Dynamic shared memory of a planner launch of this Buffer.
-int64_t mep_plan_launch_smem_bytes(const void* ctx_) {
-  const BufferCtx& c = *(const BufferCtx*)ctx_;
-  const int w = plan_rank_warps(c);            // (a lone warp counts in place)
+static int64_t plan_smem(const BufferCtx& c, bool one_device) {
+  const int w = plan_rank_warps(c, one_device);            // (a lone warp counts in place)
   int64_t more = w > 1 ? (int64_t)w * c.E : 0;
-  if (plan_tables(c) != 0) {
+  if (plan_tables(c, one_device) != 0) {
     more += 2 * (int64_t)c.R * c.E;            // the tables that are looked up, behind the counters
     if (more < solve_table_ints(c.R, c.E)) more = solve_table_ints(c.R, c.E);
   }
   return mep_plan_smem_bytes(c.R, c.E) + (int64_t)sizeof(int32_t) * more;
+}
+
+// CTAs a rank, and dynamic shared memory, of a planner launch of this Buffer.
+int mep_plan_launch_ctas(const void* ctx_) {
+  const BufferCtx& c = *(const BufferCtx*)ctx_;
+  return plan_ctas(c, c.one_device());
+}
+int64_t mep_plan_launch_smem_bytes(const void* ctx_) {
+  const BufferCtx& c = *(const BufferCtx*)ctx_;
+  return plan_smem(c, c.one_device());
 }
 
 // Fresh plan for this rank (or for all virtual ranks).  send_order [Rv][N] may be null (it is
@@ -297,12 +301,15 @@ int64_t mep_plan_launch_smem_bytes(const void* ctx_) {
 // meta chunks; they become visible with the next cross-rank barrier (the dispatch kernel's
 // exit barrier, or an explicit mep_launch_sync).  Within one device link_out and src_out [Rv][NvS] may take the
 // records of all real rows instead (the dispatch that follows sets those of padding rows): that saves
-// dispatch its exit barrier and the copies behind it, 6 - 9 us.
+// dispatch its exit barrier and the copies behind it, 6 - 9 us.  one_device != 0 only where every rank's counts are
+// memory of this device; without it the ranks exchange their counts, a virtual group's too.
 int mep_launch_plan(const void* ctx_, const int32_t* topk, const int32_t* tpe, int32_t* dst,
                     int32_t* cu_seqlens, int32_t* zero_fill, int32_t* etc, int32_t* remote_stats,
-                    int32_t* send_order, int32_t* link_out, int32_t* src_out, cudaStream_t stream) {
+                    int32_t* send_order, int32_t* link_out, int32_t* src_out, int one_device, cudaStream_t stream) {
   const BufferCtx& c = *(const BufferCtx*)ctx_;
-  if ((link_out != nullptr || src_out != nullptr) && !c.one_device())
+  const bool one = one_device != 0;
+  if (one && !c.one_device()) return fail(-2, "plan: the ranks are on several devices");
+  if ((link_out != nullptr || src_out != nullptr) && !one)
     return fail(-1, "plan: records go straight into the plan only within one device");
   PlanParams p;
   p.sync = c.sync(KID_PLAN);
@@ -313,15 +320,15 @@ int mep_launch_plan(const void* ctx_, const int32_t* topk, const int32_t* tpe, i
   p.etc = etc; p.remote_stats = remote_stats;
   p.scratch = c.plan_scratch; p.scratch_ints = c.plan_scratch_ints;
   p.send_order = send_order; p.arrive_off = c.ml.arrive_off; p.n_arrive = (int)(c.NvS / 128 + 1);
-  const size_t smem = (size_t)mep_plan_launch_smem_bytes(ctx_);
-  p.rank_warps = plan_rank_warps(c);
-  p.one_device = c.one_device();
+  const size_t smem = (size_t)plan_smem(c, one);
+  p.rank_warps = plan_rank_warps(c, one);
+  p.one_device = one;
   p.link_out = link_out; p.src_out = src_out;
-  p.tables = (int)(plan_tables(c) / sizeof(int32_t));
+  p.tables = (int)(plan_tables(c, one) / sizeof(int32_t));
   p.rank_counts = p.rank_warps > 1 ? (int)(mep_plan_smem_bytes(c.R, c.E) / sizeof(int32_t)) : 0;
   static std::atomic<unsigned long long> raised{0};
   MEP_CUDA_OK(raise_smem_limit((const void*)ep_plan_kernel, raised));
-  dim3 grid(plan_ctas(c), c.Rv());
+  dim3 grid(plan_ctas(c, one), c.Rv());
   MEP_CUDA_OK(launch_coop((const void*)ep_plan_kernel, grid, dim3(PLAN_THREADS), smem, stream, p));
   return 0;
 }
