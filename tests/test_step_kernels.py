@@ -61,13 +61,39 @@ def test_lone_dispatch_equals_dispatch(S, H, K, E, pad, shard):
     tpe = torch.bincount(topk.flatten().long(), minlength=E).to(torch.int32)
     rows, wr, cu, plan = buf.dispatch(x, w, topk, tpe)
     n = int(cu[-1])
+    real = plan.src_info[:n] >= 0
+    assert int(real.sum()) == S * K
     for keep in (True, False):
+        # what is not written shows
+        buf.hidden_view(shard).fill_(float("nan"))
+        buf.router_weight_buffer_view.fill_(float("nan"))
         rows2, wr2, cu2, plan2 = buf._dispatch_lone(x, w, topk, tpe, keep=keep, shard=shard)
         for name in ("dst", "zero_fill_ranges", "cu_seqlens"):
             assert torch.equal(getattr(plan, name), getattr(plan2, name)), name
         for name in ("link", "src_info"):
             assert torch.equal(getattr(plan, name)[:n], getattr(plan2, name)[:n]), name
-        real = plan.src_info[:n] >= 0 if not keep else slice(None)     # (padding rows keep what they hold)
         assert torch.equal(rows[:n][real], rows2[:n][real])
         assert torch.equal(wr[:n], wr2[:n])
+        padding = rows2[:n][~real]
+        assert bool(torch.isnan(padding).all() if not keep else (padding == 0).all())
+    buf.destroy()
+
+
+@pytest.mark.parametrize("fused_combine", [True, False])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_inference_reads_no_padding_row(fused_combine, in_place):
+    """A pass without a backward pass leaves padding rows as they are: whatever they hold stays out of the result."""
+    from moonep_b200 import Buffer
+    from moonep_b200.models.moe_layer import MoELayer
+    buf = Buffer(77, 256, 4, 16, 1, num_sms=8, token_padding=128, timeout_s=5.0)
+    layer = MoELayer(buf, 192, seed=1, train=False, fused_combine=fused_combine, hidden_in_place=in_place)
+    x = torch.randn(77, 256, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)).bfloat16()
+    got = []
+    for fill in (0.0, float("nan"), float("inf")):
+        for shard in range(1 + in_place):
+            buf.hidden_view(shard).fill_(fill)
+        with torch.no_grad():
+            got.append(layer(x))
+    assert bool(torch.isfinite(got[0]).all()) and bool(got[0].any())
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
     buf.destroy()
