@@ -49,13 +49,13 @@ struct GemmKParams {
   CUtensorMap a;           // weight grad: token rows of A in 64 x 64 boxes (and of B, in b)
   CUtensorMap tok[2][TG_BOXES];   // token rows in boxes of 32, 64, 96 and 128 rows (token_gemm.cuh)
   CUtensorMap b[2][2];
-  CUtensorMap b2[2][2];    // K-major B with a 128-row box
+  CUtensorMap b2[2][2];    // K-major B with a 128-row box; weight grad: grads that are added to, 32 x 32 boxes
   const int32_t* cu_seqlens;
   const int32_t* pads;     // [ngroups][2] first padding row and their number, per group; or null
   int ngroups, split, total_rows, N, K, nseg, rows_per_expert, Mw, accumulate, zero_empty_below;
   // weight grad: tiles of a unit; slots of the shared memory for k-blocks of rows and of columns, and for
-  // weight pieces of an epilogue warp (SGD)
-  int unit, row_slots, col_slots, pieces;
+  // weight pieces of an epilogue warp (SGD); warps of a row quarter that add to grads (accumulate: 1, 2, 4)
+  int unit, row_slots, col_slots, pieces, adders;
   int vec32;   // weight grad: rows of the weights allow 32-byte accesses
   int products; // weight grad: 2 = a second one with the same A (b[1], out + 2, sgd_w[1])
   // SGD kernels: 1 = only the tiles whose grads are STORED (experts with replicas, slot groups),
@@ -202,20 +202,23 @@ typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void
                              CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                              CUtensorMapFloatOOBfill);
 
-// 2-D bf16 tensor [rows][cols] (row stride ld elements), box [box_rows][box_cols], 128B swizzle.
+// 2-D tensor [rows][cols] of bf16, or with F32 of fp32 (row stride ld elements), box [box_rows][box_cols], 128B swizzle.
+template <bool F32 = false>
 static int make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int64_t ld,
-                    int box_cols, int box_rows, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
+                    int box_cols, int box_rows) {
   EncodeFn enc = (EncodeFn)driver_tensor_map_encode();
   if (!enc) return fail(-10, "CUDA driver entry cuTensorMapEncodeTiled not available");
-  if (((uintptr_t)base & 15) != 0 || (ld * 2) % 16 != 0)
+  const int bytes = F32 ? 4 : 2;
+  if (((uintptr_t)base & 15) != 0 || (ld * bytes) % 16 != 0)
     return fail(-11, "GEMM operand must be 16-byte aligned with a 16-byte multiple row stride");
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  cuuint64_t strides[1] = {(cuuint64_t)(ld * bytes)};
   cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
-                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = enc(m, F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
+                   dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   F32 ? CU_TENSOR_MAP_L2_PROMOTION_NONE : CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(-12, "cuTensorMapEncodeTiled failed with code %d", (int)r);
   return 0;
 }
@@ -297,24 +300,32 @@ static int launch_single(const void* kern, std::atomic<unsigned long long>& rais
 // than the five k-blocks that stay staged anyway (80 groups x 410 rows, 4096 x 2048: 717, 761 one by one; 32 x 1024 880,
 // 989); shorter groups lose by it (64 x 192, 4096 x 1024: 221 one by one, 252), stored grads gain nothing (32 x
 // 1024, 2048 x 1024: 159, 165), and an odd number of column tiles leaves units of unequal length (128 x 256, 2048 x 768:
-// 210, 294).
+// 210, 294).  Grads that are added to: the read-modify-writes in L2 are the kernel up to four blocks a group, and one
+// warp of a row quarter issues them without letting tiles run ahead (128 groups of 4096 x 1024: 847 us, 873 with
+// four); a few more blocks need the accumulators free earlier (6 blocks: 913 with four, 962 with one), long ones
+// the operand slots (16: 1068 with one, 1191 with four).
 static void wgrad_geometry(GemmKParams* kp, bool pair) {
   const int local = kp->split < kp->ngroups ? kp->split : kp->ngroups;
   const double kb = (double)kp->total_rows / (local > 0 ? local : 1) / BK;
   const bool sgd = kp->sgd_w[0] != nullptr, brief = kb <= 8;
-  kp->pieces = sgd ? (brief ? 2 : 1) : 0;
-  if (pair) {
-    kp->row_slots = sgd ? (brief ? 5 : 6) : 7;
-    kp->col_slots = sgd ? (brief ? 4 : 5) : 6;
+  kp->pieces = kp->adders = 0;
+  if (sgd) {
+    kp->pieces = brief ? 2 : 1;
+    kp->row_slots = (pair ? 7 : 5) - kp->pieces;
+    kp->col_slots = pair ? 6 - kp->pieces : 3;
+  } else if (kp->accumulate) {
+    kp->adders = kb < 4.5 ? 1 : kb < 10 ? 4 : kb < 14 ? 2 : 1;
+    kp->row_slots = kp->adders == 4 ? (pair ? 5 : 3) : kp->adders == 2 ? (pair ? 6 : 4) : kb < 4.5 ? 4 : (pair ? 7 : 5);
+    kp->col_slots = !pair ? 3 : kp->adders == 4 || kb < 4.5 ? 4 : 5;
   } else {
-    kp->row_slots = sgd ? (brief ? 3 : 4) : 5;
-    kp->col_slots = sgd ? 3 : 4;
+    kp->row_slots = pair ? 7 : 5;
+    kp->col_slots = pair ? 6 : 4;
   }
   kp->unit = sgd && ((kp->N + BN - 1) / BN) % 2 == 0 && kb > 5 ? 2 : 1;
 }
 static int wgrad_smem(const GemmKParams& kp, bool pair) {
   return kp.row_slots * WG_ROW_BYTES + kp.col_slots * (pair ? wg_col_bytes<true>() : wg_col_bytes<false>()) +
-         WG_EPI_WARPS * kp.pieces * WG_PIECE + 1024;
+         WG_EPI_WARPS * kp.pieces * WG_PIECE + 4 * kp.adders * WG_ADD_PIECE + 1024;
 }
 
 template <bool SGD>
@@ -413,6 +424,12 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
       if (d->ngroups > d->split && d->out[2 * i + 1] == nullptr) return fail(-8, "wgrad: groups >= split need a slot grad tensor");
       if ((((uintptr_t)d->out[2 * i] | (uintptr_t)d->out[2 * i + 1]) & 15) != 0 || d->ldc % 4 != 0)
         return fail(-11, "weight-grad output must be 16-byte aligned with a 16-byte multiple row stride");
+      if (d->accumulate) {
+        const int64_t n_local = d->split < d->ngroups ? d->split : d->ngroups;
+        if ((rc = make_map<true>(&kp.b2[i][0], d->out[2 * i], n_local * d->Mw, d->N, d->ldc, 32, 32))) return rc;
+        if (d->ngroups > d->split &&
+            (rc = make_map<true>(&kp.b2[i][1], d->out[2 * i + 1], (d->ngroups - n_local) * d->Mw, d->N, d->ldc, 32, 32))) return rc;
+      }
     }
     const bool pair = d->two_cta != 0 && grid >= 2;
     wgrad_geometry(&kp, pair);

@@ -248,6 +248,14 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
+// tiled TMA reduce-add (2-D) from this CTA's shared memory, tracked by the thread's bulk async-group.
+// x * element size must be a multiple of 16 bytes and coordinates non-negative.
+__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, int x, int y,
+                                                  const void* smem_src) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%1, %2}], [%3];"
+               ::"l"(map), "r"(x), "r"(y), "r"(smem_u32(smem_src))
+               : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }

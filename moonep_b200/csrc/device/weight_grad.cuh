@@ -18,9 +18,10 @@
 //   * sixteen epilogue warps move 16-row x 64-column pieces.  The old weights come by TMA through a ring of each
 //     warp's own, are updated as matrix fragments, and threads of a quad exchange words so that each holds 32
 //     contiguous bytes of a row: stores cover whole 128-byte lines and pass through no shared memory.  fp32 grads
-//     leave as 64-byte row segments.  (Measured and worse: a row a thread, 4.6 TB/s of stores where whole lines
-//     reach 6.1; two rows of 64 bytes a warp, 2.5; weights prefetched into registers, 2 TB/s, because
-//     outstanding loads need L1 lines and the operand slots leave 28 KB.)
+//     leave as 64-byte row segments; where they are added to grads, as 32 x 32 pieces by TMA reductions (128 groups x
+//     128 rows, 4096 x 1024: 847 us; 16-byte reductions from registers 917).  (Measured and worse: a row a thread,
+//     4.6 TB/s of stores where whole lines reach 6.1; two rows of 64 bytes a warp, 2.5; weights prefetched into
+//     registers, 2 TB/s, because outstanding loads need L1 lines and the operand slots leave 28 KB.)
 // Isolated launches, Zipf 0.5 group sizes, us before (TMA both ways, single CTAs below 512 rows) -> now.  SGD, 128 groups x
 // 256 rows, 7168 x 2048: 2020 -> 1710; 64 x 512, 4096 x 2048: 679 -> 639; 32 x 1024, 7168 x 2048: 929 -> 880; stored, 128 x
 // 256, 2048 x 768: 228 -> 210; 64 x 192, 4096 x 1024: 327 -> 227.
@@ -36,6 +37,7 @@ template <bool TWO> __host__ __device__ constexpr int wg_col_bytes() { return (T
 constexpr int WG_MAX_ROW_SLOTS = 7, WG_MAX_COL_SLOTS = 6;
 constexpr int WG_PIECE = 16 * 64 * 2;                 // weights of an epilogue step: 16 rows x 64 columns
 constexpr int WG_MAX_PIECES = WG_STEPS;
+constexpr int WG_ADD_PIECE = 32 * 32 * 4;             // grads that are added to
 
 // One tile, or two that are neighbours in the columns.
 struct WgUnit {
@@ -303,8 +305,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __g
     // SGD: a warp's weight pieces travel through a ring of its own by TMA, as far ahead as the ring is deep.
     // (Loads into registers do not: with this much shared memory in use, what is left as L1 holds 28 KB of
     // outstanding loads, which streams 2 TB/s.)
-    const int ew = warp - 2, depth = SGD ? p.pieces : 1;
-    uint8_t* wring = col_slots + NC * COL_BYTES + ew * depth * WG_PIECE;
+    // (Grads that are added to: one piece of 32 x 32 fp32 for a warp that takes part.)
+    const int ew = warp - 2, depth = p.pieces;
+    uint8_t* wring = col_slots + NC * COL_BYTES + ew * (SGD ? depth * WG_PIECE : WG_ADD_PIECE);
     const uint32_t wring_s = smem_u32(wring);
     RingSlot ws;
     auto load_piece = [&](const WgUnit& t, int ni, int k, int slot) {
@@ -339,6 +342,43 @@ __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __g
       const uint32_t tacc = tmem_base + (uint32_t)acc * BN + ((uint32_t)(q * 32) << 16) + (uint32_t)cofs;
       const bool in_rows = t.m0 < p.Mw;      // (the second CTA of a pair may have no rows left)
       bool go_on = true;
+      // the accumulator has been read: the next tile but one may overwrite it
+      auto release = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (TWO && crank != 0) mbar_arrive_remote(&acc_empty[acc], 0);   // the leader issues the MMAs
+          else mbar_arrive(&acc_empty[acc]);
+        }
+      };
+      if (!SGD && p.accumulate) {
+        // 32 x 32 pieces, a row a lane, added by TMA; p.adders warps of a row quarter share its columns
+        const int part = ew >> 2, steps = part < p.adders && t.num_kb > 0 ? BN / 32 / p.adders : 0;
+        const uint32_t tcol = tacc - (uint32_t)cofs;
+        if (steps == 0) release();
+#pragma unroll 1
+        for (int k = part * steps; k < (part + 1) * steps; ++k) {
+          uint32_t r[32];
+          __syncwarp();
+          tmem_ld_32x32(tcol + 32 * k, r);
+          tmem_ld_wait();
+          if (k == (part + 1) * steps - 1) release();
+          if (lane == 0) bulk_wait_read<0>();            // the piece before has left
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(wring + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          const int x0 = ni * BN + 32 * k;
+          if (lane == 0 && in_rows && x0 < p.N) {
+            tma_reduce_add_2d(&p.b2[t.prod][t.alloc], x0, t.g_local * p.Mw + t.m0 + q * 32, wring);
+            bulk_commit();
+          }
+        }
+        continue;
+      }
 #pragma unroll
       for (int k = 0; k < WG_STEPS; ++k) {
         uint32_t r[32];                      // column block j (of 8): [4j + 2h], [4j + 2h + 1] = columns 2c, 2c + 1 of row lane / 4 + 8h
@@ -350,14 +390,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __g
 #pragma unroll
           for (int e = 0; e < 32; ++e) r[e] = 0u;
         }
-        if (k == WG_STEPS - 1) {                        // the accumulator has been read: the next tile but one may overwrite it
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (TWO && crank != 0) mbar_arrive_remote(&acc_empty[acc], 0);   // the leader issues the MMAs
-            else mbar_arrive(&acc_empty[acc]);
-          }
-        }
+        if (k == WG_STEPS - 1) release();
         const int col = ni * BN + cofs;
         if (SGD && t.applied) {
           if (!wait(&w_full[ew][ws.slot], ws.parity, 5)) { go_on = false; break; }
@@ -409,21 +442,14 @@ __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __g
               const uint32_t g1 = __shfl_xor_sync(0xffffffffu, odd ? even_b[1] : odd_b[1], 1);
               const uint4 v = odd ? make_uint4(g0, g1, odd_b[0], odd_b[1]) : make_uint4(even_b[0], even_b[1], g0, g1);
               float* o = dst + 8ll * h * p.ldc + 16 * b;
-              if (in_rows && x0 + 16 * b < p.N) {
-                if (p.accumulate)
-                  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                               ::"l"(o), "f"(__uint_as_float(v.x)), "f"(__uint_as_float(v.y)), "f"(__uint_as_float(v.z)),
-                                 "f"(__uint_as_float(v.w))
-                               : "memory");
-                else
-                  *reinterpret_cast<uint4*>(o) = v;
-              }
+              if (in_rows && x0 + 16 * b < p.N) *reinterpret_cast<uint4*>(o) = v;
             }
         }
       }
       if (!go_on) break;
       if (SGD && next_applied && !t.applied) load_first(u, u.ni + i);
     }
+    if (!SGD && lane == 0) bulk_wait<0>();   // pieces to be added have been read and written
   }
   // ---- teardown: everything joins, in-flight work is given time to land on an abort ----------
   tc_fence_before();
