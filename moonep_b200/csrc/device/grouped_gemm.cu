@@ -54,8 +54,8 @@ struct GemmKParams {
   const int32_t* pads;     // [ngroups][2] first padding row and their number, per group; or null
   int ngroups, split, total_rows, N, K, nseg, rows_per_expert, Mw, accumulate, zero_empty_below;
   // weight grad: tiles of a unit; slots of the shared memory for k-blocks of rows and of columns, and for
-  // weight pieces of an epilogue warp (SGD); warps of a row quarter that add to grads (accumulate: 1, 2, 4)
-  int unit, row_slots, col_slots, pieces, adders;
+  // weight pieces of an epilogue warp (SGD)
+  int unit, row_slots, col_slots, pieces;
   int vec32;   // weight grad: rows of the weights allow 32-byte accesses
   int products; // weight grad: 2 = a second one with the same A (b[1], out + 2, sgd_w[1])
   // SGD kernels: 1 = only the tiles whose grads are STORED (experts with replicas, slot groups),
@@ -195,6 +195,7 @@ struct GemmDesc {
   const int32_t* disp_zero_fill;
   int32_t disp_fresh, disp_shard;
   const int32_t* pads;
+  int32_t rows_used;               // weight grad: rows that hold tokens, on the host's knowledge (0: total_rows)
 };
 
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -293,50 +294,53 @@ static int launch_single(const void* kern, std::atomic<unsigned long long>& rais
   return 0;
 }
 
-// How a weight-grad launch splits its shared memory and its tiles, by the average group (which is all the host knows;
-// every choice computes every group).  SGD: up to eight k-blocks a group the stream of old weights needs two
-// pieces a warp in flight (128 groups x 256 rows, 7168 x 2048: 1790 us, 1810 with one and more operand slots); longer
-// ones the operand slots (32 x 1024: 866, 913 with two pieces).  Two tiles a unit share staged rows: SGD with more
-// than the five k-blocks that stay staged anyway (80 groups x 410 rows, 4096 x 2048: 717, 761 one by one; 32 x 1024 880,
-// 989); shorter groups lose by it (64 x 192, 4096 x 1024: 221 one by one, 252), stored grads gain nothing (32 x
-// 1024, 2048 x 1024: 159, 165), and an odd number of column tiles leaves units of unequal length (128 x 256, 2048 x 768:
-// 210, 294).  Grads that are added to: the read-modify-writes in L2 are the kernel up to four blocks a group, and one
-// warp of a row quarter issues them without letting tiles run ahead (128 groups of 4096 x 1024: 847 us, 873 with
-// four); a few more blocks need the accumulators free earlier (6 blocks: 913 with four, 962 with one), long ones
-// the operand slots (16: 1068 with one, 1191 with four).
-static void wgrad_geometry(GemmKParams* kp, bool pair) {
+// How a weight-grad launch splits its shared memory and its tiles, by the average number of k-blocks a group: `rows`
+// is the number of rows that hold tokens, where the caller knows it.  (The length of a layer's row tensor is its
+// capacity, up to two paddings an expert more: 8 blocks a group where there are 4.)  Every choice computes every
+// group.  Figures: the three weight grads of a layer's step (down; gate and up in one launch), padding 128, Zipf 0.3 -
+// 0.9, us.
+static void wgrad_geometry(GemmKParams* kp, int rows, bool pair) {
   const int local = kp->split < kp->ngroups ? kp->split : kp->ngroups;
-  const double kb = (double)kp->total_rows / (local > 0 ? local : 1) / BK;
-  const bool sgd = kp->sgd_w[0] != nullptr, brief = kb <= 8;
-  kp->pieces = kp->adders = 0;
-  if (sgd) {
-    kp->pieces = brief ? 2 : 1;
+  const double kb = (double)rows / (local > 0 ? local : 1) / BK;
+  const int tiles_n = (kp->N + BN - 1) / BN;
+  kp->pieces = 0;
+  kp->unit = 1;
+  if (kp->sgd_w[0] != nullptr) {
+    // Up to five blocks the stream of old weights needs two pieces a warp in flight, longer groups the operand slots
+    // (128 experts, 4096 x 1024, 4 blocks 1528, 1567 with one piece; 64, 2048 x 1536, 8 blocks 809, 788).
+    kp->pieces = kb < 5 ? 2 : 1;
     kp->row_slots = (pair ? 7 : 5) - kp->pieces;
     kp->col_slots = pair ? 6 - kp->pieces : 3;
+    // Two tiles that share staged rows: with eight column tiles from two blocks on (64 experts, 7168 x 2048: 4 blocks 2683,
+    // 2513 so; 2 blocks 2146, 2133), with four and six from eight (2048 x 1536: 4 blocks 1096, 1175; 8 788, 768); not
+    // with two (1024 x 512, 8 blocks 155, 173) nor an odd number, which leaves units of unequal length (2048 x 768, 4
+    // blocks 627, 788).
+    if (tiles_n % 2 == 0 && kb >= (tiles_n >= 8 ? 1.5 : tiles_n >= 4 ? 8 : 1e9)) kp->unit = 2;
   } else if (kp->accumulate) {
-    kp->adders = kb < 4.5 ? 1 : kb < 10 ? 4 : kb < 14 ? 2 : 1;
-    kp->row_slots = kp->adders == 4 ? (pair ? 5 : 3) : kp->adders == 2 ? (pair ? 6 : 4) : kb < 4.5 ? 4 : (pair ? 7 : 5);
-    kp->col_slots = !pair ? 3 : kp->adders == 4 || kb < 4.5 ? 4 : 5;
+    // One warp of a row quarter adds; more of them, with pieces of their own, cost slots and let tiles run
+    // ahead of the read-modify-writes in L2 (2048 x 768, 64 experts x 8 blocks 586, 590 with four; 7168 x 2048, 32 x 16 3106,
+    // 4124; 4096 x 1024, 128 x 1 2569, 2602).
+    kp->row_slots = pair ? 7 : 5;
+    kp->col_slots = pair ? 5 : 3;
   } else {
     kp->row_slots = pair ? 7 : 5;
     kp->col_slots = pair ? 6 : 4;
   }
-  kp->unit = sgd && ((kp->N + BN - 1) / BN) % 2 == 0 && kb > 5 ? 2 : 1;
 }
 static int wgrad_smem(const GemmKParams& kp, bool pair) {
   return kp.row_slots * WG_ROW_BYTES + kp.col_slots * (pair ? wg_col_bytes<true>() : wg_col_bytes<false>()) +
-         WG_EPI_WARPS * kp.pieces * WG_PIECE + 4 * kp.adders * WG_ADD_PIECE + 1024;
+         WG_EPI_WARPS * kp.pieces * WG_PIECE + (kp.accumulate ? 4 * WG_ADD_PIECE : 0) + 1024;
 }
 
-template <bool SGD>
+template <int MODE>
 static int launch_wgrad(const GemmKParams& kp, bool pair, int grid, cudaStream_t stream) {
   const int smem = wgrad_smem(kp, pair);
   if (pair) {
     static PairLaunch once;
-    return launch_pair((const void*)ep_weight_grad_kernel<true, SGD>, once, kp, grid, WG_THREADS, smem, false, stream);
+    return launch_pair((const void*)ep_weight_grad_kernel<true, MODE>, once, kp, grid, WG_THREADS, smem, false, stream);
   }
   static std::atomic<unsigned long long> raised{0};
-  return launch_single((const void*)ep_weight_grad_kernel<false, SGD>, raised, kp, grid, WG_THREADS, smem, false, stream);
+  return launch_single((const void*)ep_weight_grad_kernel<false, MODE>, raised, kp, grid, WG_THREADS, smem, false, stream);
 }
 
 template <bool W_MN>
@@ -432,11 +436,10 @@ int mep_gemm_launch(const GemmDesc* d, cudaStream_t stream) {
       }
     }
     const bool pair = d->two_cta != 0 && grid >= 2;
-    wgrad_geometry(&kp, pair);
+    wgrad_geometry(&kp, d->rows_used > 0 ? d->rows_used : d->total_rows, pair);
     kp.wg_select = kp.sgd_w[0] != nullptr ? d->wg_select : 0;
-    if (kp.sgd_w[0] != nullptr)
-      return launch_wgrad<true>(kp, pair, grid, stream);
-    return launch_wgrad<false>(kp, pair, grid, stream);
+    if (kp.sgd_w[0] != nullptr) return launch_wgrad<WG_SGD>(kp, pair, grid, stream);
+    return kp.accumulate ? launch_wgrad<WG_ADD>(kp, pair, grid, stream) : launch_wgrad<WG_STORE>(kp, pair, grid, stream);
   }
   if (d->epi == EPI_F32) {
     // router logits: one group, one segment

@@ -13,6 +13,8 @@
 //   * CTA pairs (cta_group::2): each CTA stages its own 128 weight rows and half of the columns;
 //   * where reductions are long, two tiles that are neighbours in the columns share the staged rows: a chunk of
 //     the reduction for the first, then the same chunk for the second (both accumulators), 3/4 of the bytes;
+//   * beside the stream of weights (SGD), loads of groups shorter than the operand slots run one tile ahead, not several
+//     (a layer of 128 experts, 4096 x 1024: 1 block a group 1251 -> 1204 us, 4 blocks 1528 -> 1487);
 //   * loads and MMAs are issued by converged warps with one elected lane; from a single lane's branch the issuer
 //     took longer for a k-block than the tensor cores (without epilogue 32 x 1024 rows 960 -> 620 us);
 //   * sixteen epilogue warps move 16-row x 64-column pieces.  The old weights come by TMA through a ring of each
@@ -29,6 +31,7 @@
 
 namespace mep {
 
+enum { WG_STORE = 0, WG_SGD = 1, WG_ADD = 2 };        // what becomes of a tile (SGD: or stored, where it has replicas)
 constexpr int WG_EPI_WARPS = 16;
 constexpr int WG_THREADS = 64 + WG_EPI_WARPS * 32;
 constexpr int WG_STEPS = 32 / WG_EPI_WARPS;           // 16-row x 64-column pieces of a tile that a warp takes
@@ -149,8 +152,9 @@ __device__ __forceinline__ void wg_store16(__nv_bfloat16* dst, int left, bool ve
   }
 }
 
-template <bool TWO, bool SGD>
+template <bool TWO, int MODE>
 __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __grid_constant__ GemmKParams p) {
+  constexpr bool SGD = MODE == WG_SGD;
   constexpr int COL_BYTES = wg_col_bytes<TWO>();
   const int NR = p.row_slots, NC = p.col_slots;
   const int crank = TWO ? (int)cluster_cta_rank() : 0;        // 0 = leader of the pair
@@ -208,6 +212,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __g
     RingSlot row, col;
     if (issue) { tma_prefetch_desc(&p.a); tma_prefetch_desc(&p.b[0][0]); if (p.products > 1) tma_prefetch_desc(&p.b[1][0]); }
     for (; walk.find(p, s_end, s_valid, crank, u); walk.step()) {
+      const int ahead = SGD ? max(1, min(NC, u.tiles * u.num_kb)) : NC;
       const bool ok = wg_items(u, NR, row, [&](int i, int kb, const RingSlot& rs, bool first, bool) {
         const int y = u.row0 + kb * BK;
         // blocks of 64 columns of the [token rows][columns] operands
@@ -225,7 +230,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __g
               load(row_slots + rs.slot * WG_ROW_BYTES + j * 8192, &p.a, u.m0 + 64 * j, &row_full[rs.slot]);
           }
         }
-        if (!wait(&col_empty[col.slot], col.parity ^ 1u, 1)) return false;
+        // a block may be loaded when the one `ahead` before it has been multiplied, which is after its slot is free
+        const int back = col.slot - ahead;
+        if (!wait(&col_empty[back < 0 ? back + NC : back], back < 0 ? col.parity ^ 1u : col.parity, 1)) return false;
         if (issue) {
           const int n0 = (u.ni + i) * BN, mine = wg_width(p, u.ni + i) / (TWO ? 2 : 1);   // columns of this CTA
           const int blocks = (mine + 63) / 64;
@@ -305,7 +312,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __g
     // SGD: a warp's weight pieces travel through a ring of its own by TMA, as far ahead as the ring is deep.
     // (Loads into registers do not: with this much shared memory in use, what is left as L1 holds 28 KB of
     // outstanding loads, which streams 2 TB/s.)
-    // (Grads that are added to: one piece of 32 x 32 fp32 for a warp that takes part.)
+    // (Grads that are added to: one piece of 32 x 32 fp32 for each of the first four warps.)
     const int ew = warp - 2, depth = p.pieces;
     uint8_t* wring = col_slots + NC * COL_BYTES + ew * (SGD ? depth * WG_PIECE : WG_ADD_PIECE);
     const uint32_t wring_s = smem_u32(wring);
@@ -351,18 +358,17 @@ __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __g
           else mbar_arrive(&acc_empty[acc]);
         }
       };
-      if (!SGD && p.accumulate) {
-        // 32 x 32 pieces, a row a lane, added by TMA; p.adders warps of a row quarter share its columns
-        const int part = ew >> 2, steps = part < p.adders && t.num_kb > 0 ? BN / 32 / p.adders : 0;
-        const uint32_t tcol = tacc - (uint32_t)cofs;
+      if constexpr (MODE == WG_ADD) {
+        // 32 x 32 pieces, a row a lane, added by TMA: one warp of a row quarter takes all columns
+        const int steps = ew < 4 && t.num_kb > 0 ? BN / 32 : 0;
         if (steps == 0) release();
 #pragma unroll 1
-        for (int k = part * steps; k < (part + 1) * steps; ++k) {
+        for (int k = 0; k < steps; ++k) {
           uint32_t r[32];
           __syncwarp();
-          tmem_ld_32x32(tcol + 32 * k, r);
+          tmem_ld_32x32(tacc + 32 * k, r);               // (the first four warps' columns start at 0)
           tmem_ld_wait();
-          if (k == (part + 1) * steps - 1) release();
+          if (k == steps - 1) release();
           if (lane == 0) bulk_wait_read<0>();            // the piece before has left
           __syncwarp();
 #pragma unroll
@@ -442,14 +448,20 @@ __global__ void __launch_bounds__(WG_THREADS, 1) ep_weight_grad_kernel(const __g
               const uint32_t g1 = __shfl_xor_sync(0xffffffffu, odd ? even_b[1] : odd_b[1], 1);
               const uint4 v = odd ? make_uint4(g0, g1, odd_b[0], odd_b[1]) : make_uint4(even_b[0], even_b[1], g0, g1);
               float* o = dst + 8ll * h * p.ldc + 16 * b;
-              if (in_rows && x0 + 16 * b < p.N) *reinterpret_cast<uint4*>(o) = v;
+              // The arm that is never taken keeps this a branch.  Predicated, a piece's eight stores leave back to back at its
+              // end, and groups of one and two blocks take 3 - 6 % longer (a layer's step, 128 experts, 4096 x 1024: 1
+              // block 1317 against 1369 us, 2 blocks 1329 against 1424; as whole lines, two accesses a row, 1397 and 1460).
+              if (in_rows && x0 + 16 * b < p.N) {
+                if (p.unit < 0) asm volatile("membar.cta;" ::: "memory");
+                else *reinterpret_cast<uint4*>(o) = v;
+              }
             }
         }
       }
       if (!go_on) break;
       if (SGD && next_applied && !t.applied) load_first(u, u.ni + i);
     }
-    if (!SGD && lane == 0) bulk_wait<0>();   // pieces to be added have been read and written
+    if (MODE == WG_ADD && lane == 0) bulk_wait<0>();   // pieces to be added have been read and written
   }
   // ---- teardown: everything joins, in-flight work is given time to land on an abort ----------
   tc_fence_before();

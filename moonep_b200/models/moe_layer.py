@@ -207,7 +207,7 @@ class _MoEFn(torch.autograd.Function):
             sgd = lambda w: (w, fused_lr, keep)
         with tr.span("b.wgrad_down"):
             gemm.wgrad(d_out, act, cu, layer.g_down, grad_slot=gslot("down"), split=split, accumulate=acc,
-                       sgd=sgd(layer.w_down), pads=pads)
+                       sgd=sgd(layer.w_down), pads=pads, rows=buf.N)
         with tr.span("b.swiglu_bwd"):
             d_gate, d_up, d_scale = ew.swiglu_bwd(d_act, gate, up, w_nvs, rows_ptr=cu[-1:])
         ev_r = None
@@ -215,7 +215,8 @@ class _MoEFn(torch.autograd.Function):
         if fused_lr is None:
             with tr.span("b.wgrad_gateup"):
                 gemm.wgrad2(hidden, (d_gate, d_up), cu, (layer.g_gate, layer.g_up),
-                            grad_slot=(gslot("gate"), gslot("up")), split=split, accumulate=acc, pads=pads)
+                            grad_slot=(gslot("gate"), gslot("up")), split=split, accumulate=acc, pads=pads,
+                            rows=buf.N)
             if layer.hidden_in_place:  # the forward rows have had their last reader
                 buf.release_second_shard(layer)
             # the replicas' weight grads travel home on the comm stream while this stream computes dX
@@ -265,11 +266,12 @@ class _MoEFn(torch.autograd.Function):
         pools, zc = layer.pools, layer.accumulate_grads
         wg = lambda a, g, w, **kw: gemm.wgrad(hidden, a, cu, g, grad_slot=gslot(w), split=split,
                                               sgd=sgd(getattr(layer, "w_" + w)),
-                                              pads=plan.zero_fill_ranges, **kw)
+                                              pads=plan.zero_fill_ranges, rows=layer.buf.N, **kw)
         with layer.tracer.span("b.wgrad_gateup"):
             if not do_reduce:
                 gemm.wgrad2(hidden, (d_gate, d_up), cu, (layer.g_gate, layer.g_up), grad_slot=(gslot("gate"), gslot("up")),
-                            split=split, sgd=((layer.w_gate, layer.w_up), *sgd(None)[1:]), pads=plan.zero_fill_ranges)
+                            split=split, sgd=((layer.w_gate, layer.w_up), *sgd(None)[1:]), pads=plan.zero_fill_ranges,
+                            rows=layer.buf.N)
             else:
                 wg(d_gate, layer.g_gate, "gate")
                 # the gate grads travel home under the up projection's weight grad

@@ -52,7 +52,7 @@ class _GemmDesc(ctypes.Structure):
         ("disp_mode", ctypes.c_int32), ("disp_ctx", ctypes.c_void_p), ("disp_x", ctypes.c_void_p),
         ("disp_w", ctypes.c_void_p), ("disp_dst", ctypes.c_void_p), ("disp_order", ctypes.c_void_p),
         ("disp_zero_fill", ctypes.c_void_p), ("disp_fresh", ctypes.c_int32), ("disp_shard", ctypes.c_int32),
-        ("pads", ctypes.c_void_p),
+        ("pads", ctypes.c_void_p), ("rows_used", ctypes.c_int32),
     ]
 
 
@@ -274,7 +274,7 @@ def gateup_dgrad(dg, du, wg, wu, cu_seqlens, *, wg_slot=None, wu_slot=None, spli
 
 
 def wgrad(a, b, cu_seqlens, grad_local, *, grad_slot=None, split=None, accumulate=False, sgd=None,
-          grid=0, select=0, pads=None):
+          grid=0, select=0, pads=None, rows=0):
     """``grad[g] (+)= a[rows of g]^T b[rows of g]``; ``a`` [rows, M], ``b`` [rows, N], fp32 grads
     ``[G0, M, N]`` (+ slot grads for groups >= split).  Group sizes must be multiples of 64
     (padding rows must be zero in ``a`` or ``b``).  Empty groups below ``split`` are zeroed
@@ -290,24 +290,27 @@ def wgrad(a, b, cu_seqlens, grad_local, *, grad_slot=None, split=None, accumulat
     With ``sgd``, ``select=1`` computes only the groups whose grads are stored (set flags, slot
     groups) and ``select=2`` only the ones that are applied; the two launches together equal one
     with ``select=0``.  The stored grads are the ones that ``reduce_grad`` has to move, so computing
-    them first lets that transfer run beside the rest of the weight grad."""
+    them first lets that transfer run beside the rest of the weight grad.
+
+    ``rows``: how many rows of ``a`` hold tokens, where the caller knows (a Buffer's ``N``; its row tensor has
+    spare rows).  It changes no result, only how the launch is split."""
     assert select in (0, 1, 2) and (select == 0 or sgd is not None), "select splits a fused-SGD weight grad"
     w, lr, keep = (None, None, None) if sgd is None else (sgd[0], float(sgd[1]), sgd[2])
-    _wgrads(a, ((b, grad_local, grad_slot, w),), cu_seqlens, split, accumulate, lr, keep, grid, select, pads)
+    _wgrads(a, ((b, grad_local, grad_slot, w),), cu_seqlens, split, accumulate, lr, keep, grid, select, pads, rows)
     return grad_local
 
 
 def wgrad2(a, b, cu_seqlens, grad_local, *, grad_slot=(None, None), split=None, accumulate=False, sgd=None,
-           grid=0, pads=None):
+           grid=0, pads=None, rows=0):
     """Two weight grads that share ``a`` (gate and up projections) in one launch: :func:`wgrad` with pairs for
     ``b``, ``grad_local``, ``grad_slot`` and the ``weights`` of ``sgd=(weights, lr, keep)``; same results."""
     w, lr, keep = ((None, None), None, None) if sgd is None else (sgd[0], float(sgd[1]), sgd[2])
     assert b[0].shape == b[1].shape and b[0].stride() == b[1].stride()
-    _wgrads(a, tuple(zip(b, grad_local, grad_slot, w)), cu_seqlens, split, accumulate, lr, keep, grid, 0, pads)
+    _wgrads(a, tuple(zip(b, grad_local, grad_slot, w)), cu_seqlens, split, accumulate, lr, keep, grid, 0, pads, rows)
     return grad_local
 
 
-def _wgrads(a, products, cu_seqlens, split, accumulate, lr, keep, grid, select, pads):
+def _wgrads(a, products, cu_seqlens, split, accumulate, lr, keep, grid, select, pads, rows_used):
     _bf16(a, "a")
     rows, M = a.shape
     N = products[0][0].shape[1]
@@ -346,6 +349,7 @@ def _wgrads(a, products, cu_seqlens, split, accumulate, lr, keep, grid, select, 
     d.ldc = N
     d.grid = grid
     d.pads = _pads(pads, cu_seqlens)
+    d.rows_used = min(int(rows_used), rows)
     d.status = status_word(a.device).data_ptr()
     _launch(d)
 

@@ -81,3 +81,31 @@ def test_two_products_equal_one_each(M, N, two, monkeypatch):
         want += l + s + ws
         assert all(torch.equal(x, y) for x, y in zip(got, want)), form
     gemm.check_status()
+
+
+# average k-blocks that the launch is told -> with SGD two pieces and one, one and two tiles a unit (from eight blocks,
+# from two, not at all)
+@pytest.mark.parametrize("two", [0, 1])
+@pytest.mark.parametrize("blocks", [1, 4, 8])
+@pytest.mark.parametrize("M, N", [(384, 264), (256, 1000), (256, 2040)])
+def test_every_geometry_computes_every_group(M, N, blocks, two, monkeypatch):
+    """What the launch is told of the rows changes no bit, whatever the groups' real lengths."""
+    from moonep_b200.ops import gemm
+    monkeypatch.setattr(gemm, "TWO_CTA", two)
+    groups = [64, 1472, 0, 128, 448]
+    gen, ends, a, b = _inputs(groups, M, N, blocks)
+    G, rows = len(groups), 64 * blocks * len(groups)
+    spare = torch.zeros(max(0, rows - a.shape[0]), 1, device="cuda").bfloat16()      # (told rows are rows of a)
+    a, b = (torch.cat([t, spare.expand(-1, t.shape[1])]) for t in (a, b))
+    base, w = (torch.randn(G, M, N, device="cuda", generator=gen) for _ in range(2))
+    start, want = 0, torch.empty_like(base)
+    for g, n in enumerate(groups):       # each group alone, in the geometry of its own length
+        gemm.wgrad(a[start:start + n], b[start:start + n], ends[:1] * 0 + n, want[g:g + 1]) if n else want[g].zero_()
+        start += n
+    grad, acc, ws = torch.empty_like(base), base.clone(), w.bfloat16()
+    gemm.wgrad(a, b, ends, grad, rows=rows)
+    gemm.wgrad(a, b, ends, acc, accumulate=True, rows=rows)
+    gemm.wgrad(a, b, ends, base.clone(), sgd=(ws, 0.25, None), rows=rows)
+    gemm.check_status()
+    assert torch.equal(grad, want) and torch.equal(acc, base + want)
+    assert torch.equal(ws, (w.bfloat16().float() - 0.25 * want).bfloat16())
