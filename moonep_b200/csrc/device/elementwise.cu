@@ -129,9 +129,48 @@ __global__ void ep_router_topk_bwd_kernel(const float* __restrict__ weights, con
 // next to it, by issue.  A block a row left 160 of 256 threads idle at H' = 768 and met at two barriers a row: 36900
 // rows x 512 89 -> 46 us, x 2048 142 -> 134, 20000 x 1024 62 -> 48 (with the clearing of the sums in front, which the
 // kernel now does itself for the rows behind the last).  More vectors at once cost the registers of other warps (four:
-// 185 us for x 2048).  A row's sum keeps the order that it had there: eight partial sums, of the vectors with the
-// same v / 32 % 8, each over the lanes first.
-constexpr int SB_WARPS = 8, SB_DEPTH = 2;
+// 185 us for x 2048).  Few rows leave warps idle instead, and a warp's steps over a wide row are a chain of loads: up
+// to SB_WIDE rows a vector a block takes each (512 rows x 2048 15.4 -> 9.2 us, 2500 20.8 -> 18.8; 512 x 768 10.9 -> 8.2;
+// 4000 x 2048, above the line, 23.6 either way).  A row's sum has the same order either way: eight partial sums, of
+// the vectors with the same v / 32 % 8, each over the lanes first.
+constexpr int SB_WARPS = 8, SB_DEPTH = 2, SB_WIDE = 12;
+
+struct SwigluRow {
+  const uint4 *d, *g, *u;
+  uint4 *dg, *du;
+  float w;
+  __device__ __forceinline__ SwigluRow(const __nv_bfloat16* dact, const __nv_bfloat16* gate, const __nv_bfloat16* up,
+                                       __nv_bfloat16* dgate, __nv_bfloat16* dup, const float* row_scale, int r, int Hp)
+      : d((const uint4*)(dact + (size_t)r * Hp)), g((const uint4*)(gate + (size_t)r * Hp)), u((const uint4*)(up + (size_t)r * Hp)),
+        dg((uint4*)(dgate + (size_t)r * Hp)), du((uint4*)(dup + (size_t)r * Hp)), w(row_scale ? row_scale[r] : 1.f) {}
+  // gradients of vector v; its terms of the row's sum are added to acc
+  __device__ __forceinline__ void vec(int v, const uint4& d4, const uint4& g4, const uint4& u4, float& acc) const {
+    uint4 rg, ru;
+    const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&d4);
+    const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&g4);
+    const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&u4);
+    __nv_bfloat162* og2 = reinterpret_cast<__nv_bfloat162*>(&rg);
+    __nv_bfloat162* ou2 = reinterpret_cast<__nv_bfloat162*>(&ru);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float2 x = __bfloat1622float2(d2[e]), y = __bfloat1622float2(g2[e]), z = __bfloat1622float2(u2[e]);
+      float s0 = 1.f / (1.f + __expf(-y.x)), s1 = 1.f / (1.f + __expf(-y.y));
+      float sg0 = y.x * s0, sg1 = y.y * s1;
+      acc += x.x * sg0 * z.x + x.y * sg1 * z.y;
+      float dg0 = x.x * z.x * w * (s0 * (1.f + y.x * (1.f - s0)));
+      float dg1 = x.y * z.y * w * (s1 * (1.f + y.y * (1.f - s1)));
+      og2[e] = __floats2bfloat162_rn(dg0, dg1);
+      ou2[e] = __floats2bfloat162_rn(x.x * sg0 * w, x.y * sg1 * w);
+    }
+    dg[v] = rg;
+    du[v] = ru;
+  }
+};
+__device__ __forceinline__ float warp_sum(float x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
 
 __global__ void __launch_bounds__(SB_WARPS * 32, 4)
 ep_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bfloat16* __restrict__ gate,
@@ -139,67 +178,56 @@ ep_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bfloat16
                      const int32_t* __restrict__ rows_ptr, int max_rows, int Hp,
                      __nv_bfloat16* __restrict__ dgate, __nv_bfloat16* __restrict__ dup,
                      float* __restrict__ dscale) {
-  const int lane = threadIdx.x & 31;
+  __shared__ float red[SB_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rows = rows_ptr ? min(*rows_ptr, max_rows) : max_rows;
   const int nvec = Hp / 8;
-  for (int r = blockIdx.x * SB_WARPS + (threadIdx.x >> 5); r < rows; r += gridDim.x * SB_WARPS) {
-    const float w = row_scale ? row_scale[r] : 1.f;
-    const uint4* pd = reinterpret_cast<const uint4*>(dact + (size_t)r * Hp);
-    const uint4* pg = reinterpret_cast<const uint4*>(gate + (size_t)r * Hp);
-    const uint4* pu = reinterpret_cast<const uint4*>(up + (size_t)r * Hp);
-    uint4* og = reinterpret_cast<uint4*>(dgate + (size_t)r * Hp);
-    uint4* ou = reinterpret_cast<uint4*>(dup + (size_t)r * Hp);
-    float part[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) part[i] = 0.f;
-    for (int v0 = 0; v0 < nvec; v0 += 8 * 32) {
-#pragma unroll
-      for (int h = 0; h < 8; h += SB_DEPTH) {
-        if (v0 + h * 32 >= nvec) break;
-        uint4 d4[SB_DEPTH], g4[SB_DEPTH], u4[SB_DEPTH];
-#pragma unroll
-        for (int i = 0; i < SB_DEPTH; ++i) {
-          const int v = v0 + (h + i) * 32 + lane;
-          if (v < nvec) { d4[i] = pd[v]; g4[i] = pg[v]; u4[i] = pu[v]; }
-        }
-#pragma unroll
-        for (int i = 0; i < SB_DEPTH; ++i) {
-          const int v = v0 + (h + i) * 32 + lane;
-          if (v >= nvec) continue;
-          uint4 rg, ru;
-          float acc = part[h + i];
-          const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&d4[i]);
-          const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&g4[i]);
-          const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&u4[i]);
-          __nv_bfloat162* og2 = reinterpret_cast<__nv_bfloat162*>(&rg);
-          __nv_bfloat162* ou2 = reinterpret_cast<__nv_bfloat162*>(&ru);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float2 d = __bfloat1622float2(d2[e]), g = __bfloat1622float2(g2[e]), u = __bfloat1622float2(u2[e]);
-            float s0 = 1.f / (1.f + __expf(-g.x)), s1 = 1.f / (1.f + __expf(-g.y));
-            float sg0 = g.x * s0, sg1 = g.y * s1;
-            acc += d.x * sg0 * u.x + d.y * sg1 * u.y;
-            float dg0 = d.x * u.x * w * (s0 * (1.f + g.x * (1.f - s0)));
-            float dg1 = d.y * u.y * w * (s1 * (1.f + g.y * (1.f - s1)));
-            og2[e] = __floats2bfloat162_rn(dg0, dg1);
-            ou2[e] = __floats2bfloat162_rn(d.x * sg0 * w, d.y * sg1 * w);
-          }
-          part[h + i] = acc;
-          og[v] = rg;
-          ou[v] = ru;
-        }
+  if (rows <= SB_WIDE * nvec) {
+    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+      const SwigluRow row(dact, gate, up, dgate, dup, row_scale, r, Hp);
+      float part = 0.f;
+      for (int v = threadIdx.x; v < nvec; v += SB_WARPS * 32) row.vec(v, row.d[v], row.g[v], row.u[v], part);
+      if (dscale) {
+        part = warp_sum(part);
+        if (lane == 0) red[warp] = part;
+        __syncthreads();
+        if (threadIdx.x == 0)
+          dscale[r] = ((red[0] + red[4]) + (red[2] + red[6])) + ((red[1] + red[5]) + (red[3] + red[7]));
+        __syncthreads();
       }
     }
-    if (dscale) {
+  } else {
+    for (int r = blockIdx.x * SB_WARPS + warp; r < rows; r += gridDim.x * SB_WARPS) {
+      const SwigluRow row(dact, gate, up, dgate, dup, row_scale, r, Hp);
+      float part[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 8; ++i) part[i] = 0.f;
+      for (int v0 = 0; v0 < nvec; v0 += 8 * 32) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part[i] += __shfl_xor_sync(0xffffffffu, part[i], o);
+        for (int h = 0; h < 8; h += SB_DEPTH) {
+          if (v0 + h * 32 >= nvec) break;
+          uint4 d4[SB_DEPTH], g4[SB_DEPTH], u4[SB_DEPTH];
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1)
+          for (int i = 0; i < SB_DEPTH; ++i) {
+            const int v = v0 + (h + i) * 32 + lane;
+            if (v < nvec) { d4[i] = row.d[v]; g4[i] = row.g[v]; u4[i] = row.u[v]; }
+          }
 #pragma unroll
-        for (int i = 0; i < o; ++i) part[i] += part[i + o];
-      if (lane == 0) dscale[r] = part[0];
+          for (int i = 0; i < SB_DEPTH; ++i) {
+            const int v = v0 + (h + i) * 32 + lane;
+            if (v < nvec) row.vec(v, d4[i], g4[i], u4[i], part[h + i]);
+          }
+        }
+      }
+      if (dscale) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[i] = warp_sum(part[i]);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+          for (int i = 0; i < o; ++i) part[i] += part[i + o];
+        if (lane == 0) dscale[r] = part[0];
+      }
     }
   }
   // rows that hold nothing
@@ -437,7 +465,10 @@ int mep_swiglu_bwd(const void* dact, const void* gate, const void* up, const flo
                    const int32_t* rows_ptr, int max_rows, int Hp, void* dgate, void* dup,
                    float* dscale, cudaStream_t stream) {
   if (Hp % 8 != 0) return fail(-1, "swiglu_bwd: H'=%d must be a multiple of 8", Hp);
+  // as many blocks as either way of taking rows can use
+  const int wide = max_rows < SB_WIDE * (Hp / 8) ? max_rows : SB_WIDE * (Hp / 8);
   int blocks = (max_rows + SB_WARPS - 1) / SB_WARPS;
+  if (blocks < wide) blocks = wide;
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (blocks < 1) return 0;
   ep_swiglu_bwd_kernel<<<blocks, SB_WARPS * 32, 0, stream>>>(

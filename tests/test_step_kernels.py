@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("Hp", [8, 264, 520, 2048, 2312])       # part of a warp, one block of 256 columns and a bit, ...
-@pytest.mark.parametrize("rows, valid", [(1, 1), (37, 0), (300, 261)])
+@pytest.mark.parametrize("rows, valid", [(1, 1), (37, 0), (300, 261), (900, 790)])     # (wide rows a block each, else a warp)
 def test_swiglu_bwd_widths(rows, valid, Hp):
     from moonep_b200.ops import elementwise as ew
     gen = torch.Generator(device="cuda").manual_seed(Hp + rows)
