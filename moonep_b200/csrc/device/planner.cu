@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) ep_plan_kernel(const PlanPara
   const int32_t* expert_off = scratch + (size_t)3 * R * E;
 
   // running count of each expert before my slice: earlier ranks + earlier CTAs of my rank.  With few
-  // experts several threads share one's CTAs, and each has eight loads in flight.
+  // experts several threads share one's CTAs, and each has sixteen loads in flight.
   for (int e = tid; e < E; e += PLAN_THREADS) cnt[e] = rank > 0 ? tpe_cumsum[(size_t)(rank - 1) * E + e] : 0;
   __syncthreads();
   const int shares = PLAN_THREADS / E > 1 ? PLAN_THREADS / E : 1;

@@ -1,5 +1,5 @@
 // Weight-grad GEMM (groups partition the REDUCTION dimension): D[g] (+)= A[rows of g]^T * B[rows of g], both
-// operands MN-major; fp32 output, or (template SGD) the optimizer step fused in: the accumulator is applied
+// operands MN-major; fp32 output (stored, or added: WG_ADD), or WG_SGD, the optimizer step fused in: the accumulator is applied
 // straight to the bf16 weights, w = bf16(w - lr * acc), for every local expert that has no replica this step.
 //
 // A launch may compute the grads of two weights that share A (the gate and up projections): group by group, first
@@ -24,9 +24,10 @@
 //     128 rows, 4096 x 1024: 847 us; 16-byte reductions from registers 917).  (Measured and worse: a row a thread,
 //     4.6 TB/s of stores where whole lines reach 6.1; two rows of 64 bytes a warp, 2.5; weights prefetched into
 //     registers, 2 TB/s, because outstanding loads need L1 lines and the operand slots leave 28 KB.)
-// Isolated launches, Zipf 0.5 group sizes, us before (TMA both ways, single CTAs below 512 rows) -> now.  SGD, 128 groups x
-// 256 rows, 7168 x 2048: 2020 -> 1710; 64 x 512, 4096 x 2048: 679 -> 639; 32 x 1024, 7168 x 2048: 929 -> 880; stored, 128 x
-// 256, 2048 x 768: 228 -> 210; 64 x 192, 4096 x 1024: 327 -> 227.
+// The three weight grads of a layer's step, Zipf 0.3 - 0.5, us before (TMA both ways, single CTAs below 512 rows a group) ->
+// now.  SGD: 64 experts x 256 rows, 7168 x 2048 3190 -> 2450; 128 x 256, 4096 x 1024 1875 -> 1397; 128 x 64 1166 -> 1178; 64 x 32
+// rows, 7168 x 2048 2053 -> 2027.  Stored: 128 x 256, 2048 x 768 705 -> 600; 128 x 64, 4096 x 1024 1310 -> 1283.  Added: 128 x 256,
+// 4096 x 1024 2727 -> 2745; 32 x 1024, 7168 x 2048 3044 -> 3144.
 #pragma once
 
 namespace mep {

@@ -24,7 +24,9 @@ class CommPlan:
     zero_fill_ranges: torch.Tensor  # [2*epn, 2] int32
     remote_stats: torch.Tensor      # [2] int32
     cu_seqlens: torch.Tensor        # [2*epn] int32 padded group END rows
-    link: torch.Tensor              # [NvS] int32 duplicate chains of MY received rows
+    # [NvS] int32 duplicate chains of MY received rows (here and in src_info, rows behind the last group hold nothing:
+    # whatever their memory held)
+    link: torch.Tensor
     N: int
     R: int
     E: int
